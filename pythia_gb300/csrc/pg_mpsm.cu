@@ -8,10 +8,10 @@
 // (mostfreqbuildkeyoccurances) and emitting the cartesian product of equal-key
 // groups.
 //
-// Count/sum joins whose key span is 2^13..2^24 values take the bucketed form
-// further down (high-bit sort + shared-memory merge of 4096-key buckets).
+// Joins whose keys span a compact range count one side's keys in a table and
+// look the other side up (mj_dense_join further down), with no sort.
 //
-// GPU plan: sort both relations (pg_sort.cu), cut each sorted relation into
+// GPU plan otherwise: sort both relations (pg_sort.cu), cut each sorted relation into
 // equal-key runs (stream compaction of run heads: run starts and run keys),
 // match build runs to probe runs by merging the two sorted run-key arrays, scan the per-run output counts |R_k|*|S_k|, and either fold
 // count and sum (no output materialised; a build column sums as
@@ -280,119 +280,16 @@ static int mj_runs(pg_ctx* ctx, cudaStream_t s, const pg_rec* rec, uint64_t n, u
 	return PG_OK;
 }
 
-// ---------------------------------------------------------------------------
-// Count/sum without materialising, for key spans of 2^13 .. 2^24 values: both
-// relations are sorted on the bits of (key - kmin) above the low 12 (one
-// stable radix partition each, 2..4096 buckets), and each bucket pair, 4096
-// consecutive key values, is merged in shared memory: per key, the tuples on
-// each side and the summed column; then sum over keys of |R_k| * |S_k| and
-// sum_R_k * |S_k| (or sum_S_k * |R_k|). This is the sort-merge of the
-// general path with its last radix digit, run detection and run matching
-// fused into one pass over both relations.
-// ---------------------------------------------------------------------------
-#define MJ_LOCAL_BITS 12
-#define MJ_LOCAL (1u << MJ_LOCAL_BITS)
-
-__device__ __forceinline__ unsigned long long mj_tuple_col(const char* t, uint32_t off, uint32_t words)
-{
-	const uint32_t* w = reinterpret_cast<const uint32_t*>(t + off);
-	if (words == 2) return ((unsigned long long) w[1] << 32) | w[0];
-	return (unsigned long long) (long long) (int32_t) w[0];
-}
-
-__global__ void __launch_bounds__(256)
-k_mj_bucket_join(const char* __restrict__ R, const uint64_t* __restrict__ roffs, uint32_t wR, uint32_t rkoff,
-		uint32_t rkb, const char* __restrict__ S, const uint64_t* __restrict__ soffs, uint32_t wS, uint32_t skoff,
-		uint32_t skb, long long kmin, int sum_side, uint32_t soff, uint32_t swords,
-		unsigned long long* __restrict__ agg, uint64_t* __restrict__ bucket_rows)
-{
-	__shared__ unsigned long long btot;
-	extern __shared__ __align__(16) unsigned char mj_smem[];
-	unsigned long long* sm = reinterpret_cast<unsigned long long*>(mj_smem);    // [MJ_LOCAL]
-	uint32_t* cR = reinterpret_cast<uint32_t*>(sm + MJ_LOCAL);                   // [MJ_LOCAL]
-	uint32_t* cS = cR + MJ_LOCAL;                                                // [MJ_LOCAL]
-	const uint32_t b = blockIdx.x;
-	for (uint32_t k = threadIdx.x; k < MJ_LOCAL; k += blockDim.x) { sm[k] = 0; cR[k] = 0; cS[k] = 0; }
-	if (threadIdx.x == 0) btot = 0;
-	__syncthreads();
-	const uint64_t r0 = roffs[b], r1 = roffs[b + 1], s0 = soffs[b], s1 = soffs[b + 1];
-	// Eight tuples per thread are loaded before their shared-memory updates,
-	// so eight loads are in flight per thread.
-	for (int side = 0; side < 2; ++side) {
-		const char* base = side ? S : R;
-		const uint64_t lo = side ? s0 : r0, hi = side ? s1 : r1;
-		const uint32_t w = side ? wS : wR, koff = side ? skoff : rkoff, kb = side ? skb : rkb;
-		uint32_t* cnt = side ? cS : cR;
-		const bool sums = sum_side == side;
-		for (uint64_t i0 = lo + threadIdx.x; i0 < hi; i0 += 8 * (uint64_t) blockDim.x) {
-			uint32_t k[8];
-			unsigned long long v[8];
-			#pragma unroll
-			for (int u = 0; u < 8; ++u) {
-				const uint64_t i = i0 + (uint64_t) u * blockDim.x;
-				k[u] = MJ_LOCAL;
-				v[u] = 0;
-				if (i < hi) {
-					const char* t = base + i * w;
-					k[u] = (uint32_t) ((unsigned long long) (pg_load_key(t + koff, kb) - kmin) & (MJ_LOCAL - 1));
-					if (sums) v[u] = mj_tuple_col(t, soff, swords);
-				}
-			}
-			#pragma unroll
-			for (int u = 0; u < 8; ++u) {
-				if (k[u] == MJ_LOCAL) continue;
-				atomicAdd(&cnt[k[u]], 1u);
-				if (sums) atomicAdd(&sm[k[u]], v[u]);
-			}
-		}
-	}
-	__syncthreads();
-	unsigned long long c = 0, sum = 0;
-	for (uint32_t k = threadIdx.x; k < MJ_LOCAL; k += blockDim.x) {
-		const unsigned long long a = cR[k], d = cS[k];
-		c += a * d;
-		if (sum_side == 0) sum += sm[k] * d;
-		else if (sum_side == 1) sum += sm[k] * a;
-	}
-	#pragma unroll
-	for (int o = 16; o > 0; o >>= 1) {
-		c += __shfl_down_sync(0xffffffffu, c, o);
-		sum += __shfl_down_sync(0xffffffffu, sum, o);
-	}
-	if ((threadIdx.x & 31) == 0) {
-		if (c) { atomicAdd(&agg[0], c); atomicAdd(&btot, c); }
-		if (sum) atomicAdd(&agg[1], sum);
-	}
-	if (bucket_rows) {
-		__syncthreads();
-		if (threadIdx.x == 0) bucket_rows[b] = btot;
-	}
-}
-
-// offs[b] = first index of the sorted relation whose bucket (key - kmin) >>
-// MJ_LOCAL_BITS is >= b, for b in [0, B]; the relation is sorted on the bucket.
-__global__ void k_mj_bounds(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, uint32_t kbytes,
-		long long kmin, uint32_t B, uint64_t* __restrict__ offs)
-{
-	const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-	if (b > B) return;
-	uint64_t lo = 0, hi = n;
-	while (lo < hi) {
-		const uint64_t mid = (lo + hi) >> 1;
-		const unsigned long long d = (unsigned long long) (pg_load_key(in + mid * W + koff, kbytes) - kmin);
-		if ((d >> MJ_LOCAL_BITS) < b) lo = mid + 1; else hi = mid;
-	}
-	offs[b] = lo;
-}
-
-// Key range into mm[0..1] (keys ^ 2^63 as unsigned); with `unsorted`, also
-// whether some key is greater than the next one.
+// Key range of tuples 0, step, 2 step, ... into mm[0..1] (keys ^ 2^63 as
+// unsigned); with `unsorted` (step 1), also whether some key is greater than
+// the next one.
 __global__ void k_mj_minmax(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, uint32_t kbytes,
-		unsigned long long* __restrict__ mm, unsigned long long* __restrict__ unsorted)
+		uint64_t step, unsigned long long* __restrict__ mm, unsigned long long* __restrict__ unsorted)
 {
 	unsigned long long lo = ~0ull, hi = 0;
 	bool down = false;
-	for (uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; i < n; i += (uint64_t) gridDim.x * blockDim.x) {
+	for (uint64_t i = (blockIdx.x * (uint64_t) blockDim.x + threadIdx.x) * step; i < n;
+			i += (uint64_t) gridDim.x * blockDim.x * step) {
 		const long long k = pg_load_key(in + i * W + koff, kbytes);
 		const unsigned long long u = (unsigned long long) k ^ (1ull << 63);
 		lo = u < lo ? u : lo;
@@ -409,19 +306,37 @@ __global__ void k_mj_minmax(const char* __restrict__ in, uint64_t n, uint32_t W,
 	if ((threadIdx.x & 31) == 0) { atomicMin(&mm[0], lo); atomicMax(&mm[1], hi); }
 }
 
+
 // ---------------------------------------------------------------------------
-// Materialised MPSM over key buckets (16-byte tuples, 8-byte keys, 16-byte
-// output rows). After the bucket partition of both sides (as for the
-// count/sum), k_mj_bucket_join writes each bucket's output row count, a scan
-// turns them into output offsets, and k_mj_bucket_write joins each bucket
-// pair in one CTA: the build side's packed values counting-sorted by key into
-// shared memory (a run per key), then every probe tuple writes one row per
-// build tuple of its key at a block-scanned position. Output rows are in
-// bucket order; within a bucket their order is unspecified (as for every
-// join output).
+// Keys of compact range: a counting sort of one side takes the place of sorting
+// both. A table of 4-byte counts over the key window [kmin, kmin + range) is
+// filled with one L2 atomic a tuple, and the other side looks its keys up.
+//
+// - Count/sum: the side without the summed column is counted; a tuple of the
+//   other side then adds its count to the rows and count * column to the sum.
+// - Rows: the build side is counted, the counts are scanned into run starts,
+//   its packed columns are scattered into their runs, and every probe tuple
+//   writes one row per value of its key's run.
+//
+// Both relations are read once or twice and neither is written back sorted,
+// which is what the sort-merge of the same join spends its time on.
 // ---------------------------------------------------------------------------
-#define MJW_THREADS 1024
-#define MJW_CAP 24576            // build tuples of one bucket held in shared memory (192 KB)
+#define MJ_ILP 8
+#define MJ_MAX_RANGE (1ull << 30)
+#define MJ_MIN_RANGE (1ull << 24)   // window always worth a table (64 MB, kept in L2)
+#define MJ_MAX_RUN 16384            // longest build run whose rows one warp writes for a probe tuple
+
+// Key of tuple i; V16: 16-byte tuples with an 8-byte key in either half.
+template <bool V16>
+__device__ __forceinline__ int64_t mj_key(const char* __restrict__ in, uint64_t i, uint32_t W, uint32_t koff,
+		uint32_t kbytes, uint64_t pol, uint4& t)
+{
+	if (V16) {
+		t = pg_ld_hint16(in + i * 16, pol);
+		return koff == 0 ? (int64_t) (((uint64_t) t.y << 32) | t.x) : (int64_t) (((uint64_t) t.w << 32) | t.z);
+	}
+	return pg_load_key(in + i * W + koff, kbytes);
+}
 
 // The build-projected words of a row that are not the join key, packed.
 struct MjPack {
@@ -434,153 +349,304 @@ __device__ __forceinline__ uint32_t mjw_word(const uint4& t, uint32_t i)
 	return i == 0 ? t.x : i == 1 ? t.y : i == 2 ? t.z : t.w;
 }
 
-// Output word source: 0-3 probe tuple word, 4-5 packed build word.
-__device__ __forceinline__ uint32_t mjw_pick(const uint4& t, unsigned long long v, uint32_t sel)
+__device__ __forceinline__ unsigned long long mj_packed(const uint4& t, const MjPack& bp)
 {
-	return sel < 4 ? mjw_word(t, sel) : sel == 4 ? (uint32_t) v : (uint32_t) (v >> 32);
+	unsigned long long v = 0;
+	if (bp.n > 0) v = mjw_word(t, bp.roff[0]);
+	if (bp.n > 1) v |= (unsigned long long) mjw_word(t, bp.roff[1]) << 32;
+	return v;
 }
 
-// Exclusive scan of x over the CTA's MJW_THREADS threads; *total = the sum.
-// wsum: MJW_THREADS / 32 words of shared memory. Ends with a barrier.
-__device__ __forceinline__ uint32_t mjw_block_scan(uint32_t x, uint32_t* wsum, uint32_t* total)
+// cnt[key - kmin] += 1 for every tuple; a key outside the window sets *outside.
+// Lanes that hold lane 0's key add once together when there are several of
+// them, so that one key with most of the rows does not queue 32 adds a warp.
+// VALS: also the range of the packed build values, into vmm[0..1].
+template <bool V16, bool VALS>
+__global__ void __launch_bounds__(256)
+k_mj_count(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, uint32_t kbytes, long long kmin,
+		uint32_t range, uint32_t* __restrict__ cnt, unsigned int* __restrict__ outside, MjPack bp,
+		unsigned long long* __restrict__ vmm)
 {
-	const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	uint32_t inc = x;
-	#pragma unroll
-	for (int o = 1; o < 32; o <<= 1) {
-		const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-		if (lane >= (uint32_t) o) inc += y;
+	unsigned long long vlo = ~0ull, vhi = 0;
+	const uint64_t stride = (uint64_t) gridDim.x * blockDim.x, pol = pg_policy_evict_first();
+	const uint32_t lane = threadIdx.x & 31;
+	bool out = false;
+	for (uint64_t base = blockIdx.x * (uint64_t) blockDim.x; base < n; base += stride * MJ_ILP) {
+		uint32_t d[MJ_ILP];
+		#pragma unroll
+		for (int j = 0; j < MJ_ILP; ++j) {
+			const uint64_t i = base + threadIdx.x + j * stride;
+			d[j] = 0xFFFFFFFFu;
+			if (i < n) {
+				uint4 t;
+				const uint64_t x = (uint64_t) mj_key<V16>(in, i, W, koff, kbytes, pol, t) - (uint64_t) kmin;
+				if (x < range) d[j] = (uint32_t) x; else out = true;
+				if (VALS) {
+					const unsigned long long v = mj_packed(t, bp);
+					vlo = min(vlo, v);
+					vhi = max(vhi, v);
+				}
+			}
+		}
+		#pragma unroll
+		for (int j = 0; j < MJ_ILP; ++j) {
+			const uint32_t same = __ballot_sync(0xffffffffu, d[j] == __shfl_sync(0xffffffffu, d[j], 0));
+			const bool many = __popc(same) >= 4;
+			if (d[j] == 0xFFFFFFFFu || (many && lane && (same >> lane & 1))) continue;
+			atomicAdd(&cnt[d[j]], many && lane == 0 ? (uint32_t) __popc(same) : 1u);
+		}
 	}
-	if (lane == 31) wsum[warp] = inc;
+	if (out) *outside = 1;
+	if (VALS) {
+		__shared__ unsigned long long red[2][8];
+		#pragma unroll
+		for (int o = 16; o > 0; o >>= 1) {
+			vlo = min(vlo, __shfl_xor_sync(0xffffffffu, vlo, o));
+			vhi = max(vhi, __shfl_xor_sync(0xffffffffu, vhi, o));
+		}
+		if (lane == 0) { red[0][threadIdx.x >> 5] = vlo; red[1][threadIdx.x >> 5] = vhi; }
+		__syncthreads();
+		if (threadIdx.x == 0) {
+			for (int w = 1; w < 8; ++w) { vlo = min(vlo, red[0][w]); vhi = max(vhi, red[1][w]); }
+			atomicMin(&vmm[0], vlo);
+			atomicMax(&vmm[1], vhi);
+		}
+	}
+}
+
+// agg[0] += the other side's tuples of each key, agg[1] += that many times
+// column (soff, swords); swords 0: no sum.
+template <bool V16>
+__global__ void __launch_bounds__(256)
+k_mj_lookup(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, uint32_t kbytes, uint32_t soff,
+		uint32_t swords, long long kmin, uint32_t range, const uint32_t* __restrict__ cnt,
+		unsigned long long* __restrict__ agg)
+{
+	__shared__ unsigned long long red[2][8];
+	const uint64_t stride = (uint64_t) gridDim.x * blockDim.x, pol = pg_policy_evict_first();
+	const uint64_t keep = pg_policy_keep(4);
+	unsigned long long rows = 0, sum = 0;
+	for (uint64_t base = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; base < n; base += stride * MJ_ILP) {
+		uint32_t c[MJ_ILP];
+		unsigned long long v[MJ_ILP];
+		#pragma unroll
+		for (int j = 0; j < MJ_ILP; ++j) {
+			const uint64_t i = base + j * stride;
+			c[j] = 0;
+			v[j] = 0;
+			if (i < n) {
+				uint4 t;
+				const uint64_t x = (uint64_t) mj_key<V16>(in, i, W, koff, kbytes, pol, t) - (uint64_t) kmin;
+				if (V16) {
+					const uint32_t w = soff / 4;
+					const uint32_t lo = w == 0 ? t.x : w == 1 ? t.y : w == 2 ? t.z : t.w;
+					const uint32_t hi = w == 0 ? t.y : w == 1 ? t.z : t.w;
+					v[j] = swords == 2 ? ((unsigned long long) hi << 32) | lo : (unsigned long long) (long long) (int32_t) lo;
+				}
+				if (x < range) {
+					asm("ld.global.nc.L1::evict_last.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(c[j]) : "l"(cnt + x), "l"(keep));
+					if (!V16 && swords) {
+						const uint32_t* q = reinterpret_cast<const uint32_t*>(in + i * W + soff);
+						v[j] = swords == 2 ? ((unsigned long long) q[1] << 32) | q[0] : (unsigned long long) (long long) (int32_t) q[0];
+					}
+				}
+			}
+		}
+		#pragma unroll
+		for (int j = 0; j < MJ_ILP; ++j) { rows += c[j]; sum += v[j] * c[j]; }
+	}
+	#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) {
+		rows += __shfl_down_sync(0xffffffffu, rows, o);
+		sum += __shfl_down_sync(0xffffffffu, sum, o);
+	}
+	if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = rows; red[1][threadIdx.x >> 5] = sum; }
 	__syncthreads();
-	if (warp == 0) {
-		uint32_t w = lane < MJW_THREADS / 32 ? wsum[lane] : 0;
+	if (threadIdx.x < 2) {
+		unsigned long long t = 0;
+		#pragma unroll
+		for (int w = 0; w < 8; ++w) t += red[threadIdx.x][w];
+		if (t && (threadIdx.x == 0 || swords)) atomicAdd(&agg[threadIdx.x], t);
+	}
+}
+
+// Exclusive scan of the counts in place (mod 2^32; a side has fewer than 2^32
+// tuples): sums of MJ_SCAN counts, their scan (pg_scan_u64), then each
+// block's counts. The largest count goes to *mx.
+#define MJ_SCAN 4096
+__global__ void __launch_bounds__(256)
+k_mj_scan_sums(const uint32_t* __restrict__ cnt, uint32_t range, uint64_t* __restrict__ sums, unsigned int* __restrict__ mx)
+{
+	__shared__ uint32_t red[2][8];
+	const uint64_t lo = (uint64_t) blockIdx.x * MJ_SCAN;
+	uint32_t s = 0, m = 0;
+	#pragma unroll
+	for (int j = 0; j < MJ_SCAN / 256; ++j) {
+		const uint64_t i = lo + j * 256 + threadIdx.x;
+		const uint32_t c = i < range ? cnt[i] : 0;
+		s += c;
+		m = max(m, c);
+	}
+	s = __reduce_add_sync(0xffffffffu, s);
+	m = __reduce_max_sync(0xffffffffu, m);
+	if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = s; red[1][threadIdx.x >> 5] = m; }
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		for (int w = 1; w < 8; ++w) { s += red[0][w]; m = max(m, red[1][w]); }
+		sums[blockIdx.x] = s;
+		if (m > *mx) atomicMax(mx, m);
+	}
+}
+
+__global__ void __launch_bounds__(256)
+k_mj_scan_apply(uint32_t* __restrict__ cnt, uint32_t range, const uint64_t* __restrict__ sums)
+{
+	__shared__ uint32_t wt[8];
+	const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	constexpr int PER = MJ_SCAN / 256;
+	// Warp w scans its own MJ_SCAN / 8 counts, 32 at a time.
+	const uint64_t lo = (uint64_t) blockIdx.x * MJ_SCAN + warp * (MJ_SCAN / 8) + lane;
+	uint32_t c[PER], mine = 0;
+	#pragma unroll
+	for (int j = 0; j < PER; ++j) { c[j] = lo + j * 32 < range ? cnt[lo + j * 32] : 0; mine += c[j]; }
+	const uint32_t tot = __reduce_add_sync(0xffffffffu, mine);
+	if (lane == 0) wt[warp] = tot;
+	__syncthreads();
+	uint32_t run = (uint32_t) sums[blockIdx.x];
+	for (uint32_t w = 0; w < warp; ++w) run += wt[w];
+	#pragma unroll
+	for (int j = 0; j < PER; ++j) {
+		uint32_t x = c[j];
 		#pragma unroll
 		for (int o = 1; o < 32; o <<= 1) {
-			const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-			if (lane >= (uint32_t) o) w += y;
+			const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+			if (lane >= (uint32_t) o) x += y;
 		}
-		if (lane < MJW_THREADS / 32) wsum[lane] = w;
+		if (lo + j * 32 < range) cnt[lo + j * 32] = run + x - c[j];
+		run += __shfl_sync(0xffffffffu, x, 31);
 	}
-	__syncthreads();
-	const uint32_t before = (warp ? wsum[warp - 1] : 0) + inc - x;
-	*total = wsum[MJW_THREADS / 32 - 1];
-	__syncthreads();
-	return before;
 }
 
-__global__ void __launch_bounds__(MJW_THREADS, 1)
-k_mj_bucket_write(const uint4* __restrict__ R, const uint64_t* __restrict__ roffs, uint32_t rkw, MjPack bp,
-		const uint4* __restrict__ S, const uint64_t* __restrict__ soffs, uint32_t skw, long long kmin,
-		const uint64_t* __restrict__ bucket_off, uint32_t wsel, uint4* __restrict__ out, int* __restrict__ status)
+// Scatters the packed build columns into their keys' runs: pos[d] is run d's
+// first slot before and its end (the next run's start) after. Values that
+// span less than 2^32 are kept as 4-byte differences from the smallest (vmm,
+// from the counting pass): half the bytes that the scattered stores and the
+// probe's scattered reads move. Nothing is done
+// when a run is longer than MJ_MAX_RUN or a key lay outside the window
+// (meta[0], meta[1]).
+__global__ void __launch_bounds__(256)
+k_mj_fill(const char* __restrict__ R, uint64_t n, uint32_t koff, long long kmin, uint32_t range, MjPack bp,
+		uint32_t* __restrict__ pos, unsigned long long* __restrict__ val, const unsigned int* __restrict__ meta,
+		const unsigned long long* __restrict__ vmm)
 {
-	extern __shared__ __align__(16) unsigned char mw_smem[];
-	unsigned long long* rv = reinterpret_cast<unsigned long long*>(mw_smem);     // [MJW_CAP]
-	uint32_t* start = reinterpret_cast<uint32_t*>(rv + MJW_CAP);                // [MJ_LOCAL + 1]
-	uint32_t* fill = start + MJ_LOCAL + 1;                                       // [MJ_LOCAL]
-	uint32_t* wsum = fill + MJ_LOCAL;                                            // [MJW_THREADS / 32]
-	const uint32_t b = blockIdx.x, tid = threadIdx.x;
-	const uint64_t r0 = roffs[b], r1 = roffs[b + 1], s0 = soffs[b], s1 = soffs[b + 1];
-	if (r1 - r0 > MJW_CAP) {             // the host checked every bucket; never taken
-		if (tid == 0) pg_set_status(status, PG_ERR_UNSUPPORTED);
-		return;
-	}
-	const unsigned long long kbase = (unsigned long long) kmin;
-	for (uint32_t k = tid; k < MJ_LOCAL; k += MJW_THREADS) { start[k] = 0; fill[k] = 0; }
-	__syncthreads();
-	// Build side: per-key counts, their exclusive scan (run starts), then the
-	// packed values scattered into their key's run.
-	for (uint64_t i = r0 + tid; i < r1; i += MJW_THREADS) {
-		const uint4 t = R[i];
-		const unsigned long long key = ((unsigned long long) mjw_word(t, rkw + 1) << 32) | mjw_word(t, rkw);
-		atomicAdd(&start[(key - kbase) & (MJ_LOCAL - 1)], 1u);
-	}
-	__syncthreads();
-	{
-		constexpr uint32_t PER = MJ_LOCAL / MJW_THREADS;        // 4 entries per thread
-		uint32_t v[PER], run = 0;
+	if (meta[0] > MJ_MAX_RUN || meta[1]) return;
+	const unsigned long long vmin = vmm[0];
+	const bool narrow = vmm[1] - vmin < (1ull << 32);
+	const uint64_t stride = (uint64_t) gridDim.x * blockDim.x, pol = pg_policy_evict_first();
+	for (uint64_t base = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; base < n; base += stride * 4) {
+		uint4 t[4];
+		uint32_t at[4];
 		#pragma unroll
-		for (uint32_t j = 0; j < PER; ++j) { v[j] = start[tid * PER + j]; run += v[j]; }
-		uint32_t total;
-		uint32_t base = mjw_block_scan(run, wsum, &total);
+		for (int j = 0; j < 4; ++j) {
+			const uint64_t i = base + j * stride;
+			at[j] = 0xFFFFFFFFu;
+			if (i < n) {
+				const uint64_t x = (uint64_t) mj_key<true>(R, i, 16, koff, 8, pol, t[j]) - (uint64_t) kmin;
+				at[j] = (uint32_t) x;
+			}
+		}
 		#pragma unroll
-		for (uint32_t j = 0; j < PER; ++j) { start[tid * PER + j] = base; base += v[j]; }
-		if (tid == 0) start[MJ_LOCAL] = total;
+		for (int j = 0; j < 4; ++j)
+			if (at[j] < range) at[j] = atomicAdd(&pos[at[j]], 1u); else at[j] = 0xFFFFFFFFu;
+		#pragma unroll
+		for (int j = 0; j < 4; ++j) {
+			if (at[j] >= n) continue;
+			const unsigned long long v = mj_packed(t[j], bp);
+			if (narrow) reinterpret_cast<uint32_t*>(val)[at[j]] = (uint32_t) (v - vmin);
+			else val[at[j]] = v;
+		}
 	}
-	__syncthreads();
-	for (uint64_t i = r0 + tid; i < r1; i += MJW_THREADS) {
-		const uint4 t = R[i];
-		const unsigned long long key = ((unsigned long long) mjw_word(t, rkw + 1) << 32) | mjw_word(t, rkw);
-		const uint32_t k = (uint32_t) ((key - kbase) & (MJ_LOCAL - 1));
-		const uint32_t pos = start[k] + atomicAdd(&fill[k], 1u);
-		unsigned long long pv = 0;
-		if (bp.n > 0) pv = mjw_word(t, bp.roff[0]);
-		if (bp.n > 1) pv |= (unsigned long long) mjw_word(t, bp.roff[1]) << 32;
-		rv[pos] = pv;
-	}
-	__syncthreads();
-	// Probe side in chunks of MJW_THREADS tuples, the next chunk's tuples
-	// loaded while the current one is written. Tuple i of a chunk makes m_i
-	// rows (one per build tuple of its key) at its scanned offset; the rows are
-	// written load-balanced, thread j of the CTA taking the chunk's rows j,
-	// j + MJW_THREADS, ..., so a warp stores 32 consecutive rows whatever the
-	// duplicates. A row finds its probe tuple by binary search over the
-	// offsets, which reuse the fill counters' shared memory (dead after the
-	// build side).
-	uint32_t* coff = fill;                                                       // [MJW_THREADS]
-	uint32_t* crs = fill + MJW_THREADS;                                          // [MJW_THREADS]
+}
+
+// Rows of each probe tuple: one per value of its key's run [end[d - 1],
+// end[d]). A warp looks up 128 tuples at once, reserves their rows with one
+// add on the cursor, and writes them 32 at a time, each lane finding its row's
+// tuple by a search over the lanes' offsets, so that a warp stores consecutive
+// rows whatever the runs' lengths. Rows past `cap` are counted only.
+__global__ void __launch_bounds__(256)
+k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin, uint32_t range,
+		const uint32_t* __restrict__ end, const unsigned long long* __restrict__ val, uint32_t wsel,
+		uint4* __restrict__ out, uint64_t cap, unsigned long long* __restrict__ cursor, const unsigned int* __restrict__ meta,
+		const unsigned long long* __restrict__ vmm)
+{
+	if (meta[0] > MJ_MAX_RUN || meta[1]) return;
+	const unsigned long long vmin = vmm[0];
+	const bool narrow = vmm[1] - vmin < (1ull << 32);
+	const uint32_t lane = threadIdx.x & 31;
+	const uint64_t pol = pg_policy_evict_first();
+	const uint64_t nwarps = ((uint64_t) gridDim.x * blockDim.x) >> 5;
 	const uint32_t w0 = wsel & 15, w1 = (wsel >> 4) & 15, w2 = (wsel >> 8) & 15, w3 = (wsel >> 12) & 15;
-	uint64_t row = bucket_off[b];
-	uint4 tn = make_uint4(0, 0, 0, 0);
-	if (s0 + tid < s1) tn = S[s0 + tid];
-	for (uint64_t c0 = s0; c0 < s1; c0 += MJW_THREADS) {
-		const uint4 t = tn;
-		const uint64_t i = c0 + tid;
-		if (i + MJW_THREADS < s1) tn = S[i + MJW_THREADS];
-		uint32_t m = 0, rs = 0;
-		if (i < s1) {
-			const unsigned long long key = ((unsigned long long) mjw_word(t, skw + 1) << 32) | mjw_word(t, skw);
-			const uint32_t k = (uint32_t) ((key - kbase) & (MJ_LOCAL - 1));
-			rs = start[k];
-			m = start[k + 1] - rs;
+	for (uint64_t c0 = (((uint64_t) blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 128; c0 < n; c0 += nwarps * 128) {
+		uint4 t[4];
+		uint32_t lo[4], m[4];
+		#pragma unroll
+		for (int j = 0; j < 4; ++j) {
+			const uint64_t i = c0 + j * 32 + lane;
+			lo[j] = 0; m[j] = 0;
+			t[j] = make_uint4(0, 0, 0, 0);
+			if (i < n) {
+				const uint64_t x = (uint64_t) mj_key<true>(S, i, 16, koff, 8, pol, t[j]) - (uint64_t) kmin;
+				if (x < range) {
+					m[j] = __ldg(end + x);
+					if (x) lo[j] = __ldg(end + x - 1);
+				}
+			}
 		}
-		uint32_t total;
-		// The scan's barriers also order this chunk's offset writes after
-		// every thread's reads of the previous chunk's offsets.
-		const uint32_t off = mjw_block_scan(m, wsum, &total);
-		coff[tid] = off;
-		crs[tid] = rs;
-		__syncthreads();
-		for (uint32_t j = tid; j < total; j += MJW_THREADS) {
-			uint32_t x = 0;                  // the last tuple whose offset is <= j (it has m > 0)
+		uint32_t off[4], total = 0;
+		#pragma unroll
+		for (int j = 0; j < 4; ++j) {
+			m[j] -= lo[j];
+			uint32_t x = m[j];
 			#pragma unroll
-			for (uint32_t step = MJW_THREADS / 2; step; step >>= 1)
-				if (coff[x + step] <= j) x += step;
-			const unsigned long long v = rv[crs[x] + (j - coff[x])];
-			const uint4 p = S[c0 + x];
-			out[row + j] = make_uint4(mjw_pick(p, v, w0), mjw_pick(p, v, w1), mjw_pick(p, v, w2), mjw_pick(p, v, w3));
+			for (int o = 1; o < 32; o <<= 1) {
+				const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+				if (lane >= (uint32_t) o) x += y;
+			}
+			off[j] = x - m[j];
+			m[j] = __shfl_sync(0xffffffffu, x, 31);       // rows of the 32 tuples
+			total += m[j];
 		}
-		row += total;
+		unsigned long long row = 0;
+		if (lane == 0 && total) row = atomicAdd(cursor, (unsigned long long) total);
+		row = __shfl_sync(0xffffffffu, row, 0);
+		#pragma unroll
+		for (int j = 0; j < 4; ++j) {
+			for (uint32_t r0 = 0; r0 < m[j]; r0 += 32) {
+				const uint32_t r = r0 + lane;
+				uint32_t x = 0;                  // the last tuple whose offset is <= r (it has rows)
+				#pragma unroll
+				for (uint32_t step = 16; step; step >>= 1)
+					if (__shfl_sync(0xffffffffu, off[j], x + step) <= r) x += step;
+				const uint32_t at = __shfl_sync(0xffffffffu, lo[j], x) + (r - __shfl_sync(0xffffffffu, off[j], x));
+				unsigned long long v = 0;
+				if (r < m[j]) v = narrow ? vmin + __ldg(reinterpret_cast<const uint32_t*>(val) + at) : __ldg(val + at);
+				auto pick = [&](uint32_t w) -> uint32_t {
+					return w < 4 ? __shfl_sync(0xffffffffu, mjw_word(t[j], w), x) : w == 4 ? (uint32_t) v : (uint32_t) (v >> 32);
+				};
+				const uint4 o = make_uint4(pick(w0), pick(w1), pick(w2), pick(w3));
+				if (r < m[j] && row + r < cap) pg_st_hint16(out + row + r, o, pol);
+			}
+			row += m[j];
+		}
 	}
-}
-
-// Largest build-side bucket (roffs[b + 1] - roffs[b]) into *mx.
-__global__ void k_mj_max_bucket(const uint64_t* __restrict__ offs, uint32_t B, unsigned long long* __restrict__ mx)
-{
-	unsigned long long m = 0;
-	for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < B; b += gridDim.x * blockDim.x)
-		m = max(m, (unsigned long long) (offs[b + 1] - offs[b]));
-	#pragma unroll
-	for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_down_sync(0xffffffffu, m, o));
-	if ((threadIdx.x & 31) == 0 && m) atomicMax(mx, m);
 }
 
 // Word selector (4 bits per output word: 0-3 probe tuple word, 4-5 packed
 // build word) and packed build words of the 16-byte output rows of the
-// bucketed materialising join; false when the layout is not one it takes:
+// counted materialising join; false when the layout is not one it takes:
 // 16-byte tuples with 8-byte keys on both sides, 16-byte rows whose build
 // words other than the key (taken from the probe tuple's equal key) fit 8 bytes.
-static bool mj_bucket_rows_fit(const pg_rel* R, const pg_rel* S, const MjCols& pc, uint32_t* wsel, MjPack* bp)
+static bool mj_rows_fit(const pg_rel* R, const pg_rel* S, const MjCols& pc, uint32_t* wsel, MjPack* bp)
 {
 	if (R->width != 16 || S->width != 16 || R->key_bytes != 8 || S->key_bytes != 8 || (R->key_off & 7) ||
 			(S->key_off & 7) || pc.ow_words != 4 ||
@@ -612,127 +678,142 @@ static bool mj_bucket_rows_fit(const pg_rel* R, const pg_rel* S, const MjCols& p
 	return true;
 }
 
-// Joins over key buckets when the key span is 2^13..2^24 values: both sides
-// partitioned on the key bits above the low 12, then each bucket pair in
-// shared memory. Without `materialize` the per-key counts give the count and
-// sum (MjCols sum column); with it, the rows are written (16-byte layouts
-// that mj_bucket_rows_fit takes, every bucket's build side within MJW_CAP
-// tuples). *handled = false (nothing produced) when the case is not one it
-// takes: the caller then sorts.
-static int mj_bucket_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_rel* S, const MjCols& pc,
-		int sum_col, int flags, void* out, uint64_t out_capacity, pg_join_result* res, bool* handled,
-		bool* r_sorted, bool* s_sorted)
+
+static bool mj_v16(const pg_rel* r)
+{
+	return r->width == 16 && r->key_bytes == 8 && (r->key_off == 0 || r->key_off == 8) &&
+		!(reinterpret_cast<uintptr_t>(r->data) & 15);
+}
+
+// The join by a table of counts when the counted side's keys span a compact
+// range: at most 2^24 values, or 16 times its tuples (64 M x 64 M with 2^30
+// spans: the table's random accesses still cost less than sorting both sides).
+// The window comes from every 1024th tuple widened by 1/64 a side on large
+// inputs, checked by the counting pass, else from every tuple. *handled =
+// false (nothing produced): the caller sorts.
+static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_rel* S, const MjCols& pc, int sum_col,
+		int flags, void* out, uint64_t out_capacity, pg_join_result* res, bool* handled)
 {
 	*handled = false;
-	*r_sorted = *s_sorted = false;
 	const bool materialize = (flags & PG_JOIN_MATERIALIZE) != 0;
 	uint32_t wsel = 0;
-	MjPack bp;
-	const bool rows_fit = mj_bucket_rows_fit(R, S, pc, &wsel, &bp) && !(reinterpret_cast<uintptr_t>(out) & 15);
+	MjPack bp = {};
+	if (materialize && (!mj_rows_fit(R, S, pc, &wsel, &bp) || (reinterpret_cast<uintptr_t>(out) & 15)))
+		return PG_OK;
+	if (materialize && sum_col >= 0) {      // the sum as a join of its own, then the rows
+		pg_join_result a;
+		bool done = false;
+		int rs = mj_dense_join(ctx, s, R, S, pc, sum_col, flags & ~PG_JOIN_MATERIALIZE, nullptr, 0, &a, &done);
+		if (rs || !done) return rs;
+		if ((rs = mj_dense_join(ctx, s, R, S, pc, -1, flags, out, out_capacity, res, handled)) || !*handled) return rs;
+		res->sum = a.sum;
+		return PG_OK;
+	}
+	// C is counted, P looks up.
+	const bool sum_build = sum_col >= 0 && pc.side[sum_col] == 0;
+	const bool count_build = materialize || (sum_col >= 0 ? !sum_build : R->n <= S->n);
+	const pg_rel *C = count_build ? R : S, *P = count_build ? S : R;
 	int rc;
-	// [key min, key max, count, sum, largest build bucket, R unsorted, S unsorted]
+	// [key min, key max], [rows, sum], [largest count, key outside], [value min, value max]
 	unsigned long long* mm = nullptr;
 	if ((rc = pg_alloc_async(ctx, s, (void**) &mm, 64))) return rc;
-	const unsigned long long init[8] = {~0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull};
-	PG_CUDA(ctx, cudaMemcpyAsync(mm, init, 64, cudaMemcpyHostToDevice, s));
-	for (int side = 0; side < 2; ++side) {
-		const pg_rel* r = side ? S : R;
-		const bool check = (flags & (side ? PG_JOIN_PROBE_SORTED : PG_JOIN_BUILD_SORTED)) != 0;
-		const int blocks = (int) std::min<uint64_t>(pg_div_up(r->n, 256), (uint64_t) ctx->sm_count * 8);
-		k_mj_minmax<<<blocks, 256, 0, s>>>((const char*) r->data, r->n, r->width, r->key_off, r->key_bytes, mm,
-				check ? mm + 5 + side : nullptr);
+	unsigned long long* agg = mm + 2;
+	unsigned int* meta = reinterpret_cast<unsigned int*>(mm + 4);
+	unsigned long long* vmm = mm + 5;
+	for (int attempt = C->n >= (1ull << 22) ? 0 : 1; attempt < 2; ++attempt) {
+		const uint64_t step = attempt == 0 ? 1024 : 1;
+		const unsigned long long init[7] = {~0ull, 0ull, 0ull, 0ull, 0ull, ~0ull, 0ull};
+		PG_CUDA(ctx, cudaMemcpyAsync(mm, init, sizeof init, cudaMemcpyHostToDevice, s));
+		const int mblocks = (int) std::min<uint64_t>(pg_div_up(pg_div_up(C->n, step), 256), (uint64_t) ctx->sm_count * 8);
+		k_mj_minmax<<<mblocks, 256, 0, s>>>((const char*) C->data, C->n, C->width, C->key_off, C->key_bytes, step, mm, nullptr);
 		PG_LAUNCHED(ctx);
-	}
-	unsigned long long h[8];
-	PG_CUDA(ctx, cudaMemcpyAsync(h, mm, 64, cudaMemcpyDeviceToHost, s));
-	PG_CUDA(ctx, cudaStreamSynchronize(s));
-	// A side confirmed sorted skips its sort (here: its bucket partition).
-	*r_sorted = (flags & PG_JOIN_BUILD_SORTED) && !h[5];
-	*s_sorted = (flags & PG_JOIN_PROBE_SORTED) && !h[6];
-	if (materialize && !rows_fit) { pg_free_async(ctx, s, mm); return PG_OK; }
-	const unsigned long long span = h[1] - h[0];
-	const int bits = span == 0 ? 0 : 64 - __builtin_clzll(span);
-	if (bits <= (int) MJ_LOCAL_BITS || bits > (int) MJ_LOCAL_BITS + 12) { pg_free_async(ctx, s, mm); return PG_OK; }
-	const long long kmin = (long long) (h[0] ^ (1ull << 63));
-	const int hb = bits - MJ_LOCAL_BITS;
-	const uint32_t B = 1u << hb;
-	// Stable radix passes over the bucket bits (one of up to 8 bits, or two
-	// halves of at most 6: the fast partition shapes), then the bucket
-	// bounds by binary search.
-	const int npass = hb <= 8 ? 1 : 2;
-	const int d0 = npass == 1 ? hb : hb / 2;
-	char *pR = nullptr, *pS = nullptr, *tmp = nullptr;
-	uint64_t *oR = nullptr, *oS = nullptr, *brows = nullptr;
-	auto release = [&]() {
-		for (void* p : {(void*) pR, (void*) pS, (void*) tmp, (void*) oR, (void*) oS, (void*) brows, (void*) mm})
-			pg_free_async(ctx, s, p);
-	};
-	if (!*r_sorted && (rc = pg_alloc_async(ctx, s, (void**) &pR, R->n * R->width))) return rc;
-	if (!*s_sorted && (rc = pg_alloc_async(ctx, s, (void**) &pS, S->n * S->width))) return rc;
-	if (npass == 2 && !(*r_sorted && *s_sorted) &&
-			(rc = pg_alloc_async(ctx, s, (void**) &tmp, std::max(R->n * R->width, S->n * S->width)))) return rc;
-	if ((rc = pg_alloc_async(ctx, s, (void**) &oR, (B + 1) * 8))) return rc;
-	if ((rc = pg_alloc_async(ctx, s, (void**) &oS, (B + 1) * 8))) return rc;
-	if (materialize && (rc = pg_alloc_async(ctx, s, (void**) &brows, (B + 1) * 8))) return rc;
-	const char* bR = *r_sorted ? (const char*) R->data : pR;   // each side in bucket order
-	const char* bS = *s_sorted ? (const char*) S->data : pS;
-	for (int side = 0; side < 2; ++side) {
-		const pg_rel* in = side ? S : R;
-		char* dst = side ? pS : pR;
-		pg_rel cur = *in;
-		const bool sorted = side ? *s_sorted : *r_sorted;
-		for (int p = 0; p < npass && !sorted; ++p) {
-			const int d = p == 0 ? d0 : hb - d0;
-			pg_hashfn f;
-			f.fn = PG_FN_PARAMMODULO;
-			f.skipbits = MJ_LOCAL_BITS + (p == 0 ? 0 : d0);
-			f.k = (int64_t) ((1u << d) - 1) << f.skipbits;
-			f.min = kmin;
-			f.max = 0; f.bucketrange = 0;
-			f.nbuckets = 1u << d;
-			char* o = (npass == 2 && p == 0) ? tmp : dst;
-			if ((rc = pg_partition_fn(ctx, s, &cur, f, o, nullptr))) return rc;
-			cur.data = o;
+		unsigned long long h[4];
+		PG_CUDA(ctx, cudaMemcpyAsync(h, mm, 16, cudaMemcpyDeviceToHost, s));
+		PG_CUDA(ctx, cudaStreamSynchronize(s));
+		if (step > 1) {
+			const unsigned long long slack = (h[1] - h[0]) / 64 + 64;
+			h[0] = h[0] > slack ? h[0] - slack : 0;
+			h[1] = ~0ull - h[1] > slack ? h[1] + slack : ~0ull;
 		}
-		k_mj_bounds<<<(B + 256) / 256, 256, 0, s>>>(side ? bS : bR, in->n, in->width, in->key_off, in->key_bytes,
-				kmin, B, side ? oS : oR);
+		const unsigned long long span = h[1] - h[0];
+		// A sample's span is at most the exact one: too wide ends both attempts.
+		if (span >= MJ_MAX_RANGE || span >= std::max<unsigned long long>(MJ_MIN_RANGE + (MJ_MIN_RANGE >> 4), 16 * C->n)) break;
+		const uint32_t range = (uint32_t) span + 1;
+		const long long kmin = (long long) (h[0] ^ (1ull << 63));
+		uint32_t* cnt = nullptr;
+		uint64_t* sums = nullptr;
+		unsigned long long* val = nullptr;
+		auto release = [&]() { for (void* p : {(void*) cnt, (void*) sums, (void*) val}) pg_free_async(ctx, s, p); };
+		if ((rc = pg_alloc_async(ctx, s, (void**) &cnt, (uint64_t) range * 4))) return rc;
+		PG_CUDA(ctx, cudaMemsetAsync(cnt, 0, (uint64_t) range * 4, s));
+		const int cblocks = (int) std::min<uint64_t>(pg_div_up(C->n, 256 * MJ_ILP), (uint64_t) ctx->sm_count * 16);
+		const int pblocks = (int) std::min<uint64_t>(pg_div_up(P->n, 256 * MJ_ILP), (uint64_t) ctx->sm_count * 16);
+#define MJ_COUNT(V, VALS) k_mj_count<V, VALS><<<cblocks, 256, 0, s>>>((const char*) C->data, C->n, C->width, C->key_off, \
+				C->key_bytes, kmin, range, cnt, meta + 1, bp, vmm)
+		if (materialize) MJ_COUNT(true, true);
+		else if (mj_v16(C)) MJ_COUNT(true, false);
+		else MJ_COUNT(false, false);
+#undef MJ_COUNT
 		PG_LAUNCHED(ctx);
-	}
-	PG_CUDA(ctx, cudaMemsetAsync(mm + 2, 0, 24, s));
-	const int sum_side = sum_col < 0 ? -1 : (int) pc.side[sum_col];
-	const size_t smem = MJ_LOCAL * (8 + 4 + 4);
-	PG_CUDA(ctx, cudaFuncSetAttribute(k_mj_bucket_join, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-	k_mj_bucket_join<<<B, 256, smem, s>>>(bR, oR, R->width, R->key_off, R->key_bytes, bS, oS, S->width, S->key_off,
-			S->key_bytes, kmin, sum_side, sum_col >= 0 ? pc.off[sum_col] : 0, sum_col >= 0 ? pc.words[sum_col] : 0,
-			mm + 2, brows);
-	PG_LAUNCHED(ctx);
-	if (materialize) {
-		if ((rc = pg_scan_u64(ctx, s, brows, B, nullptr))) { release(); return rc; }
-		k_mj_max_bucket<<<(B + 255) / 256, 256, 0, s>>>(oR, B, mm + 4);
-		PG_LAUNCHED(ctx);
-	}
-	unsigned long long o[3];
-	PG_CUDA(ctx, cudaMemcpyAsync(o, mm + 2, 24, cudaMemcpyDeviceToHost, s));
-	if ((rc = pg_check_status(ctx, s, "pg_mpsm_join"))) { release(); return rc; }
-	if (materialize && o[2] > MJW_CAP) { release(); return PG_OK; }     // a bucket too large: sort instead
-	res->n_out = o[0];
-	res->sum = (int64_t) o[1];
-	*handled = true;
-	if (materialize && o[0]) {
-		if (o[0] > out_capacity) {
-			release();
-			return pg_fail(ctx, PG_ERR_OUTPUT_FULL, "pg_mpsm_join: output capacity too small");
+		if (!materialize) {
+			const uint32_t soff = sum_col >= 0 ? pc.off[sum_col] : 0, swords = sum_col >= 0 ? pc.words[sum_col] : 0;
+			if (mj_v16(P)) k_mj_lookup<true><<<pblocks, 256, 0, s>>>((const char*) P->data, P->n, 16, P->key_off, 8, soff,
+					swords, kmin, range, cnt, agg);
+			else k_mj_lookup<false><<<pblocks, 256, 0, s>>>((const char*) P->data, P->n, P->width, P->key_off, P->key_bytes,
+					soff, swords, kmin, range, cnt, agg);
+			PG_LAUNCHED(ctx);
+		} else {
+			const uint64_t nb = pg_div_up(range, MJ_SCAN);
+			if ((rc = pg_alloc_async(ctx, s, (void**) &sums, nb * 8)) ||
+					(rc = pg_alloc_async(ctx, s, (void**) &val, C->n * 8))) { release(); return rc; }
+			k_mj_scan_sums<<<(unsigned) nb, 256, 0, s>>>(cnt, range, sums, meta);
+			PG_LAUNCHED(ctx);
+			if ((rc = pg_scan_u64(ctx, s, sums, nb, nullptr))) { release(); return rc; }
+			k_mj_scan_apply<<<(unsigned) nb, 256, 0, s>>>(cnt, range, sums);
+			PG_LAUNCHED(ctx);
+			const int fblocks = (int) std::min<uint64_t>(pg_div_up(C->n, 256 * 4), (uint64_t) ctx->sm_count * 16);
+			k_mj_fill<<<fblocks, 256, 0, s>>>((const char*) C->data, C->n, C->key_off, kmin, range, bp, cnt, val, meta, vmm);
+			PG_LAUNCHED(ctx);
+			const int rblocks = (int) std::min<uint64_t>(pg_div_up(P->n, 128 * 8), (uint64_t) ctx->sm_count * 24);
+			k_mj_rows<<<rblocks, 256, 0, s>>>((const char*) P->data, P->n, P->key_off, kmin, range, cnt, val, wsel,
+					reinterpret_cast<uint4*>(out), out_capacity, agg, meta, vmm);
+			PG_LAUNCHED(ctx);
 		}
-		const size_t wsmem = MJW_CAP * 8 + (2 * MJ_LOCAL + 1) * 4 + (MJW_THREADS / 32) * 4;
-		PG_CUDA(ctx, cudaFuncSetAttribute(k_mj_bucket_write, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) wsmem));
-		k_mj_bucket_write<<<B, MJW_THREADS, wsmem, s>>>(reinterpret_cast<const uint4*>(bR), oR, R->key_off / 4, bp,
-				reinterpret_cast<const uint4*>(bS), oS, S->key_off / 4, kmin, brows, wsel,
-				reinterpret_cast<uint4*>(out), ctx->d_status);
-		PG_LAUNCHED(ctx);
+		unsigned long long o[3];     // rows, sum, (largest count, key outside)
+		PG_CUDA(ctx, cudaMemcpyAsync(o, agg, 24, cudaMemcpyDeviceToHost, s));
 		rc = pg_check_status(ctx, s, "pg_mpsm_join");
+		release();
+		if (rc) { pg_free_async(ctx, s, mm); return rc; }
+		if (o[2] >> 32) continue;                                         // the sample missed a key
+		if (materialize && (uint32_t) o[2] > MJ_MAX_RUN) break;
+		res->n_out = o[0];
+		res->sum = (int64_t) o[1];
+		*handled = true;
+		if (materialize && o[0] > out_capacity)
+			rc = pg_fail(ctx, PG_ERR_OUTPUT_FULL, "pg_mpsm_join: output capacity too small");
+		break;
 	}
-	release();
+	pg_free_async(ctx, s, mm);
 	return rc;
+}
+
+// Whether a side flagged as sorted is, on the device.
+static int mj_confirm_sorted(pg_ctx* ctx, cudaStream_t s, const pg_rel* r, bool* sorted)
+{
+	int rc;
+	unsigned long long* mm = nullptr;
+	if ((rc = pg_alloc_async(ctx, s, (void**) &mm, 32))) return rc;
+	const unsigned long long init[3] = {~0ull, 0ull, 0ull};
+	PG_CUDA(ctx, cudaMemcpyAsync(mm, init, sizeof init, cudaMemcpyHostToDevice, s));
+	const int blocks = (int) std::min<uint64_t>(pg_div_up(r->n, 256), (uint64_t) ctx->sm_count * 8);
+	k_mj_minmax<<<blocks, 256, 0, s>>>((const char*) r->data, r->n, r->width, r->key_off, r->key_bytes, 1, mm, mm + 2);
+	PG_LAUNCHED(ctx);
+	unsigned long long down = 0;
+	PG_CUDA(ctx, cudaMemcpyAsync(&down, mm + 2, 8, cudaMemcpyDeviceToHost, s));
+	PG_CUDA(ctx, cudaStreamSynchronize(s));
+	pg_free_async(ctx, s, mm);
+	*sorted = !down;
+	return PG_OK;
 }
 
 extern "C" int pg_mpsm_join(pg_ctx* ctx, pg_stream stream, const pg_rel* R, const pg_rel* S,
@@ -766,9 +847,10 @@ extern "C" int pg_mpsm_join(pg_ctx* ctx, pg_stream stream, const pg_rel* R, cons
 	bool r_sorted = false, s_sorted = false;   // confirmed on the device
 	if (R->n < (1ull << 32) && S->n < (1ull << 32)) {
 		bool handled = false;
-		if ((rc = mj_bucket_join(ctx, s, R, S, pc, sum_col, flags, out, out_capacity, res, &handled, &r_sorted,
-				&s_sorted))) return rc;
+		if ((rc = mj_dense_join(ctx, s, R, S, pc, sum_col, flags, out, out_capacity, res, &handled))) return rc;
 		if (handled) return PG_OK;
+		if ((flags & PG_JOIN_BUILD_SORTED) && (rc = mj_confirm_sorted(ctx, s, R, &r_sorted))) return rc;
+		if ((flags & PG_JOIN_PROBE_SORTED) && (rc = mj_confirm_sorted(ctx, s, S, &s_sorted))) return rc;
 	}
 	// A sorted 16-byte tuple keyed at offset 0 is its own sorted record array.
 	pg_rec *rr = nullptr, *sr = nullptr;
