@@ -357,6 +357,21 @@ __device__ __forceinline__ unsigned long long mj_packed(const uint4& t, const Mj
 	return v;
 }
 
+// Table loads, kept in L2 while the relations stream past.
+__device__ __forceinline__ uint32_t mj_ld32(const uint32_t* p, uint64_t pol)
+{
+	uint32_t v;
+	asm("ld.global.nc.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
+	return v;
+}
+
+__device__ __forceinline__ unsigned long long mj_ld64(const unsigned long long* p, uint64_t pol)
+{
+	unsigned long long v;
+	asm("ld.global.nc.L2::cache_hint.u64 %0, [%1], %2;" : "=l"(v) : "l"(p), "l"(pol));
+	return v;
+}
+
 // cnt[key - kmin] += 1 for every tuple; a key outside the window sets *outside.
 // Lanes that hold lane 0's key add once together when there are several of
 // them, so that one key with most of the rows does not queue 32 adds a warp.
@@ -583,7 +598,7 @@ k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin,
 	const unsigned long long vmin = vmm[0];
 	const bool narrow = vmm[1] - vmin < (1ull << 32);
 	const uint32_t lane = threadIdx.x & 31;
-	const uint64_t pol = pg_policy_evict_first();
+	const uint64_t pol = pg_policy_evict_first(), keep = pg_policy_keep(4);
 	const uint64_t nwarps = ((uint64_t) gridDim.x * blockDim.x) >> 5;
 	const uint32_t w0 = wsel & 15, w1 = (wsel >> 4) & 15, w2 = (wsel >> 8) & 15, w3 = (wsel >> 12) & 15;
 	for (uint64_t c0 = (((uint64_t) blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 128; c0 < n; c0 += nwarps * 128) {
@@ -597,8 +612,8 @@ k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin,
 			if (i < n) {
 				const uint64_t x = (uint64_t) mj_key<true>(S, i, 16, koff, 8, pol, t[j]) - (uint64_t) kmin;
 				if (x < range) {
-					m[j] = __ldg(end + x);
-					if (x) lo[j] = __ldg(end + x - 1);
+					m[j] = mj_ld32(end + x, keep);
+					if (x) lo[j] = mj_ld32(end + x - 1, keep);
 				}
 			}
 		}
@@ -629,7 +644,7 @@ k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin,
 					if (__shfl_sync(0xffffffffu, off[j], x + step) <= r) x += step;
 				const uint32_t at = __shfl_sync(0xffffffffu, lo[j], x) + (r - __shfl_sync(0xffffffffu, off[j], x));
 				unsigned long long v = 0;
-				if (r < m[j]) v = narrow ? vmin + __ldg(reinterpret_cast<const uint32_t*>(val) + at) : __ldg(val + at);
+				if (r < m[j]) v = narrow ? vmin + mj_ld32(reinterpret_cast<const uint32_t*>(val) + at, keep) : mj_ld64(val + at, keep);
 				auto pick = [&](uint32_t w) -> uint32_t {
 					return w < 4 ? __shfl_sync(0xffffffffu, mjw_word(t[j], w), x) : w == 4 ? (uint32_t) v : (uint32_t) (v >> 32);
 				};
