@@ -355,6 +355,31 @@ __device__ __forceinline__ void pg_bulk_wait_read() { asm volatile("cp.async.bul
 // Waits until every committed bulk store has completed.
 __device__ __forceinline__ void pg_bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
+// Words that blocks of one launch exchange.
+__device__ __forceinline__ unsigned long long pg_ld_relaxed(const unsigned long long* p)
+{
+	unsigned long long v;
+	asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+	return v;
+}
+
+__device__ __forceinline__ uint32_t pg_ld_relaxed(const uint32_t* p)
+{
+	uint32_t v;
+	asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+	return v;
+}
+
+__device__ __forceinline__ void pg_st_relaxed(unsigned long long* p, unsigned long long v)
+{
+	asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" :: "l"(p), "l"(v) : "memory");
+}
+
+__device__ __forceinline__ void pg_st_relaxed(uint32_t* p, uint32_t v)
+{
+	asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
+}
+
 __host__ __device__ __forceinline__ uint64_t pg_div_up(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 __host__ __device__ __forceinline__ uint64_t pg_min64(uint64_t a, uint64_t b) { return a < b ? a : b; }
 __host__ __device__ __forceinline__ uint32_t pg_min32(uint32_t a, uint32_t b) { return a < b ? a : b; }

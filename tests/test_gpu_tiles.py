@@ -1,0 +1,107 @@
+"""Edges of the tiled and counted kernels: sizes around tile boundaries, widths
+that change the copy unit, unaligned bases, key windows at their limits."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from oracle import oracle as orc
+from pythia_gb300 import datagen as dg
+from pythia_gb300 import gpu
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows(n, width, seed):
+    """n rows of `width` bytes whose first int32 is uniform in [0, 1000)."""
+    rng = np.random.default_rng(seed)
+    a = rng.integers(-(1 << 31), 1 << 31, size=(n, width // 4), dtype=np.int64).astype(np.int32)
+    a[:, 0] = rng.integers(0, 1000, size=n)
+    return a
+
+
+# Tiles hold (24 KB / width) rows rounded down to 32, at least 32; over 1024
+# bytes a thread copies each tuple.
+@pytest.mark.parametrize("width", [4, 8, 12, 16, 24, 40, 136, 1024, 1028])
+@pytest.mark.parametrize("shift", [0, 4, 8])
+def test_filter_and_project_tile_edges(ctx, width, shift):
+    L = gpu.lib()
+    tile = max(32, 24 * 1024 // width // 32 * 32)
+    for n in (1, 31, 33, tile - 1, tile, tile + 1, 5 * tile + 7):
+        rows = _rows(n, width, width * 1000 + n)
+        src, dst = ctx.alloc(rows.nbytes + 64), ctx.alloc(rows.nbytes + 64)
+        ctx._check(L.pg_h2d(ctx.h, ctx.stream, src.ptr + shift, rows.ctypes.data, rows.nbytes))
+        r = gpu.Rel(src.ptr + shift, n, width, 0, 0)
+        for limit in (0, 300, 1000):                       # none, some, every row
+            pr, npr = gpu.preds([("int", "<", 0, limit)])
+            m = ctypes.c_uint64()
+            ctx._check(L.pg_filter(ctx.h, ctx.stream, ctypes.byref(r), pr, npr, dst.ptr + shift, ctypes.byref(m)))
+            got = np.empty((m.value, width // 4), dtype=np.int32)
+            if m.value:
+                ctx._check(L.pg_d2h(ctx.h, ctx.stream, got.ctypes.data, dst.ptr + shift, got.nbytes))
+                ctx.sync()
+            assert np.array_equal(got, rows[rows[:, 0] < limit])
+        cols = [(width - 4, 4)] if width < 16 else [(width - 8, 8), (0, 4), (8, 4)]
+        c = (gpu.Col * len(cols))(*[gpu.Col(0, o, b) for o, b in cols])
+        ctx._check(L.pg_project(ctx.h, ctx.stream, ctypes.byref(r), c, len(cols), dst.ptr + shift))
+        want = np.concatenate([rows[:, o // 4:(o + b) // 4] for o, b in cols], axis=1)
+        got = np.empty_like(want)
+        ctx._check(L.pg_d2h(ctx.h, ctx.stream, got.ctypes.data, dst.ptr + shift, got.nbytes))
+        ctx.sync()
+        assert np.array_equal(got, want)
+
+
+def _mpsm(ctx, R, S, **kw):
+    proj = (("P", 8, 8), ("B", 8, 8))
+    got, n, _ = ctx.mpsm(R, S, proj=proj, **kw)
+    want, wn, _ = orc.mergejoin(R, S, proj=proj)
+    assert n == wn and np.array_equal(orc.canonical(got), orc.canonical(want))
+    for sc in (0, 1):
+        _, n2, s2 = ctx.mpsm(R, S, proj=proj, flags=gpu.JOIN_COUNT | gpu.JOIN_SUM, sum_col=sc)
+        assert (n2, s2) == orc.mergejoin(R, S, proj=proj, materialise=False, sum_col=sc)[1:]
+
+
+# Key windows at the counted join's limits (2^24 values whatever the size, 16
+# tuples' worth beyond), either side of the scan's blocks, values that do and
+# do not fit 4 bytes, and runs either side of the longest one warp writes.
+@pytest.mark.parametrize("case", ["one_key", "scan_edge", "widest", "too_wide", "wide_values", "extremes", "run_limit",
+                                  "over_run_limit"])
+def test_mpsm_counted_window(ctx, case):
+    n = 30_000
+    R, S = dg.uniform_keys(n, 4096, dg.seed_for(201)), dg.uniform_keys(n, 4096, dg.seed_for(202))
+    if case == "one_key":
+        R, S = R[:300], S[:200]
+        R[:, 0] = S[:, 0] = -7
+    elif case == "scan_edge":
+        R[0, 0], R[1, 0] = 0, 4096                          # 4097 counts: one in the second block
+        S[0, 0] = 4096
+    elif case == "widest":
+        R[0, 0], R[1, 0] = 0, (1 << 24) - 1
+    elif case == "too_wide":
+        R[0, 0], R[1, 0] = 0, 1 << 40
+        S[5, 0] = 1 << 40
+    elif case == "wide_values":
+        R[::2, 1] = -R[::2, 1]
+        R[0, 1], R[1, 1] = np.iinfo(np.int64).min, np.iinfo(np.int64).max
+    elif case == "extremes":
+        R[:, 0] += np.iinfo(np.int64).max - 5000
+        S[:, 0] += np.iinfo(np.int64).max - 5000
+        S[3, 0] = np.iinfo(np.int64).min
+    else:
+        R[: 16384 + (case == "over_run_limit"), 0] = 99
+        S = S[:500]
+        S[:3, 0] = 99
+    _mpsm(ctx, R, S)
+
+
+def test_mpsm_key_outside_the_sampled_window(ctx):
+    # Over 4M tuples the window comes from every 1024th; a matching key far from
+    # the rest and off the sample must still join.
+    n = (1 << 22) + 5
+    R, S = dg.uniform_keys(n, 1 << 20, dg.seed_for(203)), dg.uniform_keys(1000, 1 << 20, dg.seed_for(204))
+    R[1025, 0] = S[7, 0] = 3 << 20
+    _, n2, s2 = ctx.mpsm(R, S, flags=gpu.JOIN_COUNT | gpu.JOIN_SUM, sum_col=0)
+    assert (n2, s2) == orc.mergejoin(R, S, materialise=False, sum_col=0)[1:]
+    got, n3, _ = ctx.mpsm(R, S)
+    want, _, _ = orc.mergejoin(R, S)
+    assert n3 == n2 and np.array_equal(orc.canonical(got), orc.canonical(want))
