@@ -158,10 +158,9 @@ enum {
 	                                    table loads kept in L1 (dense-table probes); 0 = the built-in
 	                                    4/8 evict-last with L1 (bits 4-7 = 0xC), 256 = all bits clear */
 	PG_TUNE_PROBE_PASSES = 8,        /* dense-table probe passes: 1, 2 (half the table each), 0 by size */
-	PG_TUNE_GROUPBY_PATH = 9,        /* group-by: 0 by key range and size, 1 hashed global table, 2 partitioned,
-	                                    3 hashed global without warp combining, 4 partitioned without warp
-	                                    combining, 6 dense when the key range allows, 7 as 6 without the
-	                                    shared-memory tables of windows up to 4096 keys */
+	PG_TUNE_GROUPBY_PATH = 9,        /* group-by: 0 by key range and size, 1 to 5 hashed table, 6 dense when the
+	                                    key range allows, 7 as 6 without the shared-memory tables of windows up
+	                                    to 4096 keys */
 	PG_TUNE_PROBE_WIDE = 10,         /* probe of tuples or rows other than 16 bytes: 0 materialised rows of dense
 	                                    tables staged through shared memory where the width allows, everything
 	                                    else per-thread loads; 1 per-thread loads; 2 staged, 4 lookups per
@@ -182,7 +181,7 @@ enum {
 	                                    inputs of at most 2^18 tuples whose span needs over 32 bits), 1 radix
 	                                    whenever the span fits 63 bits, 2 bitonic tiles and merges always */
 	PG_TUNE_GROUPBY_ILP = 15,        /* rows in flight per thread of the dense group-by over a global table: 4
-	                                    or 8 (0: built-in, 4 for dec sums, 8 otherwise) */
+	                                    or 8 (0: built-in, 4) */
 	PG_TUNE_HASH_PARTITION = 16,     /* hashed tables: 2 partitions the probe side (and R, for packed values) on
 	                                    the keys' hash first, so that each partition uses a 16 MB slice of the
 	                                    table; 0 (built-in) or 1: not (measured slower on the 16M x 256M

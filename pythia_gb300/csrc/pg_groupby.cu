@@ -19,16 +19,13 @@
 // exact sum. The unit comes from the largest exponent of the column (sampled,
 // with a margin, on large inputs; a value above the bound makes the operator
 // redo the sum with the exact bound). Infinities and NaNs are summed on the
-// side and patch their groups' results. Lanes of a warp that carry the same
-// key are combined first (warp match), which cuts atomics on skewed keys;
-// with few groups each CTA aggregates into a shared-memory table and merges
-// once.
+// side and patch their groups' results. Blocks add the rows of groups they
+// meet often in shared memory first, which cuts L2 atomics on skewed keys.
 #include "pg_internal.cuh"
 #include <algorithm>
 
 #define GB_THREADS 256
 #define GB_DEC (VT == PG_VAL_DEC && AGG == PG_AGG_SUM)     // inside templates on VT, AGG
-#define GB_SMEM_SLOTS 4096
 
 // An open-addressing group table. A group's aggregate is one word of acc (a
 // count, a long sum, an int sum in its low 4 bytes) or, for a dec sum, the
@@ -57,6 +54,18 @@ __device__ __forceinline__ void fold_slot(unsigned long long* acc, uint64_t wstr
 	else if (VT == PG_VAL_LONG) atomicAdd(&acc[slot], v.i);
 	else if (VT == PG_VAL_INT) atomicAdd(reinterpret_cast<unsigned int*>(&acc[slot]), (unsigned int) v.i);
 	else pg_fx_atomic_add(&acc[slot], wstride, v.f);
+}
+
+// v added to a 64-bit word in shared memory by its 32-bit halves: a shared
+// 64-bit add is a compare-and-swap loop, a 32-bit one a single instruction, and
+// the upper half needs one only for a carry or a large value. The word is right
+// once every add is in.
+__device__ __forceinline__ void gb_shared_add64(unsigned long long* p, unsigned long long v)
+{
+	unsigned int* const q = reinterpret_cast<unsigned int*>(p);
+	const unsigned int lo = (unsigned int) v, old = atomicAdd(q, lo);
+	const unsigned int hi = (unsigned int) (v >> 32) + (old + lo < lo);
+	if (hi) atomicAdd(q + 1, hi);
 }
 
 // A dec sum's count from table words acc[slot + k * wstride].
@@ -117,191 +126,32 @@ __device__ __forceinline__ void warp_combine(uint32_t peers, GbVal& v)
 	v = t;
 }
 
-template <int VT, int AGG, bool HASKEY, bool SMEM>
+// No GROUP BY: one group. Warps fold their rows, then each block adds once.
+template <int VT, int AGG>
 __global__ void __launch_bounds__(GB_THREADS)
-k_gb_insert(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, uint32_t kbytes,
-		uint32_t voff, GbTable t, uint32_t smem_log2, PgFx fx, int* __restrict__ status)
+k_gb_single(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t voff, GbTable t, PgFx fx)
 {
-	extern __shared__ __align__(16) unsigned char sm[];
-	const uint32_t sc1 = SMEM ? (1u << smem_log2) + 1 : 0;
-	unsigned long long* skeys = reinterpret_cast<unsigned long long*>(sm);
-	unsigned long long* sacc = skeys + sc1;                 // [PG_FX_WORDS sc1]: a dec sum's words sc1 apart
-	__shared__ int s_sentinel;
-	if (SMEM) {
-		for (uint32_t i = threadIdx.x; i < sc1; i += blockDim.x) skeys[i] = (unsigned long long) PG_EMPTY_KEY;
-		for (uint32_t i = threadIdx.x; i < PG_FX_WORDS * sc1; i += blockDim.x) sacc[i] = 0;
-		if (threadIdx.x == 0) s_sentinel = 0;
-		__syncthreads();
-	}
-	bool full = false;
+	__shared__ unsigned long long sacc[PG_FX_WORDS];
+	if (threadIdx.x < PG_FX_WORDS) sacc[threadIdx.x] = 0;
+	__syncthreads();
 	uint32_t fl = 0;
 	const int fs = GB_DEC ? fx.p[0] : 0, fb = GB_DEC ? fx.p[1] : 0;
-	const int lane = threadIdx.x & 31;
+	GbVal v = {0, {0, 0, 0, 0}};
 	const uint64_t stride = (uint64_t) gridDim.x * blockDim.x;
-	const uint64_t n_round = pg_div_up(n, 32) * 32;
-	for (uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; i < n_round; i += stride) {
-		bool valid = i < n;
-		int64_t k = 0;
-		GbVal v = {0, {0, 0, 0, 0}};
-		if (valid) {
-			const char* r = in + i * W;
-			if (HASKEY) k = pg_load_key(r + koff, kbytes);
-			v = gb_load_val<VT, AGG>(r, voff, fs, fb, fl);
-		}
-		// Lanes with the same key fold together first.
-		uint32_t active = __ballot_sync(0xffffffffu, valid);
-		if (!valid) continue;
-		uint32_t peers = HASKEY ? __match_any_sync(active, (unsigned long long) k) : active;
-		warp_combine<VT, AGG>(peers, v);
-		if (lane != __ffs(peers) - 1) continue;
-		if (SMEM) {
-			uint64_t s = HASKEY ? gb_slot(skeys, smem_log2, k, &s_sentinel) : 0;
-			if (s == UINT64_MAX) { full = true; continue; }
-			fold_slot<VT, AGG>(sacc, sc1, s, v);
-		} else {
-			uint64_t s = HASKEY ? gb_slot(t.keys, t.log2cap, k, t.sentinel_used) : 0;
-			if (s == UINT64_MAX) { full = true; continue; }
-			fold_slot<VT, AGG>(t.acc, t.wstride(), s, v);
-		}
+	for (uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; i < n; i += stride) {
+		const GbVal x = gb_load_val<VT, AGG>(in + i * W, voff, fs, fb, fl);
+		if (GB_DEC) pg_fx_add4(v.f, x.f);
+		else v.i += x.i;
 	}
-	if (full) pg_set_status(status, PG_ERR_TABLE_FULL);
+	warp_combine<VT, AGG>(0xffffffffu, v);
+	if ((threadIdx.x & 31) == 0) fold_slot<VT, AGG>(sacc, 1, 0, v);
 	if (fl) atomicOr(reinterpret_cast<unsigned int*>(fx.p + 2), fl);
-	if (SMEM) {
-		// Merge this CTA's partial groups into the global table.
-		__syncthreads();
-		const uint32_t sc = 1u << smem_log2;
-		for (uint32_t i = threadIdx.x; i <= sc; i += blockDim.x) {
-			bool used = HASKEY ? ((i < sc) ? skeys[i] != (unsigned long long) PG_EMPTY_KEY : s_sentinel != 0)
-			                   : i == 0;
-			if (!used) continue;
-			int64_t k = (i < sc) ? (int64_t) skeys[i] : PG_EMPTY_KEY;
-			uint64_t s = HASKEY ? gb_slot(t.keys, t.log2cap, k, t.sentinel_used) : 0;
-			if (s == UINT64_MAX) { pg_set_status(status, PG_ERR_TABLE_FULL); continue; }
-			GbVal v = {sacc[i], {0, 0, 0, 0}};
-			if (GB_DEC) v.f = gb_table_count(sacc, sc1, i);
-			fold_slot<VT, AGG>(t.acc, t.wstride(), s, v);
-		}
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		GbVal s = {sacc[0], {0, 0, 0, 0}};
+		if (GB_DEC) s.f = gb_table_count(sacc, 1, 0);
+		fold_slot<VT, AGG>(t.acc, t.wstride(), 0, s);
 	}
-}
-
-// Global-table insert with four independent rows per thread per iteration:
-// their key loads, slot reads and accumulator atomics are issued together, so
-// the chains of dependent L2 round trips overlap instead of running one row
-// at a time.
-template <int VT, int AGG, bool MATCH, int GB_ILP>
-__global__ void __launch_bounds__(GB_THREADS)
-k_gb_insert_ilp(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, uint32_t kbytes,
-		uint32_t voff, GbTable t, PgFx fx, int* __restrict__ status)
-{
-	const uint64_t cap = 1ull << t.log2cap, mask = cap - 1;
-	const uint64_t stride = (uint64_t) gridDim.x * blockDim.x;
-	const uint64_t step = stride * GB_ILP;
-	bool full = false;
-	uint32_t fl = 0;
-	const int fs = GB_DEC ? fx.p[0] : 0, fb = GB_DEC ? fx.p[1] : 0;
-	const int lane = threadIdx.x & 31;
-	for (uint64_t base = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; base < pg_div_up(n, 32) * 32;
-			base += step) {
-		int64_t k[GB_ILP];
-		GbVal v[GB_ILP];
-		bool lead[GB_ILP];
-		#pragma unroll
-		for (int j = 0; j < GB_ILP; ++j) {
-			const uint64_t i = base + j * stride;
-			const bool valid = i < n;
-			k[j] = 0; v[j] = GbVal{0, {0, 0, 0, 0}}; lead[j] = false;
-			if (valid) {
-				const char* r = in + i * W;
-				k[j] = pg_load_key(r + koff, kbytes);
-				v[j] = gb_load_val<VT, AGG>(r, voff, fs, fb, fl);
-			}
-			if (MATCH) {
-				const uint32_t active = __ballot_sync(0xffffffffu, valid);
-				if (valid) {
-					const uint32_t peers = __match_any_sync(active, (unsigned long long) k[j]);
-					warp_combine<VT, AGG>(peers, v[j]);
-					lead[j] = lane == __ffs(peers) - 1;
-				}
-			} else {
-				lead[j] = valid;
-			}
-		}
-		uint64_t slot[GB_ILP];
-		unsigned long long cur[GB_ILP];
-		#pragma unroll
-		for (int j = 0; j < GB_ILP; ++j) {
-			if (!lead[j]) continue;
-			if (k[j] == PG_EMPTY_KEY) { slot[j] = cap; cur[j] = 0; continue; }
-			slot[j] = pg_mix64((uint64_t) k[j]) >> (64 - t.log2cap);
-			cur[j] = t.keys[slot[j]];
-		}
-		#pragma unroll
-		for (int j = 0; j < GB_ILP; ++j) {
-			if (!lead[j]) continue;
-			if (slot[j] == cap) { if (!*t.sentinel_used) atomicExch(t.sentinel_used, 1); continue; }
-			uint64_t probe = 0;
-			for (; probe < cap; ++probe) {
-				if (cur[j] == (unsigned long long) k[j]) break;
-				if (cur[j] == (unsigned long long) PG_EMPTY_KEY) {
-					const unsigned long long old = atomicCAS(&t.keys[slot[j]], (unsigned long long) PG_EMPTY_KEY,
-							(unsigned long long) k[j]);
-					if (old == (unsigned long long) PG_EMPTY_KEY || old == (unsigned long long) k[j]) break;
-					cur[j] = old;
-					continue;
-				}
-				slot[j] = (slot[j] + 1) & mask;
-				cur[j] = t.keys[slot[j]];
-			}
-			if (probe == cap) { full = true; lead[j] = false; }
-		}
-		if (GB_DEC) {
-			pg_fx4 f[GB_ILP];
-			#pragma unroll
-			for (int j = 0; j < GB_ILP; ++j) f[j] = v[j].f;
-			pg_fx_atomic_add_rows<GB_ILP>(t.acc, t.wstride(), slot, 1, lead, f, nullptr);
-		} else {
-			#pragma unroll
-			for (int j = 0; j < GB_ILP; ++j)
-				if (lead[j]) fold_slot<VT, AGG>(t.acc, 1, slot[j], v[j]);
-		}
-	}
-	if (full) pg_set_status(status, PG_ERR_TABLE_FULL);
-	if (fl) atomicOr(reinterpret_cast<unsigned int*>(fx.p + 2), fl);
-}
-
-// ---------------------------------------------------------------------------
-// High-cardinality path: rows are first radix-partitioned on the top bits of
-// the key mix (PG_FN_MIXRADIX) so that each partition holds about 1K groups;
-// then one CTA per partition aggregates it in a shared-memory table with the
-// same integer atomics, on shared instead of L2 atomics, and writes its
-// groups out. A partition whose groups overflow the shared table sends the
-// excess keys to the global table (emitted afterwards).
-// ---------------------------------------------------------------------------
-#define GBP_THREADS 512
-// Slots of a partition's shared-memory table: 4096 (64 KB, three CTAs per
-// SM), or 2048 for dec sums (key and the four words of the chained form,
-// pg_fx_chain_add: 80 KB, two CTAs per SM); a partition holds about 1K groups
-// either way.
-#define GBP_SLOTS (GB_DEC ? 2048u : 4096u)
-#define GBP_GROUPS 1024u
-
-// Slot of key k in a per-partition table: low bits of the mix (the top bits
-// are the partition number).
-template <uint32_t SLOTS>
-__device__ __forceinline__ uint32_t gbp_slot(unsigned long long* keys, int64_t k, int* sentinel)
-{
-	if (k == PG_EMPTY_KEY) { if (!*sentinel) atomicExch(sentinel, 1); return SLOTS; }
-	uint32_t s = (uint32_t) (pg_mix64((uint64_t) k) & (SLOTS - 1));
-	for (uint32_t probe = 0; probe < SLOTS; ++probe) {
-		const unsigned long long cur = keys[s];
-		if (cur == (unsigned long long) k) return s;
-		if (cur == (unsigned long long) PG_EMPTY_KEY) {
-			const unsigned long long old = atomicCAS(&keys[s], (unsigned long long) PG_EMPTY_KEY, (unsigned long long) k);
-			if (old == (unsigned long long) PG_EMPTY_KEY || old == (unsigned long long) k) return s;
-		}
-		s = (s + 1) & (SLOTS - 1);
-	}
-	return UINT32_MAX;
 }
 
 // Writes one group's row: kbytes of key (none for 0), then its aggregate:
@@ -320,95 +170,6 @@ __device__ __forceinline__ void gb_write_agg(char* o, uint32_t kbytes, int64_t k
 	if (GB_DEC) a = (unsigned long long) __double_as_longlong(pg_fx_double4(c, fx_s));
 	reinterpret_cast<uint32_t*>(o)[0] = (uint32_t) a;
 	reinterpret_cast<uint32_t*>(o)[1] = (uint32_t) (a >> 32);
-}
-
-template <int VT, int AGG, bool MATCH>
-__global__ void __launch_bounds__(GBP_THREADS)
-k_gb_part_agg(const char* __restrict__ rows, const uint64_t* __restrict__ offs, uint32_t P, uint32_t W,
-		uint32_t koff, uint32_t kbytes, uint32_t voff, GbTable t, PgFx fx, char* __restrict__ out, uint64_t out_cap,
-		unsigned long long* __restrict__ cursor, int* __restrict__ overflow, int* __restrict__ status)
-{
-	extern __shared__ __align__(16) unsigned char sm[];
-	constexpr uint32_t SW = GBP_SLOTS + 1;                                         // a dec sum's word stride
-	unsigned long long* skeys = reinterpret_cast<unsigned long long*>(sm);        // [SLOTS + 1]
-	unsigned long long* sacc = skeys + SW;                                         // [SLOTS + 1], 4 [SLOTS + 1] for dec
-	__shared__ int s_sent;
-	__shared__ uint32_t wtot[GBP_THREADS / 32];
-	__shared__ unsigned long long s_base;
-	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-	const uint32_t ow = kbytes + ((AGG == PG_AGG_SUM && VT == PG_VAL_INT) ? 4 : 8);
-	uint32_t fl = 0;
-	const int fs = GB_DEC ? fx.p[0] : 0, fb = GB_DEC ? fx.p[1] : 0;
-	for (uint32_t part = blockIdx.x; part < P; part += gridDim.x) {
-		for (uint32_t i = tid; i <= GBP_SLOTS; i += blockDim.x) {
-			skeys[i] = (unsigned long long) PG_EMPTY_KEY; sacc[i] = 0;
-			if (GB_DEC) { sacc[i + SW] = 0; sacc[i + 2 * SW] = 0; sacc[i + 3 * SW] = 0; }
-		}
-		if (tid == 0) s_sent = 0;
-		__syncthreads();
-		const uint64_t lo = offs[part], hi = offs[part + 1];
-		bool spilled = false;
-		for (uint64_t i = lo + tid; i < lo + pg_div_up(hi - lo, 32) * 32; i += blockDim.x) {
-			const bool valid = i < hi;
-			int64_t k = 0;
-			GbVal v = {0, {0, 0, 0, 0}};
-			if (valid) {
-				const char* r = rows + i * W;
-				k = pg_load_key(r + koff, kbytes);
-				v = gb_load_val<VT, AGG>(r, voff, fs, fb, fl);
-			}
-			if (MATCH) {
-				const uint32_t active = __ballot_sync(0xffffffffu, valid);
-				if (!valid) continue;
-				const uint32_t peers = __match_any_sync(active, (unsigned long long) k);
-				warp_combine<VT, AGG>(peers, v);
-				if (lane != __ffs(peers) - 1) continue;
-			} else if (!valid) {
-				continue;
-			}
-			const uint32_t s = gbp_slot<GBP_SLOTS>(skeys, k, &s_sent);
-			if (s != UINT32_MAX) {
-				if (GB_DEC) pg_fx_atomic_chain_add(&sacc[s], SW, v.f);
-				else fold_slot<VT, AGG>(sacc, SW, s, v);
-				continue;
-			}
-			// Shared table full: this key lives in the global table.
-			const uint64_t g = gb_slot(t.keys, t.log2cap, k, t.sentinel_used);
-			if (g == UINT64_MAX) { pg_set_status(status, PG_ERR_TABLE_FULL); continue; }
-			fold_slot<VT, AGG>(t.acc, t.wstride(), g, v);
-			spilled = true;
-		}
-		if (spilled) atomicExch(overflow, 1);
-		__syncthreads();
-		// Emit: count used slots per thread, scan, reserve, write.
-		uint32_t mine = 0;
-		for (uint32_t i = tid; i <= GBP_SLOTS; i += blockDim.x)
-			mine += (i < GBP_SLOTS) ? (skeys[i] != (unsigned long long) PG_EMPTY_KEY) : (s_sent != 0);
-		uint32_t x = mine;
-		#pragma unroll
-		for (int o = 1; o < 32; o <<= 1) {
-			const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-			if (lane >= o) x += y;
-		}
-		if (lane == 31) wtot[warp] = x;
-		__syncthreads();
-		uint32_t before = 0, total = 0;
-		for (int w = 0; w < GBP_THREADS / 32; ++w) { const uint32_t c = wtot[w]; before += w < warp ? c : 0; total += c; }
-		if (tid == 0) s_base = total ? atomicAdd(cursor, (unsigned long long) total) : 0;
-		__syncthreads();
-		uint64_t pos = s_base + before + x - mine;
-		for (uint32_t i = tid; i <= GBP_SLOTS; i += blockDim.x) {
-			const bool used = (i < GBP_SLOTS) ? (skeys[i] != (unsigned long long) PG_EMPTY_KEY) : (s_sent != 0);
-			if (!used) continue;
-			if (pos < out_cap)
-				gb_write_agg<VT, AGG>(out + pos * ow, kbytes, i < GBP_SLOTS ? (int64_t) skeys[i] : PG_EMPTY_KEY,
-						sacc[i], GB_DEC ? pg_fx_from_chain(reinterpret_cast<const uint64_t*>(sacc + i), SW)
-						                : pg_fx4{0, 0, 0, 0}, fs);
-			++pos;
-		}
-		__syncthreads();
-	}
-	if (fl) atomicOr(reinterpret_cast<unsigned int*>(fx.p + 2), fl);
 }
 
 template <int VT, int AGG, bool HASKEY>
@@ -447,8 +208,8 @@ __global__ void k_gb_emit(GbTable t, uint32_t kbytes, char* __restrict__ out, ui
 // Dense key domain (keys span at most a few times the group count, e.g.
 // group numbers 0..G-1 or surrogate keys): a min/max pass, then the slot of a
 // row is key - kmin. No probing and no key words: a row costs its atomics
-// (one for a typical dec value, as for the integer aggregates) and, for
-// sums, a byte store marking the group present. A dec sum's table keeps
+// (one for a typical dec value, as for the integer aggregates); a sum's first
+// add marks the group present. A dec sum's table keeps
 // each of its PG_FX_WORDS words in an array of its own (word k of slot i at
 // acc[i + k * range]), so the word every row adds into takes 8 bytes a group
 // of L2.
@@ -503,6 +264,140 @@ __device__ __forceinline__ void gb_row_kv(const char* __restrict__ in, uint64_t 
 	}
 }
 
+// ---------------------------------------------------------------------------
+// Hashed groups: a table of 4-key buckets, so that one 32-byte load finds a
+// row's group (at load 1/2 a key's home bucket overflows for one key in 20;
+// slot-by-slot probing made the 32 lanes of a warp wait for the longest of
+// their probe sequences), then one atomic. In front of it every block keeps
+// the groups it met first in a small direct-mapped table in shared memory and
+// adds their rows there: keys that many rows share, which would queue at one
+// L2 address, are met early.
+//
+// Bound by L2 (a random bucket read and an atomic a row). One row in flight a
+// thread, six blocks on an SM and about 64 blocks per SM in turn measured
+// best: 20M rows in 250,000 groups 320 us, against 530 with six blocks per SM
+// and 1010 with four rows a thread in three resident blocks. Partitioning the
+// rows first (shared-memory tables per partition) took 850 us, and 9.5 ms for
+// 64M rows in 4M groups where this takes 1.3.
+// ---------------------------------------------------------------------------
+#define GBH_CACHE_LOG2 8                    // groups kept per block: 256 (4 KB, 10 KB for dec)
+#define GBH_BLOCKS_PER_SM 64
+// Few groups: room for all of them in every block (32 KB, 40 KB for dec), and
+// fewer blocks, which each end by adding their groups to the table. 20M rows
+// in 1000 groups: 180 us, 527 with 256 places.
+#define GBH_FEW 1024u
+#define GBH_FEW_LOG2 (GB_DEC ? 10 : 11)
+#define GBH_FEW_PROBES 4
+#define GBH_FEW_BLOCKS_PER_SM 24
+
+// The bucket's keys straight from L2 (other blocks insert concurrently; an
+// empty slot seen late only costs the atomicCAS that finds it taken).
+__device__ __forceinline__ pg_u64x4 gbh_bucket(const unsigned long long* p)
+{
+	pg_u64x4 v;
+	asm volatile("ld.relaxed.gpu.global.v4.u64 {%0,%1,%2,%3}, [%4];" : "=l"(v.a), "=l"(v.b), "=l"(v.c), "=l"(v.d) : "l"(p) : "memory");
+	return v;
+}
+
+// Slot of key k (not the empty marker), whose home bucket b0 was read as v:
+// found or claimed there, else in the buckets after it. UINT64_MAX when every
+// bucket is full.
+__device__ __forceinline__ uint64_t gbh_slot(unsigned long long* keys, uint32_t log2cap, unsigned long long k, uint64_t b,
+		pg_u64x4 v)
+{
+	const uint64_t nb = 1ull << (log2cap - 2);
+	for (uint64_t probe = 0; probe < nb; ++probe) {
+		if (v.a == k) return 4 * b;
+		if (v.b == k) return 4 * b + 1;
+		if (v.c == k) return 4 * b + 2;
+		if (v.d == k) return 4 * b + 3;
+		// Slots fill in order: claim the first empty one, or find there the
+		// key that took it meanwhile.
+		const unsigned long long empty = (unsigned long long) PG_EMPTY_KEY;
+		#pragma unroll
+		for (int i = 0; i < 4; ++i) {
+			const unsigned long long cur = i == 0 ? v.a : i == 1 ? v.b : i == 2 ? v.c : v.d;
+			if (cur != empty) continue;
+			const unsigned long long old = atomicCAS(&keys[4 * b + i], empty, k);
+			if (old == empty || old == k) return 4 * b + i;
+		}
+		b = (b + 1) & (nb - 1);
+		v = gbh_bucket(keys + 4 * b);
+	}
+	return UINT64_MAX;
+}
+
+template <int VT, int AGG, bool VEC16>
+__global__ void __launch_bounds__(GB_THREADS, 6)
+k_gb_hash(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, uint32_t kbytes, uint32_t voff,
+		GbTable t, uint32_t places, uint32_t probes, PgFx fx, int* __restrict__ status)
+{
+	extern __shared__ __align__(16) unsigned char gbh_sm[];
+	unsigned long long* const skeys = reinterpret_cast<unsigned long long*>(gbh_sm);   // [places], a power of two
+	unsigned long long* const sacc = skeys + places;                                  // [places], for dec 4 words places apart
+	for (uint32_t i = threadIdx.x; i < places; i += blockDim.x) skeys[i] = (unsigned long long) PG_EMPTY_KEY;
+	for (uint32_t i = threadIdx.x; i < (GB_DEC ? 4 : 1) * places; i += blockDim.x) sacc[i] = 0;
+	__syncthreads();
+	const uint64_t stride = (uint64_t) gridDim.x * blockDim.x;
+	bool full = false;
+	uint32_t fl = 0;
+	const int fs = GB_DEC ? fx.p[0] : 0, fb = GB_DEC ? fx.p[1] : 0;
+	for (uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; i < n; i += stride) {
+		int64_t k;
+		uint64_t vbits = 0;
+		if (AGG == PG_AGG_COUNT && !VEC16) k = pg_load_key(in + i * W + koff, kbytes);
+		else gb_row_kv<VT, VEC16>(in, i, W, koff, kbytes, voff, k, vbits);
+		GbVal v = {AGG == PG_AGG_COUNT ? 1 : vbits, {0, 0, 0, 0}};
+		pg_fx3 f = {0, 0, 0};
+		if (GB_DEC) f = pg_fx_take(vbits, fs, fb, fl);
+		if (k == PG_EMPTY_KEY) {
+			if (!*t.sentinel_used) atomicExch(t.sentinel_used, 1);
+			v.f = pg_fx_widen(f);
+			fold_slot<VT, AGG>(t.acc, t.wstride(), 1ull << t.log2cap, v);
+			continue;
+		}
+		const uint64_t h = pg_mix64((uint64_t) k);
+		uint32_t c = (uint32_t) h & (places - 1);
+		bool here = false;
+		for (uint32_t p = 0; p < probes; ++p, c = (c + 1) & (places - 1)) {
+			unsigned long long cur = *(volatile unsigned long long*) &skeys[c];
+			if (cur == (unsigned long long) PG_EMPTY_KEY) {
+				cur = atomicCAS(&skeys[c], (unsigned long long) PG_EMPTY_KEY, (unsigned long long) k);
+				if (cur == (unsigned long long) PG_EMPTY_KEY) cur = (unsigned long long) k;
+			}
+			if (cur == (unsigned long long) k) { here = true; break; }
+		}
+		if (here) {
+			if (GB_DEC) pg_fx_atomic_chain_add(&sacc[c], places, pg_fx_widen(f));
+			else if (VT == PG_VAL_INT && AGG == PG_AGG_SUM) fold_slot<VT, AGG>(sacc, places, c, v);
+			else gb_shared_add64(&sacc[c], v.i);
+			continue;
+		}
+		const uint64_t b = h >> (66 - t.log2cap);
+		const uint64_t slot = gbh_slot(t.keys, t.log2cap, (unsigned long long) k, b, gbh_bucket(t.keys + 4 * b));
+		if (slot == UINT64_MAX) { full = true; continue; }
+		if (GB_DEC) {
+			const uint64_t at[1] = {slot};
+			const bool ok[1] = {true};
+			const pg_fx3 x[1] = {f};
+			pg_fx_atomic_add_rows<1>(t.acc, t.wstride(), at, 1, ok, x, nullptr);
+		} else fold_slot<VT, AGG>(t.acc, t.wstride(), slot, v);
+	}
+	__syncthreads();
+	for (uint32_t i = threadIdx.x; i < places; i += blockDim.x) {
+		const unsigned long long k = skeys[i];
+		if (k == (unsigned long long) PG_EMPTY_KEY) continue;
+		const uint64_t b = pg_mix64(k) >> (66 - t.log2cap);
+		const uint64_t slot = gbh_slot(t.keys, t.log2cap, k, b, gbh_bucket(t.keys + 4 * b));
+		if (slot == UINT64_MAX) { full = true; continue; }
+		GbVal v = {sacc[i], {0, 0, 0, 0}};
+		if (GB_DEC) v.f = pg_fx_from_chain(reinterpret_cast<const uint64_t*>(sacc + i), places);
+		fold_slot<VT, AGG>(t.acc, t.wstride(), slot, v);
+	}
+	if (full) pg_set_status(status, PG_ERR_TABLE_FULL);
+	if (fl) atomicOr(reinterpret_cast<unsigned int*>(fx.p + 2), fl);
+}
+
 #define GBD_ILP 4
 // ILP rows per thread in flight (their loads and atomics issued together).
 template <int VT, int AGG, bool VEC16, int ILP>
@@ -538,13 +433,23 @@ k_gb_dense(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, u
 		if (GB_DEC) {
 			pg_fx_atomic_add_rows<ILP>(acc, range, d, 1, ok, f, present);
 		} else {
+			// A sum's first add returns the initial 0 and marks its group: a
+			// byte store a row beside an add that returns nothing took longer
+			// (3.10 against 2.50 ms for 256M rows in 1M groups).
+			unsigned long long old[ILP];
 			#pragma unroll
 			for (int j = 0; j < ILP; ++j) {
+				old[j] = 1;
 				if (!ok[j]) continue;
-				if (VT == PG_VAL_INT && AGG == PG_AGG_SUM)
-					atomicAdd(reinterpret_cast<unsigned int*>(&acc[d[j]]), (unsigned int) iv[j]);
-				else atomicAdd(&acc[d[j]], iv[j]);
-				if (AGG == PG_AGG_SUM) present[d[j]] = 1;
+				if (AGG == PG_AGG_COUNT) atomicAdd(&acc[d[j]], iv[j]);
+				else if (VT == PG_VAL_INT)
+					old[j] = atomicAdd(reinterpret_cast<unsigned int*>(&acc[d[j]]), (unsigned int) iv[j]);
+				else old[j] = atomicAdd(&acc[d[j]], iv[j]);
+			}
+			if (AGG == PG_AGG_SUM) {
+				#pragma unroll
+				for (int j = 0; j < ILP; ++j)
+					if (old[j] == 0) present[d[j]] = 1;
 			}
 		}
 	}
@@ -603,7 +508,7 @@ k_gb_dense_smem(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t ko
 			if (GB_DEC) pg_fx_atomic_add(&sacc[d[j]], range, pg_fx_widen(f[j]));
 			else if (VT == PG_VAL_INT && AGG == PG_AGG_SUM)
 				atomicAdd(reinterpret_cast<unsigned int*>(&sacc[d[j]]), (unsigned int) iv[j]);
-			else atomicAdd(&sacc[d[j]], iv[j]);
+			else gb_shared_add64(&sacc[d[j]], iv[j]);
 			if (AGG == PG_AGG_SUM) spres[d[j]] = 1;
 		}
 	}
@@ -786,6 +691,15 @@ int pg_fx_patch_specials(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint32_t
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
+// Rows that gb_row_kv reads with one 16-byte load.
+template <int VT, int AGG>
+static bool gb_vec16(const pg_rel* in, uint32_t voff)
+{
+	return in->width == 16 && (in->key_off == 0 || in->key_off == 8) && in->key_bytes == 8 &&
+		(reinterpret_cast<uintptr_t>(in->data) & 15) == 0 &&
+		(AGG == PG_AGG_COUNT || (VT == PG_VAL_INT ? (voff & 3) == 0 : (voff == 0 || voff == 8)));
+}
+
 // One dense aggregation over the key window [kmin, kmin + range): table, fill,
 // aggregation, emission. *overflow: some key lay outside the window (nothing
 // of this run is usable then); *fxfl: the dec sum's flags (fx).
@@ -822,13 +736,13 @@ static int gb_dense_window(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint32
 				in->width, in->key_off, in->key_bytes, voff, kmin, (uint32_t) range, acc, fx, present, oflag);
 		PG_LAUNCHED(ctx);
 	} else {
-		// Rows in flight per thread: eight for counts and integer sums, four for
-		// dec sums, whose kernel holds more registers a row (85 at eight rows:
-		// 3.60 against 2.74 ms at four for 256M rows in 1M groups).
+		// Four rows in flight a thread and many blocks in turn: 256M rows in 1M
+		// groups 2.52 ms (dec) and 2.44 (long), against 2.64 and 2.55 with eight
+		// blocks per SM; eight rows hold too many registers for dec sums.
 		const int64_t knob = ctx->tune[PG_TUNE_GROUPBY_ILP];
-		const int ilp = knob == 4 ? GBD_ILP : knob == 8 ? 8 : GB_DEC ? GBD_ILP : 8;
+		const int ilp = knob == 8 ? 8 : GBD_ILP;
 		const int gblocks = (int) std::min<uint64_t>(pg_div_up(in->n, (uint64_t) GB_THREADS * ilp),
-				(uint64_t) ctx->sm_count * 8);
+				(uint64_t) ctx->sm_count * 128);
 #define GBD_LAUNCH(V, I) k_gb_dense<VT, AGG, V, I><<<gblocks, GB_THREADS, 0, s>>>((const char*) in->data, in->n, \
 				in->width, in->key_off, in->key_bytes, voff, kmin, range, acc, fx, present, oflag)
 		if (vec16 && ilp == 8) GBD_LAUNCH(true, 8);
@@ -886,9 +800,7 @@ static int gb_dense(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint32_t voff
 {
 	*done = false;
 	int rc;
-	const bool vec16 = in->width == 16 && (in->key_off == 0 || in->key_off == 8) && in->key_bytes == 8 &&
-		(reinterpret_cast<uintptr_t>(in->data) & 15) == 0 &&
-		(AGG == PG_AGG_COUNT || (VT == PG_VAL_INT ? (voff & 3) == 0 : (voff == 0 || voff == 8)));
+	const bool vec16 = gb_vec16<VT, AGG>(in, voff);
 	const uint64_t limit = std::max<uint64_t>(4 * std::max<uint64_t>(hint, 1), std::min<uint64_t>(2 * in->n, 1ull << 22));
 	unsigned long long h[2];
 	if (in->n >= (1ull << 22)) {
@@ -908,6 +820,8 @@ static int gb_dense(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint32_t voff
 				return pg_check_status(ctx, s, "pg_groupby");
 			}
 		}
+		// The sampled keys alone span too much: so do all.
+		if (span >= limit || span >= (1ull << 28)) return PG_OK;
 	}
 	if ((rc = gb_key_range(ctx, s, in, vec16, 1, h))) return rc;
 	const long long kmin = (long long) (h[0] ^ (1ull << 63)), kmax = (long long) (h[1] ^ (1ull << 63));
@@ -941,94 +855,32 @@ static int gb_run(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint32_t voff, 
 		t.log2cap = lg;
 		char* mem = nullptr;
 		int rc;
-		size_t bytes = (cap + 1) * 8 * (1 + PG_FX_WORDS) + 64;
+		const uint64_t aw = GB_DEC ? PG_FX_WORDS : 1;                  // accumulator words a slot
+		size_t bytes = (cap + 4) * 8 + (cap + 1) * 8 * aw + 64;
 		if ((rc = pg_alloc_async(ctx, s, (void**) &mem, bytes))) return rc;
 		t.keys = reinterpret_cast<unsigned long long*>(mem);
-		t.acc = t.keys + cap + 1;
-		t.sentinel_used = reinterpret_cast<int*>(t.acc + PG_FX_WORDS * (cap + 1));
+		t.acc = t.keys + cap + 4;
+		t.sentinel_used = reinterpret_cast<int*>(t.acc + aw * (cap + 1));
 		unsigned long long* cursor = reinterpret_cast<unsigned long long*>(t.sentinel_used + 2);
 		PG_CUDA(ctx, cudaMemsetAsync(t.keys, 0xFF, (cap + 1) * 8, s));
-		PG_CUDA(ctx, cudaMemsetAsync(t.acc, 0, (cap + 1) * 8 * PG_FX_WORDS + 64, s));
-		const bool smem = groups <= GB_SMEM_SLOTS / (GB_DEC ? 8 : 2);       // tables up to 66 KB
-		// Path knob: 0 by size, 1 global table (warp-combined), 2 partitioned,
-		// 3 global table without the warp combine.
-		const int64_t path = ctx->tune[PG_TUNE_GROUPBY_PATH];
-		const bool part_ok = haskey && !smem && in->n < (1ull << 32) && in->width <= 1024;
+		PG_CUDA(ctx, cudaMemsetAsync(t.acc, 0, (cap + 1) * 8 * aw + 64, s));
 		unsigned int f = 0;
-		if (part_ok && (path == 2 || path == 4 || (path == 0 && in->n >= 4 * groups))) {
-			// High cardinality: partition by key hash, aggregate per partition.
-			uint32_t lp = 1;
-			while ((1ull << lp) < groups / GBP_GROUPS && lp < 12) ++lp;
-			const uint32_t P = 1u << lp;
-			char* prow = nullptr;
-			uint64_t* poffs = nullptr;
-			int* oflag = reinterpret_cast<int*>(cursor + 1);
-			if ((rc = pg_alloc_async(ctx, s, (void**) &prow, in->n * in->width))) return rc;
-			if ((rc = pg_alloc_async(ctx, s, (void**) &poffs, (P + 1) * 8))) return rc;
-			pg_hashfn fn;
-			fn.fn = PG_FN_MIXRADIX; fn.k = 0; fn.min = 0; fn.max = 0; fn.bucketrange = 0;
-			fn.skipbits = 64 - lp; fn.nbuckets = P;
-			if ((rc = pg_partition_fn(ctx, s, in, fn, prow, poffs))) return rc;
-			const size_t psm = (size_t) (GBP_SLOTS + 1) * (GB_DEC ? 40 : 16);
-			const int pblocks = (int) std::min<uint64_t>(P, (uint64_t) ctx->sm_count * (GB_DEC ? 2 : 3));   // CTAs per SM
-			if (path == 4) {
-				PG_CUDA(ctx, cudaFuncSetAttribute(k_gb_part_agg<VT, AGG, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) psm));
-				k_gb_part_agg<VT, AGG, false><<<pblocks, GBP_THREADS, psm, s>>>(prow, poffs, P, in->width, in->key_off,
-						in->key_bytes, voff, t, fx, (char*) out, out_cap, cursor, oflag, ctx->d_status);
-			} else {
-				PG_CUDA(ctx, cudaFuncSetAttribute(k_gb_part_agg<VT, AGG, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) psm));
-				k_gb_part_agg<VT, AGG, true><<<pblocks, GBP_THREADS, psm, s>>>(prow, poffs, P, in->width, in->key_off,
-						in->key_bytes, voff, t, fx, (char*) out, out_cap, cursor, oflag, ctx->d_status);
-			}
+		if (in->n && haskey) {
+			const bool few = groups <= GBH_FEW;
+			const uint32_t places = 1u << (few ? GBH_FEW_LOG2 : GBH_CACHE_LOG2), probes = few ? GBH_FEW_PROBES : 1;
+			const size_t smem = (size_t) places * (GB_DEC ? 40 : 16);
+			const int blocks = (int) std::min<uint64_t>(pg_div_up(in->n, GB_THREADS),
+					(uint64_t) ctx->sm_count * (few ? GBH_FEW_BLOCKS_PER_SM : GBH_BLOCKS_PER_SM));
+			if (gb_vec16<VT, AGG>(in, voff))
+				k_gb_hash<VT, AGG, true><<<blocks, GB_THREADS, smem, s>>>((const char*) in->data, in->n, in->width, in->key_off,
+						in->key_bytes, voff, t, places, probes, fx, ctx->d_status);
+			else
+				k_gb_hash<VT, AGG, false><<<blocks, GB_THREADS, smem, s>>>((const char*) in->data, in->n, in->width, in->key_off,
+						in->key_bytes, voff, t, places, probes, fx, ctx->d_status);
 			PG_LAUNCHED(ctx);
-			int hflag = 0;
-			PG_CUDA(ctx, cudaMemcpyAsync(&hflag, oflag, 4, cudaMemcpyDeviceToHost, s));
-			rc = pg_check_status(ctx, s, "pg_groupby");
-			pg_free_async(ctx, s, prow);
-			pg_free_async(ctx, s, poffs);
-			if (rc == PG_ERR_TABLE_FULL) { pg_free_async(ctx, s, mem); groups *= 4; continue; }
-			if (rc) { pg_free_async(ctx, s, mem); return rc; }
-			if (hflag) {   // groups that overflowed a partition's table
-				int eblocks = (int) std::min<uint64_t>(pg_div_up(cap + 1, 256), (uint64_t) ctx->sm_count * 8);
-				k_gb_emit<VT, AGG, true><<<eblocks, 256, 0, s>>>(t, in->key_bytes, (char*) out, out_cap, cursor, 0, fx);
-				PG_LAUNCHED(ctx);
-			}
-			unsigned long long ng = 0;
-			PG_CUDA(ctx, cudaMemcpyAsync(&ng, cursor, 8, cudaMemcpyDeviceToHost, s));
-			if (GB_DEC) PG_CUDA(ctx, cudaMemcpyAsync(&f, fx.p + 2, 4, cudaMemcpyDeviceToHost, s));
-			PG_CUDA(ctx, cudaStreamSynchronize(s));
-			pg_free_async(ctx, s, mem);
-			*ngroups = ng;
-			*fxfl |= f;
-			if (ng > out_cap) return pg_fail(ctx, PG_ERR_OUTPUT_FULL, "pg_groupby: output capacity too small");
-			return PG_OK;
-		}
-		uint32_t slg = 1;
-		while ((1u << slg) < 2 * groups) ++slg;
-		if (!haskey) slg = 0;
-		const size_t smem_bytes = smem ? ((size_t) (1u << slg) + 1) * 8 * (1 + PG_FX_WORDS) : 0;
-		int blocks = (int) std::min<uint64_t>(pg_div_up(std::max<uint64_t>(in->n, 1), GB_THREADS),
-				(uint64_t) ctx->sm_count * (smem ? 4 : 8));
-		if (in->n) {
-			#define GB_LAUNCH(HK, SM) cudaFuncSetAttribute(k_gb_insert<VT, AGG, HK, SM>, \
-					cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem_bytes); \
-					k_gb_insert<VT, AGG, HK, SM><<<blocks, GB_THREADS, smem_bytes, s>>>( \
-					(const char*) in->data, in->n, in->width, in->key_off, in->key_bytes, voff, t, slg, fx, ctx->d_status)
-			if (haskey && smem) { GB_LAUNCH(true, true); }
-			else if (haskey && (path == 3 || path == 5)) {
-				if (path == 5)
-					k_gb_insert_ilp<VT, AGG, false, 8><<<blocks, GB_THREADS, 0, s>>>((const char*) in->data, in->n,
-							in->width, in->key_off, in->key_bytes, voff, t, fx, ctx->d_status);
-				else
-					k_gb_insert_ilp<VT, AGG, false, 4><<<blocks, GB_THREADS, 0, s>>>((const char*) in->data, in->n,
-							in->width, in->key_off, in->key_bytes, voff, t, fx, ctx->d_status);
-			}
-			else if (haskey) {
-				k_gb_insert_ilp<VT, AGG, true, 4><<<blocks, GB_THREADS, 0, s>>>((const char*) in->data, in->n,
-						in->width, in->key_off, in->key_bytes, voff, t, fx, ctx->d_status);
-			}
-			else { GB_LAUNCH(false, true); }
-			#undef GB_LAUNCH
+		} else if (in->n) {
+			const int blocks = (int) std::min<uint64_t>(pg_div_up(in->n, GB_THREADS), (uint64_t) ctx->sm_count * 4);
+			k_gb_single<VT, AGG><<<blocks, GB_THREADS, 0, s>>>((const char*) in->data, in->n, in->width, voff, t, fx);
 			PG_LAUNCHED(ctx);
 		}
 		rc = pg_check_status(ctx, s, "pg_groupby");
