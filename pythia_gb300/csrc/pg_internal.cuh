@@ -75,6 +75,16 @@ int pg_partition_fn(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, const pg_hash
 // the 64-bit key mix, skipbits = 64 - log2(buckets). Spreads any key domain
 // evenly, for partitions that feed per-partition tables.
 #define PG_FN_MIXRADIX 64
+// Another: the digit of key - min (mod 2^64) that starts at bit skipbits, k its
+// mask (at most 8 bits).
+#define PG_FN_DIGIT 65
+
+// Pass `pass` of a stable LSD radix sort of 16-byte tuples on key - base (mod
+// 2^64), 8 bits a pass (pg_partition.cu). With `refuted`, the pass first
+// confirms that every key lies in [base, base + 2^window) (one readback);
+// *refuted and nothing written when one does not.
+bool pg_radix_pass_takes(const pg_rel* in, const void* out);
+int pg_radix_pass(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, int64_t base, int pass, int window, bool* refuted, void* out);
 
 __device__ __forceinline__ uint64_t pg_mix64(uint64_t k);
 
@@ -88,30 +98,23 @@ __device__ __forceinline__ int64_t pg_load_key(const char* p, uint32_t bytes)
 	return (int64_t) (((uint64_t) q[1] << 32) | q[0]);
 }
 
-// Bucket of one field value; mirrors the reference's arithmetic exactly,
-// including its unsigned-int truncations.
-__device__ __forceinline__ uint32_t pg_hash_field(const pg_hashfn& f, const char* p, uint32_t size)
+// Bucket of an int, long or date field of `size` bytes (4 or 8) whose value,
+// widened, is v; mirrors the reference's arithmetic exactly, including its
+// unsigned-int truncations.
+__device__ __forceinline__ uint32_t pg_hash_value(const pg_hashfn& f, int64_t v, uint32_t size)
 {
 	switch (f.fn) {
 	case PG_FN_BYTES: {
 		uint64_t h = 14695981039346656037ull;
 		for (uint32_t i = 0; i < size; ++i) {
-			h ^= (uint64_t) (int64_t) (signed char) p[i];
+			h ^= (uint64_t) (int64_t) (signed char) (v >> (8 * i));
 			h += (h << 1) + (h << 4) + (h << 5) + (h << 7) + (h << 8) + (h << 40);
 		}
 		return (uint32_t) (((h >> f.k) ^ h) & ((1ull << f.k) - 1));
 	}
-	case PG_FN_MIXRADIX:
-		return (uint32_t) (pg_mix64((uint64_t) pg_load_key(p, size)) >> f.skipbits);
-	case PG_FN_TPCHQ1MAGIC: {
-		uint32_t v = *reinterpret_cast<const uint32_t*>(p);
-		return (((v >> 4) | (v >> 16)) & 0x1u) | ((v >> 1) & 0x2u);
-	}
+	case PG_FN_MIXRADIX: return (uint32_t) (pg_mix64((uint64_t) v) >> f.skipbits);
+	case PG_FN_TPCHQ1MAGIC: return ((((uint32_t) v >> 4) | ((uint32_t) v >> 16)) & 0x1u) | (((uint32_t) v >> 1) & 0x2u);
 	case PG_FN_ALWAYSZERO: return 0;
-	default: break;
-	}
-	int64_t v = pg_load_key(p, size);
-	switch (f.fn) {
 	case PG_FN_MODULO: return (uint32_t) (v & f.k);
 	case PG_FN_RANGE: {
 		int64_t val = (int64_t) ((uint64_t) (v - f.min) << f.k);
@@ -137,6 +140,22 @@ __device__ __forceinline__ uint32_t pg_hash_field(const pg_hashfn& f, const char
 	}
 	default: return 0;
 	}
+}
+
+// Bucket of one field at p; a char column (any size) hashes its bytes.
+__device__ __forceinline__ uint32_t pg_hash_field(const pg_hashfn& f, const char* p, uint32_t size)
+{
+	if (f.fn == PG_FN_BYTES) {
+		uint64_t h = 14695981039346656037ull;
+		for (uint32_t i = 0; i < size; ++i) {
+			h ^= (uint64_t) (int64_t) (signed char) p[i];
+			h += (h << 1) + (h << 4) + (h << 5) + (h << 7) + (h << 8) + (h << 40);
+		}
+		return (uint32_t) (((h >> f.k) ^ h) & ((1ull << f.k) - 1));
+	}
+	if (f.fn == PG_FN_ALWAYSZERO) return 0;
+	if (f.fn == PG_FN_TPCHQ1MAGIC) return pg_hash_value(f, *reinterpret_cast<const int32_t*>(p), 4);
+	return pg_hash_value(f, pg_load_key(p, size), size);
 }
 
 // 64-bit finaliser of MurmurHash3 (Appleby): slot placement for the

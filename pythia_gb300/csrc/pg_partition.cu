@@ -18,6 +18,7 @@
 // (write-combining through shared memory).
 #include "pg_internal.cuh"
 #include <algorithm>
+#include <type_traits>
 
 #define PART_MAX_BUCKETS 4096
 #define PART_TILE_BYTES (20 * 1024)     // measured best: 4 CTAs per SM
@@ -282,6 +283,328 @@ static size_t part_smem_bytes(uint32_t tile, uint32_t W, uint32_t B, int NW)
 	return s;
 }
 
+// ---------------------------------------------------------------------------
+// 16-byte tuples and at most 256 buckets. k_chunk_hist counts every block's
+// chunk of the input per bucket (at the copy rate); a block of k_part_sweep
+// adds up the chunks before its own and goes through its chunk in tiles:
+//
+// - the next tile arrives by a bulk copy while this one is worked on;
+// - every warp takes its rows of the tile 32 at a time: lanes of the same bucket
+//   are found with one ballot a bucket bit, and a counter per warp and bucket
+//   gives each row its rank;
+// - a thread a bucket turns the warps' counts into each warp's first slot of the
+//   bucket in the grouped tile and the bucket's first output row;
+// - the rows, still in registers, go to their slots, over the tile itself;
+// - a thread a bucket stores the bucket's rows of the tile with one bulk copy.
+//
+// Every row keeps its order within its bucket. 100M tuples in 256 buckets:
+// counting 230 us (the copy rate), partitioning 660 us, against 909 us with
+// 20 KB tiles, a slot -> row permutation and a store a row; two thirds of that
+// is the scattered stores (the same rows stored in tile order: 560 us). Tiles of
+// 3072 rows, two blocks on an SM: smaller ones cost more in barriers (256 x 8 in
+// three blocks 780 us), more threads in registers (512 x 6 670 us, 1024 x 3
+// 1030 us). One-sweep forms with a look-back instead of the counting pass took
+// as long a pass or longer (DRAM rows are no better used and every tile waits).
+// ---------------------------------------------------------------------------
+#define SW_BUCKETS 256
+#define PG_FN_DIGIT32 66              // PG_FN_DIGIT within the key's low 32 bits
+#define SW_CHECKED(FN) ((FN) != PG_FN_DIGIT && (FN) != PG_FN_DIGIT32)   // the bucket may be out of range
+#define SW_THREADS 384
+#define SW_ITEMS 8
+#define SW_BLOCKS_PER_SM 2
+#define SW_WARPS (SW_THREADS / 32)
+#define SW_TILE (SW_THREADS * SW_ITEMS)
+#define SW_HIST_SPLIT 2             // blocks of k_chunk_hist per chunk
+
+// Key of a tuple (4 or 8 bytes at word kw), widened. K0: 8 bytes at word 0.
+template <bool K0>
+__device__ __forceinline__ int64_t sw_key(const uint4& t, uint32_t kw, uint32_t kbytes)
+{
+	if (K0) return (int64_t) (((uint64_t) t.y << 32) | t.x);
+	const uint32_t lo = kw == 0 ? t.x : kw == 1 ? t.y : kw == 2 ? t.z : t.w;
+	const uint32_t hi = kw == 0 ? t.y : kw == 1 ? t.z : t.w;
+	return kbytes == 4 ? (int64_t) (int32_t) lo : (int64_t) (((uint64_t) hi << 32) | lo);
+}
+
+// Bucket of a key. PG_FN_DIGIT is taken from 32-bit words: only its low bits
+// after the shift are kept.
+template <int FN>
+__device__ __forceinline__ uint32_t sw_bucket(const pg_hashfn& f, int64_t v, uint32_t kbytes)
+{
+	// All of the digit in the low word: the borrow does not matter.
+	if (FN == PG_FN_DIGIT32) return (((uint32_t) v - (uint32_t) f.min) >> f.skipbits) & (uint32_t) f.k;
+	if (FN == PG_FN_DIGIT) {
+		const uint64_t x = (uint64_t) v - (uint64_t) f.min;
+		const bool upper = f.skipbits >= 32;
+		return __funnelshift_r(upper ? (uint32_t) (x >> 32) : (uint32_t) x, upper ? 0u : (uint32_t) (x >> 32),
+				f.skipbits & 31) & (uint32_t) f.k;
+	}
+	if (FN == PG_FN_MIXRADIX) return (uint32_t) (pg_mix64((uint64_t) v) >> f.skipbits);
+	return pg_hash_value(f, v, kbytes);
+}
+
+// Lanes of the warp whose 8-bit value equals b, among `valid`: a ballot a bit.
+__device__ __forceinline__ uint32_t sw_peers(uint32_t b, uint32_t valid)
+{
+	uint32_t peers = valid;
+	#pragma unroll
+	for (int k = 0; k < 8; ++k) {
+		const bool on = (b >> k) & 1u;
+		const uint32_t m = __ballot_sync(0xffffffffu, on);
+		peers &= on ? m : ~m;
+	}
+	return peers;
+}
+
+// counts[c][b]: rows of bucket b in chunk c (chunk_rows rows each). With
+// `outside`, a key outside [f.min, f.min + 2^window) sets it.
+template <int FN, bool K0>
+__global__ void __launch_bounds__(512)
+k_chunk_hist(const uint4* __restrict__ in, uint32_t n, uint32_t kw, uint32_t kbytes, pg_hashfn f, uint32_t chunk_rows,
+		uint32_t* __restrict__ counts, uint32_t window, int* __restrict__ outside, int* __restrict__ status)
+{
+	__shared__ uint32_t h[SW_BUCKETS];
+	if (threadIdx.x < SW_BUCKETS) h[threadIdx.x] = 0;
+	__syncthreads();
+	const uint32_t lo = blockIdx.x * chunk_rows, hi = (uint32_t) pg_min64(n, (uint64_t) lo + chunk_rows);
+	bool bad = false, out = false;
+	for (uint64_t i0 = (uint64_t) lo + blockIdx.y * 512 + threadIdx.x; i0 < hi; i0 += 4 * SW_HIST_SPLIT * 512) {
+		uint4 t[4];
+		#pragma unroll
+		for (int j = 0; j < 4; ++j) {
+			const uint64_t i = i0 + j * (SW_HIST_SPLIT * 512);
+			t[j] = i < hi ? pg_ld_stream16(in + i) : make_uint4(0, 0, 0, 0);
+		}
+		#pragma unroll
+		for (int j = 0; j < 4; ++j) {
+			if (i0 + j * (SW_HIST_SPLIT * 512) >= hi) continue;
+			const int64_t key = sw_key<K0>(t[j], kw, kbytes);
+			const uint32_t b = sw_bucket<FN>(f, key, kbytes);
+			if (b < f.nbuckets) atomicAdd(&h[b], 1u); else bad = true;
+			if (outside && window < 64 && ((uint64_t) key - (uint64_t) f.min) >> window) out = true;
+		}
+	}
+	if (bad) pg_set_status(status, PG_ERR_ARG);
+	if (out) *outside = 1;
+	__syncthreads();
+	if (threadIdx.x < SW_BUCKETS && h[threadIdx.x]) atomicAdd(&counts[blockIdx.x * SW_BUCKETS + threadIdx.x], h[threadIdx.x]);
+}
+
+// Exclusive scan of x over threads 0..255 (the others must not call it). wt: 8
+// words of shared memory.
+__device__ __forceinline__ uint32_t sw_scan256(uint32_t x, uint32_t* wt)
+{
+	const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	uint32_t inc = x;
+	#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+		if (lane >= (uint32_t) o) inc += y;
+	}
+	if (lane == 31) wt[warp] = inc;
+	asm volatile("bar.sync 1, 256;" ::: "memory");
+	uint32_t before = 0;
+	#pragma unroll
+	for (int w = 0; w < 8; ++w) before += (uint32_t) w < warp ? wt[w] : 0;
+	return before + inc - x;                // the caller's next block barrier frees wt
+}
+
+struct SwShared {
+	uint4 tile[2][SW_TILE];
+	uint16_t slot[SW_WARPS][SW_BUCKETS];    // a warp's count of a bucket, then its first slot
+	uint32_t wt[8];
+	uint64_t bar[2];
+};
+
+template <int FN, bool K0>
+__global__ void __launch_bounds__(SW_THREADS, SW_BLOCKS_PER_SM)
+k_part_sweep(const uint4* __restrict__ in, uint32_t n, uint32_t kw, uint32_t kbytes, pg_hashfn f, uint32_t chunk_tiles,
+		const uint32_t* __restrict__ counts, uint64_t* __restrict__ offsets, uint4* __restrict__ out, int* __restrict__ status)
+{
+	static_assert(SW_THREADS > SW_BUCKETS, "a thread a bucket, and a warp that waits for the first tile");
+	extern __shared__ __align__(128) unsigned char sw_sm[];
+	SwShared& sm = *reinterpret_cast<SwShared*>(sw_sm);
+	const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, B = f.nbuckets;
+	const uint32_t t0 = blockIdx.x * chunk_tiles;
+	const uint32_t tiles = (uint32_t) pg_min64(chunk_tiles, pg_div_up(n, SW_TILE) - t0);
+	auto rows_of = [&](uint32_t k) -> uint32_t { return pg_min32(SW_TILE, n - (t0 + k) * SW_TILE); };
+	auto issue = [&](uint32_t k) {
+		const uint32_t bytes = rows_of(k) * 16;
+		pg_mbar_expect_tx(&sm.bar[k & 1], bytes);
+		pg_bulk_g2s_hint(sm.tile[k & 1], in + (uint64_t) (t0 + k) * SW_TILE, bytes, &sm.bar[k & 1], pg_policy_evict_first());
+	};
+	if (tid == 0) {
+		pg_mbar_init(&sm.bar[0], 1);
+		pg_mbar_init(&sm.bar[1], 1);
+		pg_fence_mbar_init();
+		issue(0);
+		if (tiles > 1) issue(1);
+	}
+	for (uint32_t i = tid; i < SW_WARPS * SW_BUCKETS / 2; i += SW_THREADS) reinterpret_cast<uint32_t*>(sm.slot)[i] = 0;
+	__syncthreads();
+	const uint32_t spin = pg_spin_knob(status);
+	// Thread b keeps bucket b's next output row: the rows of lower buckets and
+	// those of earlier chunks come before this chunk's. The other warps wait for
+	// the first tile meanwhile.
+	uint32_t next = 0;
+	if (tid >= SW_BUCKETS) pg_mbar_wait_timed(&sm.bar[0], 0, spin, status);
+	else {
+		uint32_t total = 0;
+		if (tid < B)
+			#pragma unroll 8
+			for (uint32_t c = 0; c < gridDim.x; ++c) {
+				const uint32_t x = __ldg(counts + c * SW_BUCKETS + tid);
+				total += x;
+				next += c < blockIdx.x ? x : 0;
+			}
+		const uint32_t first = sw_scan256(total, sm.wt);
+		if (offsets && blockIdx.x == 0) {
+			if (tid < B) offsets[tid] = first;
+			if (tid == 0) offsets[B] = n;
+		}
+		next += first;
+	}
+	__syncthreads();
+	const uint64_t pol = pg_policy_evict_first();
+	uint16_t* const slot = sm.slot[warp];
+	const uint32_t r0 = warp * (SW_ITEMS * 32) + lane;      // item j: row r0 + 32 j of the tile
+	for (uint32_t k = 0; k < tiles; ++k) {
+		const uint32_t rows = rows_of(k);
+		uint4* const tile = sm.tile[k & 1];
+		// A wait past the context's limit records PG_ERR_TIMEOUT and goes on until
+		// the copy lands; the rows are unspecified if it never does.
+		pg_mbar_wait_timed(&sm.bar[k & 1], (k >> 1) & 1, spin, status);
+		auto work = [&](auto whole) {
+			constexpr bool FULL = decltype(whole)::value;
+			uint4 t[SW_ITEMS];
+			uint32_t br[SW_ITEMS];                       // bucket, rank in the warp's rows of it << 8
+			uint32_t first = 0, tot = 0, row = 0;        // thread b: bucket b's first slot, rows, first output row
+			#pragma unroll
+			for (int j = 0; j < SW_ITEMS; ++j) {
+				const bool mine = FULL || r0 + j * 32 < rows;
+				t[j] = tile[r0 + j * 32];
+				uint32_t b = sw_bucket<FN>(f, sw_key<K0>(t[j], kw, kbytes), kbytes);
+				if (SW_CHECKED(FN) && b >= B) b = 0;     // the histogram reported it
+				const uint32_t peers = sw_peers(b, FULL ? 0xffffffffu : __ballot_sync(0xffffffffu, mine));
+				const uint32_t at = slot[b], below = __popc(peers & ((1u << lane) - 1));
+				__syncwarp();
+				if (mine && below == 0) slot[b] = (uint16_t) (at + __popc(peers));
+				__syncwarp();
+				br[j] = b | ((at + below) << 8);
+			}
+			__syncthreads();
+			if (tid < SW_BUCKETS) {
+				uint32_t c[SW_WARPS];
+				#pragma unroll
+				for (int w = 0; w < SW_WARPS; ++w) { c[w] = sm.slot[w][tid]; tot += c[w]; }
+				first = sw_scan256(tot, sm.wt);
+				row = next;
+				next += tot;
+				uint32_t at = first;
+				#pragma unroll
+				for (int w = 0; w < SW_WARPS; ++w) { sm.slot[w][tid] = (uint16_t) at; at += c[w]; }
+			}
+			__syncthreads();
+			#pragma unroll
+			for (int j = 0; j < SW_ITEMS; ++j) {
+				const uint32_t s = slot[br[j] & 255] + (br[j] >> 8);
+				if ((FULL || r0 + j * 32 < rows) && s < SW_TILE) tile[s] = t[j];
+			}
+			pg_fence_proxy_async_smem();
+			__syncthreads();
+			// (Past n only when a copy gave up above.)
+			if (tot && (uint64_t) row + tot <= n) pg_bulk_s2g_hint(out + row, tile + first, tot * 16, pol);
+			// The counters for the next tile.
+			#pragma unroll
+			for (uint32_t i = tid; i < SW_WARPS * SW_BUCKETS / 2; i += SW_THREADS) reinterpret_cast<uint32_t*>(sm.slot)[i] = 0;
+			pg_bulk_wait_read();
+		};
+		if (rows == SW_TILE) work(std::true_type());
+		else work(std::false_type());
+		// The buffer's next copy comes after this tile's stores have read it.
+		__syncthreads();
+		if (tid == 0 && k + 2 < tiles) issue(k + 2);
+	}
+}
+
+// Whether k_part_sweep takes a partition of `in` into `out`.
+static bool sw_takes(const pg_rel* in, const void* out, uint32_t buckets)
+{
+	return in->width == 16 && (in->key_off & 3) == 0 && buckets <= SW_BUCKETS &&
+		!((reinterpret_cast<uintptr_t>(in->data) | reinterpret_cast<uintptr_t>(out)) & 15);
+}
+
+// `check` (pg_radix_pass): the key window is confirmed before the rows move;
+// *refuted and nothing written when it is not.
+struct SwCheck { uint32_t window; bool* refuted; };
+
+template <int FN, bool K0>
+static int sw_partition_as(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, const pg_hashfn& f, void* out, uint64_t* offsets,
+		const SwCheck* check)
+{
+	const uint32_t n = (uint32_t) in->n, ntiles = (uint32_t) pg_div_up(n, SW_TILE);
+	const uint32_t chunk = (uint32_t) pg_div_up(ntiles, ctx->sm_count * SW_BLOCKS_PER_SM), G = (uint32_t) pg_div_up(ntiles, chunk);
+	int rc;
+	uint32_t* counts = nullptr;               // [G][256], then the flag of a key outside the window
+	const size_t bytes = (size_t) G * SW_BUCKETS * 4 + 4;
+	if ((rc = pg_alloc_async(ctx, s, (void**) &counts, bytes))) return rc;
+	int* outside = reinterpret_cast<int*>(counts + (size_t) G * SW_BUCKETS);
+	PG_CUDA(ctx, cudaMemsetAsync(counts, 0, bytes, s));
+	k_chunk_hist<FN, K0><<<dim3(G, SW_HIST_SPLIT), 512, 0, s>>>((const uint4*) in->data, n, in->key_off / 4, in->key_bytes, f,
+			chunk * SW_TILE, counts, check ? check->window : 64, check ? outside : nullptr, ctx->d_status);
+	PG_LAUNCHED(ctx);
+	if (check) {
+		int bad = 0;
+		PG_CUDA(ctx, cudaMemcpyAsync(&bad, outside, 4, cudaMemcpyDeviceToHost, s));
+		PG_CUDA(ctx, cudaStreamSynchronize(s));
+		if (bad) { *check->refuted = true; pg_free_async(ctx, s, counts); return PG_OK; }
+	}
+	PG_CUDA(ctx, cudaFuncSetAttribute(k_part_sweep<FN, K0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(SwShared)));
+	k_part_sweep<FN, K0><<<G, SW_THREADS, sizeof(SwShared), s>>>((const uint4*) in->data, n, in->key_off / 4, in->key_bytes,
+			f, chunk, counts, offsets, (uint4*) out, ctx->d_status);
+	PG_LAUNCHED(ctx);
+	pg_free_async(ctx, s, counts);
+	return PG_OK;
+}
+
+static int sw_partition_digit(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, const pg_hashfn& f, uint32_t bits, void* out,
+		uint64_t* offsets, const SwCheck* check)
+{
+	const bool k0 = in->key_off == 0 && in->key_bytes == 8;
+	if (f.skipbits + bits <= 32)
+		return k0 ? sw_partition_as<PG_FN_DIGIT32, true>(ctx, s, in, f, out, offsets, check)
+		          : sw_partition_as<PG_FN_DIGIT32, false>(ctx, s, in, f, out, offsets, check);
+	return k0 ? sw_partition_as<PG_FN_DIGIT, true>(ctx, s, in, f, out, offsets, check)
+	          : sw_partition_as<PG_FN_DIGIT, false>(ctx, s, in, f, out, offsets, check);
+}
+
+// The functions that are one run of bits of key - min (modulo, and
+// parammodulo whose bits lie below the sign bit: its signed shift then equals
+// the unsigned one) go as PG_FN_DIGIT.
+static int sw_partition(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, pg_hashfn f, void* out, uint64_t* offsets)
+{
+	uint32_t lg = 0;
+	while ((1u << lg) < f.nbuckets) ++lg;
+	if (f.fn == PG_FN_MODULO) { f.fn = PG_FN_DIGIT; f.min = 0; f.skipbits = 0; }
+	else if (f.fn == PG_FN_PARAMMODULO && f.skipbits + lg < 64) f.fn = PG_FN_DIGIT;
+	if (f.fn == PG_FN_DIGIT) {
+		f.k = f.nbuckets - 1;
+		return sw_partition_digit(ctx, s, in, f, lg, out, offsets, nullptr);
+	}
+	if (f.fn == PG_FN_MIXRADIX) return sw_partition_as<PG_FN_MIXRADIX, false>(ctx, s, in, f, out, offsets, nullptr);
+	return sw_partition_as<PART_FN_ANY, false>(ctx, s, in, f, out, offsets, nullptr);
+}
+
+bool pg_radix_pass_takes(const pg_rel* in, const void* out) { return sw_takes(in, out, SW_BUCKETS) && in->n < (1ull << 32); }
+
+int pg_radix_pass(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, int64_t base, int pass, int window, bool* refuted, void* out)
+{
+	pg_hashfn f = {};
+	f.fn = PG_FN_DIGIT; f.min = base; f.skipbits = 8 * pass; f.nbuckets = SW_BUCKETS; f.k = SW_BUCKETS - 1;
+	const SwCheck check = {(uint32_t) window, refuted};
+	return sw_partition_digit(ctx, s, in, f, 8, out, nullptr, refuted ? &check : nullptr);
+}
+
 extern "C" int pg_partition(pg_ctx* ctx, pg_stream stream, const pg_rel* in,
 		const pg_hashcfg* cfg, void* out, uint64_t* offsets)
 {
@@ -311,6 +634,7 @@ int pg_partition_fn(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, const pg_hash
 		if (offsets) PG_CUDA(ctx, cudaMemsetAsync(offsets, 0, (B + 1) * sizeof(uint64_t), s));
 		return PG_OK;
 	}
+	if (sw_takes(in, out, B)) return sw_partition(ctx, s, in, f, out, offsets);
 	const int NW = B <= 1024 ? 8 : 4;
 	const int64_t tb = ctx->tune[PG_TUNE_PARTITION_TILE];
 	uint32_t tile = (uint32_t) (tb > 0 ? std::min<int64_t>(65536, std::max<int64_t>(8192, tb)) : PART_TILE_BYTES) / W;

@@ -175,11 +175,11 @@ __global__ void k_records_to_tuples(const pg_rec* __restrict__ rec, uint64_t n, 
 // (hash.cpp:237-267) driven to completion. Ties keep input order.
 // ---------------------------------------------------------------------------
 __global__ void k_sort_minmax(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff,
-		uint32_t kbytes, unsigned long long* __restrict__ mm)
+		uint32_t kbytes, uint64_t step, unsigned long long* __restrict__ mm)
 {
 	unsigned long long lo = ~0ull, hi = 0;
-	for (uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; i < n;
-			i += (uint64_t) gridDim.x * blockDim.x) {
+	for (uint64_t i = (blockIdx.x * (uint64_t) blockDim.x + threadIdx.x) * step; i < n;
+			i += (uint64_t) gridDim.x * blockDim.x * step) {
 		const unsigned long long u = (unsigned long long) pg_load_key(in + i * W + koff, kbytes) ^ (1ull << 63);
 		lo = u < lo ? u : lo;
 		hi = u > hi ? u : hi;
@@ -212,6 +212,42 @@ __global__ void k_make_records(const char* __restrict__ in, uint64_t n, uint32_t
 	}
 }
 
+// Smallest and largest key of rows 0, step, 2 step, ... (step 1: every row),
+// sign bit flipped (unsigned order = signed order). One host round trip.
+static int sort_key_range(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint64_t step, unsigned long long (&h)[2])
+{
+	int rc;
+	unsigned long long* mm = nullptr;
+	if ((rc = pg_alloc_async(ctx, s, (void**) &mm, 16))) return rc;
+	const unsigned long long init[2] = {~0ull, 0ull};
+	PG_CUDA(ctx, cudaMemcpyAsync(mm, init, 16, cudaMemcpyHostToDevice, s));
+	const int blocks = (int) std::min<uint64_t>(pg_div_up(pg_div_up(in->n, step), 256), (uint64_t) ctx->sm_count * 8);
+	k_sort_minmax<<<blocks, 256, 0, s>>>((const char*) in->data, in->n, in->width, in->key_off, in->key_bytes, step, mm);
+	PG_LAUNCHED(ctx);
+	PG_CUDA(ctx, cudaMemcpyAsync(h, mm, 16, cudaMemcpyDeviceToHost, s));
+	PG_CUDA(ctx, cudaStreamSynchronize(s));
+	pg_free_async(ctx, s, mm);
+	return PG_OK;
+}
+
+static int bits_of(unsigned long long x) { return x == 0 ? 0 : 64 - __builtin_clzll(x); }
+
+// The passes over the low `bits` bits of key - base, the last into `out`. With
+// `refuted`, the first one confirms that no key lies outside.
+static int radix_passes(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, int64_t base, int bits, void* out, void* tmp,
+		bool* refuted)
+{
+	const int passes = (bits + 7) / 8;
+	pg_rel cur = *in;
+	for (int p = 0; p < passes; ++p) {
+		void* dst = (passes - 1 - p) % 2 == 0 ? out : tmp;
+		if (int rc = pg_radix_pass(ctx, s, &cur, base, p, bits, p == 0 ? refuted : nullptr, dst)) return rc;
+		if (p == 0 && refuted && *refuted) return PG_OK;
+		cur.data = dst;
+	}
+	return PG_OK;
+}
+
 // Sorts `in` into `out` by radix passes when the key span allows; returns
 // PG_OK with *done = false (nothing queued) when it does not. `tmp` holds n
 // tuples of scratch.
@@ -220,27 +256,42 @@ static int radix_sort(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, void* out, 
 	*done = false;
 	const uint64_t n = in->n;
 	if (n == 0 || n >= (1ull << 32)) return PG_OK;
+	const int64_t path = ctx->tune[PG_TUNE_SORT_PATH];
+	if (path == 2) return PG_OK;
+	const int64_t tb = ctx->tune[PG_TUNE_RADIX_BITS];
+	const int digit = tb >= 4 && tb <= 12 ? (int) tb : 8;
+	const bool sweep = digit == 8 && pg_radix_pass_takes(in, out) && pg_radix_pass_takes(in, tmp);
 	int rc;
-	unsigned long long* mm = nullptr;
-	if ((rc = pg_alloc_async(ctx, s, (void**) &mm, 16))) return rc;
-	const unsigned long long init[2] = {~0ull, 0ull};
-	PG_CUDA(ctx, cudaMemcpyAsync(mm, init, 16, cudaMemcpyHostToDevice, s));
-	const int blocks = (int) std::min<uint64_t>(pg_div_up(n, 256), (uint64_t) ctx->sm_count * 8);
-	k_sort_minmax<<<blocks, 256, 0, s>>>((const char*) in->data, n, in->width, in->key_off, in->key_bytes, mm);
-	PG_LAUNCHED(ctx);
 	unsigned long long h[2];
-	PG_CUDA(ctx, cudaMemcpyAsync(h, mm, 16, cudaMemcpyDeviceToHost, s));
-	PG_CUDA(ctx, cudaStreamSynchronize(s));
-	pg_free_async(ctx, s, mm);
-	const unsigned long long span = h[1] - h[0];
-	const int bits = span == 0 ? 0 : 64 - __builtin_clzll(span);
-	// LSD radix over the bits of key - min while they fit 63 bits (the digit
-	// function masks a signed difference). Bitonic tiles and merge-path
+	if (sweep && n >= (1ull << 22)) {
+		// Large inputs: the window of the digits from every 1024th row, checked
+		// by the first pass, instead of a pass for the exact
+		// range: the aligned power of two around the sample, or the sample
+		// widened by 1/256 a side, whichever needs no more passes than the
+		// sample's own span.
+		if ((rc = sort_key_range(ctx, s, in, 1024, h))) return rc;
+		const unsigned long long span = h[1] - h[0], slack = span / 256 + 64;
+		const int want = (bits_of(span) + 7) / 8, ab = bits_of(h[0] ^ h[1]);
+		const unsigned long long lo = h[0] > slack ? h[0] - slack : 0, hi = ~0ull - h[1] > slack ? h[1] + slack : ~0ull;
+		const int wb = bits_of(hi - lo);
+		unsigned long long base = 0;
+		int bits = 0;
+		if ((ab + 7) / 8 == want) { bits = ab; base = ab == 64 ? 0 : h[0] >> ab << ab; }
+		else if ((wb + 7) / 8 == want) { bits = wb; base = lo; }
+		if (bits) {
+			bool refuted = false;
+			if ((rc = radix_passes(ctx, s, in, (int64_t) (base ^ (1ull << 63)), bits, out, tmp, &refuted))) return rc;
+			if (!refuted) { *done = true; return PG_OK; }
+		}
+	}
+	if ((rc = sort_key_range(ctx, s, in, 1, h))) return rc;
+	const int bits = bits_of(h[1] - h[0]);
+	// LSD radix over the bits of key - min (while they fit 63 bits for other
+	// tuples than 16 bytes, whose digit function masks a signed difference). Bitonic tiles and merge-path
 	// merges instead for wider spans, and for small inputs whose span needs
 	// more than four 8-bit passes: there the few merge passes cost less than
 	// the radix passes (a histogram read and a scatter each).
-	const int64_t path = ctx->tune[PG_TUNE_SORT_PATH];
-	if (path == 2 || bits > 63) return PG_OK;
+	if (bits > 63 && !sweep) return PG_OK;
 	if (path == 0 && bits > 32 && n <= (1ull << 18)) return PG_OK;
 	const long long kmin = (long long) (h[0] ^ (1ull << 63));
 	if (bits == 0) {   // one key value: already sorted
@@ -248,8 +299,11 @@ static int radix_sort(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, void* out, 
 		*done = true;
 		return PG_OK;
 	}
-	const int64_t tb = ctx->tune[PG_TUNE_RADIX_BITS];
-	const int digit = tb >= 4 && tb <= 12 ? (int) tb : 8;
+	if (sweep) {
+		if ((rc = radix_passes(ctx, s, in, kmin, bits, out, tmp, nullptr))) return rc;
+		*done = true;
+		return PG_OK;
+	}
 	const int passes = (bits + digit - 1) / digit;
 	pg_rel cur = *in;
 	for (int p = 0; p < passes; ++p) {

@@ -105,3 +105,46 @@ def test_mpsm_key_outside_the_sampled_window(ctx):
     got, n3, _ = ctx.mpsm(R, S)
     want, _, _ = orc.mergejoin(R, S)
     assert n3 == n2 and np.array_equal(orc.canonical(got), orc.canonical(want))
+
+
+# 16-byte tuples and at most 256 buckets: tiles of 3072 rows over two blocks an
+# SM. Sizes around one tile, a chunk of several, keys in any word, 4-byte keys
+# and every kind of bucket function.
+@pytest.mark.parametrize("n", [1, 31, 3071, 3072, 3073, 304 * 3072 + 1, 2 * 304 * 3072 - 5])
+@pytest.mark.parametrize("cfg", [("parammodulo", dict(buckets=256)), ("parammodulo", dict(buckets=256, skipbits=28, offset=9)),
+                                 ("parammodulo", dict(buckets=128, skipbits=40)), ("modulo", dict(buckets=8)),
+                                 ("exactrange", dict(buckets=231, min=-(1 << 40), max=1 << 40)), ("knuth", dict(buckets=64)),
+                                 ("alwayszero", dict())])
+def test_partition_16_byte_tiles(ctx, n, cfg):
+    rows = dg.uniform_keys(n, 1 << 41, dg.seed_for(205))
+    rows[:, 0] -= 1 << 40
+    fn, kw = cfg
+    for key in ((0, 8), (8, 8), (4, 8), (12, 4)):
+        if fn == "exactrange" and key != (0, 8):
+            continue
+        got, offs = ctx.partition(rows, gpu.hashcfg(fn, **kw), *key)
+        want, woffs = orc.partition(rows, orc.hashcfg(fn, **kw), key)
+        assert np.array_equal(offs, woffs)
+        assert np.array_equal(got.view(np.uint8), want.view(np.uint8))
+
+
+# From 4M tuples the sort's digits come from a sampled key window: an aligned
+# one, one that straddles zero, one that a key off the sample refutes, and spans
+# over 63 bits. Ties keep input order.
+@pytest.mark.parametrize("case", ["aligned", "straddling", "refuted", "power_of_two_edge", "one_value", "full_span"])
+def test_sort_key_windows(ctx, case):
+    n = (1 << 22) + 77
+    rows = dg.uniform_keys(n, 1 << 20, dg.seed_for(206))
+    if case == "straddling":
+        rows[:, 0] -= 1 << 19
+    elif case == "refuted":
+        rows[1025, 0], rows[2050, 0] = 1 << 45, -5
+    elif case == "power_of_two_edge":
+        rows[5, 0] = 1 << 20
+    elif case == "one_value":
+        rows[:, 0] = 42
+    elif case == "full_span":
+        rows[:, 0] *= -7046029254386353131
+        rows[3, 0], rows[4, 0] = np.iinfo(np.int64).min, np.iinfo(np.int64).max
+    want = rows[np.argsort(rows[:, 0], kind="stable")]
+    assert np.array_equal(ctx.sort(rows), want)
