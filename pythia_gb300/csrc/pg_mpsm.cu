@@ -321,7 +321,8 @@ __global__ void k_mj_minmax(const char* __restrict__ in, uint64_t n, uint32_t W,
 // Both relations are read once or twice and neither is written back sorted,
 // which is what the sort-merge of the same join spends its time on.
 // ---------------------------------------------------------------------------
-#define MJ_ILP 8
+#define MJ_ILP 2                    // tuples in flight a thread of the counting and lookup passes
+#define MJ_BLOCKS_PER_SM 64         // blocks of those passes: many short ones (64M x 64M: 0.75 ms; 8 and 16: 0.92)
 #define MJ_MAX_RANGE (1ull << 30)
 #define MJ_MIN_RANGE (1ull << 24)   // window always worth a table (64 MB, kept in L2)
 #define MJ_MAX_RUN 16384            // longest build run whose rows one warp writes for a probe tuple
@@ -761,8 +762,8 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 		auto release = [&]() { for (void* p : {(void*) cnt, (void*) sums, (void*) val}) pg_free_async(ctx, s, p); };
 		if ((rc = pg_alloc_async(ctx, s, (void**) &cnt, (uint64_t) range * 4))) return rc;
 		PG_CUDA(ctx, cudaMemsetAsync(cnt, 0, (uint64_t) range * 4, s));
-		const int cblocks = (int) std::min<uint64_t>(pg_div_up(C->n, 256 * MJ_ILP), (uint64_t) ctx->sm_count * 16);
-		const int pblocks = (int) std::min<uint64_t>(pg_div_up(P->n, 256 * MJ_ILP), (uint64_t) ctx->sm_count * 16);
+		const int cblocks = (int) std::min<uint64_t>(pg_div_up(C->n, 256 * MJ_ILP), (uint64_t) ctx->sm_count * MJ_BLOCKS_PER_SM);
+		const int pblocks = (int) std::min<uint64_t>(pg_div_up(P->n, 256 * MJ_ILP), (uint64_t) ctx->sm_count * MJ_BLOCKS_PER_SM);
 #define MJ_COUNT(V, VALS) k_mj_count<V, VALS><<<cblocks, 256, 0, s>>>((const char*) C->data, C->n, C->width, C->key_off, \
 				C->key_bytes, kmin, range, cnt, meta + 1, bp, vmm)
 		if (materialize) MJ_COUNT(true, true);
