@@ -101,7 +101,8 @@ __device__ __forceinline__ uint64_t hj_pack(const char* t, uint32_t code)
 // so the L2 round trips of several inserts overlap instead of running one
 // tuple at a time. A key already present is inserted again (duplicates are
 // kept) and flags the table as not unique.
-#define HT_ILP 4
+#define HT_ILP 2
+#define HT_BLOCKS_PER_SM 64
 __global__ void __launch_bounds__(256)
 k_ht_build(const char* __restrict__ R, uint64_t n, uint32_t W, uint32_t koff,
 		uint32_t kbytes, uint32_t pcode, bool inline_val, unsigned long long* __restrict__ slots,
@@ -385,7 +386,8 @@ __global__ void __launch_bounds__(1024) k_dense_prep16(const uint4* __restrict__
 	const unsigned long long vspan = vhi - vlo;
 	h.vmin = 0;
 	if (h.drange == 0 || vspan >= 0xFFFFFFFEull) {
-		h.flags = 4;
+		// 8: the sampled keys alone span more than a dense table takes.
+		h.flags = 4 | (hi - lo >= (2 * n > 64 ? 2 * n : 64) ? 8 : 0);
 		h.drange = 0;
 	} else {
 		const unsigned long long slack = m == n ? 0 : (0xFFFFFFFEull - vspan) / 2;
@@ -1491,6 +1493,66 @@ __device__ __forceinline__ void hj_st_stream(char* p, uint4 v, uint64_t pol)
 			:: "l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "l"(pol));
 }
 
+// ---------------------------------------------------------------------------
+// Count and sum of a probe of 16-byte tuples against a hashed table of unique
+// keys: one tuple in flight a thread, straight from global memory, in many short
+// blocks. Random bucket loads bound it (38 of its 54 DRAM bytes a tuple on a
+// 128 MB table, at 0.74 of the copy rate), so what counts is how many warps wait
+// for them at once: 48M probes 520 us, against 580 staged through shared memory
+// with sixteen warps on an SM (k_probe16_warp) and 840 with two tuples a thread
+// (spills at this occupancy).
+// ---------------------------------------------------------------------------
+#define HA_BLOCKS_PER_SM 64
+__global__ void __launch_bounds__(256, 6)
+k_probe16_hash_agg(const char* __restrict__ S, uint64_t n, uint32_t koff, const HjProbeTable tb, uint32_t wsel,
+		uint32_t sum_w0, uint32_t sum_words, unsigned long long* __restrict__ agg, int sum_col)
+{
+	__shared__ unsigned long long red[2][8];
+	const uint64_t mask = (1ull << tb.log2cap) - 1;
+	const uint64_t stride = (uint64_t) gridDim.x * blockDim.x;
+	const uint64_t keep = pg_policy_keep((tb.cache >> 4) & 7), stream = pg_policy_evict_first();
+	unsigned long long cnt = 0, sum = 0;
+	for (uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; i < n; i += stride) {
+		const uint4 t = hj_ld_stream(S + i * 16, stream);
+		const int64_t key = koff == 0 ? (int64_t) (((uint64_t) t.y << 32) | t.x) : (int64_t) (((uint64_t) t.w << 32) | t.z);
+		uint64_t val = 0;
+		bool hit = false;
+		if (key == PG_EMPTY_KEY) {
+			if (tb.nside) { hit = true; val = tb.side[0]; }
+		} else {
+			uint64_t slot = hj_slot0(key, tb.log2cap);
+			for (uint64_t round = 0; round <= (mask >> 1); ++round) {
+				const pg_u64x4 bk = pg_ld_bucket32(tb.slots + 2 * slot, keep);
+				if ((long long) bk.a == key) { hit = true; val = bk.b; break; }
+				if (bk.a == (unsigned long long) PG_EMPTY_KEY) break;
+				if ((long long) bk.c == key) { hit = true; val = bk.d; break; }
+				if (bk.c == (unsigned long long) PG_EMPTY_KEY) break;
+				slot = (slot + 2) & mask;
+			}
+		}
+		if (!hit) continue;
+		++cnt;
+		if (sum_col < 0) continue;
+		const uint32_t lo = hj_pick(t, val, (wsel >> (4 * sum_w0)) & 15);
+		if (sum_words == 2)
+			sum += ((unsigned long long) hj_pick(t, val, (wsel >> (4 * sum_w0 + 4)) & 15) << 32) | lo;
+		else sum += (unsigned long long) (long long) (int32_t) lo;
+	}
+	#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) {
+		cnt += __shfl_down_sync(0xffffffffu, cnt, o);
+		sum += __shfl_down_sync(0xffffffffu, sum, o);
+	}
+	if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = cnt; red[1][threadIdx.x >> 5] = sum; }
+	__syncthreads();
+	if (threadIdx.x < 2) {
+		unsigned long long x = 0;
+		#pragma unroll
+		for (int w = 0; w < 8; ++w) x += red[threadIdx.x][w];
+		if (x) atomicAdd(&agg[threadIdx.x], x);
+	}
+}
+
 // STD: the output row is (probe words 2-3, value) = the (P$1, B$1) projection
 // of 16-byte tuples, picked without the general word selector.
 // PRED: probe tuples failing the predicates `pr` skip their lookup (a Filter
@@ -2000,13 +2062,14 @@ static uint32_t hj_probe_partition_bits(const pg_ctx* ctx, const pg_hashtable* h
 
 // The table of R with host round trips: exact key and value ranges read back
 // first, then a dense layout (duplicates counted and read back) or the hashed
-// table. Fills the layout fields of `ht`.
-static int hj_build_exact(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, pg_hashtable* ht)
+// table. `hashed`: the key range is known to be too wide for a dense layout.
+// Fills the layout fields of `ht`.
+static int hj_build_exact(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, pg_hashtable* ht, bool hashed)
 {
 	int rc;
 	ht->dense = false; ht->dense_val = nullptr; ht->dense_bits = nullptr; ht->dense32 = nullptr; ht->vmin = 0;
 	ht->slots = nullptr; ht->side = nullptr; ht->nside = 0;
-	if (R->n && ht->inline_val && ctx->tune[PG_TUNE_DENSE] != 2) {
+	if (R->n && ht->inline_val && !hashed && ctx->tune[PG_TUNE_DENSE] != 2) {
 		// Dense key domain (unique keys spanning at most 2|R| values, e.g. a
 		// surrogate primary key 1..N): index by key - min, no hashing. Only
 		// for packed values: the unique-key probe kernels read them inline.
@@ -2108,7 +2171,7 @@ static int hj_build_exact(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, pg_hasht
 		PG_CUDA(ctx, cudaMemsetAsync(ht->slots, 0xFF, ht->capacity * 16, s));
 		PG_CUDA(ctx, cudaMemsetAsync(side_count, 0, 8, s));
 		if (R->n) {
-			int blocks = (int) std::min<uint64_t>(pg_div_up(R->n, 256 * HT_ILP), (uint64_t) ctx->sm_count * 16);
+			int blocks = (int) std::min<uint64_t>(pg_div_up(R->n, 256 * HT_ILP), (uint64_t) ctx->sm_count * HT_BLOCKS_PER_SM);
 			k_ht_build<<<blocks, 256, 0, s>>>(Rb, R->n, R->width, R->key_off, R->key_bytes,
 					hj_pack_code(ht->bcols), ht->inline_val, ht->slots, ht->log2cap, ht->side, ht->side_cap,
 					side_count, flags, ctx->d_status);
@@ -2211,7 +2274,7 @@ int hj_settle(pg_ctx* ctx, pg_hashtable* ht)
 	// header see it refuted and touch no entry, so the window can go.
 	pg_free_async(ctx, s, ht->dense32_base);
 	ht->dense32_base = nullptr; ht->dense32 = nullptr;
-	int rc = hj_build_exact(ctx, s, &ht->rel, ht);
+	int rc = hj_build_exact(ctx, s, &ht->rel, ht, (h.flags & 8) != 0);
 	ht->spec.store(false, std::memory_order_release);
 	return rc;
 }
@@ -2247,7 +2310,7 @@ extern "C" int pg_hashjoin_build(pg_ctx* ctx, pg_stream stream, const pg_rel* R,
 			(spec == 1 || R->n >= HJ_SPEC_MIN_TUPLES))
 		rc = hj_build_spec(ctx, s, R, ht);
 	else
-		rc = hj_build_exact(ctx, s, R, ht);
+		rc = hj_build_exact(ctx, s, R, ht, false);
 	if (rc) { pg_hashtable_free(ctx, ht); return rc; }
 	*out = ht;
 	return PG_OK;
@@ -2396,6 +2459,13 @@ static int hj_launch_unique(pg_ctx* ctx, cudaStream_t s, const pg_hashtable* ht,
 			const int passes = mode == 0 || pk == 1 ? 1
 				: (pk == 2 || (!direct && tbytes > HJ_TWO_PASS_MIN_BYTES && tbytes <= HJ_TWO_PASS_MAX_BYTES)) ? 2 : 1;
 			const uint64_t dr = mode == 0 ? 0 : ht->drange;
+			// Counts and sums over a hashed table (knob 1: the staged probe).
+			if (mode == 0 && !materialize && var != 1) {
+				const int ablocks = (int) std::min<uint64_t>(pg_div_up(n, 256), (uint64_t) ctx->sm_count * HA_BLOCKS_PER_SM);
+				k_probe16_hash_agg<<<ablocks, 256, 0, s>>>(S, n, koff, tb, wsel, sum_w0, sum_words, acc + 1, sum_col);
+				PG_LAUNCHED(ctx);
+				return PG_OK;
+			}
 			// Only the register-loading dense kernels read a speculative
 			// table's window from its header.
 			if (spec && (!direct || pred || passes != 1)) return HJ_NEED_SETTLE;
