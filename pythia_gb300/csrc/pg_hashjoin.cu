@@ -396,6 +396,105 @@ __global__ void __launch_bounds__(1024) k_dense_prep16(const uint4* __restrict__
 	*hdr = h;
 }
 
+// The same for few tuples in one launch of one CTA, exactly: ranges over every
+// tuple, window, fill, store and count, with block barriers where the form for
+// large inputs has launches, and where no dense layout fits (keys too far apart or
+// repeated) the hashed table, which the first use then finds ready. Joins of 1000
+// tuples with 10,000: dense keys 73 -> 41 us, far ones 106 -> 74; of 8000 with 50,000:
+// 80 -> 44 and 112 -> 106. From 16,000 tuples far apart one SM's random atomics take
+// longer than the launches and round trips they save (111 -> 135).
+#define HJ_SMALL_TUPLES 8192
+__global__ void __launch_bounds__(1024) k_dense_small16(const uint4* __restrict__ R, uint32_t n, uint32_t kw,
+		uint32_t pk, uint64_t cap, uint32_t* __restrict__ table, unsigned long long* __restrict__ slots, uint32_t log2cap,
+		HjDenseHdr* __restrict__ hdr)
+{
+	__shared__ unsigned long long red[4][32];
+	__shared__ HjDenseHdr h;
+	const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	unsigned long long lo = ~0ull, hi = 0, vlo = ~0ull, vhi = 0;
+	#pragma unroll 8
+	for (uint32_t i = tid; i < n; i += 1024) {
+		const uint4 v = __ldg(R + i);
+		const unsigned long long k = (((unsigned long long) hj_word4(v, kw + 1) << 32) | hj_word4(v, kw)) ^ (1ull << 63);
+		const unsigned long long p = hj_pack16(v, pk);
+		lo = k < lo ? k : lo; hi = k > hi ? k : hi;
+		vlo = p < vlo ? p : vlo; vhi = p > vhi ? p : vhi;
+	}
+	hj_minmax4(lo, hi, vlo, vhi);
+	if (lane == 0) { red[0][warp] = lo; red[1][warp] = hi; red[2][warp] = vlo; red[3][warp] = vhi; }
+	__syncthreads();
+	if (warp == 0) {
+		lo = red[0][lane]; hi = red[1][lane]; vlo = red[2][lane]; vhi = red[3][lane];
+		hj_minmax4(lo, hi, vlo, vhi);
+		if (lane == 0) {
+			const bool wide = hi - lo >= (2 * (uint64_t) n > 64 ? 2 * (uint64_t) n : 64) || hi - lo >= cap;
+			h.n = n; h.present = 0; h.kmin = lo; h.kmax = hi; h.vlo = vlo; h.vhi = vhi; h.pad = 0;
+			h.dmin = (long long) (lo ^ (1ull << 63));
+			h.vmin = vlo;
+			h.flags = wide ? 4 | 8 : vhi - vlo >= 0xFFFFFFFFull ? 4 : 0;
+			h.drange = h.flags ? 0 : hi - lo + 1;
+		}
+	}
+	__syncthreads();
+	bool dense = h.flags == 0;
+	if (dense) {
+		const uint32_t range = (uint32_t) h.drange;
+		for (uint32_t i = tid; i < (range + 3) / 4; i += 1024)
+			reinterpret_cast<uint4*>(table)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+		__syncthreads();
+		#pragma unroll 4
+		for (uint32_t i = tid; i < n; i += 1024) {
+			const uint4 v = __ldg(R + i);
+			const unsigned long long k = ((unsigned long long) hj_word4(v, kw + 1) << 32) | hj_word4(v, kw);
+			table[k - (unsigned long long) h.dmin] = (uint32_t) (hj_pack16(v, pk) - h.vmin);
+		}
+		__syncthreads();
+		uint32_t c = 0;
+		for (uint32_t i = tid; i < range; i += 1024) c += *(volatile uint32_t*) (table + i) != 0xFFFFFFFFu;
+		c = __reduce_add_sync(0xffffffffu, c);
+		if (lane == 0) red[0][warp] = c;
+		__syncthreads();
+		if (tid == 0) {
+			unsigned long long t = 0;
+			for (int w = 0; w < 32; ++w) t += red[0][w];
+			h.present = t;
+		}
+		__syncthreads();
+		dense = h.present == n;
+	}
+	// Wide values keep a dense layout of their own, made by the exact build;
+	// so do keys equal to the empty marker, with their side list.
+	if (!dense && (h.flags == 0 || (h.flags & 8)) && h.kmin <= ((1ull << 63) - 1) && h.kmax >= ((1ull << 63) - 1)) {
+		int marker = 0;
+		for (uint32_t i = tid; i < n; i += 1024) {
+			const uint4 v = __ldg(R + i);
+			marker |= (hj_word4(v, kw + 1) & hj_word4(v, kw)) == ~0u;
+		}
+		if (__syncthreads_or(marker)) {
+			if (tid == 0) *hdr = h;
+			return;
+		}
+	}
+	if (!dense && (h.flags == 0 || (h.flags & 8))) {
+		const uint32_t mask = (1u << log2cap) - 1;
+		for (uint32_t i = tid; i <= mask; i += 1024) reinterpret_cast<uint4*>(slots)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+		__syncthreads();
+		int dup = 0;
+		for (uint32_t i = tid; i < n; i += 1024) {
+			const uint4 v = __ldg(R + i);
+			const unsigned long long k = ((unsigned long long) hj_word4(v, kw + 1) << 32) | hj_word4(v, kw);
+			for (uint32_t s = (uint32_t) hj_slot0((int64_t) k, log2cap);; s = (s + 1) & mask) {   // at most half full
+				const unsigned long long old = atomicCAS(&slots[2 * (uint64_t) s], (unsigned long long) PG_EMPTY_KEY, k);
+				if (old == (unsigned long long) PG_EMPTY_KEY) { slots[2 * (uint64_t) s + 1] = hj_pack16(v, pk); break; }
+				if (old == k) dup = 1;
+			}
+		}
+		dup = __syncthreads_or(dup);
+		if (tid == 0) h.flags |= 16 | (dup ? 32 : 0);
+	}
+	if (tid == 0) *hdr = h;
+}
+
 // All ones over the window's entries (nothing when the sample ruled it out).
 __global__ void k_dense_fill16(uint32_t* __restrict__ table, const HjDenseHdr* __restrict__ hdr)
 {
@@ -2060,6 +2159,14 @@ static uint32_t hj_probe_partition_bits(const pg_ctx* ctx, const pg_hashtable* h
 	return std::min<uint32_t>(std::max<uint32_t>(lp, 1), 8);
 }
 
+// Hashed slots for n tuples: at most half full.
+static uint32_t hj_log2cap(uint64_t n)
+{
+	uint32_t lg = 10;
+	while ((1ull << lg) < 2 * n) ++lg;
+	return lg;
+}
+
 // The table of R with host round trips: exact key and value ranges read back
 // first, then a dense layout (duplicates counted and read back) or the hashed
 // table. `hashed`: the key range is known to be too wide for a dense layout.
@@ -2142,10 +2249,7 @@ static int hj_build_exact(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, pg_hasht
 		}
 		pg_free_async(ctx, s, mm);
 	}
-	uint64_t want = std::max<uint64_t>(1024, 2 * R->n);
-	uint32_t lg = 10;
-	while ((1ull << lg) < want) ++lg;
-	ht->log2cap = lg; ht->capacity = 1ull << lg;
+	ht->log2cap = hj_log2cap(R->n); ht->capacity = 1ull << ht->log2cap;
 	ht->side_cap = HJ_SIDE_CAP0;
 	if ((rc = pg_alloc_async(ctx, s, (void**) &ht->slots, ht->capacity * 16))) return rc;
 	if ((rc = pg_alloc_async(ctx, s, (void**) &ht->side, ht->side_cap * 8 + 64))) return rc;
@@ -2211,6 +2315,22 @@ static int hj_build_spec(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, pg_hashta
 	ht->dmin = 0; ht->drange = cap; ht->vmin = 0; ht->vlo = 0; ht->vmax = 0;     // bounds until settled
 	const uint32_t kw = R->key_off / 4;
 	const uint32_t pk = hj_pack16_code(ht->bcols);
+	auto built = [&]() {
+		// Probes on other streams wait for these kernels (the build returns
+		// without synchronising).
+		PG_CUDA(ctx, cudaEventCreateWithFlags(&ht->built, cudaEventDisableTiming));
+		PG_CUDA(ctx, cudaEventRecord(ht->built, s));
+		ht->spec.store(true, std::memory_order_release);
+		return PG_OK;
+	};
+	if (R->n <= HJ_SMALL_TUPLES && ctx->tune[PG_TUNE_BUILD_SPEC] != 1) {
+		ht->log2cap = hj_log2cap(R->n);
+		if ((rc = pg_alloc_async(ctx, s, (void**) &ht->small_slots, 16ull << ht->log2cap))) return rc;
+		k_dense_small16<<<1, 1024, 0, s>>>((const uint4*) R->data, (uint32_t) R->n, kw, pk, cap, ht->dense32_base,
+				ht->small_slots, ht->log2cap, ht->hdr);
+		PG_LAUNCHED(ctx);
+		return built();
+	}
 	k_dense_prep16<<<1, 1024, 0, s>>>((const uint4*) R->data, R->n, kw, pk, cap, ht->hdr);
 	PG_LAUNCHED(ctx);
 	const int fgrid = (int) std::min<uint64_t>(pg_div_up(cap / 4 + 1, 256), (uint64_t) ctx->sm_count * 8);
@@ -2221,12 +2341,7 @@ static int hj_build_spec(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, pg_hashta
 	PG_LAUNCHED(ctx);
 	k_dense32_count_spec<<<fgrid, 256, 0, s>>>(ht->dense32_base, ht->hdr);
 	PG_LAUNCHED(ctx);
-	// Probes on other streams wait for these kernels (the build returns
-	// without synchronising).
-	PG_CUDA(ctx, cudaEventCreateWithFlags(&ht->built, cudaEventDisableTiming));
-	PG_CUDA(ctx, cudaEventRecord(ht->built, s));
-	ht->spec.store(true, std::memory_order_release);
-	return PG_OK;
+	return built();
 }
 
 static bool hj_hdr_ok(const HjDenseHdr& h)
@@ -2234,15 +2349,21 @@ static bool hj_hdr_ok(const HjDenseHdr& h)
 	return h.flags == 0 && h.present == h.n;
 }
 
-int hj_settle(pg_ctx* ctx, pg_hashtable* ht)
+// `refuted`: the header's flags, present entries and tuples as a probe read
+// them back when its checks failed (no second round trip), else null.
+static int hj_settle_known(pg_ctx* ctx, pg_hashtable* ht, const unsigned long long* refuted)
 {
 	if (!ht || !ht->spec.load(std::memory_order_acquire)) return PG_OK;
 	std::lock_guard<std::mutex> g(ht->mu);
 	if (!ht->spec.load(std::memory_order_relaxed)) return PG_OK;
 	cudaStream_t s = ht->stream;
 	HjDenseHdr h;
-	PG_CUDA(ctx, cudaMemcpyAsync(&h, ht->hdr, sizeof h, cudaMemcpyDeviceToHost, s));
-	PG_CUDA(ctx, cudaStreamSynchronize(s));
+	if (refuted) {
+		h.flags = (int) refuted[0]; h.present = refuted[1]; h.n = refuted[2];
+	} else {
+		PG_CUDA(ctx, cudaMemcpyAsync(&h, ht->hdr, sizeof h, cudaMemcpyDeviceToHost, s));
+		PG_CUDA(ctx, cudaStreamSynchronize(s));
+	}
 	if (hj_hdr_ok(h)) {
 		// Exact layout, as hj_build_exact would have made it: the window
 		// narrowed to the keys present, entries based on the smallest value.
@@ -2274,10 +2395,26 @@ int hj_settle(pg_ctx* ctx, pg_hashtable* ht)
 	// header see it refuted and touch no entry, so the window can go.
 	pg_free_async(ctx, s, ht->dense32_base);
 	ht->dense32_base = nullptr; ht->dense32 = nullptr;
-	int rc = hj_build_exact(ctx, s, &ht->rel, ht, (h.flags & 8) != 0);
+	if (h.flags & 16) {          // the build kernel filled the hashed table
+		int rc;
+		if ((rc = pg_alloc_async(ctx, s, (void**) &ht->side, HJ_SIDE_CAP0 * 8 + 64))) return rc;
+		ht->side_cap = HJ_SIDE_CAP0; ht->nside = 0;
+		ht->dense = false; ht->dense_val = nullptr; ht->dense_bits = nullptr; ht->vmin = 0;
+		ht->log2cap = hj_log2cap(ht->rel.n); ht->capacity = 1ull << ht->log2cap;
+		ht->slots = ht->small_slots;
+		ht->small_slots = nullptr;
+		ht->unique = (h.flags & 32) == 0;
+		ht->spec.store(false, std::memory_order_release);
+		return PG_OK;
+	}
+	// Keys spanning too much, or repeated (none outside the window and fewer
+	// entries than tuples), leave the hashed table only.
+	int rc = hj_build_exact(ctx, s, &ht->rel, ht, (h.flags & 8) != 0 || h.flags == 0);
 	ht->spec.store(false, std::memory_order_release);
 	return rc;
 }
+
+int hj_settle(pg_ctx* ctx, pg_hashtable* ht) { return hj_settle_known(ctx, ht, nullptr); }
 
 extern "C" int pg_hashjoin_build(pg_ctx* ctx, pg_stream stream, const pg_rel* R,
 		const pg_col* proj, int nproj, pg_hashtable** out)
@@ -2304,10 +2441,10 @@ extern "C" int pg_hashjoin_build(pg_ctx* ctx, pg_stream stream, const pg_rel* R,
 	ht->inline_val = bbytes <= 8;
 	ht->rel = *R;
 	ht->spec.store(false); ht->hdr = nullptr; ht->dense32_base = nullptr; ht->dense32_copy = nullptr;
-	ht->built = nullptr;
+	ht->built = nullptr; ht->small_slots = nullptr;
 	const int64_t spec = ctx->tune[PG_TUNE_BUILD_SPEC];
 	if (R->n && ht->inline_val && ctx->tune[PG_TUNE_DENSE] != 2 && spec != 2 && hj_vec16(R, ht->bcols) &&
-			(spec == 1 || R->n >= HJ_SPEC_MIN_TUPLES))
+			(spec == 1 || R->n >= HJ_SPEC_MIN_TUPLES || R->n <= HJ_SMALL_TUPLES))
 		rc = hj_build_spec(ctx, s, R, ht);
 	else
 		rc = hj_build_exact(ctx, s, R, ht, false);
@@ -2333,6 +2470,7 @@ extern "C" int pg_hashtable_free(pg_ctx* ctx, pg_hashtable* ht)
 		pg_free_async(ctx, ht->stream, ht->dense32);
 	}
 	pg_free_async(ctx, ht->stream, ht->hdr);
+	pg_free_async(ctx, ht->stream, ht->small_slots);
 	if (ht->built) cudaEventDestroy(ht->built);
 	delete ht;
 	return PG_OK;
@@ -2661,7 +2799,8 @@ static int hj_readback(pg_ctx* ctx, cudaStream_t s, unsigned long long* acc, con
 // (only for the dense 16-byte layouts the register-loading kernels handle).
 static int hj_probe_run(pg_ctx* ctx, pg_stream stream, pg_hashtable* ht,
 		const pg_rel* S_in, const pg_col* proj, int nproj,
-		void* out, uint64_t out_capacity, int flags, int sum_col, pg_join_result* res, const PgPred16* pred)
+		void* out, uint64_t out_capacity, int flags, int sum_col, pg_join_result* res, const PgPred16* pred,
+		unsigned long long (&checks)[3])
 {
 	if (!ctx || !ht || !res) return pg_fail(ctx, PG_ERR_ARG, "pg_hashjoin_probe: null argument");
 	int rc;
@@ -2713,6 +2852,7 @@ static int hj_probe_run(pg_ctx* ctx, pg_stream stream, pg_hashtable* ht,
 			if ((rc = hj_readback(ctx, s, acc, hdr, host_acc, &refuted, "pg_hashjoin_probe"))) return rc;
 			if (refuted) {
 				pg_free_async(ctx, s, counts); pg_free_async(ctx, s, acc);
+				for (int i = 0; i < 3; ++i) checks[i] = host_acc[4 + i];
 				return HJ_SPEC_REFUTED;
 			}
 			res->n_out = host_acc[0];
@@ -2738,6 +2878,7 @@ static int hj_probe_run(pg_ctx* ctx, pg_stream stream, pg_hashtable* ht,
 			if ((rc = hj_readback(ctx, s, acc, hdr, host_acc, &refuted, "pg_hashjoin_probe"))) return rc;
 			if (refuted) {
 				pg_free_async(ctx, s, acc);
+				for (int i = 0; i < 3; ++i) checks[i] = host_acc[4 + i];
 				return HJ_SPEC_REFUTED;
 			}
 			res->n_out = host_acc[1];
@@ -2785,10 +2926,11 @@ static int hj_probe(pg_ctx* ctx, pg_stream stream, pg_hashtable* ht,
 		const pg_rel* S, const pg_col* proj, int nproj,
 		void* out, uint64_t out_capacity, int flags, int sum_col, pg_join_result* res, const PgPred16* pred)
 {
-	int rc = hj_probe_run(ctx, stream, ht, S, proj, nproj, out, out_capacity, flags, sum_col, res, pred);
+	unsigned long long checks[3];
+	int rc = hj_probe_run(ctx, stream, ht, S, proj, nproj, out, out_capacity, flags, sum_col, res, pred, checks);
 	if (rc != HJ_NEED_SETTLE && rc != HJ_SPEC_REFUTED) return rc;
-	if ((rc = hj_settle(ctx, ht))) return rc;
-	return hj_probe_run(ctx, stream, ht, S, proj, nproj, out, out_capacity, flags, sum_col, res, pred);
+	if ((rc = hj_settle_known(ctx, ht, rc == HJ_SPEC_REFUTED ? checks : nullptr))) return rc;
+	return hj_probe_run(ctx, stream, ht, S, proj, nproj, out, out_capacity, flags, sum_col, res, pred, checks);
 }
 
 extern "C" int pg_hashjoin_probe(pg_ctx* ctx, pg_stream stream, pg_hashtable* ht,

@@ -29,7 +29,9 @@ struct HjDenseHdr {
 	unsigned long long kmin, kmax;   // exact key range (keys ^ 2^63, as unsigned), store pass
 	unsigned long long vlo, vhi;     // exact packed-value range, store pass
 	int flags;                   // 1 key outside the window, 2 value outside the entry range,
-	                             // 4 sample: window larger than the allocation or values too wide
+	                             // 4 sample: window larger than the allocation or values too wide,
+	                             // 8 the keys read span more than any dense table takes,
+	                             // 16 small_slots hold the hashed table (32: of repeated keys)
 	int pad;
 };
 
@@ -78,6 +80,7 @@ struct pg_hashtable {
 	HjDenseHdr* hdr;
 	uint32_t* dense32_base;
 	uint32_t* dense32_copy;
+	unsigned long long* small_slots;  // few tuples: slots the build kernel fills when no dense layout fits
 	cudaEvent_t built;          // recorded after the speculative build's kernels (null otherwise)
 	pg_rel rel;                 // the build relation, for an exact rebuild
 };

@@ -148,3 +148,52 @@ def test_sort_key_windows(ctx, case):
         rows[3, 0], rows[4, 0] = np.iinfo(np.int64).min, np.iinfo(np.int64).max
     want = rows[np.argsort(rows[:, 0], kind="stable")]
     assert np.array_equal(ctx.sort(rows), want)
+
+
+def _same_join(ctx, R, S, **kw):
+    got, n, _ = ctx.hashjoin(R, S, **kw)
+    want, wn, _ = orc.hashjoin(R, S, hash=orc.hashcfg("modulo", 1 << 12), **kw)
+    assert n == wn and np.array_equal(orc.canonical(got), orc.canonical(want))
+    for sc in (0, 1):
+        _, n2, s2 = ctx.hashjoin(R, S, flags=gpu.JOIN_COUNT | gpu.JOIN_SUM, sum_col=sc, **kw)
+        assert (n2, s2) == orc.hashjoin(R, S, materialise=False, sum_col=sc, hash=orc.hashcfg("modulo", 1 << 12), **kw)[1:]
+
+
+# Builds of up to 8192 tuples are one launch, which makes either layout: dense,
+# or hashed for keys too far apart or repeated; wide values and the empty-marker
+# key (-1) beside far keys go back to the exact build.
+@pytest.mark.parametrize("n", [1, 2, 33, 1024, 1025, 8192, 8193])
+@pytest.mark.parametrize("case", ["dense", "far", "repeated", "far_repeated", "marker", "marker_far", "wide_values", "extremes"])
+def test_join_small_builds(ctx, n, case):
+    R = dg.build_relation(n, dg.seed_for(207))
+    S = dg.probe_uniform(3 * n + 5, R, dg.seed_for(208))
+    if case in ("far", "far_repeated", "marker_far"):
+        R[:, 0] *= -7046029254386353131
+        S[:, 0] *= -7046029254386353131
+    if case in ("repeated", "far_repeated"):
+        R[n // 2:, 0] = R[: n - n // 2, 0]
+    elif case in ("marker", "marker_far"):
+        R[n // 3, 0] = S[1, 0] = -1
+        if case == "marker":
+            R[:, 0] = np.arange(-2, n - 2)
+    elif case == "wide_values":
+        R[0, 1] = -5
+    elif case == "extremes":
+        R[0, 0], R[-1, 0] = np.iinfo(np.int64).min, np.iinfo(np.int64).max
+        S[0, 0], S[2, 0] = R[0, 0], R[-1, 0]
+    S[::5, 0] += 1                                          # some misses
+    _same_join(ctx, R, S)
+
+
+# Hashed counts and sums: one tuple a thread in blocks of 256, 64 blocks an SM.
+@pytest.mark.parametrize("m", [1, 255, 257, 152 * 64 * 256 + 3])
+def test_join_hashed_agg_sizes(ctx, m):
+    R = dg.build_relation(70_000, dg.seed_for(209))
+    S = dg.probe_uniform(m, R, dg.seed_for(210))
+    R[:, 0] *= -7046029254386353131
+    S[:, 0] *= -7046029254386353131
+    R[9, 0] = -1
+    S[:: max(1, m // 7), 0] = -1
+    for sc in (0, 1):
+        _, n2, s2 = ctx.hashjoin(R, S, flags=gpu.JOIN_COUNT | gpu.JOIN_SUM, sum_col=sc)
+        assert (n2, s2) == orc.hashjoin(R, S, materialise=False, sum_col=sc, hash=orc.hashcfg("modulo", 1 << 16))[1:]
