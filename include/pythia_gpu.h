@@ -176,10 +176,10 @@ enum {
 	PG_TUNE_L2_FETCH = 13,           /* L2 fetch granularity hint of the context in bytes: 0 leaves the CUDA
 	                                    default, else 32, 64 or 128 (cudaLimitMaxL2FetchGranularity, a limit of
 	                                    the calling process that ends with it) */
-	PG_TUNE_SORT_PATH = 14,          /* page sort and the MPSM's sorts: 0 LSD radix over key - min while the span
-	                                    fits 63 bits (bitonic tiles and merge-path merges for wider spans and for
-	                                    inputs of at most 2^18 tuples whose span needs over 32 bits), 1 radix
-	                                    whenever the span fits 63 bits, 2 bitonic tiles and merges always */
+	PG_TUNE_SORT_PATH = 14,          /* page sort and the MPSM's sorts: 0 LSD radix over key - min, in one cooperative
+	                                    launch up to 2^20 tuples, other than 16-byte tuples as (key, row) records;
+	                                    1 a launch per radix pass over the tuples themselves while the span fits
+	                                    them (63 bits; 64 for 16-byte tuples), else 2 bitonic tiles and merges */
 	PG_TUNE_GROUPBY_ILP = 15,        /* rows in flight per thread of the dense group-by over a global table: 4
 	                                    or 8 (0: built-in, 4) */
 	PG_TUNE_HASH_PARTITION = 16,     /* hashed tables: 2 partitions the probe side (and R, for packed values) on

@@ -197,3 +197,26 @@ def test_join_hashed_agg_sizes(ctx, m):
     for sc in (0, 1):
         _, n2, s2 = ctx.hashjoin(R, S, flags=gpu.JOIN_COUNT | gpu.JOIN_SUM, sum_col=sc)
         assert (n2, s2) == orc.hashjoin(R, S, materialise=False, sum_col=sc, hash=orc.hashcfg("modulo", 1 << 16))[1:]
+
+
+# Up to 2^20 tuples sort in one cooperative launch: one block of 4096 rows, every
+# block with four or eight rows a thread, one pass, eight passes, one value; then
+# the first size past it. Other widths go by (key, row) records. Ties keep order.
+@pytest.mark.parametrize("n", [1, 31, 4096, 4097, 150_000, 152 * 4096, 152 * 4096 + 1, 1 << 20, (1 << 20) + 1])
+@pytest.mark.parametrize("bits", [0, 1, 8, 9, 30, 64])
+def test_sort_one_launch(ctx, n, bits):
+    rows = dg.uniform_keys(n, 1 << min(bits, 40), dg.seed_for(211))
+    if bits == 64:
+        rows[:, 0] *= -7046029254386353131
+        rows[0, 0], rows[-1, 0] = np.iinfo(np.int64).max, np.iinfo(np.int64).min
+    else:
+        rows[:, 0] -= 1 << bits >> 1
+    assert np.array_equal(ctx.sort(rows), rows[np.argsort(rows[:, 0], kind="stable")])
+    if n <= 150_000:
+        assert np.array_equal(ctx.sort(rows, (8, 8)), rows[np.argsort(rows[:, 1], kind="stable")])
+        words = rows.view(np.int32).reshape(n, 4)
+        for width, off in ((12, 0), (24, 8), (20, 4)):
+            t = np.zeros((n, width // 4), dtype=np.int32)
+            t[:, 0], t[:, -1] = np.arange(n), np.arange(n)
+            t[:, off // 4:off // 4 + 2] = words[:, :2]
+            assert np.array_equal(ctx.sort(t, (off, 8)), t[np.argsort(rows[:, 0], kind="stable")])
