@@ -149,6 +149,24 @@ int pg_check_status(pg_ctx* ctx, cudaStream_t s, const char* what)
 	return PG_OK;
 }
 
+__global__ void k_collect(unsigned long long* __restrict__ dst, const int* __restrict__ status, const int* __restrict__ flag)
+{
+	dst[0] = flag ? (unsigned long long) (unsigned) *flag : 0;
+	dst[1] = (unsigned long long) (unsigned) *status;
+}
+
+int pg_readback(pg_ctx* ctx, cudaStream_t s, unsigned long long* dev, int n, const int* flag, unsigned long long* host,
+		const char* what)
+{
+	k_collect<<<1, 1, 0, s>>>(dev + n, ctx->d_status, flag);
+	PG_LAUNCHED(ctx);
+	unsigned long long h[16];
+	PG_CUDA(ctx, cudaMemcpyAsync(h, dev, (n + 2) * 8, cudaMemcpyDeviceToHost, s));
+	PG_CUDA(ctx, cudaStreamSynchronize(s));
+	for (int i = 0; i <= n; ++i) host[i] = h[i];
+	return h[n + 1] ? pg_status_fail(ctx, s, (int) h[n + 1], what) : PG_OK;
+}
+
 extern "C" int pg_stream_create(pg_ctx* ctx, pg_stream* s)
 {
 	if (!ctx || !s) return PG_ERR_ARG;

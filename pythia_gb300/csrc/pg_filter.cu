@@ -319,20 +319,21 @@ extern "C" int pg_filter(pg_ctx* ctx, pg_stream stream, const pg_rel* in, const 
 		P.chars = chars;
 	}
 	uint64_t* scratch = nullptr;
-	const unsigned long long* count = nullptr;
+	unsigned long long* count = nullptr;
 	const uint32_t rows = fl_tile_rows(w, FL_TILE_BYTES);
 	const uint64_t ntiles = pg_div_up(in->n, w <= FL_MAX_WIDTH ? rows : FL_TILE);
 	if (w <= FL_MAX_WIDTH && ntiles < (1ull << 31) - 1) {
-		// [total, ticket, first output row of each tile, survivors of each tile]
-		if ((rc = pg_alloc_async(ctx, s, (void**) &scratch, 16 + ntiles * 12))) return rc;
-		PG_CUDA(ctx, cudaMemsetAsync(scratch, 0, 16 + ntiles * 12, s));
+		// [total, two words of pg_readback, ticket, first output row of each tile,
+		// survivors of each tile]
+		if ((rc = pg_alloc_async(ctx, s, (void**) &scratch, 32 + ntiles * 12))) return rc;
+		PG_CUDA(ctx, cudaMemsetAsync(scratch, 0, 32 + ntiles * 12, s));
 		unsigned long long* total = reinterpret_cast<unsigned long long*>(scratch);
 		const size_t smem = (size_t) rows * w + rows / 32 * 8 + rows * 2;
 		const uintptr_t o = reinterpret_cast<uintptr_t>(out);
 #define FL_LAUNCH(U) do { \
 		PG_CUDA(ctx, cudaFuncSetAttribute(k_filter<U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)); \
 		k_filter<U><<<(unsigned) ntiles + 1, FL_THREADS, smem, s>>>((const char*) in->data, in->n, w, rows, P, \
-				reinterpret_cast<uint32_t*>(total + 2 + ntiles), total + 2, reinterpret_cast<unsigned int*>(total + 1), (char*) out, total, ctx->d_status); } while (0)
+				reinterpret_cast<uint32_t*>(total + 4 + ntiles), total + 4, reinterpret_cast<unsigned int*>(total + 3), (char*) out, total, ctx->d_status); } while (0)
 		if (!(w & 15) && !(o & 15)) FL_LAUNCH(uint4);
 		else if (!(w & 7) && !(o & 7)) FL_LAUNCH(uint2);
 		else FL_LAUNCH(uint32_t);
@@ -340,7 +341,7 @@ extern "C" int pg_filter(pg_ctx* ctx, pg_stream stream, const pg_rel* in, const 
 		PG_LAUNCHED(ctx);
 		count = total;
 	} else {
-		if ((rc = pg_alloc_async(ctx, s, (void**) &scratch, (ntiles + 1) * 8))) return rc;
+		if ((rc = pg_alloc_async(ctx, s, (void**) &scratch, (ntiles + 3) * 8))) return rc;
 		k_filter_count<<<(unsigned) ntiles, FL_THREADS, 0, s>>>((const char*) in->data, in->n, w, P, scratch);
 		PG_LAUNCHED(ctx);
 		if ((rc = pg_scan_u64(ctx, s, scratch, ntiles, scratch + ntiles))) return rc;
@@ -348,12 +349,12 @@ extern "C" int pg_filter(pg_ctx* ctx, pg_stream stream, const pg_rel* in, const 
 		PG_LAUNCHED(ctx);
 		count = reinterpret_cast<unsigned long long*>(scratch + ntiles);
 	}
-	uint64_t total = 0;
-	PG_CUDA(ctx, cudaMemcpyAsync(&total, count, 8, cudaMemcpyDeviceToHost, s));
+	unsigned long long h[2];
+	rc = pg_readback(ctx, s, count, 1, nullptr, h, "pg_filter");
 	pg_free_async(ctx, s, scratch);
 	pg_free_async(ctx, s, chars);
-	if ((rc = pg_check_status(ctx, s, "pg_filter"))) return rc;
-	*n_out = total;
+	if (rc) return rc;
+	*n_out = h[0];
 	return PG_OK;
 }
 

@@ -241,7 +241,7 @@ __global__ void k_gb_key_minmax(const char* __restrict__ in, uint64_t n, uint32_
 		lo = a < lo ? a : lo;
 		hi = b > hi ? b : hi;
 	}
-	if ((threadIdx.x & 31) == 0) { atomicMin(&mm[0], lo); atomicMax(&mm[1], hi); }
+	if ((threadIdx.x & 31) == 0) { atomicMax(&mm[0], ~lo); atomicMax(&mm[1], hi); }      // zero before
 }
 
 // Key and value words of row i: the 8-byte key at koff and the value at voff
@@ -710,12 +710,12 @@ static int gb_dense_window(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint32
 	int rc;
 	char* mem = nullptr;
 	const uint64_t words = range * (GB_DEC ? PG_FX_WORDS : 1);
-	const size_t bytes = words * 8 + range + 128;
+	const size_t bytes = words * 8 + 32 + range;
 	if ((rc = pg_alloc_async(ctx, s, (void**) &mem, bytes))) return rc;
 	unsigned long long* acc = reinterpret_cast<unsigned long long*>(mem);      // a dec sum: word k of slot i at acc[i + k range]
 	unsigned long long* cursor = acc + words;
-	unsigned char* present = reinterpret_cast<unsigned char*>(cursor + 1);
-	unsigned int* oflag = reinterpret_cast<unsigned int*>((reinterpret_cast<uintptr_t>(present + range) + 15) & ~uintptr_t(15));
+	unsigned int* oflag = reinterpret_cast<unsigned int*>(cursor + 1);         // then two words of pg_readback
+	unsigned char* present = reinterpret_cast<unsigned char*>(cursor + 4);
 	PG_CUDA(ctx, cudaMemsetAsync(mem, 0, bytes, s));
 	if (range <= (GB_DEC ? GBS_MAX_SLOTS_DEC : GBS_MAX_SLOTS) && ctx->tune[PG_TUNE_GROUPBY_PATH] != 7) {
 		// Few groups: per-CTA tables in shared memory, one flush each.
@@ -756,17 +756,13 @@ static int gb_dense_window(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint32
 	k_gb_dense_emit<VT, AGG><<<eblocks, 256, 0, s>>>(acc, fx, present, range, kmin, in->key_bytes, (char*) out,
 			out_cap, cursor);
 	PG_LAUNCHED(ctx);
-	unsigned long long h[2] = {0, 0};
-	unsigned int f = 0;
-	PG_CUDA(ctx, cudaMemcpyAsync(&h[0], cursor, 8, cudaMemcpyDeviceToHost, s));
-	PG_CUDA(ctx, cudaMemcpyAsync(&h[1], oflag, 4, cudaMemcpyDeviceToHost, s));
-	if (GB_DEC) PG_CUDA(ctx, cudaMemcpyAsync(&f, fx.p + 2, 4, cudaMemcpyDeviceToHost, s));
-	PG_CUDA(ctx, cudaStreamSynchronize(s));
+	unsigned long long h[3];
+	rc = pg_readback(ctx, s, cursor, 2, GB_DEC ? fx.p + 2 : nullptr, h, "pg_groupby");
 	pg_free_async(ctx, s, mem);
 	*ngroups = h[0];
-	*overflow = (h[1] & 0xFFFFFFFFull) != 0;
-	*fxfl |= f;
-	return PG_OK;
+	*overflow = h[1] != 0;
+	*fxfl |= (uint32_t) h[2];
+	return rc;
 }
 
 // Key range of rows 0, step, 2 step, ...: h[0], h[1] = min and max with the
@@ -776,8 +772,7 @@ static int gb_key_range(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, bool vec1
 	int rc;
 	unsigned long long* mm = nullptr;
 	if ((rc = pg_alloc_async(ctx, s, (void**) &mm, 32))) return rc;
-	const unsigned long long init[2] = {~0ull, 0ull};
-	PG_CUDA(ctx, cudaMemcpyAsync(mm, init, 16, cudaMemcpyHostToDevice, s));
+	PG_CUDA(ctx, cudaMemsetAsync(mm, 0, 16, s));
 	const uint64_t ns = pg_div_up(in->n, step);
 	const int blocks = (int) std::max<uint64_t>(1, std::min<uint64_t>(pg_div_up(ns, 256), (uint64_t) ctx->sm_count * 8));
 	if (vec16) k_gb_key_minmax<true><<<blocks, 256, 0, s>>>((const char*) in->data, in->n, in->width, in->key_off,
@@ -788,6 +783,7 @@ static int gb_key_range(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, bool vec1
 	PG_CUDA(ctx, cudaMemcpyAsync(h, mm, 16, cudaMemcpyDeviceToHost, s));
 	PG_CUDA(ctx, cudaStreamSynchronize(s));
 	pg_free_async(ctx, s, mm);
+	h[0] = ~h[0];
 	return PG_OK;
 }
 
@@ -817,7 +813,7 @@ static int gb_dense(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint32_t voff
 			if (!overflow) {
 				*done = true;
 				if (*ngroups > out_cap) return pg_fail(ctx, PG_ERR_OUTPUT_FULL, "pg_groupby: output capacity too small");
-				return pg_check_status(ctx, s, "pg_groupby");
+				return PG_OK;
 			}
 		}
 		// The sampled keys alone span too much: so do all.
@@ -832,7 +828,7 @@ static int gb_dense(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint32_t voff
 			fx, fxfl))) return rc;
 	*done = true;
 	if (*ngroups > out_cap) return pg_fail(ctx, PG_ERR_OUTPUT_FULL, "pg_groupby: output capacity too small");
-	return pg_check_status(ctx, s, "pg_groupby");
+	return PG_OK;
 }
 
 template <int VT, int AGG>
@@ -864,7 +860,6 @@ static int gb_run(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint32_t voff, 
 		unsigned long long* cursor = reinterpret_cast<unsigned long long*>(t.sentinel_used + 2);
 		PG_CUDA(ctx, cudaMemsetAsync(t.keys, 0xFF, (cap + 1) * 8, s));
 		PG_CUDA(ctx, cudaMemsetAsync(t.acc, 0, (cap + 1) * 8 * aw + 64, s));
-		unsigned int f = 0;
 		if (in->n && haskey) {
 			const bool few = groups <= GBH_FEW;
 			const uint32_t places = 1u << (few ? GBH_FEW_LOG2 : GBH_CACHE_LOG2), probes = few ? GBH_FEW_PROBES : 1;
@@ -883,21 +878,20 @@ static int gb_run(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint32_t voff, 
 			k_gb_single<VT, AGG><<<blocks, GB_THREADS, 0, s>>>((const char*) in->data, in->n, in->width, voff, t, fx);
 			PG_LAUNCHED(ctx);
 		}
-		rc = pg_check_status(ctx, s, "pg_groupby");
-		if (rc == PG_ERR_TABLE_FULL) { pg_free_async(ctx, s, mem); groups *= 4; continue; }
-		if (rc) { pg_free_async(ctx, s, mem); return rc; }
+		// The groups are written out before the table is known to have held them
+		// all; one that was full is enlarged and filled again.
 		int eblocks = (int) std::min<uint64_t>(pg_div_up(cap + 1, 256), (uint64_t) ctx->sm_count * 8);
 		if (haskey) k_gb_emit<VT, AGG, true><<<eblocks, 256, 0, s>>>(t, in->key_bytes, (char*) out, out_cap, cursor, 0, fx);
 		else k_gb_emit<VT, AGG, false><<<1, 32, 0, s>>>(t, 0, (char*) out, out_cap, cursor, in->n, fx);
 		PG_LAUNCHED(ctx);
-		unsigned long long ng = 0;
-		PG_CUDA(ctx, cudaMemcpyAsync(&ng, cursor, 8, cudaMemcpyDeviceToHost, s));
-		if (GB_DEC) PG_CUDA(ctx, cudaMemcpyAsync(&f, fx.p + 2, 4, cudaMemcpyDeviceToHost, s));
-		PG_CUDA(ctx, cudaStreamSynchronize(s));
+		unsigned long long h[2];
+		rc = pg_readback(ctx, s, cursor, 1, GB_DEC ? fx.p + 2 : nullptr, h, "pg_groupby");
 		pg_free_async(ctx, s, mem);
-		*ngroups = ng;
-		*fxfl |= f;
-		if (ng > out_cap) return pg_fail(ctx, PG_ERR_OUTPUT_FULL, "pg_groupby: output capacity too small");
+		if (rc == PG_ERR_TABLE_FULL) { groups *= 4; continue; }
+		if (rc) return rc;
+		*ngroups = h[0];
+		*fxfl |= (uint32_t) h[1];
+		if (h[0] > out_cap) return pg_fail(ctx, PG_ERR_OUTPUT_FULL, "pg_groupby: output capacity too small");
 		return PG_OK;
 	}
 	return pg_fail(ctx, PG_ERR_TABLE_FULL, "pg_groupby: group table kept overflowing");

@@ -3295,12 +3295,12 @@ extern "C" int pg_hashjoin_groupby(pg_ctx* ctx, pg_stream stream, pg_hashtable* 
 	const bool dec = agg == PG_AGG_SUM && val_type == PG_VAL_DEC;
 	char* mem = nullptr;
 	const uint64_t words = vrange * (dec ? PG_FX_WORDS : 1);
-	const size_t pres_end = (words + 1) * 8 + ((vrange + 15) & ~15ull);
+	const size_t pres_end = (words + 3) * 8 + ((vrange + 15) & ~15ull);
 	const size_t bytes = pres_end + 16;
 	if ((rc = pg_alloc_async(ctx, s, (void**) &mem, bytes))) return rc;
 	unsigned long long* acc = reinterpret_cast<unsigned long long*>(mem);   // a dec sum: word k of group g at acc[g + k vrange]
 	unsigned long long* cursor = acc + words;
-	unsigned char* present = reinterpret_cast<unsigned char*>(cursor + 1);
+	unsigned char* present = reinterpret_cast<unsigned char*>(cursor + 3);     // two words of pg_readback between
 	PgFx fx = {reinterpret_cast<int*>(mem + pres_end)};
 	// A dec sum's unit: the probe column's largest exponent, from every 1024th
 	// tuple (4x margin) on large inputs; redone exactly if a value lies above.
@@ -3324,11 +3324,13 @@ extern "C" int pg_hashjoin_groupby(pg_ctx* ctx, pg_stream stream, pg_hashtable* 
 		}
 		if ((rc = pg_dense_groups_emit(ctx, s, acc, fx, present, vrange, (long long) ht->vlo, gbytes, val_type, agg,
 				out, out_capacity, cursor))) return rc;
-		unsigned long long ng = 0;
-		unsigned int fl = 0;
-		PG_CUDA(ctx, cudaMemcpyAsync(&ng, cursor, 8, cudaMemcpyDeviceToHost, s));
-		if (dec) PG_CUDA(ctx, cudaMemcpyAsync(&fl, fx.p + 2, 4, cudaMemcpyDeviceToHost, s));
-		if ((rc = pg_check_status(ctx, s, "pg_hashjoin_groupby"))) return rc;
+		unsigned long long h[2];
+		if ((rc = pg_readback(ctx, s, cursor, 1, dec ? fx.p + 2 : nullptr, h, "pg_hashjoin_groupby"))) {
+			pg_free_async(ctx, s, mem);
+			return rc;
+		}
+		const unsigned long long ng = h[0];
+		const unsigned int fl = (unsigned int) h[1];
 		*ngroups = ng;
 		if ((fl & PG_FX_RANGE) && pass == 0) continue;
 		pg_free_async(ctx, s, mem);

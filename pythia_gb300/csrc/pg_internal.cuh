@@ -53,6 +53,13 @@ int pg_check_status(pg_ctx* ctx, cudaStream_t s, const char* what);
 // Clears a non-zero status `st` read back by the caller and reports it.
 int pg_status_fail(pg_ctx* ctx, cudaStream_t s, int st, const char* what);
 
+// A call's n result words (at most 13) at `dev` in one copy, host[0..n), with
+// host[n] = *flag (0 without one), and the status word as the return code; two
+// spare words follow the results. A copy of a few bytes costs the host about as
+// much as a launch and a half, and these calls made three or four.
+int pg_readback(pg_ctx* ctx, cudaStream_t s, unsigned long long* dev, int n, const int* flag, unsigned long long* host,
+		const char* what);
+
 // ---------------------------------------------------------------------------
 // Bucket functions (hash.h:51-479) in the form their constructors leave them.
 // ---------------------------------------------------------------------------

@@ -280,8 +280,8 @@ static int mj_runs(pg_ctx* ctx, cudaStream_t s, const pg_rec* rec, uint64_t n, u
 	return PG_OK;
 }
 
-// Key range of tuples 0, step, 2 step, ... into mm[0..1] (keys ^ 2^63 as
-// unsigned); with `unsorted` (step 1), also whether some key is greater than
+// Key range of tuples 0, step, 2 step, ... (keys ^ 2^63 as unsigned) into mm =
+// [~smallest, largest], zero before; with `unsorted` (step 1), also whether some key is greater than
 // the next one.
 __global__ void k_mj_minmax(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, uint32_t kbytes,
 		uint64_t step, unsigned long long* __restrict__ mm, unsigned long long* __restrict__ unsorted)
@@ -303,7 +303,7 @@ __global__ void k_mj_minmax(const char* __restrict__ in, uint64_t n, uint32_t W,
 		lo = a < lo ? a : lo;
 		hi = b > hi ? b : hi;
 	}
-	if ((threadIdx.x & 31) == 0) { atomicMin(&mm[0], lo); atomicMax(&mm[1], hi); }
+	if ((threadIdx.x & 31) == 0) { atomicMax(&mm[0], ~lo); atomicMax(&mm[1], hi); }
 }
 
 
@@ -376,7 +376,8 @@ __device__ __forceinline__ unsigned long long mj_ld64(const unsigned long long* 
 // cnt[key - kmin] += 1 for every tuple; a key outside the window sets *outside.
 // Lanes that hold lane 0's key add once together when there are several of
 // them, so that one key with most of the rows does not queue 32 adds a warp.
-// VALS: also the range of the packed build values, into vmm[0..1].
+// VALS: also the range of the packed build values, into vmm = [~smallest, largest],
+// zero before.
 template <bool V16, bool VALS>
 __global__ void __launch_bounds__(256)
 k_mj_count(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, uint32_t kbytes, long long kmin,
@@ -424,7 +425,7 @@ k_mj_count(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, u
 		__syncthreads();
 		if (threadIdx.x == 0) {
 			for (int w = 1; w < 8; ++w) { vlo = min(vlo, red[0][w]); vhi = max(vhi, red[1][w]); }
-			atomicMin(&vmm[0], vlo);
+			atomicMax(&vmm[0], ~vlo);
 			atomicMax(&vmm[1], vhi);
 		}
 	}
@@ -556,7 +557,7 @@ k_mj_fill(const char* __restrict__ R, uint64_t n, uint32_t koff, long long kmin,
 		const unsigned long long* __restrict__ vmm)
 {
 	if (meta[0] > MJ_MAX_RUN || meta[1]) return;
-	const unsigned long long vmin = vmm[0];
+	const unsigned long long vmin = ~vmm[0];
 	const bool narrow = vmm[1] - vmin < (1ull << 32);
 	const uint64_t stride = (uint64_t) gridDim.x * blockDim.x, pol = pg_policy_evict_first();
 	for (uint64_t base = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; base < n; base += stride * 4) {
@@ -596,7 +597,7 @@ k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin,
 		const unsigned long long* __restrict__ vmm)
 {
 	if (meta[0] > MJ_MAX_RUN || meta[1]) return;
-	const unsigned long long vmin = vmm[0];
+	const unsigned long long vmin = ~vmm[0];
 	const bool narrow = vmm[1] - vmin < (1ull << 32);
 	const uint32_t lane = threadIdx.x & 31;
 	const uint64_t pol = pg_policy_evict_first(), keep = pg_policy_keep(4);
@@ -730,22 +731,23 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 	const bool count_build = materialize || (sum_col >= 0 ? !sum_build : R->n <= S->n);
 	const pg_rel *C = count_build ? R : S, *P = count_build ? S : R;
 	int rc;
-	// [key min, key max], [rows, sum], [largest count, key outside], [value min, value max]
+	// [~key min, key max], [rows, sum], [largest count, key outside], two words of
+	// pg_readback, [~value min, value max]
 	unsigned long long* mm = nullptr;
-	if ((rc = pg_alloc_async(ctx, s, (void**) &mm, 64))) return rc;
+	if ((rc = pg_alloc_async(ctx, s, (void**) &mm, 72))) return rc;
 	unsigned long long* agg = mm + 2;
 	unsigned int* meta = reinterpret_cast<unsigned int*>(mm + 4);
-	unsigned long long* vmm = mm + 5;
+	unsigned long long* vmm = mm + 7;
 	for (int attempt = C->n >= (1ull << 22) ? 0 : 1; attempt < 2; ++attempt) {
 		const uint64_t step = attempt == 0 ? 1024 : 1;
-		const unsigned long long init[7] = {~0ull, 0ull, 0ull, 0ull, 0ull, ~0ull, 0ull};
-		PG_CUDA(ctx, cudaMemcpyAsync(mm, init, sizeof init, cudaMemcpyHostToDevice, s));
+		PG_CUDA(ctx, cudaMemsetAsync(mm, 0, 72, s));
 		const int mblocks = (int) std::min<uint64_t>(pg_div_up(pg_div_up(C->n, step), 256), (uint64_t) ctx->sm_count * 8);
 		k_mj_minmax<<<mblocks, 256, 0, s>>>((const char*) C->data, C->n, C->width, C->key_off, C->key_bytes, step, mm, nullptr);
 		PG_LAUNCHED(ctx);
 		unsigned long long h[4];
 		PG_CUDA(ctx, cudaMemcpyAsync(h, mm, 16, cudaMemcpyDeviceToHost, s));
 		PG_CUDA(ctx, cudaStreamSynchronize(s));
+		h[0] = ~h[0];
 		if (step > 1) {
 			const unsigned long long slack = (h[1] - h[0]) / 64 + 64;
 			h[0] = h[0] > slack ? h[0] - slack : 0;
@@ -795,9 +797,8 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 					reinterpret_cast<uint4*>(out), out_capacity, agg, meta, vmm);
 			PG_LAUNCHED(ctx);
 		}
-		unsigned long long o[3];     // rows, sum, (largest count, key outside)
-		PG_CUDA(ctx, cudaMemcpyAsync(o, agg, 24, cudaMemcpyDeviceToHost, s));
-		rc = pg_check_status(ctx, s, "pg_mpsm_join");
+		unsigned long long o[4];     // rows, sum, (largest count, key outside)
+		rc = pg_readback(ctx, s, agg, 3, nullptr, o, "pg_mpsm_join");
 		release();
 		if (rc) { pg_free_async(ctx, s, mm); return rc; }
 		if (o[2] >> 32) continue;                                         // the sample missed a key
@@ -819,8 +820,7 @@ static int mj_confirm_sorted(pg_ctx* ctx, cudaStream_t s, const pg_rel* r, bool*
 	int rc;
 	unsigned long long* mm = nullptr;
 	if ((rc = pg_alloc_async(ctx, s, (void**) &mm, 32))) return rc;
-	const unsigned long long init[3] = {~0ull, 0ull, 0ull};
-	PG_CUDA(ctx, cudaMemcpyAsync(mm, init, sizeof init, cudaMemcpyHostToDevice, s));
+	PG_CUDA(ctx, cudaMemsetAsync(mm, 0, 32, s));
 	const int blocks = (int) std::min<uint64_t>(pg_div_up(r->n, 256), (uint64_t) ctx->sm_count * 8);
 	k_mj_minmax<<<blocks, 256, 0, s>>>((const char*) r->data, r->n, r->width, r->key_off, r->key_bytes, 1, mm, mm + 2);
 	PG_LAUNCHED(ctx);

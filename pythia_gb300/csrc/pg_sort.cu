@@ -198,7 +198,7 @@ __global__ void k_sort_minmax(const char* __restrict__ in, uint64_t n, uint32_t 
 		lo = a < lo ? a : lo;
 		hi = b > hi ? b : hi;
 	}
-	if ((threadIdx.x & 31) == 0) { atomicMin(&mm[0], lo); atomicMax(&mm[1], hi); }
+	if ((threadIdx.x & 31) == 0) { atomicMax(&mm[0], ~lo); atomicMax(&mm[1], hi); }      // zero before
 }
 
 // (key, other half) or (key, row index) records for layouts other than a
@@ -227,14 +227,14 @@ static int sort_key_range(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint64_
 	int rc;
 	unsigned long long* mm = nullptr;
 	if ((rc = pg_alloc_async(ctx, s, (void**) &mm, 16))) return rc;
-	const unsigned long long init[2] = {~0ull, 0ull};
-	PG_CUDA(ctx, cudaMemcpyAsync(mm, init, 16, cudaMemcpyHostToDevice, s));
+	PG_CUDA(ctx, cudaMemsetAsync(mm, 0, 16, s));
 	const int blocks = (int) std::min<uint64_t>(pg_div_up(pg_div_up(in->n, step), 256), (uint64_t) ctx->sm_count * 8);
 	k_sort_minmax<<<blocks, 256, 0, s>>>((const char*) in->data, in->n, in->width, in->key_off, in->key_bytes, step, mm);
 	PG_LAUNCHED(ctx);
 	PG_CUDA(ctx, cudaMemcpyAsync(h, mm, 16, cudaMemcpyDeviceToHost, s));
 	PG_CUDA(ctx, cudaStreamSynchronize(s));
 	pg_free_async(ctx, s, mm);
+	h[0] = ~h[0];
 	return PG_OK;
 }
 
