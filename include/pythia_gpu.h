@@ -165,10 +165,10 @@ enum {
 	                                    tables staged through shared memory where the width allows, everything
 	                                    else per-thread loads; 1 per-thread loads; 2 staged, 4 lookups per
 	                                    thread; 3 staged, 2 lookups per thread */
-	PG_TUNE_BUILD_SPEC = 11,         /* narrow dense build of 16-byte tuples: 0 on the device alone for up to 8192
-	                                    tuples (one launch) and from 65,536 (key window from a sample), checked by
-	                                    the table's first use; 1 from a sample at every size; 2 exact key range
-	                                    read back to the host first */
+	PG_TUNE_BUILD_SPEC = 11,         /* narrow dense build of 16-byte tuples: 0 on the device alone, up to 2^20 tuples
+	                                    exactly in one cooperative launch, larger from a sample, checked by the
+	                                    table's first use; 1 from a sample at every size; 2 exact key range read
+	                                    back to the host first */
 	PG_TUNE_SPIN_LIMIT = 12,         /* polls a device-side wait for a bulk copy makes before the call fails with
 	                                    PG_ERR_TIMEOUT (the copy is still waited for, so the kernel ends
 	                                    cleanly): 0 the built-in limit (2^26 blocking polls), else that many

@@ -329,7 +329,6 @@ __global__ void k_dense32_count(const uint32_t* __restrict__ table, uint64_t ran
 // exactly. Four launches: sample, fill, store, count.
 // ---------------------------------------------------------------------------
 #define HJ_SPEC_SAMPLE 4096
-#define HJ_SPEC_MIN_TUPLES 65536
 
 __device__ __forceinline__ void hj_minmax4(unsigned long long& lo, unsigned long long& hi, unsigned long long& vlo,
 		unsigned long long& vhi)
@@ -396,103 +395,124 @@ __global__ void __launch_bounds__(1024) k_dense_prep16(const uint4* __restrict__
 	*hdr = h;
 }
 
-// The same for few tuples in one launch of one CTA, exactly: ranges over every
-// tuple, window, fill, store and count, with block barriers where the form for
-// large inputs has launches, and where no dense layout fits (keys too far apart or
-// repeated) the hashed table, which the first use then finds ready. Joins of 1000
-// tuples with 10,000: dense keys 73 -> 41 us, far ones 106 -> 74; of 8000 with 50,000:
-// 80 -> 44 and 112 -> 106. From 16,000 tuples far apart one SM's random atomics take
-// longer than the launches and round trips they save (111 -> 135).
-#define HJ_SMALL_TUPLES 8192
-__global__ void __launch_bounds__(1024) k_dense_small16(const uint4* __restrict__ R, uint32_t n, uint32_t kw,
+// The same for smaller inputs in one cooperative launch, exactly: ranges over
+// every tuple, window, fill, store and count, with grid barriers where the form
+// for large inputs has launches, and where no dense layout fits (keys too far apart
+// or repeated) the hashed table, which the first use then finds ready. One block
+// per 2048 tuples (a single one's barriers are block barriers). Whole joins of
+// 1000 tuples with 10,000: dense keys 73 -> 42 us, far ones 107 -> 78; of 16,000 with
+// 100,000: 84 -> 48 and 112 -> 90 (exact ranges and duplicate counts read back by the
+// host before). From 65,536 tuples the sampled form, used there before, takes as
+// long for dense keys (140,000 with 800,000: 58 us) and longer for far ones (167,
+// now 87), up to 2^20: the spare hashed slots are 32 MB then.
+#define HJ_SMALL_PER_BLOCK 2048
+#define HJ_SMALL_TUPLES (1u << 20)
+
+// What the blocks of k_build_small gather, zero before (G > 1).
+struct HjSmallShared {
+	unsigned long long nkmin, kmax, nvmin, vmax;     // ~smallest and largest key (^ 2^63) and value
+	unsigned long long present;
+	unsigned int marker, dup;
+	unsigned int lost;                               // a block gave up on a barrier
+	unsigned int bar;
+};
+
+__global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict__ R, uint32_t n, uint32_t kw,
 		uint32_t pk, uint64_t cap, uint32_t* __restrict__ table, unsigned long long* __restrict__ slots, uint32_t log2cap,
-		HjDenseHdr* __restrict__ hdr)
+		HjDenseHdr* __restrict__ hdr, HjSmallShared* g, int* __restrict__ status)
 {
 	__shared__ unsigned long long red[4][32];
-	__shared__ HjDenseHdr h;
+	__shared__ HjSmallShared mine;
 	const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	const uint32_t first = blockIdx.x * 1024 + tid, stride = gridDim.x * 1024;
+	const bool alone = gridDim.x == 1;
+	const uint32_t spin = pg_spin_knob(status);
+	uint32_t epoch = 0;
+	bool dead = false;
+	HjSmallShared* const acc = alone ? &mine : g;
+	if (alone && tid == 0) mine = HjSmallShared{0, 0, 0, 0, 0, 0, 0, 0, 0};
+	auto meet = [&]() {
+		pg_grid_sync(&g->bar, epoch, dead, spin, status);
+		if (dead) atomicOr(&acc->lost, 1u);          // before this block's next arrival
+	};
+	auto key_of = [&](const uint4& v) { return ((unsigned long long) hj_word4(v, kw + 1) << 32) | hj_word4(v, kw); };
 	unsigned long long lo = ~0ull, hi = 0, vlo = ~0ull, vhi = 0;
-	#pragma unroll 8
-	for (uint32_t i = tid; i < n; i += 1024) {
+	int marker = 0;
+	#pragma unroll 4
+	for (uint32_t i = first; i < n; i += stride) {
 		const uint4 v = __ldg(R + i);
-		const unsigned long long k = (((unsigned long long) hj_word4(v, kw + 1) << 32) | hj_word4(v, kw)) ^ (1ull << 63);
-		const unsigned long long p = hj_pack16(v, pk);
-		lo = k < lo ? k : lo; hi = k > hi ? k : hi;
+		const unsigned long long k = key_of(v), u = k ^ (1ull << 63), p = hj_pack16(v, pk);
+		lo = u < lo ? u : lo; hi = u > hi ? u : hi;
 		vlo = p < vlo ? p : vlo; vhi = p > vhi ? p : vhi;
+		marker |= k == (unsigned long long) PG_EMPTY_KEY;
 	}
 	hj_minmax4(lo, hi, vlo, vhi);
 	if (lane == 0) { red[0][warp] = lo; red[1][warp] = hi; red[2][warp] = vlo; red[3][warp] = vhi; }
-	__syncthreads();
+	marker = __syncthreads_or(marker);
 	if (warp == 0) {
 		lo = red[0][lane]; hi = red[1][lane]; vlo = red[2][lane]; vhi = red[3][lane];
 		hj_minmax4(lo, hi, vlo, vhi);
 		if (lane == 0) {
-			const bool wide = hi - lo >= (2 * (uint64_t) n > 64 ? 2 * (uint64_t) n : 64) || hi - lo >= cap;
-			h.n = n; h.present = 0; h.kmin = lo; h.kmax = hi; h.vlo = vlo; h.vhi = vhi; h.pad = 0;
-			h.dmin = (long long) (lo ^ (1ull << 63));
-			h.vmin = vlo;
-			h.flags = wide ? 4 | 8 : vhi - vlo >= 0xFFFFFFFFull ? 4 : 0;
-			h.drange = h.flags ? 0 : hi - lo + 1;
+			atomicMax(&acc->nkmin, ~lo); atomicMax(&acc->kmax, hi);
+			atomicMax(&acc->nvmin, ~vlo); atomicMax(&acc->vmax, vhi);
+			if (marker) atomicOr(&acc->marker, 1u);
 		}
 	}
-	__syncthreads();
-	bool dense = h.flags == 0;
-	if (dense) {
+	meet();
+	volatile HjSmallShared* const va = acc;
+	HjDenseHdr h;
+	h.n = n; h.present = 0; h.kmin = ~va->nkmin; h.kmax = va->kmax; h.vlo = ~va->nvmin; h.vhi = va->vmax; h.pad = 0;
+	h.dmin = (long long) (h.kmin ^ (1ull << 63));
+	h.vmin = h.vlo;
+	const unsigned long long span = h.kmax - h.kmin;
+	const bool wide = span >= (2 * (uint64_t) n > 64 ? 2 * (uint64_t) n : 64) || span >= cap;
+	h.flags = wide ? 4 | 8 : h.vhi - h.vlo >= 0xFFFFFFFFull ? 4 : 0;
+	h.drange = h.flags ? 0 : span + 1;
+	if (h.flags == 0) {
 		const uint32_t range = (uint32_t) h.drange;
-		for (uint32_t i = tid; i < (range + 3) / 4; i += 1024)
+		for (uint32_t i = first; i < (range + 3) / 4; i += stride)
 			reinterpret_cast<uint4*>(table)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
-		__syncthreads();
+		meet();
 		#pragma unroll 4
-		for (uint32_t i = tid; i < n; i += 1024) {
+		for (uint32_t i = first; i < n; i += stride) {
 			const uint4 v = __ldg(R + i);
-			const unsigned long long k = ((unsigned long long) hj_word4(v, kw + 1) << 32) | hj_word4(v, kw);
-			table[k - (unsigned long long) h.dmin] = (uint32_t) (hj_pack16(v, pk) - h.vmin);
+			const unsigned long long d = key_of(v) - (unsigned long long) h.dmin;
+			if (d < range) table[d] = (uint32_t) (hj_pack16(v, pk) - h.vmin);
 		}
-		__syncthreads();
+		meet();
 		uint32_t c = 0;
-		for (uint32_t i = tid; i < range; i += 1024) c += *(volatile uint32_t*) (table + i) != 0xFFFFFFFFu;
+		for (uint32_t i = first; i < range; i += stride) c += __ldcg(table + i) != 0xFFFFFFFFu;
 		c = __reduce_add_sync(0xffffffffu, c);
-		if (lane == 0) red[0][warp] = c;
-		__syncthreads();
-		if (tid == 0) {
-			unsigned long long t = 0;
-			for (int w = 0; w < 32; ++w) t += red[0][w];
-			h.present = t;
-		}
-		__syncthreads();
-		dense = h.present == n;
+		if (lane == 0 && c) atomicAdd(&acc->present, (unsigned long long) c);
+		meet();
+		h.present = va->present;
 	}
-	// Wide values keep a dense layout of their own, made by the exact build;
-	// so do keys equal to the empty marker, with their side list.
-	if (!dense && (h.flags == 0 || (h.flags & 8)) && h.kmin <= ((1ull << 63) - 1) && h.kmax >= ((1ull << 63) - 1)) {
-		int marker = 0;
-		for (uint32_t i = tid; i < n; i += 1024) {
-			const uint4 v = __ldg(R + i);
-			marker |= (hj_word4(v, kw + 1) & hj_word4(v, kw)) == ~0u;
-		}
-		if (__syncthreads_or(marker)) {
-			if (tid == 0) *hdr = h;
-			return;
-		}
-	}
-	if (!dense && (h.flags == 0 || (h.flags & 8))) {
+	// The hashed table, unless the tuples have a dense layout (of wide values: by
+	// the exact build) or a key equal to the empty marker (the exact build's list).
+	if (h.flags != 4 && h.present != n && !va->marker) {
 		const uint32_t mask = (1u << log2cap) - 1;
-		for (uint32_t i = tid; i <= mask; i += 1024) reinterpret_cast<uint4*>(slots)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
-		__syncthreads();
-		int dup = 0;
-		for (uint32_t i = tid; i < n; i += 1024) {
+		for (uint32_t i = first; i <= mask; i += stride) reinterpret_cast<uint4*>(slots)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+		meet();
+		bool dup = false;
+		for (uint32_t i = first; i < n; i += stride) {
 			const uint4 v = __ldg(R + i);
-			const unsigned long long k = ((unsigned long long) hj_word4(v, kw + 1) << 32) | hj_word4(v, kw);
-			for (uint32_t s = (uint32_t) hj_slot0((int64_t) k, log2cap);; s = (s + 1) & mask) {   // at most half full
+			const unsigned long long k = key_of(v);
+			uint32_t s = (uint32_t) hj_slot0((int64_t) k, log2cap);
+			for (uint32_t tries = 0; tries <= mask; ++tries, s = (s + 1) & mask) {       // at most half full
 				const unsigned long long old = atomicCAS(&slots[2 * (uint64_t) s], (unsigned long long) PG_EMPTY_KEY, k);
 				if (old == (unsigned long long) PG_EMPTY_KEY) { slots[2 * (uint64_t) s + 1] = hj_pack16(v, pk); break; }
-				if (old == k) dup = 1;
+				if (old == k) dup = true;
 			}
 		}
-		dup = __syncthreads_or(dup);
-		if (tid == 0) h.flags |= 16 | (dup ? 32 : 0);
+		if (dup) atomicOr(&acc->dup, 1u);
+		meet();
+		h.flags |= 16 | (va->dup ? 32 : 0);
 	}
-	if (tid == 0) *hdr = h;
+	// Past a lost barrier (the status says so) neither layout can be trusted.
+	if (blockIdx.x == 0 && tid == 0) {
+		if (va->lost) h.flags = 4;
+		*hdr = h;
+	}
 }
 
 // All ones over the window's entries (nothing when the sample ruled it out).
@@ -2309,7 +2329,7 @@ static int hj_build_spec(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, pg_hashta
 	ht->slots = nullptr; ht->side = nullptr; ht->nside = 0; ht->log2cap = 1; ht->capacity = 0;
 	ht->dense_val = nullptr; ht->dense_bits = nullptr;
 	ht->hdr = nullptr; ht->dense32_base = nullptr; ht->dense32 = nullptr;
-	if ((rc = pg_alloc_async(ctx, s, (void**) &ht->hdr, sizeof(HjDenseHdr)))) return rc;
+	if ((rc = pg_alloc_async(ctx, s, (void**) &ht->hdr, sizeof(HjDenseHdr) + sizeof(HjSmallShared)))) return rc;
 	if ((rc = pg_alloc_async(ctx, s, (void**) &ht->dense32_base, cap * 4))) return rc;
 	ht->dense32 = ht->dense32_base;
 	ht->dmin = 0; ht->drange = cap; ht->vmin = 0; ht->vlo = 0; ht->vmax = 0;     // bounds until settled
@@ -2323,11 +2343,23 @@ static int hj_build_spec(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, pg_hashta
 		ht->spec.store(true, std::memory_order_release);
 		return PG_OK;
 	};
-	if (R->n <= HJ_SMALL_TUPLES && ctx->tune[PG_TUNE_BUILD_SPEC] != 1) {
+	// Where the spare slots do not fit in memory the sampled form does without.
+	bool small = R->n <= HJ_SMALL_TUPLES && ctx->tune[PG_TUNE_BUILD_SPEC] != 1;
+	if (small && pg_alloc_async(ctx, s, (void**) &ht->small_slots, 16ull << hj_log2cap(R->n)) != PG_OK) {
+		cudaGetLastError();
+		ht->small_slots = nullptr;
+		small = false;
+	}
+	if (small) {
 		ht->log2cap = hj_log2cap(R->n);
-		if ((rc = pg_alloc_async(ctx, s, (void**) &ht->small_slots, 16ull << ht->log2cap))) return rc;
-		k_dense_small16<<<1, 1024, 0, s>>>((const uint4*) R->data, (uint32_t) R->n, kw, pk, cap, ht->dense32_base,
-				ht->small_slots, ht->log2cap, ht->hdr);
+		uint32_t G = (uint32_t) std::min<uint64_t>(pg_div_up(R->n, HJ_SMALL_PER_BLOCK), ctx->sm_count);
+		HjSmallShared* g = reinterpret_cast<HjSmallShared*>(ht->hdr + 1);
+		if (G > 1) PG_CUDA(ctx, cudaMemsetAsync(g, 0, sizeof(HjSmallShared), s));
+		const uint4* rd = (const uint4*) R->data;
+		uint32_t n = (uint32_t) R->n, kww = kw, pkk = pk, lg = ht->log2cap;
+		uint64_t capp = cap;
+		void* args[] = {&rd, &n, &kww, &pkk, &capp, &ht->dense32_base, &ht->small_slots, &lg, &ht->hdr, &g, &ctx->d_status};
+		PG_CUDA(ctx, cudaLaunchCooperativeKernel((void*) k_build_small, dim3(G), dim3(1024), args, 0, s));
 		PG_LAUNCHED(ctx);
 		return built();
 	}
@@ -2363,6 +2395,10 @@ static int hj_settle_known(pg_ctx* ctx, pg_hashtable* ht, const unsigned long lo
 	} else {
 		PG_CUDA(ctx, cudaMemcpyAsync(&h, ht->hdr, sizeof h, cudaMemcpyDeviceToHost, s));
 		PG_CUDA(ctx, cudaStreamSynchronize(s));
+	}
+	if (!(h.flags & 16)) {       // spare slots that no probe will read
+		pg_free_async(ctx, s, ht->small_slots);
+		ht->small_slots = nullptr;
 	}
 	if (hj_hdr_ok(h)) {
 		// Exact layout, as hj_build_exact would have made it: the window
@@ -2443,8 +2479,7 @@ extern "C" int pg_hashjoin_build(pg_ctx* ctx, pg_stream stream, const pg_rel* R,
 	ht->spec.store(false); ht->hdr = nullptr; ht->dense32_base = nullptr; ht->dense32_copy = nullptr;
 	ht->built = nullptr; ht->small_slots = nullptr;
 	const int64_t spec = ctx->tune[PG_TUNE_BUILD_SPEC];
-	if (R->n && ht->inline_val && ctx->tune[PG_TUNE_DENSE] != 2 && spec != 2 && hj_vec16(R, ht->bcols) &&
-			(spec == 1 || R->n >= HJ_SPEC_MIN_TUPLES || R->n <= HJ_SMALL_TUPLES))
+	if (R->n && ht->inline_val && ctx->tune[PG_TUNE_DENSE] != 2 && spec != 2 && hj_vec16(R, ht->bcols))
 		rc = hj_build_spec(ctx, s, R, ht);
 	else
 		rc = hj_build_exact(ctx, s, R, ht, false);

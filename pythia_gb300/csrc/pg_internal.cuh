@@ -406,6 +406,31 @@ __device__ __forceinline__ void pg_st_relaxed(uint32_t* p, uint32_t v)
 	asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
 }
 
+#define PG_GRID_SPIN_LIMIT (1u << 22)
+// All blocks of the cooperative launch meet; what they stored before is
+// visible after. Bounded: past the limit the status records PG_ERR_TIMEOUT and
+// this block no longer waits, so callers keep every access in bounds whatever the
+// others have done.
+__device__ __forceinline__ void pg_grid_sync(uint32_t* bar, uint32_t& epoch, bool& dead, uint32_t spin, int* status)
+{
+	__syncthreads();
+	++epoch;
+	if (gridDim.x > 1 && threadIdx.x == 0) {
+		__threadfence();
+		atomicAdd(bar, 1u);
+		for (uint32_t polls = 0; !dead;) {
+			uint32_t v;
+			asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+			if (v >= epoch * gridDim.x) break;
+			++polls;
+			if (polls == (spin ? spin : PG_GRID_SPIN_LIMIT)) pg_set_status(status, PG_ERR_TIMEOUT);
+			if (polls >= PG_GRID_SPIN_LIMIT) { pg_set_status(status, PG_ERR_TIMEOUT); dead = true; }
+		}
+		__threadfence();
+	}
+	__syncthreads();
+}
+
 __host__ __device__ __forceinline__ uint64_t pg_div_up(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 __host__ __device__ __forceinline__ uint64_t pg_min64(uint64_t a, uint64_t b) { return a < b ? a : b; }
 __host__ __device__ __forceinline__ uint32_t pg_min32(uint32_t a, uint32_t b) { return a < b ? a : b; }

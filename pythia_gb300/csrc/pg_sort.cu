@@ -254,31 +254,6 @@ static int bits_of(unsigned long long x) { return x == 0 ? 0 : 64 - __builtin_cl
 #define SS_THREADS 1024
 #define SS_WARPS (SS_THREADS / 32)
 #define SS_MAX_ROWS (1u << 20)
-#define SS_SPIN_LIMIT (1u << 22)
-
-// All blocks of the cooperative launch meet; what they stored before is
-// visible after. Bounded: past the limit the status records PG_ERR_TIMEOUT and
-// this block no longer waits (every access below stays in bounds whatever the
-// others have done).
-__device__ __forceinline__ void ss_grid_sync(uint32_t* bar, uint32_t& epoch, bool& dead, uint32_t spin, int* status)
-{
-	__syncthreads();
-	++epoch;
-	if (gridDim.x > 1 && threadIdx.x == 0) {
-		__threadfence();
-		atomicAdd(bar, 1u);
-		for (uint32_t polls = 0; !dead;) {
-			uint32_t v;
-			asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-			if (v >= epoch * gridDim.x) break;
-			++polls;
-			if (polls == (spin ? spin : SS_SPIN_LIMIT)) pg_set_status(status, PG_ERR_TIMEOUT);
-			if (polls >= SS_SPIN_LIMIT) { pg_set_status(status, PG_ERR_TIMEOUT); dead = true; }
-		}
-		__threadfence();
-	}
-	__syncthreads();
-}
 
 __device__ __forceinline__ unsigned long long ss_key(const uint4& t, uint32_t kw, uint32_t kbytes)
 {
@@ -329,7 +304,7 @@ k_sort_small(const uint4* __restrict__ in, uint32_t n, uint32_t kw, uint32_t kby
 	}
 	if (G > 1) {
 		if (tid == 0) { atomicMax(&mm[0], ~lo); atomicMax(&mm[1], hi); }
-		ss_grid_sync(bar, epoch, dead, spin, status);
+		pg_grid_sync(bar, epoch, dead, spin, status);
 		lo = ~pg_ld_relaxed(mm);
 		hi = pg_ld_relaxed(mm + 1);
 	}
@@ -383,7 +358,7 @@ k_sort_small(const uint4* __restrict__ in, uint32_t n, uint32_t kw, uint32_t kby
 		}
 		uint32_t total = 0, before = 0;
 		if (G > 1) {
-			ss_grid_sync(bar, epoch, dead, spin, status);
+			pg_grid_sync(bar, epoch, dead, spin, status);
 			#pragma unroll 8
 			for (uint32_t k = q; k < G; k += 4) {
 				const uint32_t x = __ldcg(counts + k * 256 + b);
@@ -418,7 +393,7 @@ k_sort_small(const uint4* __restrict__ in, uint32_t n, uint32_t kw, uint32_t kby
 			if (row < n) __stcg(dst + row, t[j]);
 		}
 		if (p + 1 == passes) return;
-		ss_grid_sync(bar, epoch, dead, spin, status);
+		pg_grid_sync(bar, epoch, dead, spin, status);
 		#pragma unroll
 		for (int j = 0; j < ITEMS; ++j)
 			if (r0 + j * 32 < n) t[j] = __ldcg(dst + r0 + j * 32);

@@ -159,11 +159,14 @@ def _same_join(ctx, R, S, **kw):
         assert (n2, s2) == orc.hashjoin(R, S, materialise=False, sum_col=sc, hash=orc.hashcfg("modulo", 1 << 12), **kw)[1:]
 
 
-# Builds of up to 8192 tuples are one launch, which makes either layout: dense,
-# or hashed for keys too far apart or repeated; wide values and the empty-marker
-# key (-1) beside far keys go back to the exact build.
-@pytest.mark.parametrize("n", [1, 2, 33, 1024, 1025, 8192, 8193])
-@pytest.mark.parametrize("case", ["dense", "far", "repeated", "far_repeated", "marker", "marker_far", "wide_values", "extremes"])
+# Builds of up to 2^20 tuples are one cooperative launch of a block per 2048, which
+# makes either layout: dense, or hashed for keys too far apart or repeated; wide
+# values and the empty-marker key (-1) beside far keys go back to the exact build.
+BUILDS = ["dense", "far", "repeated", "far_repeated", "marker", "marker_far", "wide_values", "extremes"]
+
+
+@pytest.mark.parametrize("n,case", [(n, c) for n in (1, 2, 33, 2048, 2049, 70_001) for c in BUILDS] +
+                         [(n, c) for n in (1 << 20, (1 << 20) + 1) for c in ("dense", "far")])
 def test_join_small_builds(ctx, n, case):
     R = dg.build_relation(n, dg.seed_for(207))
     S = dg.probe_uniform(3 * n + 5, R, dg.seed_for(208))
