@@ -359,6 +359,13 @@ __device__ __forceinline__ unsigned long long mj_packed(const uint4& t, const Mj
 }
 
 // Table loads, kept in L2 while the relations stream past.
+__device__ __forceinline__ uint32_t mj_ld16(const uint16_t* p, uint64_t pol)
+{
+	uint16_t v;
+	asm("ld.global.nc.L2::cache_hint.u16 %0, [%1], %2;" : "=h"(v) : "l"(p), "l"(pol));
+	return v;
+}
+
 __device__ __forceinline__ uint32_t mj_ld32(const uint32_t* p, uint64_t pol)
 {
 	uint32_t v;
@@ -544,13 +551,22 @@ k_mj_scan_apply(uint32_t* __restrict__ cnt, uint32_t range, const uint64_t* __re
 	}
 }
 
+// Bytes of a value slot: values that span less than 2^16 or 2^32 are kept as
+// differences from the smallest (vmm, from the counting pass). The scattered stores
+// and the probe's scattered reads then move fewer bytes and stay in L2 for more
+// tuples: 16M x 16M with four duplicates a key and values below 1000, 2 bytes
+// against 4: 245 -> 208 us the fill, 562 -> 522 the rows.
+__device__ __forceinline__ uint32_t mj_val_bytes(unsigned long long span)
+{
+	return span < (1u << 16) ? 2 : span < (1ull << 32) ? 4 : 8;
+}
+
 // Scatters the packed build columns into their keys' runs: pos[d] is run d's
-// first slot before and its end (the next run's start) after. Values that
-// span less than 2^32 are kept as 4-byte differences from the smallest (vmm,
-// from the counting pass): half the bytes that the scattered stores and the
-// probe's scattered reads move. Nothing is done
-// when a run is longer than MJ_MAX_RUN or a key lay outside the window
-// (meta[0], meta[1]).
+// first slot before and its end (the next run's start) after. One tuple a thread
+// in many blocks: each waits for its returning add (four a thread: 10 us more).
+// Nothing is done when a run is longer than MJ_MAX_RUN or a key lay outside the
+// window (meta[0], meta[1]).
+#define MJ_FILL_BLOCKS_PER_SM 64
 __global__ void __launch_bounds__(256)
 k_mj_fill(const char* __restrict__ R, uint64_t n, uint32_t koff, long long kmin, uint32_t range, MjPack bp,
 		uint32_t* __restrict__ pos, unsigned long long* __restrict__ val, const unsigned int* __restrict__ meta,
@@ -558,39 +574,33 @@ k_mj_fill(const char* __restrict__ R, uint64_t n, uint32_t koff, long long kmin,
 {
 	if (meta[0] > MJ_MAX_RUN || meta[1]) return;
 	const unsigned long long vmin = ~vmm[0];
-	const bool narrow = vmm[1] - vmin < (1ull << 32);
+	const uint32_t bytes = mj_val_bytes(vmm[1] - vmin);
 	const uint64_t stride = (uint64_t) gridDim.x * blockDim.x, pol = pg_policy_evict_first();
-	for (uint64_t base = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; base < n; base += stride * 4) {
-		uint4 t[4];
-		uint32_t at[4];
-		#pragma unroll
-		for (int j = 0; j < 4; ++j) {
-			const uint64_t i = base + j * stride;
-			at[j] = 0xFFFFFFFFu;
-			if (i < n) {
-				const uint64_t x = (uint64_t) mj_key<true>(R, i, 16, koff, 8, pol, t[j]) - (uint64_t) kmin;
-				at[j] = (uint32_t) x;
-			}
-		}
-		#pragma unroll
-		for (int j = 0; j < 4; ++j)
-			if (at[j] < range) at[j] = atomicAdd(&pos[at[j]], 1u); else at[j] = 0xFFFFFFFFu;
-		#pragma unroll
-		for (int j = 0; j < 4; ++j) {
-			if (at[j] >= n) continue;
-			const unsigned long long v = mj_packed(t[j], bp);
-			if (narrow) reinterpret_cast<uint32_t*>(val)[at[j]] = (uint32_t) (v - vmin);
-			else val[at[j]] = v;
-		}
+	for (uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; i < n; i += stride) {
+		uint4 t;
+		const uint64_t x = (uint64_t) mj_key<true>(R, i, 16, koff, 8, pol, t) - (uint64_t) kmin;
+		if (x >= range) continue;
+		const uint32_t at = atomicAdd(&pos[x], 1u);
+		if (at >= n) continue;
+		const unsigned long long v = mj_packed(t, bp);
+		if (bytes == 2) reinterpret_cast<uint16_t*>(val)[at] = (uint16_t) (v - vmin);
+		else if (bytes == 4) reinterpret_cast<uint32_t*>(val)[at] = (uint32_t) (v - vmin);
+		else val[at] = v;
 	}
 }
 
 // Rows of each probe tuple: one per value of its key's run [end[d - 1],
-// end[d]). A warp looks up 128 tuples at once, reserves their rows with one
+// end[d]). A warp looks up 64 tuples at once, reserves their rows with one
 // add on the cursor, and writes them 32 at a time, each lane finding its row's
 // tuple by a search over the lanes' offsets, so that a warp stores consecutive
 // rows whatever the runs' lengths. Rows past `cap` are counted only.
-__global__ void __launch_bounds__(256)
+// Bound by DRAM: the values' scattered reads miss L2 under the stream of rows
+// (16M tuples, 64M rows, 4-byte values: 1.36 GB read and 1.07 written). The whole join
+// above with its group-by: 128 tuples a warp and no limit on registers 1220 us, with 6
+// blocks an SM 1180, 64 tuples 1123 (32: 1345), in one wave of blocks 1109.
+#define MJ_ROWS_TUPLES 2                             // a lane
+#define MJ_ROWS_BLOCKS_PER_SM 6
+__global__ void __launch_bounds__(256, MJ_ROWS_BLOCKS_PER_SM)
 k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin, uint32_t range,
 		const uint32_t* __restrict__ end, const unsigned long long* __restrict__ val, uint32_t wsel,
 		uint4* __restrict__ out, uint64_t cap, unsigned long long* __restrict__ cursor, const unsigned int* __restrict__ meta,
@@ -598,16 +608,16 @@ k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin,
 {
 	if (meta[0] > MJ_MAX_RUN || meta[1]) return;
 	const unsigned long long vmin = ~vmm[0];
-	const bool narrow = vmm[1] - vmin < (1ull << 32);
+	const uint32_t bytes = mj_val_bytes(vmm[1] - vmin);
 	const uint32_t lane = threadIdx.x & 31;
 	const uint64_t pol = pg_policy_evict_first(), keep = pg_policy_keep(4);
 	const uint64_t nwarps = ((uint64_t) gridDim.x * blockDim.x) >> 5;
 	const uint32_t w0 = wsel & 15, w1 = (wsel >> 4) & 15, w2 = (wsel >> 8) & 15, w3 = (wsel >> 12) & 15;
-	for (uint64_t c0 = (((uint64_t) blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 128; c0 < n; c0 += nwarps * 128) {
-		uint4 t[4];
-		uint32_t lo[4], m[4];
+	for (uint64_t c0 = (((uint64_t) blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (32 * MJ_ROWS_TUPLES); c0 < n; c0 += nwarps * (32 * MJ_ROWS_TUPLES)) {
+		uint4 t[MJ_ROWS_TUPLES];
+		uint32_t lo[MJ_ROWS_TUPLES], m[MJ_ROWS_TUPLES];
 		#pragma unroll
-		for (int j = 0; j < 4; ++j) {
+		for (int j = 0; j < MJ_ROWS_TUPLES; ++j) {
 			const uint64_t i = c0 + j * 32 + lane;
 			lo[j] = 0; m[j] = 0;
 			t[j] = make_uint4(0, 0, 0, 0);
@@ -619,9 +629,9 @@ k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin,
 				}
 			}
 		}
-		uint32_t off[4], total = 0;
+		uint32_t off[MJ_ROWS_TUPLES], total = 0;
 		#pragma unroll
-		for (int j = 0; j < 4; ++j) {
+		for (int j = 0; j < MJ_ROWS_TUPLES; ++j) {
 			m[j] -= lo[j];
 			uint32_t x = m[j];
 			#pragma unroll
@@ -637,7 +647,7 @@ k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin,
 		if (lane == 0 && total) row = atomicAdd(cursor, (unsigned long long) total);
 		row = __shfl_sync(0xffffffffu, row, 0);
 		#pragma unroll
-		for (int j = 0; j < 4; ++j) {
+		for (int j = 0; j < MJ_ROWS_TUPLES; ++j) {
 			for (uint32_t r0 = 0; r0 < m[j]; r0 += 32) {
 				const uint32_t r = r0 + lane;
 				uint32_t x = 0;                  // the last tuple whose offset is <= r (it has rows)
@@ -646,7 +656,11 @@ k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin,
 					if (__shfl_sync(0xffffffffu, off[j], x + step) <= r) x += step;
 				const uint32_t at = __shfl_sync(0xffffffffu, lo[j], x) + (r - __shfl_sync(0xffffffffu, off[j], x));
 				unsigned long long v = 0;
-				if (r < m[j]) v = narrow ? vmin + mj_ld32(reinterpret_cast<const uint32_t*>(val) + at, keep) : mj_ld64(val + at, keep);
+				if (r < m[j]) {
+					if (bytes == 2) v = vmin + mj_ld16(reinterpret_cast<const uint16_t*>(val) + at, keep);
+					else if (bytes == 4) v = vmin + mj_ld32(reinterpret_cast<const uint32_t*>(val) + at, keep);
+					else v = mj_ld64(val + at, keep);
+				}
 				auto pick = [&](uint32_t w) -> uint32_t {
 					return w < 4 ? __shfl_sync(0xffffffffu, mjw_word(t[j], w), x) : w == 4 ? (uint32_t) v : (uint32_t) (v >> 32);
 				};
@@ -789,10 +803,11 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 			if ((rc = pg_scan_u64(ctx, s, sums, nb, nullptr))) { release(); return rc; }
 			k_mj_scan_apply<<<(unsigned) nb, 256, 0, s>>>(cnt, range, sums);
 			PG_LAUNCHED(ctx);
-			const int fblocks = (int) std::min<uint64_t>(pg_div_up(C->n, 256 * 4), (uint64_t) ctx->sm_count * 16);
+			const int fblocks = (int) std::min<uint64_t>(pg_div_up(C->n, 256), (uint64_t) ctx->sm_count * MJ_FILL_BLOCKS_PER_SM);
 			k_mj_fill<<<fblocks, 256, 0, s>>>((const char*) C->data, C->n, C->key_off, kmin, range, bp, cnt, val, meta, vmm);
 			PG_LAUNCHED(ctx);
-			const int rblocks = (int) std::min<uint64_t>(pg_div_up(P->n, 128 * 8), (uint64_t) ctx->sm_count * 24);
+			const int rblocks = (int) std::min<uint64_t>(pg_div_up(P->n, 256 * MJ_ROWS_TUPLES),
+					(uint64_t) ctx->sm_count * MJ_ROWS_BLOCKS_PER_SM);
 			k_mj_rows<<<rblocks, 256, 0, s>>>((const char*) P->data, P->n, P->key_off, kmin, range, cnt, val, wsel,
 					reinterpret_cast<uint4*>(out), out_capacity, agg, meta, vmm);
 			PG_LAUNCHED(ctx);

@@ -94,6 +94,18 @@ def test_mpsm_counted_window(ctx, case):
     _mpsm(ctx, R, S)
 
 
+# The rows' values are kept as 2- or 4-byte differences where their span allows;
+# a warp takes 64 probe tuples, a block 512.
+@pytest.mark.parametrize("span", [0, (1 << 16) - 1, 1 << 16, (1 << 32) - 1, 1 << 32])
+@pytest.mark.parametrize("n", [1, 64, 65, 512, 513, 40_003])
+def test_mpsm_value_spans(ctx, n, span):
+    R, S = dg.uniform_keys(n, n // 3 + 1, dg.seed_for(208)), dg.uniform_keys(n + 1, n // 3 + 1, dg.seed_for(209))
+    R[:, 1] = 77 + R[:, 1] % (span + 1)
+    R[0, 1], R[-1, 1] = 77, 77 + span
+    S[0, 0], S[-1, 0] = R[0, 0], R[-1, 0]
+    _mpsm(ctx, R, S)
+
+
 def test_mpsm_key_outside_the_sampled_window(ctx):
     # Over 4M tuples the window comes from every 1024th; a matching key far from
     # the rest and off the sample must still join.
