@@ -159,8 +159,8 @@ enum {
 	                                    4/8 evict-last with L1 (bits 4-7 = 0xC), 256 = all bits clear */
 	PG_TUNE_PROBE_PASSES = 8,        /* dense-table probe passes: 1, 2 (half the table each), 0 by size */
 	PG_TUNE_GROUPBY_PATH = 9,        /* group-by: 0 by key range and size, 1 to 5 hashed table, 6 dense when the
-	                                    key range allows, 7 as 6 without the shared-memory tables of windows up
-	                                    to 4096 keys */
+	                                    key range allows, 7 as 6 without the shared-memory tables of windows
+	                                    that fit there */
 	PG_TUNE_PROBE_WIDE = 10,         /* probe of tuples or rows other than 16 bytes: 0 materialised rows of dense
 	                                    tables staged through shared memory where the width allows, everything
 	                                    else per-thread loads; 1 per-thread loads; 2 staged, 4 lookups per

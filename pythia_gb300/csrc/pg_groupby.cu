@@ -457,74 +457,99 @@ k_gb_dense(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, u
 	if (fl) atomicOr(reinterpret_cast<unsigned int*>(fx.p + 2), fl);
 }
 
-// Dense group-by over a window of at most GBS_MAX_SLOTS keys: each CTA sums
-// its rows into a copy of the table in shared memory (dec sums' seven table
-// words, int sums in the low 4 bytes, counts and long sums in 8), then adds
-// each slot it saw into the global table once. Few groups otherwise put every
-// row's atomic on a handful of L2 lines.
-#define GBS_MAX_SLOTS 4096
-#define GBS_MAX_SLOTS_DEC 1536                     // 57 bytes a slot: two CTAs per SM
-template <int VT, int AGG, bool VEC16>
-__global__ void __launch_bounds__(GB_THREADS)
+// Dense group-by over a window whose table fits in shared memory: each CTA sums
+// its rows into a copy there, then adds each slot it saw into the global table once.
+// Few groups otherwise put every row's atomic on a handful of L2 lines. A slot is
+// 32-bit words, which take native adds: a count or an int sum one word, a long sum
+// two, a dec sum its t2 word in two and t2's overflows in a third; the chunks of a
+// value far below the column's largest, rare, go to the global table's lazy words,
+// or with few groups, where those are hot lines too, to lazy words here (LAZY).
+// The first add into a sum's slot returns the initial 0 and marks it seen.
+// Int and long sums are bound by the read, dec ones by instructions (137 a row, 59%
+// of issue): 64M rows in 300 groups 223, 224 and 352 us, as before but for dec's 520; in
+// 3000 (over 1500 in L2 before, dec at 57 bytes a slot) 223, 224 and 351 from 1540 to
+// 1750; in 12,000, long and dec with one CTA an SM, 230, 328 and 438 from 1550, 1550 and
+// 1000. One row a thread, the next one loaded, and 64 warps an SM: dec 352, four rows
+// and 32 warps 466. Several copies against equal keys: no faster.
+#define GBS_THREADS 1024
+#define GBS_MAX_BYTES (224 * 1024)
+#define GBS_LAZY_BYTES (8 * PG_FX_LAZY)
+template <int VT, int AGG>
+__host__ __device__ constexpr uint32_t gbs_words() { return GB_DEC ? 3 : AGG == PG_AGG_COUNT || VT == PG_VAL_INT ? 1 : 2; }
+template <int VT, int AGG>
+__host__ __device__ constexpr uint32_t gbs_slot_bytes() { return 4 * gbs_words<VT, AGG>() + (AGG == PG_AGG_SUM ? 1 : 0); }
+
+template <int VT, int AGG, bool VEC16, bool LAZY>
+__global__ void __launch_bounds__(GBS_THREADS, 2)
 k_gb_dense_smem(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, uint32_t kbytes, uint32_t voff,
 		long long kmin, uint32_t range, unsigned long long* __restrict__ acc, PgFx fx,
 		unsigned char* __restrict__ present, unsigned int* __restrict__ overflow)
 {
-	constexpr uint32_t SW = GB_DEC ? PG_FX_WORDS : 1;                                 // shared words per slot
+	constexpr uint32_t LW = LAZY ? 2 * PG_FX_LAZY : 0, SW = gbs_words<VT, AGG>();
 	extern __shared__ __align__(16) unsigned char gsm[];
-	unsigned long long* const sacc = reinterpret_cast<unsigned long long*>(gsm);
-	unsigned char* const spres = gsm + (size_t) range * SW * 8;
-	for (uint32_t i = threadIdx.x; i < range * SW; i += blockDim.x) sacc[i] = 0;
-	for (uint32_t i = threadIdx.x; i < range; i += blockDim.x) spres[i] = 0;
+	unsigned long long* const sl = reinterpret_cast<unsigned long long*>(gsm);         // lazy word c of slot d at sl[d + c range]
+	uint32_t* const sw = reinterpret_cast<uint32_t*>(gsm) + (size_t) range * LW;       // word w of slot d at sw[d + w range]
+	unsigned char* const spres = reinterpret_cast<unsigned char*>(sw + range * SW);
+	for (uint32_t d = threadIdx.x; d < range * (LW + SW); d += blockDim.x) reinterpret_cast<uint32_t*>(gsm)[d] = 0;
+	if (AGG == PG_AGG_SUM) for (uint32_t d = threadIdx.x; d < range; d += blockDim.x) spres[d] = 0;
 	__syncthreads();
 	const uint64_t stride = (uint64_t) gridDim.x * blockDim.x;
 	bool outside = false;
 	uint32_t fl = 0;
 	const int fs = GB_DEC ? fx.p[0] : 0, fb = GB_DEC ? fx.p[1] : 0;
-	for (uint64_t base = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; base < n; base += stride * GBD_ILP) {
-		uint32_t d[GBD_ILP];
-		unsigned long long iv[GBD_ILP];
-		pg_fx3 f[GBD_ILP];
-		bool ok[GBD_ILP];
-		#pragma unroll
-		for (int j = 0; j < GBD_ILP; ++j) {
-			const uint64_t i = base + j * stride;
-			ok[j] = i < n;
-			d[j] = 0; iv[j] = 0; f[j] = pg_fx3{0, 0, 0};
-			if (!ok[j]) continue;
-			int64_t k;
-			uint64_t vbits;
-			gb_row_kv<VT, VEC16>(in, i, W, koff, kbytes, voff, k, vbits);
-			const uint64_t dd = (uint64_t) k - (uint64_t) kmin;
-			if (dd >= range) { ok[j] = false; outside = true; continue; }   // key outside the table
-			d[j] = (uint32_t) dd;
-			if (AGG == PG_AGG_COUNT) iv[j] = 1;
-			else if (GB_DEC) f[j] = pg_fx_take(vbits, fs, fb, fl);
-			else iv[j] = vbits;
+	int64_t k = 0;
+	uint64_t vbits = 0;
+	uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x;
+	if (i < n) gb_row_kv<VT, VEC16>(in, i, W, koff, kbytes, voff, k, vbits);
+	for (; i < n; i += stride) {
+		const uint64_t dd = (uint64_t) k - (uint64_t) kmin;
+		uint64_t v = vbits;
+		if (i + stride < n) gb_row_kv<VT, VEC16>(in, i + stride, W, koff, kbytes, voff, k, vbits);
+		if (dd >= range) { outside = true; continue; }      // key outside the table
+		const uint32_t d = (uint32_t) dd;
+		if (AGG == PG_AGG_COUNT) { atomicAdd(&sw[d], 1u); continue; }
+		if (GB_DEC) {
+			const pg_fx3 f = pg_fx_take(v, fs, fb, fl);
+			v = f.w2;
+			if (f.w0 | f.w1) {
+				#pragma unroll
+				for (int c = 0; c < PG_FX_LAZY; ++c) {
+					const uint64_t x = pg_fx_chunk(f.w0, f.w1, c);
+					if (!x) continue;
+					if (LAZY) gb_shared_add64(&sl[d + c * range], x);
+					else atomicAdd(&acc[d + (uint64_t) (PG_FX_L0 + c) * range], (unsigned long long) x);
+				}
+			}
 		}
-		#pragma unroll
-		for (int j = 0; j < GBD_ILP; ++j) {
-			if (!ok[j]) continue;
-			if (GB_DEC) pg_fx_atomic_add(&sacc[d[j]], range, pg_fx_widen(f[j]));
-			else if (VT == PG_VAL_INT && AGG == PG_AGG_SUM)
-				atomicAdd(reinterpret_cast<unsigned int*>(&sacc[d[j]]), (unsigned int) iv[j]);
-			else gb_shared_add64(&sacc[d[j]], iv[j]);
-			if (AGG == PG_AGG_SUM) spres[d[j]] = 1;
-		}
+		const uint32_t lo = (uint32_t) v, old = atomicAdd(&sw[d], lo);
+		if (old == 0) spres[d] = 1;
+		const uint32_t hi = SW == 1 ? 0 : (uint32_t) (v >> 32) + (old + lo < lo);
+		if (!hi) continue;
+		const uint32_t oh = atomicAdd(&sw[d + range], hi);
+		if (!GB_DEC) continue;
+		// A value's part of t2 is within +-2^60: hi did not wrap.
+		const int32_t was = (int32_t) oh, is = (int32_t) (oh + hi);
+		if ((int32_t) hi > 0 ? is < was : is > was) atomicAdd(&sw[d + 2 * range], (int32_t) hi > 0 ? 1u : ~0u);
 	}
 	if (outside) *overflow = 1;
 	if (fl) atomicOr(reinterpret_cast<unsigned int*>(fx.p + 2), fl);
 	__syncthreads();
-	for (uint32_t i = threadIdx.x; i < range; i += blockDim.x) {
+	for (uint32_t d = threadIdx.x; d < range; d += blockDim.x) {
 		if (AGG == PG_AGG_COUNT) {
-			if (sacc[i]) atomicAdd(&acc[i], sacc[i]);
+			if (sw[d]) atomicAdd(&acc[d], (unsigned long long) sw[d]);
 			continue;
 		}
-		if (!spres[i]) continue;
-		if (GB_DEC) pg_fx_atomic_add(&acc[i], range, gb_table_count(sacc, range, i));
-		else if (VT == PG_VAL_INT) atomicAdd(reinterpret_cast<unsigned int*>(&acc[i]), (unsigned int) sacc[i]);
-		else atomicAdd(&acc[i], sacc[i]);
-		present[i] = 1;
+		if (!spres[d]) continue;
+		const unsigned long long v = SW == 1 ? sw[d] : ((unsigned long long) sw[d + range] << 32) | sw[d];
+		if (GB_DEC) {
+			const uint64_t t3 = (uint64_t) (int64_t) (int32_t) sw[d + 2 * range];
+			pg_fx_atomic_add(&acc[d], range, pg_fx4{0, 0, v, t3 - (v >> 63)});
+			#pragma unroll
+			for (int c = 0; c < (LAZY ? PG_FX_LAZY : 0); ++c)
+				if (sl[d + c * range]) atomicAdd(&acc[d + (uint64_t) (PG_FX_L0 + c) * range], sl[d + c * range]);
+		} else if (VT == PG_VAL_INT) atomicAdd(reinterpret_cast<unsigned int*>(&acc[d]), (unsigned int) v);
+		else atomicAdd(&acc[d], v);
+		present[d] = 1;
 	}
 }
 
@@ -717,23 +742,26 @@ static int gb_dense_window(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint32
 	unsigned int* oflag = reinterpret_cast<unsigned int*>(cursor + 1);         // then two words of pg_readback
 	unsigned char* present = reinterpret_cast<unsigned char*>(cursor + 4);
 	PG_CUDA(ctx, cudaMemsetAsync(mem, 0, bytes, s));
-	if (range <= (GB_DEC ? GBS_MAX_SLOTS_DEC : GBS_MAX_SLOTS) && ctx->tune[PG_TUNE_GROUPBY_PATH] != 7) {
-		// Few groups: per-CTA tables in shared memory, one flush each.
-		const int sbytes = (int) (range * (GB_DEC ? 8 * PG_FX_WORDS + 1 : 9));
+	// Few groups: per-CTA tables in shared memory, one flush each, while the
+	// flushes are fewer than the rows (1M rows in 4000 groups take 79 us in L2, with
+	// more slots to flush than rows 90). A table of half the SM's shared memory or less
+	// lets two CTAs share it; dec sums keep lazy words there when they fit in that half.
+	uint64_t sbytes = range * gbs_slot_bytes<VT, AGG>();
+	const bool lazy = GB_DEC && sbytes + range * GBS_LAZY_BYTES <= GBS_MAX_BYTES / 2;
+	if (lazy) sbytes += range * GBS_LAZY_BYTES;
+	int sblocks = 0;
+	auto* const kernel = vec16 ? lazy ? k_gb_dense_smem<VT, AGG, true, GB_DEC> : k_gb_dense_smem<VT, AGG, true, false>
+	                           : lazy ? k_gb_dense_smem<VT, AGG, false, GB_DEC> : k_gb_dense_smem<VT, AGG, false, false>;
+	if (sbytes <= GBS_MAX_BYTES && ctx->tune[PG_TUNE_GROUPBY_PATH] != 7) {
 		int per_sm = 0;
-		if (vec16) {
-			PG_CUDA(ctx, cudaFuncSetAttribute(k_gb_dense_smem<VT, AGG, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sbytes));
-			PG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gb_dense_smem<VT, AGG, true>, GB_THREADS, sbytes));
-		} else {
-			PG_CUDA(ctx, cudaFuncSetAttribute(k_gb_dense_smem<VT, AGG, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sbytes));
-			PG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gb_dense_smem<VT, AGG, false>, GB_THREADS, sbytes));
-		}
-		const int sblocks = (int) std::min<uint64_t>(pg_div_up(in->n, (uint64_t) GB_THREADS * GBD_ILP),
+		PG_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GBS_MAX_BYTES));
+		PG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, GBS_THREADS, sbytes));
+		sblocks = (int) std::min<uint64_t>(pg_div_up(in->n, GBS_THREADS),
 				(uint64_t) ctx->sm_count * std::max(per_sm, 1));
-		if (vec16) k_gb_dense_smem<VT, AGG, true><<<sblocks, GB_THREADS, sbytes, s>>>((const char*) in->data, in->n,
-				in->width, in->key_off, in->key_bytes, voff, kmin, (uint32_t) range, acc, fx, present, oflag);
-		else k_gb_dense_smem<VT, AGG, false><<<sblocks, GB_THREADS, sbytes, s>>>((const char*) in->data, in->n,
-				in->width, in->key_off, in->key_bytes, voff, kmin, (uint32_t) range, acc, fx, present, oflag);
+	}
+	if (sblocks && range * sblocks <= in->n) {
+		kernel<<<sblocks, GBS_THREADS, sbytes, s>>>((const char*) in->data, in->n, in->width, in->key_off, in->key_bytes,
+				voff, kmin, (uint32_t) range, acc, fx, present, oflag);
 		PG_LAUNCHED(ctx);
 	} else {
 		// Four rows in flight a thread and many blocks in turn: 256M rows in 1M

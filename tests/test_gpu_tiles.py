@@ -235,3 +235,47 @@ def test_sort_one_launch(ctx, n, bits):
             t[:, 0], t[:, -1] = np.arange(n), np.arange(n)
             t[:, off // 4:off // 4 + 2] = words[:, :2]
             assert np.array_equal(ctx.sort(t, (off, 8)), t[np.argsort(rows[:, 0], kind="stable")])
+
+
+# Dense group tables in shared memory: 224 KB a CTA, two CTAs an SM up to half of
+# that. Slots of 4 (counts), 5 (int), 9 (long) and 13 bytes (dec, 53 up to 2163 slots
+# with the words of small values); larger windows go to the global table. Dec sums
+# all of one sign overflow their word, tiny values and zeros need the lazy words.
+@pytest.mark.parametrize("val,groups", [("count", 27_000), ("int", 1), ("int", 22_938), ("long", 3), ("long", 12_743),
+                                        ("long", 12_744), ("long", 25_486), ("long", 25_487), ("dec", 2), ("dec", 2163),
+                                        ("dec", 2164), ("dec", 8822), ("dec", 8823), ("dec", 17_644), ("dec", 17_645)])
+def test_groupby_shared_table_sizes(ctx, val, groups):
+    n = (1 << 22) - 1                                       # the exact key window
+    rng = np.random.default_rng(groups)
+    rows = np.empty((n, 2), dtype=np.int64)
+    rows[:, 0] = rng.integers(0, groups, size=n) - 5
+    rows[:groups, 0] = np.arange(groups) - 5
+    if val == "dec":
+        v = rng.uniform(0.5, 1.0, size=n) * np.where(rows[:, 0] % 2, 1e4, -1e4)
+        v[::37] *= 1e-9
+        v[::1001] = 0.0
+        v[rows[:, 0] == 1] = 0.0                            # a group that adds nothing
+        rows[:, 1] = v.view(np.int64)
+        got = np.ascontiguousarray(ctx.groupby(rows, val=(8, "dec"))).view(np.int64).reshape(-1, 2)
+        want = orc.groupby_exact(rows).view(np.int64).reshape(-1, 2)
+        assert np.array_equal(got[np.argsort(got[:, 0], kind="stable")], want)
+        return
+    rows[:, 1] = rng.integers(-(1 << 62), 1 << 62, size=n)
+    agg, vtype = ("count", "long") if val == "count" else ("sum", val)
+    got = ctx.groupby(rows, val=(8, vtype), agg=agg)
+    want = orc.groupby(rows, val=(8, vtype), agg=agg, hash=orc.hashcfg("modulo", 1024))
+    assert np.array_equal(orc.canonical(got), orc.canonical(want))
+
+
+# Tuples that are not 16 bytes load key and value apart.
+@pytest.mark.parametrize("val", ["int", "long", "dec"])
+@pytest.mark.parametrize("n", [1, 1023, 1025, 50_001])
+def test_groupby_shared_table_24_byte_rows(ctx, n, val):
+    a = dg.groupby_rows(n, 7, 1e4, dg.seed_for(211)) if val == "dec" else dg.uniform_keys(n, 7, dg.seed_for(211))
+    rows = np.ascontiguousarray(np.concatenate([a, a[:, :1]], axis=1))
+    got = np.ascontiguousarray(ctx.groupby(rows, val=(8, val)))
+    if val == "dec":
+        g = got.view(np.int64).reshape(-1, 2)
+        assert np.array_equal(g[np.argsort(g[:, 0], kind="stable")], orc.groupby_exact(a).view(np.int64).reshape(-1, 2))
+    else:
+        assert np.array_equal(orc.canonical(got), orc.canonical(orc.groupby(rows, val=(8, val))))
