@@ -21,11 +21,9 @@
 // redo the sum with the exact bound). Infinities and NaNs are summed on the
 // side and patch their groups' results. Blocks add the rows of groups they
 // meet often in shared memory first, which cuts L2 atomics on skewed keys.
-#include "pg_internal.cuh"
-#include <algorithm>
+#include "pg_groupshared.cuh"
 
 #define GB_THREADS 256
-#define GB_DEC (VT == PG_VAL_DEC && AGG == PG_AGG_SUM)     // inside templates on VT, AGG
 
 // An open-addressing group table. A group's aggregate is one word of acc (a
 // count, a long sum, an int sum in its low 4 bytes) or, for a dec sum, the
@@ -54,18 +52,6 @@ __device__ __forceinline__ void fold_slot(unsigned long long* acc, uint64_t wstr
 	else if (VT == PG_VAL_LONG) atomicAdd(&acc[slot], v.i);
 	else if (VT == PG_VAL_INT) atomicAdd(reinterpret_cast<unsigned int*>(&acc[slot]), (unsigned int) v.i);
 	else pg_fx_atomic_add(&acc[slot], wstride, v.f);
-}
-
-// v added to a 64-bit word in shared memory by its 32-bit halves: a shared
-// 64-bit add is a compare-and-swap loop, a 32-bit one a single instruction, and
-// the upper half needs one only for a carry or a large value. The word is right
-// once every add is in.
-__device__ __forceinline__ void gb_shared_add64(unsigned long long* p, unsigned long long v)
-{
-	unsigned int* const q = reinterpret_cast<unsigned int*>(p);
-	const unsigned int lo = (unsigned int) v, old = atomicAdd(q, lo);
-	const unsigned int hi = (unsigned int) (v >> 32) + (old + lo < lo);
-	if (hi) atomicAdd(q + 1, hi);
 }
 
 // A dec sum's count from table words acc[slot + k * wstride].
@@ -457,100 +443,36 @@ k_gb_dense(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, u
 	if (fl) atomicOr(reinterpret_cast<unsigned int*>(fx.p + 2), fl);
 }
 
-// Dense group-by over a window whose table fits in shared memory: each CTA sums
-// its rows into a copy there, then adds each slot it saw into the global table once.
-// Few groups otherwise put every row's atomic on a handful of L2 lines. A slot is
-// 32-bit words, which take native adds: a count or an int sum one word, a long sum
-// two, a dec sum its t2 word in two and t2's overflows in a third; the chunks of a
-// value far below the column's largest, rare, go to the global table's lazy words,
-// or with few groups, where those are hot lines too, to lazy words here (LAZY).
-// The first add into a sum's slot returns the initial 0 and marks it seen.
-// Int and long sums are bound by the read, dec ones by instructions (137 a row, 59%
-// of issue): 64M rows in 300 groups 223, 224 and 352 us, as before but for dec's 520; in
-// 3000 (over 1500 in L2 before, dec at 57 bytes a slot) 223, 224 and 351 from 1540 to
-// 1750; in 12,000, long and dec with one CTA an SM, 230, 328 and 438 from 1550, 1550 and
-// 1000. One row a thread, the next one loaded, and 64 warps an SM: dec 352, four rows
-// and 32 warps 466. Several copies against equal keys: no faster.
-#define GBS_THREADS 1024
-#define GBS_MAX_BYTES (224 * 1024)
-#define GBS_LAZY_BYTES (8 * PG_FX_LAZY)
-template <int VT, int AGG>
-__host__ __device__ constexpr uint32_t gbs_words() { return GB_DEC ? 3 : AGG == PG_AGG_COUNT || VT == PG_VAL_INT ? 1 : 2; }
-template <int VT, int AGG>
-__host__ __device__ constexpr uint32_t gbs_slot_bytes() { return 4 * gbs_words<VT, AGG>() + (AGG == PG_AGG_SUM ? 1 : 0); }
-
+// Dense group-by over a window whose table fits in shared memory (GbShared). Int and
+// long sums are bound by the read, dec ones by instructions (137 a row, 59% of issue):
+// 64M rows in 300 groups 223, 224 and 352 us, as before but for dec's 520; in 3000 (over
+// 1500 in L2 before, dec at 57 bytes a slot) 223, 224 and 351 from 1540 to 1750; in
+// 12,000, long and dec with one CTA an SM, 230, 328 and 438 from 1550, 1550 and 1000. One
+// row a thread, the next one loaded, and 64 warps an SM: dec 352, four rows and 32 warps
+// 466.
 template <int VT, int AGG, bool VEC16, bool LAZY>
 __global__ void __launch_bounds__(GBS_THREADS, 2)
 k_gb_dense_smem(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, uint32_t kbytes, uint32_t voff,
 		long long kmin, uint32_t range, unsigned long long* __restrict__ acc, PgFx fx,
 		unsigned char* __restrict__ present, unsigned int* __restrict__ overflow)
 {
-	constexpr uint32_t LW = LAZY ? 2 * PG_FX_LAZY : 0, SW = gbs_words<VT, AGG>();
 	extern __shared__ __align__(16) unsigned char gsm[];
-	unsigned long long* const sl = reinterpret_cast<unsigned long long*>(gsm);         // lazy word c of slot d at sl[d + c range]
-	uint32_t* const sw = reinterpret_cast<uint32_t*>(gsm) + (size_t) range * LW;       // word w of slot d at sw[d + w range]
-	unsigned char* const spres = reinterpret_cast<unsigned char*>(sw + range * SW);
-	for (uint32_t d = threadIdx.x; d < range * (LW + SW); d += blockDim.x) reinterpret_cast<uint32_t*>(gsm)[d] = 0;
-	if (AGG == PG_AGG_SUM) for (uint32_t d = threadIdx.x; d < range; d += blockDim.x) spres[d] = 0;
-	__syncthreads();
+	GbShared<VT, AGG, LAZY> t(gsm, range, acc, fx);
 	const uint64_t stride = (uint64_t) gridDim.x * blockDim.x;
 	bool outside = false;
-	uint32_t fl = 0;
-	const int fs = GB_DEC ? fx.p[0] : 0, fb = GB_DEC ? fx.p[1] : 0;
 	int64_t k = 0;
 	uint64_t vbits = 0;
 	uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x;
 	if (i < n) gb_row_kv<VT, VEC16>(in, i, W, koff, kbytes, voff, k, vbits);
 	for (; i < n; i += stride) {
-		const uint64_t dd = (uint64_t) k - (uint64_t) kmin;
-		uint64_t v = vbits;
+		const uint64_t d = (uint64_t) k - (uint64_t) kmin, v = vbits;
 		if (i + stride < n) gb_row_kv<VT, VEC16>(in, i + stride, W, koff, kbytes, voff, k, vbits);
-		if (dd >= range) { outside = true; continue; }      // key outside the table
-		const uint32_t d = (uint32_t) dd;
-		if (AGG == PG_AGG_COUNT) { atomicAdd(&sw[d], 1u); continue; }
-		if (GB_DEC) {
-			const pg_fx3 f = pg_fx_take(v, fs, fb, fl);
-			v = f.w2;
-			if (f.w0 | f.w1) {
-				#pragma unroll
-				for (int c = 0; c < PG_FX_LAZY; ++c) {
-					const uint64_t x = pg_fx_chunk(f.w0, f.w1, c);
-					if (!x) continue;
-					if (LAZY) gb_shared_add64(&sl[d + c * range], x);
-					else atomicAdd(&acc[d + (uint64_t) (PG_FX_L0 + c) * range], (unsigned long long) x);
-				}
-			}
-		}
-		const uint32_t lo = (uint32_t) v, old = atomicAdd(&sw[d], lo);
-		if (old == 0) spres[d] = 1;
-		const uint32_t hi = SW == 1 ? 0 : (uint32_t) (v >> 32) + (old + lo < lo);
-		if (!hi) continue;
-		const uint32_t oh = atomicAdd(&sw[d + range], hi);
-		if (!GB_DEC) continue;
-		// A value's part of t2 is within +-2^60: hi did not wrap.
-		const int32_t was = (int32_t) oh, is = (int32_t) (oh + hi);
-		if ((int32_t) hi > 0 ? is < was : is > was) atomicAdd(&sw[d + 2 * range], (int32_t) hi > 0 ? 1u : ~0u);
+		if (d < range) t.add((uint32_t) d, v);
+		else outside = true;                                // key outside the table
 	}
 	if (outside) *overflow = 1;
-	if (fl) atomicOr(reinterpret_cast<unsigned int*>(fx.p + 2), fl);
-	__syncthreads();
-	for (uint32_t d = threadIdx.x; d < range; d += blockDim.x) {
-		if (AGG == PG_AGG_COUNT) {
-			if (sw[d]) atomicAdd(&acc[d], (unsigned long long) sw[d]);
-			continue;
-		}
-		if (!spres[d]) continue;
-		const unsigned long long v = SW == 1 ? sw[d] : ((unsigned long long) sw[d + range] << 32) | sw[d];
-		if (GB_DEC) {
-			const uint64_t t3 = (uint64_t) (int64_t) (int32_t) sw[d + 2 * range];
-			pg_fx_atomic_add(&acc[d], range, pg_fx4{0, 0, v, t3 - (v >> 63)});
-			#pragma unroll
-			for (int c = 0; c < (LAZY ? PG_FX_LAZY : 0); ++c)
-				if (sl[d + c * range]) atomicAdd(&acc[d + (uint64_t) (PG_FX_L0 + c) * range], sl[d + c * range]);
-		} else if (VT == PG_VAL_INT) atomicAdd(reinterpret_cast<unsigned int*>(&acc[d]), (unsigned int) v);
-		else atomicAdd(&acc[d], v);
-		present[d] = 1;
-	}
+	if (t.fl) atomicOr(reinterpret_cast<unsigned int*>(fx.p + 2), t.fl);
+	t.flush(present);
 }
 
 template <int VT, int AGG>
@@ -742,26 +664,15 @@ static int gb_dense_window(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint32
 	unsigned int* oflag = reinterpret_cast<unsigned int*>(cursor + 1);         // then two words of pg_readback
 	unsigned char* present = reinterpret_cast<unsigned char*>(cursor + 4);
 	PG_CUDA(ctx, cudaMemsetAsync(mem, 0, bytes, s));
-	// Few groups: per-CTA tables in shared memory, one flush each, while the
-	// flushes are fewer than the rows (1M rows in 4000 groups take 79 us in L2, with
-	// more slots to flush than rows 90). A table of half the SM's shared memory or less
-	// lets two CTAs share it; dec sums keep lazy words there when they fit in that half.
-	uint64_t sbytes = range * gbs_slot_bytes<VT, AGG>();
-	const bool lazy = GB_DEC && sbytes + range * GBS_LAZY_BYTES <= GBS_MAX_BYTES / 2;
-	if (lazy) sbytes += range * GBS_LAZY_BYTES;
+	const GbsPlan plan = gbs_plan<VT, AGG>(range);
+	auto* const kernel = vec16
+			? plan.lazy ? k_gb_dense_smem<VT, AGG, true, GB_DEC> : k_gb_dense_smem<VT, AGG, true, false>
+			: plan.lazy ? k_gb_dense_smem<VT, AGG, false, GB_DEC> : k_gb_dense_smem<VT, AGG, false, false>;
 	int sblocks = 0;
-	auto* const kernel = vec16 ? lazy ? k_gb_dense_smem<VT, AGG, true, GB_DEC> : k_gb_dense_smem<VT, AGG, true, false>
-	                           : lazy ? k_gb_dense_smem<VT, AGG, false, GB_DEC> : k_gb_dense_smem<VT, AGG, false, false>;
-	if (sbytes <= GBS_MAX_BYTES && ctx->tune[PG_TUNE_GROUPBY_PATH] != 7) {
-		int per_sm = 0;
-		PG_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GBS_MAX_BYTES));
-		PG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, GBS_THREADS, sbytes));
-		sblocks = (int) std::min<uint64_t>(pg_div_up(in->n, GBS_THREADS),
-				(uint64_t) ctx->sm_count * std::max(per_sm, 1));
-	}
-	if (sblocks && range * sblocks <= in->n) {
-		kernel<<<sblocks, GBS_THREADS, sbytes, s>>>((const char*) in->data, in->n, in->width, in->key_off, in->key_bytes,
-				voff, kmin, (uint32_t) range, acc, fx, present, oflag);
+	if (ctx->tune[PG_TUNE_GROUPBY_PATH] != 7 && (rc = gbs_blocks(ctx, kernel, plan, range, in->n, &sblocks))) return rc;
+	if (sblocks) {
+		kernel<<<sblocks, GBS_THREADS, plan.bytes, s>>>((const char*) in->data, in->n, in->width, in->key_off,
+				in->key_bytes, voff, kmin, (uint32_t) range, acc, fx, present, oflag);
 		PG_LAUNCHED(ctx);
 	} else {
 		// Four rows in flight a thread and many blocks in turn: 256M rows in 1M

@@ -279,3 +279,32 @@ def test_groupby_shared_table_24_byte_rows(ctx, n, val):
         assert np.array_equal(g[np.argsort(g[:, 0], kind="stable")], orc.groupby_exact(a).view(np.int64).reshape(-1, 2))
     else:
         assert np.array_equal(orc.canonical(got), orc.canonical(orc.groupby(rows, val=(8, val))))
+
+
+# Join then group-by with each CTA's groups in shared memory, for as many as fit and
+# flush fewer slots than there are probe tuples; the global table past that. Sizes
+# around a block's 1024 tuples, and probe misses.
+@pytest.mark.parametrize("probe,groups", [(1, 1), (1023, 5), (1025, 9), (3_000_000, 2163), (3_000_000, 2164),
+                                          (3_000_000, 17_644), (3_000_000, 17_645)])
+@pytest.mark.parametrize("swap", [False, True])
+def test_hashjoin_groupby_shared_tables(ctx, probe, groups, swap):
+    build = 2 * groups + 1
+    rng = np.random.default_rng(probe + groups)
+    R = np.stack([rng.permutation(build), np.arange(build) % groups + 40], axis=1).astype(np.int64)
+    keys = rng.integers(-3, build + 3, size=probe)
+    keys[0] = 0
+    dec = rng.uniform(0.5, 1.0, size=probe) * np.where(keys % 2, 1e6, -1e6)
+    dec[::41] *= 1e-12
+    whole = rng.integers(-(1 << 62), 1 << 62, size=probe)
+    group = np.full(build, -1, dtype=np.int64)
+    group[R[:, 0]] = R[:, 1]
+    hit = (keys >= 0) & (keys < build)
+    for vtype, v in (("dec", dec.view(np.int64)), ("long", whole), ("int", whole), ("count", whole)):
+        cols = [v, keys] if swap else [keys, v]
+        S = np.ascontiguousarray(np.stack(cols, axis=1).astype(np.int64))
+        pkey, val = ((8, 8), 0) if swap else ((0, 8), 8)
+        joined = np.ascontiguousarray(np.stack([group[keys[hit]], v[hit]], axis=1))
+        agg, t = ("count", "long") if vtype == "count" else ("sum", vtype)
+        got = np.ascontiguousarray(ctx.hashjoin_groupby(R, S, pkey=pkey, val=(val, t), agg=agg))
+        want = orc.groupby_exact(joined) if t == "dec" else orc.groupby(joined, val=(8, t), agg=agg)
+        assert np.array_equal(orc.canonical(got), orc.canonical(want))
