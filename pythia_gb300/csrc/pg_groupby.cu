@@ -54,6 +54,42 @@ __device__ __forceinline__ void fold_slot(unsigned long long* acc, uint64_t wstr
 	else pg_fx_atomic_add(&acc[slot], wstride, v.f);
 }
 
+// The same with the carry out of the 64 bits.
+__device__ __forceinline__ uint64_t gb_shared_add64_carry(unsigned long long* p, unsigned long long v)
+{
+	unsigned int* const q = reinterpret_cast<unsigned int*>(p);
+	const unsigned int lo = (unsigned int) v, old = atomicAdd(q, lo);
+	const unsigned long long hi = (v >> 32) + (old + lo < lo);          // up to 2^32
+	if ((unsigned int) hi == 0) return hi >> 32;
+	const unsigned int oh = atomicAdd(q + 1, (unsigned int) hi);
+	return oh + (unsigned int) hi < oh;
+}
+
+// Adds count a into four chained words t[k * stride] in shared memory, as
+// pg_fx_chain_add does one add at a time: a carry or overflow goes on with the add
+// that made it. A value near the column's largest is two 32-bit adds on t2, where 64-bit
+// ones were compare-and-swap loops: 20M rows hashed into 10 groups 403 -> 208 us, into
+// 300 408 -> 387, into 100,000 536 -> 514.
+__device__ __forceinline__ void gb_shared_chain_add(unsigned long long* t, uint32_t stride, const pg_fx3& a)
+{
+	uint64_t c = 0;
+	if (a.w0) c = gb_shared_add64_carry(t, a.w0);
+	const uint64_t x1 = a.w1 + c;
+	c = x1 < c;
+	if (x1) c += gb_shared_add64_carry(t + stride, x1);
+	const uint64_t l = a.w2 + c;                       // within +-2^61
+	if (l) {
+		unsigned int* const q = reinterpret_cast<unsigned int*>(t + 2 * stride);
+		const unsigned int lo = (unsigned int) l, old = atomicAdd(q, lo);
+		const unsigned int hi = (unsigned int) (l >> 32) + (old + lo < lo);
+		if (hi) {
+			const unsigned int oh = atomicAdd(q + 1, hi);
+			const int32_t was = (int32_t) oh, is = (int32_t) (oh + hi);
+			if ((int32_t) hi > 0 ? is < was : is > was) gb_shared_add64(t + 3 * stride, (int32_t) hi > 0 ? 1ull : ~0ull);
+		}
+	}
+}
+
 // A dec sum's count from table words acc[slot + k * wstride].
 __device__ __forceinline__ pg_fx4 gb_table_count(const unsigned long long* acc, uint64_t wstride, uint64_t slot)
 {
@@ -269,9 +305,13 @@ __device__ __forceinline__ void gb_row_kv(const char* __restrict__ in, uint64_t 
 #define GBH_CACHE_LOG2 8                    // groups kept per block: 256 (4 KB, 10 KB for dec)
 #define GBH_BLOCKS_PER_SM 64
 // Few groups: room for all of them in every block (32 KB, 40 KB for dec), and
-// fewer blocks, which each end by adding their groups to the table. 20M rows
-// in 1000 groups: 180 us, 527 with 256 places.
+// fewer blocks, which each end by adding their groups to the table: eight rows a
+// block for every group, unless that would leave an SM without its five blocks (1M rows in
+// 300 groups 113 -> 94 us, dec 149 -> 119). 20M rows in 1000 groups: 180 us, 527 with 256
+// places.
 #define GBH_FEW 1024u
+#define GBH_FEW_ROWS 8
+#define GBH_FEW_RESIDENT 5
 #define GBH_FEW_LOG2 (GB_DEC ? 10 : 11)
 #define GBH_FEW_PROBES 4
 #define GBH_FEW_BLOCKS_PER_SM 24
@@ -354,7 +394,7 @@ k_gb_hash(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, ui
 			if (cur == (unsigned long long) k) { here = true; break; }
 		}
 		if (here) {
-			if (GB_DEC) pg_fx_atomic_chain_add(&sacc[c], places, pg_fx_widen(f));
+			if (GB_DEC) gb_shared_chain_add(&sacc[c], places, f);
 			else if (VT == PG_VAL_INT && AGG == PG_AGG_SUM) fold_slot<VT, AGG>(sacc, places, c, v);
 			else gb_shared_add64(&sacc[c], v.i);
 			continue;
@@ -803,8 +843,9 @@ static int gb_run(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint32_t voff, 
 			const bool few = groups <= GBH_FEW;
 			const uint32_t places = 1u << (few ? GBH_FEW_LOG2 : GBH_CACHE_LOG2), probes = few ? GBH_FEW_PROBES : 1;
 			const size_t smem = (size_t) places * (GB_DEC ? 40 : 16);
-			const int blocks = (int) std::min<uint64_t>(pg_div_up(in->n, GB_THREADS),
-					(uint64_t) ctx->sm_count * (few ? GBH_FEW_BLOCKS_PER_SM : GBH_BLOCKS_PER_SM));
+			uint64_t most = (uint64_t) ctx->sm_count * (few ? GBH_FEW_BLOCKS_PER_SM : GBH_BLOCKS_PER_SM);
+			if (few) most = std::min(most, std::max<uint64_t>(in->n / (GBH_FEW_ROWS * groups), (uint64_t) ctx->sm_count * GBH_FEW_RESIDENT));
+			const int blocks = (int) std::min<uint64_t>(pg_div_up(in->n, GB_THREADS), most);
 			if (gb_vec16<VT, AGG>(in, voff))
 				k_gb_hash<VT, AGG, true><<<blocks, GB_THREADS, smem, s>>>((const char*) in->data, in->n, in->width, in->key_off,
 						in->key_bytes, voff, t, places, probes, fx, ctx->d_status);
