@@ -590,17 +590,18 @@ k_mj_fill(const char* __restrict__ R, uint64_t n, uint32_t koff, long long kmin,
 }
 
 // Rows of each probe tuple: one per value of its key's run [end[d - 1],
-// end[d]). A warp looks up 64 tuples at once, reserves their rows with one
+// end[d]). A warp looks up 32 T tuples at once, reserves their rows with one
 // add on the cursor, and writes them 32 at a time, each lane finding its row's
 // tuple by a search over the lanes' offsets, so that a warp stores consecutive
 // rows whatever the runs' lengths. Rows past `cap` are counted only.
 // Bound by DRAM: the values' scattered reads miss L2 under the stream of rows
 // (16M tuples, 64M rows, 4-byte values: 1.36 GB read and 1.07 written). The whole join
-// above with its group-by: 128 tuples a warp and no limit on registers 1220 us, with 6
-// blocks an SM 1180, 64 tuples 1123 (32: 1345), in one wave of blocks 1109.
-#define MJ_ROWS_TUPLES 2                             // a lane
-#define MJ_ROWS_BLOCKS_PER_SM 6
-__global__ void __launch_bounds__(256, MJ_ROWS_BLOCKS_PER_SM)
+// above with its group-by: no limit on registers 1214 us, with 6 blocks an SM 1160, and
+// two tuples a lane instead of four 1105; of keys with one row 1484, 1513 and 1590, so
+// those take four.
+#define MJ_ROWS_BLOCKS_PER_SM 24
+template <int T>                                      // tuples a lane
+__global__ void __launch_bounds__(256, 6)
 k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin, uint32_t range,
 		const uint32_t* __restrict__ end, const unsigned long long* __restrict__ val, uint32_t wsel,
 		uint4* __restrict__ out, uint64_t cap, unsigned long long* __restrict__ cursor, const unsigned int* __restrict__ meta,
@@ -613,11 +614,11 @@ k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin,
 	const uint64_t pol = pg_policy_evict_first(), keep = pg_policy_keep(4);
 	const uint64_t nwarps = ((uint64_t) gridDim.x * blockDim.x) >> 5;
 	const uint32_t w0 = wsel & 15, w1 = (wsel >> 4) & 15, w2 = (wsel >> 8) & 15, w3 = (wsel >> 12) & 15;
-	for (uint64_t c0 = (((uint64_t) blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (32 * MJ_ROWS_TUPLES); c0 < n; c0 += nwarps * (32 * MJ_ROWS_TUPLES)) {
-		uint4 t[MJ_ROWS_TUPLES];
-		uint32_t lo[MJ_ROWS_TUPLES], m[MJ_ROWS_TUPLES];
+	for (uint64_t c0 = (((uint64_t) blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (32 * T); c0 < n; c0 += nwarps * (32 * T)) {
+		uint4 t[T];
+		uint32_t lo[T], m[T];
 		#pragma unroll
-		for (int j = 0; j < MJ_ROWS_TUPLES; ++j) {
+		for (int j = 0; j < T; ++j) {
 			const uint64_t i = c0 + j * 32 + lane;
 			lo[j] = 0; m[j] = 0;
 			t[j] = make_uint4(0, 0, 0, 0);
@@ -629,9 +630,9 @@ k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin,
 				}
 			}
 		}
-		uint32_t off[MJ_ROWS_TUPLES], total = 0;
+		uint32_t off[T], total = 0;
 		#pragma unroll
-		for (int j = 0; j < MJ_ROWS_TUPLES; ++j) {
+		for (int j = 0; j < T; ++j) {
 			m[j] -= lo[j];
 			uint32_t x = m[j];
 			#pragma unroll
@@ -647,7 +648,7 @@ k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin,
 		if (lane == 0 && total) row = atomicAdd(cursor, (unsigned long long) total);
 		row = __shfl_sync(0xffffffffu, row, 0);
 		#pragma unroll
-		for (int j = 0; j < MJ_ROWS_TUPLES; ++j) {
+		for (int j = 0; j < T; ++j) {
 			for (uint32_t r0 = 0; r0 < m[j]; r0 += 32) {
 				const uint32_t r = r0 + lane;
 				uint32_t x = 0;                  // the last tuple whose offset is <= r (it has rows)
@@ -716,6 +717,12 @@ static bool mj_v16(const pg_rel* r)
 		!(reinterpret_cast<uintptr_t>(r->data) & 15);
 }
 
+// Rows of more tuples than this partition both sides first: 64M x 64M with four
+// duplicates a key 6.83 -> 4.40 ms (4-byte values; by sorting both sides in buckets 5.98),
+// 48M with 2-byte values and a group-by 4.76 -> 3.80; 32M 2.33 -> 2.74 with 2-byte values,
+// 4.16 -> 3.74 with 4-byte ones.
+#define MJ_SPLIT_TUPLES (32ull << 20)
+
 // The join by a table of counts when the counted side's keys span a compact
 // range: at most 2^24 values, or 16 times its tuples (64 M x 64 M with 2^30
 // spans: the table's random accesses still cost less than sorting both sides).
@@ -775,12 +782,42 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 		uint32_t* cnt = nullptr;
 		uint64_t* sums = nullptr;
 		unsigned long long* val = nullptr;
-		auto release = [&]() { for (void* p : {(void*) cnt, (void*) sums, (void*) val}) pg_free_async(ctx, s, p); };
+		char* split[2] = {nullptr, nullptr};
+		auto release = [&]() {
+			for (void* p : {(void*) cnt, (void*) sums, (void*) val, (void*) split[0], (void*) split[1]}) pg_free_async(ctx, s, p);
+		};
+		// Rows of more tuples than L2 holds values of: both sides by the top 8 bits of
+		// the window first (without memory for the copies, as they are), then one piece of
+		// the input a block, so that the blocks in flight use the same part of the table.
+		bool parted = false;
+		if (materialize && C->n > MJ_SPLIT_TUPLES && P->n > MJ_SPLIT_TUPLES / 4) {
+			if (pg_alloc_async(ctx, s, (void**) &split[0], C->n * 16) == PG_OK &&
+					pg_alloc_async(ctx, s, (void**) &split[1], P->n * 16) == PG_OK) {
+				pg_hashfn f = {};
+				f.fn = PG_FN_PARAMMODULO;
+				f.nbuckets = 256;
+				f.min = kmin;
+				f.skipbits = range > 256 ? 24 - __builtin_clz(range - 1) : 0;
+				f.k = (int64_t) 255 << f.skipbits;
+				if ((rc = pg_partition_fn(ctx, s, C, f, split[0], nullptr)) ||
+						(rc = pg_partition_fn(ctx, s, P, f, split[1], nullptr))) { release(); pg_free_async(ctx, s, mm); return rc; }
+				parted = true;
+			} else {
+				cudaGetLastError();
+				if (split[0]) { pg_free_async(ctx, s, split[0]); split[0] = nullptr; }
+				split[1] = nullptr;
+			}
+		}
+		const char* const cdata = (const char*) (parted ? split[0] : C->data);
+		const char* const pdata = (const char*) (parted ? split[1] : P->data);
+		auto grid = [&](uint64_t n, uint32_t per_block, uint32_t per_sm) -> int {
+			const uint64_t b = pg_div_up(n, per_block);
+			return (int) (parted ? b : std::min<uint64_t>(b, (uint64_t) ctx->sm_count * per_sm));
+		};
 		if ((rc = pg_alloc_async(ctx, s, (void**) &cnt, (uint64_t) range * 4))) return rc;
 		PG_CUDA(ctx, cudaMemsetAsync(cnt, 0, (uint64_t) range * 4, s));
-		const int cblocks = (int) std::min<uint64_t>(pg_div_up(C->n, 256 * MJ_ILP), (uint64_t) ctx->sm_count * MJ_BLOCKS_PER_SM);
-		const int pblocks = (int) std::min<uint64_t>(pg_div_up(P->n, 256 * MJ_ILP), (uint64_t) ctx->sm_count * MJ_BLOCKS_PER_SM);
-#define MJ_COUNT(V, VALS) k_mj_count<V, VALS><<<cblocks, 256, 0, s>>>((const char*) C->data, C->n, C->width, C->key_off, \
+		const int cblocks = grid(C->n, 256 * MJ_ILP, MJ_BLOCKS_PER_SM), pblocks = grid(P->n, 256 * MJ_ILP, MJ_BLOCKS_PER_SM);
+#define MJ_COUNT(V, VALS) k_mj_count<V, VALS><<<cblocks, 256, 0, s>>>(cdata, C->n, C->width, C->key_off, \
 				C->key_bytes, kmin, range, cnt, meta + 1, bp, vmm)
 		if (materialize) MJ_COUNT(true, true);
 		else if (mj_v16(C)) MJ_COUNT(true, false);
@@ -803,13 +840,14 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 			if ((rc = pg_scan_u64(ctx, s, sums, nb, nullptr))) { release(); return rc; }
 			k_mj_scan_apply<<<(unsigned) nb, 256, 0, s>>>(cnt, range, sums);
 			PG_LAUNCHED(ctx);
-			const int fblocks = (int) std::min<uint64_t>(pg_div_up(C->n, 256), (uint64_t) ctx->sm_count * MJ_FILL_BLOCKS_PER_SM);
-			k_mj_fill<<<fblocks, 256, 0, s>>>((const char*) C->data, C->n, C->key_off, kmin, range, bp, cnt, val, meta, vmm);
+			const int fblocks = grid(C->n, 256, MJ_FILL_BLOCKS_PER_SM);
+			k_mj_fill<<<fblocks, 256, 0, s>>>(cdata, C->n, C->key_off, kmin, range, bp, cnt, val, meta, vmm);
 			PG_LAUNCHED(ctx);
-			const int rblocks = (int) std::min<uint64_t>(pg_div_up(P->n, 256 * MJ_ROWS_TUPLES),
-					(uint64_t) ctx->sm_count * MJ_ROWS_BLOCKS_PER_SM);
-			k_mj_rows<<<rblocks, 256, 0, s>>>((const char*) P->data, P->n, P->key_off, kmin, range, cnt, val, wsel,
-					reinterpret_cast<uint4*>(out), out_capacity, agg, meta, vmm);
+#define MJ_ROWS(T) k_mj_rows<T><<<grid(P->n, 256 * T, MJ_ROWS_BLOCKS_PER_SM), 256, 0, s>>>(pdata, P->n, P->key_off, kmin, \
+				range, cnt, val, wsel, reinterpret_cast<uint4*>(out), out_capacity, agg, meta, vmm)
+			if (!parted && C->n / 2 >= range) MJ_ROWS(2);
+			else MJ_ROWS(4);
+#undef MJ_ROWS
 			PG_LAUNCHED(ctx);
 		}
 		unsigned long long o[4];     // rows, sum, (largest count, key outside)

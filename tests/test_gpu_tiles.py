@@ -119,6 +119,30 @@ def test_mpsm_key_outside_the_sampled_window(ctx):
     assert n3 == n2 and np.array_equal(orc.canonical(got), orc.canonical(want))
 
 
+# Rows of over 32M build and 8M probe tuples go by a partition of both sides; a key off
+# the sampled window sends them to the exact one.
+@pytest.mark.parametrize("far", [False, True])
+def test_mpsm_rows_partitioned_first(ctx, far):
+    n, m = (32 << 20) + 3, (8 << 20) + 5
+    rng = np.random.default_rng(212)
+    R = np.stack([rng.permutation(n) - 9, rng.integers(0, 1 << 31, size=n)], axis=1)
+    S = np.stack([rng.integers(0, n, size=m) - 9, np.arange(m)], axis=1)
+    want = np.empty(n, dtype=np.int64)
+    want[R[:, 0] + 9] = R[:, 1]
+    want = want[S[:, 0] + 9]
+    if far:
+        old = R[1025, 0]
+        R[1025, 0] = 3 * n
+        S[S[:, 0] == old, 0] = 3 * n
+        S[5, 0], want[5] = 3 * n, R[1025, 1]
+    got, rows, _ = ctx.mpsm(R, S, proj=(("P", 8, 8), ("B", 8, 8)))
+    assert rows == m
+    got = np.ascontiguousarray(got).view(np.int64).reshape(-1, 2)
+    seen = np.full(m, -1, dtype=np.int64)
+    seen[got[:, 0]] = got[:, 1]
+    assert np.array_equal(seen, want)
+
+
 # 16-byte tuples and at most 256 buckets: tiles of 3072 rows over two blocks an
 # SM. Sizes around one tile, a chunk of several, keys in any word, 4-byte keys
 # and every kind of bucket function.
