@@ -81,9 +81,9 @@ typedef struct {
 enum { PG_JOIN_MATERIALIZE = 1, PG_JOIN_COUNT = 2, PG_JOIN_SUM = 4 };
 /* pg_mpsm_join only: that side is already sorted on its key, as a plan's
  * buildpresorted / probepresorted = "yes" states (SortMergeJoinOp::init,
- * operators/join.cpp:750-762). The device confirms it while it reads the key
- * range and then skips that side's sort or partition; a side that is not
- * sorted is sorted as usual, so the result never depends on the flags. */
+ * operators/join.cpp:750-762). Where the join sorts, the device confirms it and
+ * then skips that side's sort; a side that is not sorted is sorted as usual, so the
+ * result never depends on the flags. */
 enum { PG_JOIN_BUILD_SORTED = 8, PG_JOIN_PROBE_SORTED = 16 };
 
 /* ---------------------------------------------------------------------- */
@@ -147,8 +147,9 @@ enum {
 	                                    for other projections), 4 register loads without prefetch, 5 deeper
 	                                    pipeline (default for (P$1, B$1) rows of narrow dense tables) */
 	PG_TUNE_DENSE = 2,               /* 1: allow dense tables (default), 2: always hash */
-	PG_TUNE_PARTITION_TILE = 3,      /* partition tile bytes (8192..65536) */
-	PG_TUNE_GROUPBY_SMEM_GROUPS = 4, /* largest group count aggregated in shared memory first */
+	PG_TUNE_PARTITION_TILE = 3,      /* partition tile bytes (8192..65536), other than 16-byte tuples in at
+	                                    most 256 buckets */
+	PG_TUNE_GROUPBY_SMEM_GROUPS = 4, /* no effect: what fits in shared memory is aggregated there */
 	PG_TUNE_RADIX_BITS = 5,          /* radix sort digit: 4..12 bits (partition fan-out 2^bits) */
 	PG_TUNE_PROBE_ITEMS = 6,         /* dense-table lookups in flight per lane of the 16-byte probe: 4 or 8 */
 	PG_TUNE_PROBE_CACHE = 7,         /* 16-byte probe L2 policies: bits 0-1 table loads (0 evict-last,
@@ -370,9 +371,8 @@ int pg_hashjoin_groupby(pg_ctx* ctx, pg_stream stream, pg_hashtable* ht, const p
 /* ---------------------------------------------------------------------- */
 /* Page sort: TupleBuffer::sort<KeyT> / sortAllInPage (util/buffer.inl:135-292,
  * operators/join.cpp:893-912) and the bitonic block sort
- * (util/bitonicsort.cpp:371-443): bitonic sort of `tile`-tuple pages in
- * shared memory, then merge-path merges. Ascending signed key; ties in
- * unspecified order. `out` may not alias `in`.                            */
+ * (util/bitonicsort.cpp:371-443), by LSD radix passes. Ascending signed key; ties
+ * in unspecified order. `out` may not alias `in`.                         */
 /* ---------------------------------------------------------------------- */
 int pg_sort_pages(pg_ctx* ctx, pg_stream stream, const pg_rel* in, void* out);
 

@@ -30,8 +30,9 @@
 // value near the column's largest, whose low bits are zero, costs one
 // returning atomic, t2 overflows only about once per 2^(64 - PG_FX_TOP) such
 // values, and values far below the largest add fire-and-forget chunks.
-// Tables in shared memory, where returning adds are cheap, use a compact
-// four-word chained form instead (pg_fx_chain_add).
+// Tables in shared memory, where returning adds are cheap, keep less: the dense
+// group-by t2 and its overflows, the hashed one's caches a four-word chained form
+// (pg_fx_chain_add).
 //
 // Host and device: the host test checks quantisation, both table forms' adds
 // and the rounding against exact rational arithmetic.

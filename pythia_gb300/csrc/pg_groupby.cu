@@ -484,7 +484,7 @@ k_gb_dense(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, u
 }
 
 // Dense group-by over a window whose table fits in shared memory (GbShared). Int and
-// long sums are bound by the read, dec ones by instructions (137 a row, 59% of issue):
+// long sums are bound by the read, dec ones by instructions (75% of issue):
 // 64M rows in 300 groups 223, 224 and 352 us, as before but for dec's 520; in 3000 (over
 // 1500 in L2 before, dec at 57 bytes a slot) 223, 224 and 351 from 1540 to 1750; in
 // 12,000, long and dec with one CTA an SM, 230, 328 and 438 from 1550, 1550 and 1000. One

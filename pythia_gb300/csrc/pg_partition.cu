@@ -8,14 +8,17 @@
 // exactly what the reference produces when its threads read consecutive
 // slices.
 //
-// Pass 1 (k_part_hist) counts tuples per (bucket, CTA). An exclusive scan over
-// the bucket-major counts gives every CTA its first output slot per bucket.
-// Pass 2 (k_part_scatter) streams the chunk again in tiles staged in shared
-// memory by bulk copies (cp.async.bulk + mbarrier, double-buffered), ranks
-// tuples within the tile per bucket (per-warp ballots over the bucket bits +
-// per-warp counters, which keeps the order stable), and writes each tile out grouped by bucket so a
-// warp's stores go to consecutive addresses of one partition
-// (write-combining through shared memory).
+// 16-byte tuples and at most 256 buckets: k_chunk_hist counts tuples per (bucket,
+// block), an exclusive scan over the bucket-major counts gives every block its first
+// output slot per bucket, and k_part_sweep streams the block's tiles again, ranks
+// their tuples and stores each bucket's rows of a tile as one run.
+//
+// Other widths and fan-outs: k_part_hist counts and k_part_scatter moves tiles staged
+// in shared memory by bulk copies (cp.async.bulk + mbarrier, double-buffered). It ranks
+// tuples within the tile per bucket (per-warp ballots over the bucket bits + per-warp
+// counters, which keeps the order stable) and writes each tile out grouped by bucket, so a
+// warp's stores go to consecutive addresses of one partition (write-combining through
+// shared memory).
 #include "pg_internal.cuh"
 #include <algorithm>
 #include <type_traits>

@@ -1,22 +1,22 @@
-// Page sort on sm_103a: bitonic tile sort in shared memory + merge-path merges.
+// Page sort on sm_103a: LSD radix passes over key - min.
 //
 // Replaces TupleBuffer::sort<KeyT> (util/buffer.inl:135-292, std::sort on the
 // key at keyoffset, reached through sortAllInPage, operators/join.cpp:893-912)
 // and the SSE bitonic block sort (util/bitonicsort.cpp:371-443), which sorts
 // 4096-record cache blocks with a bitonic network and then merges blocks
-// pairwise. The same structure here: a CTA stages a 4096-tuple page in shared
-// memory (bulk copy, cp.async.bulk + mbarrier), sorts (key, position) pairs
-// with a bitonic network, and writes the page in key order; then log2(n/4096)
-// merge passes, each CTA producing 2048 outputs of a run pair located by a
-// merge-path binary search (Odeh et al., "Merge Path", 2012).
+// pairwise.
 //
-// Keys spanning at most 2^32 values take an LSD radix path instead (see
-// radix_sort below). Tuples travel as 16-byte records {int64 key, uint64 val}. A 16-byte tuple
-// with an 8-byte key is its own record (the key half first); any other layout
-// sorts (widened key, row index) records and gathers rows at the end. Ties are
-// left in unspecified order, as std::sort leaves them. Unlike the reference's
-// bitonic path (asserting power-of-two sizes above 4096 records,
-// util/buffer.cpp:101-104) any n is accepted, including n = 4096.
+// Up to 2^20 tuples take one cooperative launch (k_sort_small); more take stable
+// 256-way passes of the partition, over a key window from a sample that the first
+// pass checks (radix_passes). Tuples travel as 16-byte records {int64 key, uint64 val}: a
+// 16-byte tuple with an 8-byte key is its own record; any other layout sorts (widened
+// key, row index) records and gathers rows at the end. The reference's structure, 4096-tuple
+// bitonic pages and log2(n/4096) merge passes, each CTA producing 2048 outputs of a
+// run pair located by a merge-path binary search (Odeh et al., "Merge Path", 2012), stays
+// behind PG_TUNE_SORT_PATH. Ties are left in unspecified
+// order, as std::sort leaves them. Unlike the reference's bitonic path (asserting
+// power-of-two sizes above 4096 records, util/buffer.cpp:101-104) any n is accepted,
+// including n = 4096.
 #include "pg_internal.cuh"
 #include "pg_sort.cuh"
 #include <algorithm>
