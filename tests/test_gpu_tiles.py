@@ -309,7 +309,7 @@ def test_groupby_shared_table_24_byte_rows(ctx, n, val):
 # flush fewer slots than there are probe tuples; the global table past that. Sizes
 # around a block's 1024 tuples, and probe misses.
 @pytest.mark.parametrize("probe,groups", [(1, 1), (1023, 5), (1025, 9), (3_000_000, 2163), (3_000_000, 2164),
-                                          (3_000_000, 17_644), (3_000_000, 17_645)])
+                                          (3_000_000, 17_644), (3_000_000, 17_645), (3_000_000, 46_000)])
 @pytest.mark.parametrize("swap", [False, True])
 def test_hashjoin_groupby_shared_tables(ctx, probe, groups, swap):
     build = 2 * groups + 1
