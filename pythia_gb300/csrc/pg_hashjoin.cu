@@ -2542,7 +2542,8 @@ static int hj_make_cols(pg_ctx* ctx, const pg_hashtable* ht, const pg_col* proj,
 #define HJ_TWO_PASS_MAX_BYTES (112ull << 20)  // ... up to this (half must fit in L2)
 
 // Launches the unique-key probe over n tuples at S (device) into `out`;
-// counts/sums accumulate in acc[1..2], the output cursor is acc[0].
+// counts/sums accumulate in acc[1..2], the output cursor is acc[0]. `spec`: the
+// table was seen unsettled (hj_view).
 // With `counts` (device, one word per 256-tuple chunk) and cap >= n, 16-byte
 // probes use the warp-independent kernel and write rows positionally; the
 // caller then compacts when fewer than n rows matched (*positional = true).
@@ -2565,7 +2566,7 @@ static int hjg_launch(pg_ctx* ctx, cudaStream_t s, const char* S, uint64_t n, ui
 	return PG_OK;
 }
 
-static int hj_launch_unique(pg_ctx* ctx, cudaStream_t s, const pg_hashtable* ht, const char* S,
+static int hj_launch_unique(pg_ctx* ctx, cudaStream_t s, const pg_hashtable* ht, bool spec, const char* S,
 		uint64_t n, uint32_t W, uint32_t koff, uint32_t kbytes, const HjCols& pc, char* out,
 		uint64_t cap, unsigned long long* acc, bool materialize, int sum_col,
 		uint64_t* counts = nullptr, bool* positional = nullptr, const PgPred16* pred = nullptr)
@@ -2573,9 +2574,8 @@ static int hj_launch_unique(pg_ctx* ctx, cudaStream_t s, const pg_hashtable* ht,
 	if (positional) *positional = false;
 	const uint64_t ntiles = pg_div_up(n, HJ_TILE);
 	HjProbeTable tb;
-	// A speculative table is described by its header and window base alone
-	// (read once: another thread may settle it meanwhile).
-	const bool spec = ht->spec.load(std::memory_order_acquire);
+	// A speculative table (`spec`, as the caller saw it) is described by its header
+	// and window base alone: another thread may settle it meanwhile.
 	if (spec) {
 		tb = HjProbeTable();
 		tb.hdr = ht->hdr; tb.dense32 = ht->dense32_base;
@@ -2624,7 +2624,8 @@ static int hj_launch_unique(pg_ctx* ctx, cudaStream_t s, const pg_hashtable* ht,
 			// Two passes over half the table each when the dense table is
 			// larger than L2 keeps next to the streams (knob: 1 one pass,
 			// 2 two passes, 0 by table size).
-			const uint64_t tbytes = mode == 2 ? ht->drange * 4 : ht->drange * 8;
+			const uint64_t dr = spec || mode == 0 ? 0 : ht->drange;
+			const uint64_t tbytes = mode == 2 ? dr * 4 : dr * 8;
 			const int64_t pk = pred ? 1 : ctx->tune[PG_TUNE_PROBE_PASSES];
 			// Dense tables take the register-loading probe unless the knob asks
 			// for the staged one (1) or the non-prefetching one (4).
@@ -2632,7 +2633,6 @@ static int hj_launch_unique(pg_ctx* ctx, cudaStream_t s, const pg_hashtable* ht,
 			const bool direct = mode != 0 && (var == 0 || var == 3 || var == 4 || var == 5);
 			const int passes = mode == 0 || pk == 1 ? 1
 				: (pk == 2 || (!direct && tbytes > HJ_TWO_PASS_MIN_BYTES && tbytes <= HJ_TWO_PASS_MAX_BYTES)) ? 2 : 1;
-			const uint64_t dr = mode == 0 ? 0 : ht->drange;
 			// Counts and sums over a hashed table (knob 1: the staged probe).
 			if (mode == 0 && !materialize && var != 1) {
 				const int ablocks = (int) std::min<uint64_t>(pg_div_up(n, 256), (uint64_t) ctx->sm_count * HA_BLOCKS_PER_SM);
@@ -2854,7 +2854,8 @@ static int hj_probe_run(pg_ctx* ctx, pg_stream stream, pg_hashtable* ht,
 	pg_rel Sloc = *S_in;
 	const pg_rel* S = &Sloc;
 	HjScratch part_buf(ctx, s);
-	if (const uint32_t lp = hj_probe_partition_bits(ctx, ht, S_in->n)) {
+	const HjView view = hj_view(*ht);
+	if (const uint32_t lp = view.spec ? 0 : hj_probe_partition_bits(ctx, ht, S_in->n)) {
 		if ((rc = pg_alloc_async(ctx, s, &part_buf.p, S_in->n * S_in->width))) return rc;
 		pg_hashfn f;
 		f.fn = PG_FN_MIXRADIX; f.k = 0; f.min = 0; f.max = 0; f.bucketrange = 0;
@@ -2868,11 +2869,11 @@ static int hj_probe_run(pg_ctx* ctx, pg_stream stream, pg_hashtable* ht,
 	const uint64_t ntiles = pg_div_up(S->n, HJ_TILE);
 	unsigned long long host_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 
-	if (ht->unique && ht->inline_val) {
+	if (view.unique && ht->inline_val) {
 		const char* Sd = (const char*) S->data;
 		// A speculative table's checks come back with the counts; when they
 		// failed, the kernels wrote nothing and the caller rebuilds.
-		const bool spec = ht->spec.load(std::memory_order_acquire);
+		const bool spec = view.spec;
 		const HjDenseHdr* hdr = spec ? ht->hdr : nullptr;
 		bool refuted = false;
 		if (spec) PG_CUDA(ctx, cudaStreamWaitEvent(s, ht->built, 0));
@@ -2880,7 +2881,7 @@ static int hj_probe_run(pg_ctx* ctx, pg_stream stream, pg_hashtable* ht,
 			uint64_t* counts = nullptr;
 			bool positional = false;
 			if ((rc = pg_alloc_async(ctx, s, (void**) &counts, pg_div_up(S->n, PW_CHUNK) * 8))) return rc;
-			if ((rc = hj_launch_unique(ctx, s, ht, Sd, S->n, S->width, S->key_off, S->key_bytes, pc,
+			if ((rc = hj_launch_unique(ctx, s, ht, spec, Sd, S->n, S->width, S->key_off, S->key_bytes, pc,
 					(char*) out, out_capacity, acc, true, -1, counts, &positional, pred))) {
 				pg_free_async(ctx, s, counts); pg_free_async(ctx, s, acc);
 				return rc;
@@ -2899,14 +2900,14 @@ static int hj_probe_run(pg_ctx* ctx, pg_stream stream, pg_hashtable* ht,
 			pg_free_async(ctx, s, counts);
 			if (sum_col >= 0 || (flags & PG_JOIN_COUNT)) {
 				// Fold count/sum with a second, non-materialising pass.
-				if ((rc = hj_launch_unique(ctx, s, ht, Sd, S->n, S->width, S->key_off, S->key_bytes, pc,
+				if ((rc = hj_launch_unique(ctx, s, ht, spec, Sd, S->n, S->width, S->key_off, S->key_bytes, pc,
 						nullptr, 0, acc, false, sum_col, nullptr, nullptr, pred))) return rc;
 				PG_CUDA(ctx, cudaMemcpyAsync(host_acc, acc, 32, cudaMemcpyDeviceToHost, s));
 				if ((rc = pg_check_status(ctx, s, "pg_hashjoin_probe"))) return rc;
 				res->sum = (int64_t) host_acc[2];
 			}
 		} else {
-			if ((rc = hj_launch_unique(ctx, s, ht, Sd, S->n, S->width, S->key_off, S->key_bytes, pc,
+			if ((rc = hj_launch_unique(ctx, s, ht, spec, Sd, S->n, S->width, S->key_off, S->key_bytes, pc,
 					nullptr, 0, acc, false, sum_col, nullptr, nullptr, pred))) {
 				pg_free_async(ctx, s, acc);
 				return rc;
@@ -3057,7 +3058,7 @@ extern "C" int pg_hashjoin_probe_spans(pg_ctx* ctx, pg_stream stream, pg_hashtab
 		for (int i = 0; i < nspans && !rc; ++i) {
 			const pg_rel& S = spans[i];
 			if (!S.n) continue;
-			rc = hj_launch_unique(ctx, s, ht, (const char*) S.data, S.n, S.width, S.key_off, S.key_bytes, pc,
+			rc = hj_launch_unique(ctx, s, ht, false, (const char*) S.data, S.n, S.width, S.key_off, S.key_bytes, pc,
 					m ? (char*) out : nullptr, m ? out_capacity : 0, acc, m, m ? -1 : sum_col);
 		}
 	}
@@ -3174,10 +3175,10 @@ extern "C" int pg_hashjoin_host(pg_ctx* ctx, const pg_rel* Rh, const pg_rel* Sh,
 		HJH_TRY(cudaStreamWaitEvent(scomp, ev_in[b], 0));
 		if (c >= 2) HJH_TRY(cudaStreamWaitEvent(scomp, ev_out[b], 0));   // output buffer free
 		HJH_TRY(cudaMemsetAsync(acc + 4 * b, 0, 32, scomp));
-		if (materialize && hj_launch_unique(ctx, scomp, ht, dS[b], rows, Sh->width, Sh->key_off, Sh->key_bytes,
+		if (materialize && hj_launch_unique(ctx, scomp, ht, false, dS[b], rows, Sh->width, Sh->key_off, Sh->key_bytes,
 				pc, dO[b], CH, acc + 4 * b, true, -1, dC[b], &posit[b])) { cleanup(); return PG_ERR_CUDA; }
 		if ((!materialize || sum_col >= 0 || (flags & PG_JOIN_COUNT)) &&
-				hj_launch_unique(ctx, scomp, ht, dS[b], rows, Sh->width, Sh->key_off, Sh->key_bytes,
+				hj_launch_unique(ctx, scomp, ht, false, dS[b], rows, Sh->width, Sh->key_off, Sh->key_bytes,
 				pc, nullptr, 0, acc + 4 * b, false, sum_col)) { cleanup(); return PG_ERR_CUDA; }
 		HJH_TRY(cudaGetLastError());
 		HJH_TRY(cudaMemcpyAsync(hacc + 4 * b, acc + 4 * b, 32, cudaMemcpyDeviceToHost, scomp));

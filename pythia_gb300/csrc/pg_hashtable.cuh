@@ -4,6 +4,7 @@
 #define PG_HASHTABLE_CUH
 
 #include "pg_internal.cuh"
+#include "pg_tableview.h"
 #include <atomic>
 #include <mutex>
 

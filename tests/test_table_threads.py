@@ -1,0 +1,90 @@
+"""Join tables whose first uses come from several threads at once: the order in
+which a probe reads a table that another thread settles (on the host, with a fake
+table), and probes of fresh tables of repeated keys from threads of their own."""
+import ctypes
+import os
+import shutil
+import subprocess
+import threading
+
+import numpy as np
+import pytest
+
+from pythia_gb300 import datagen as dg
+from pythia_gb300 import gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def test_a_table_settled_between_two_reads_is_never_seen_settled_and_unique(tmp_path):
+    cxx = shutil.which("g++")
+    if not cxx:
+        pytest.skip("no host C++ compiler")
+    so = str(tmp_path / "libtableview.so")
+    subprocess.run([cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-I" + os.path.join(ROOT, "pythia_gb300", "csrc"),
+                    os.path.join(ROOT, "tests", "native", "tableview_shim.cpp"), "-o", so], check=True)
+    L = ctypes.CDLL(so)
+    for k in range(4):                          # before the first read .. after the last
+        v = L.tableview_settled_before(k)
+        spec, unique = bool(v & 1), bool(v & 2)
+        assert spec or not unique, k            # repeated keys: unique only while the header checks it
+        assert not spec or unique, k            # an unsettled table goes by its header
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", ["dense", "repeated", "far", "wide"])
+def test_first_probes_from_several_threads(ctx, case):
+    # Every build of 16-byte tuples is first used unsettled: four threads, each on a
+    # stream of its own, count and sum a fresh table's matches at once.
+    L, threads, n = gpu.lib(), 4, 3000
+    R = dg.build_relation(n, dg.seed_for(301))
+    S = dg.probe_uniform(2 * n, R, dg.seed_for(302))
+    if case == "repeated":
+        R[n // 2:, 0] = R[: n // 2, 0]
+    elif case == "far":
+        R[:, 0] *= -7046029254386353131
+        S[:, 0] *= -7046029254386353131
+    elif case == "wide":
+        R[0, 1] = -5
+    order = np.argsort(R[:, 0], kind="stable")
+    keys, vals = R[order, 0], R[order, 1].astype(np.uint64)
+    lo, hi = np.searchsorted(keys, S[:, 0], "left"), np.searchsorted(keys, S[:, 0], "right")
+    pre = np.concatenate([np.zeros(1, np.uint64), np.cumsum(vals, dtype=np.uint64)])
+    want = (int((hi - lo).sum()), int((pre[hi] - pre[lo]).sum(dtype=np.uint64).astype(np.int64)))
+    dR, dS = ctx.upload(R), ctx.upload(S)
+    rR, rS = ctx.rel(dR, n, 16), ctx.rel(dS, 2 * n, 16)
+    c, nc = gpu.cols((("P", 8, 8), ("B", 8, 8)))
+    streams = []
+    for _ in range(threads):
+        s = ctypes.c_void_p()
+        ctx._check(L.pg_stream_create(ctx.h, ctypes.byref(s)))
+        streams.append(s.value)
+    bad = []
+    gate, done = threading.Barrier(threads + 1), threading.Barrier(threads + 1)
+    state = {"ht": None, "rounds": 300}
+
+    def probe(k):
+        for _ in range(state["rounds"]):
+            gate.wait()
+            res = gpu.JoinResult()
+            rc = L.pg_hashjoin_probe(ctx.h, streams[k], state["ht"], ctypes.byref(rS), c, nc, None, 0,
+                                     gpu.JOIN_COUNT | gpu.JOIN_SUM, 1, ctypes.byref(res))
+            if rc or (res.n_out, res.sum) != want:
+                bad.append((k, rc, res.n_out, res.sum))
+            done.wait()
+
+    workers = [threading.Thread(target=probe, args=(k,), daemon=True) for k in range(threads)]
+    for t in workers:
+        t.start()
+    for _ in range(state["rounds"]):
+        ht = ctypes.c_void_p()
+        ctx._check(L.pg_hashjoin_build(ctx.h, ctx.stream, ctypes.byref(rR), c, nc, ctypes.byref(ht)))
+        state["ht"] = ht.value
+        gate.wait()
+        done.wait()
+        L.pg_hashtable_free(ctx.h, ht)
+    for t in workers:
+        t.join()
+    for s in streams:
+        L.pg_stream_destroy(ctx.h, s)
+    assert not bad, bad[:5]
