@@ -29,6 +29,7 @@
 #include "pg_groupshared.cuh"
 #include "pg_pred.cuh"
 #include <algorithm>
+#include <cstddef>
 #include <vector>
 
 #define HJ_THREADS 256
@@ -2382,18 +2383,50 @@ static bool hj_hdr_ok(const HjDenseHdr& h)
 	return h.flags == 0 && h.present == h.n;
 }
 
-// `refuted`: the header's flags, present entries and tuples as a probe read
-// them back when its checks failed (no second round trip), else null.
-static int hj_settle_known(pg_ctx* ctx, pg_hashtable* ht, const unsigned long long* refuted)
+// Whether a good table's narrowed window needs a copy of its entries: based on the
+// smallest value, and on a 16-byte boundary (table readers, the image checksum's
+// 8-byte words and vector loads, rely on the alignment of an allocation).
+static bool hj_hdr_rebase(const HjDenseHdr& h)
+{
+	return h.vlo != h.vmin || (((h.kmin ^ (1ull << 63)) - (unsigned long long) h.dmin) & 3) != 0;
+}
+
+// The exact layout of a good table, as hj_build_exact would have made it: the
+// window `win` narrowed to the keys present, entries based on the smallest value.
+static void hj_settle_good(pg_hashtable* ht, const HjDenseHdr& h, uint32_t* win)
+{
+	ht->dense32 = win;
+	ht->dmin = (long long) (h.kmin ^ (1ull << 63));
+	ht->drange = h.kmax - h.kmin + 1;
+	ht->vmin = h.vlo; ht->vlo = h.vlo; ht->vmax = h.vhi;
+	ht->spec.store(false, std::memory_order_release);
+}
+
+// After a probe on stream s read back a good header (the build is over then): the
+// table is settled at once where no copy is needed, which always holds for builds of
+// up to 2^20 tuples. Later probes then take it as it is, and the spare slots, 32 of a
+// 1M-tuple table's 41 MB, are given back.
+static void hj_settle_probed(pg_ctx* ctx, cudaStream_t s, pg_hashtable* ht, const HjDenseHdr& h)
+{
+	if (hj_hdr_rebase(h)) return;
+	std::lock_guard<std::mutex> g(ht->mu);
+	if (!ht->spec.load(std::memory_order_relaxed)) return;
+	pg_free_async(ctx, s, ht->small_slots);
+	ht->small_slots = nullptr;
+	hj_settle_good(ht, h, ht->dense32_base + (h.kmin ^ (1ull << 63)) - (unsigned long long) h.dmin);
+}
+
+// `refuted`: the header as a probe read it back when its checks failed (no second
+// round trip), else null.
+static int hj_settle_known(pg_ctx* ctx, pg_hashtable* ht, const HjDenseHdr* refuted)
 {
 	if (!ht || !ht->spec.load(std::memory_order_acquire)) return PG_OK;
 	std::lock_guard<std::mutex> g(ht->mu);
 	if (!ht->spec.load(std::memory_order_relaxed)) return PG_OK;
 	cudaStream_t s = ht->stream;
 	HjDenseHdr h;
-	if (refuted) {
-		h.flags = (int) refuted[0]; h.present = refuted[1]; h.n = refuted[2];
-	} else {
+	if (refuted) h = *refuted;
+	else {
 		PG_CUDA(ctx, cudaMemcpyAsync(&h, ht->hdr, sizeof h, cudaMemcpyDeviceToHost, s));
 		PG_CUDA(ctx, cudaStreamSynchronize(s));
 	}
@@ -2402,16 +2435,9 @@ static int hj_settle_known(pg_ctx* ctx, pg_hashtable* ht, const unsigned long lo
 		ht->small_slots = nullptr;
 	}
 	if (hj_hdr_ok(h)) {
-		// Exact layout, as hj_build_exact would have made it: the window
-		// narrowed to the keys present, entries based on the smallest value.
-		const long long kmin = (long long) (h.kmin ^ (1ull << 63)), kmax = (long long) (h.kmax ^ (1ull << 63));
-		const unsigned long long off = (unsigned long long) kmin - (unsigned long long) h.dmin;
-		uint32_t* win = ht->dense32_base + off;
-		const unsigned long long range = (unsigned long long) kmax - (unsigned long long) kmin + 1;
-		// A copy too when the narrowed window would not start on a 16-byte
-		// boundary: table readers (the image checksum's 8-byte words, vector
-		// loads) rely on the alignment of an allocation.
-		if (h.vlo != h.vmin || (off & 3) != 0) {
+		uint32_t* win = ht->dense32_base + (h.kmin ^ (1ull << 63)) - (unsigned long long) h.dmin;
+		if (hj_hdr_rebase(h)) {
+			const unsigned long long range = h.kmax - h.kmin + 1;
 			int rc;
 			if ((rc = pg_alloc_async(ctx, s, (void**) &ht->dense32_copy, range * 4))) return rc;
 			const int grid = (int) std::min<uint64_t>(pg_div_up(range, 256), (uint64_t) ctx->sm_count * 8);
@@ -2420,11 +2446,7 @@ static int hj_settle_known(pg_ctx* ctx, pg_hashtable* ht, const unsigned long lo
 			PG_CUDA(ctx, cudaStreamSynchronize(s));      // users on other streams read the copy next
 			win = ht->dense32_copy;
 		}
-		ht->dense32 = win;
-		ht->dmin = kmin;
-		ht->drange = range;
-		ht->vmin = h.vlo; ht->vlo = h.vlo; ht->vmax = h.vhi;
-		ht->spec.store(false, std::memory_order_release);
+		hj_settle_good(ht, h, win);
 		return PG_OK;
 	}
 	// Refuted (a repeated key, a key or value the sample missed): rebuild
@@ -2805,29 +2827,34 @@ static int hj_compact(pg_ctx* ctx, cudaStream_t s, char* out, uint64_t n, uint64
 	return PG_OK;
 }
 
-// The probe's accumulators acc[0..3] with, in acc[4..7], a speculative
-// table's checks (flags, present entries, tuples) and the context's status
-// word, so that one copy brings all of them back.
+// The probe's accumulators acc[0..3] with, from acc[4] on, the context's status word
+// and a speculative table's header, so that one copy brings all of them back.
+struct HjReadback {
+	unsigned long long acc[4];        // [cursor, count, sum, spare]
+	unsigned long long status;
+	HjDenseHdr hdr;
+};
 __global__ void k_probe_tail(unsigned long long* __restrict__ acc, const HjDenseHdr* __restrict__ hdr,
 		const int* __restrict__ status)
 {
-	acc[4] = hdr ? (unsigned long long) (unsigned) hdr->flags : 0;
-	acc[5] = hdr ? hdr->present : 0;
-	acc[6] = hdr ? hdr->n : 0;
-	acc[7] = (unsigned long long) (unsigned) *status;
+	HjReadback* const r = reinterpret_cast<HjReadback*>(acc);
+	r->status = (unsigned long long) (unsigned) *status;
+	if (hdr) r->hdr = *hdr;
 }
 
-// One round trip after a probe: h = acc[0..7]; a non-zero status fails the
-// call; *refuted: the speculative table's checks failed (nothing was probed).
-static int hj_readback(pg_ctx* ctx, cudaStream_t s, unsigned long long* acc, const HjDenseHdr* hdr,
-		unsigned long long (&h)[8], bool* refuted, const char* what)
+// One round trip after a probe of `ht` (seen unsettled: hdr, else null); a non-zero
+// status fails the call; *refuted: the table's checks failed and nothing was probed,
+// else it may be settled now.
+static int hj_readback(pg_ctx* ctx, cudaStream_t s, unsigned long long* acc, pg_hashtable* ht, const HjDenseHdr* hdr,
+		HjReadback& h, bool* refuted, const char* what)
 {
 	k_probe_tail<<<1, 1, 0, s>>>(acc, hdr, ctx->d_status);
 	PG_LAUNCHED(ctx);
-	PG_CUDA(ctx, cudaMemcpyAsync(h, acc, sizeof h, cudaMemcpyDeviceToHost, s));
+	PG_CUDA(ctx, cudaMemcpyAsync(&h, acc, hdr ? sizeof h : offsetof(HjReadback, hdr), cudaMemcpyDeviceToHost, s));
 	PG_CUDA(ctx, cudaStreamSynchronize(s));
-	if (h[7]) return pg_status_fail(ctx, s, (int) h[7], what);
-	*refuted = hdr && !(h[4] == 0 && h[5] == h[6]);
+	if (h.status) return pg_status_fail(ctx, s, (int) h.status, what);
+	*refuted = hdr && !hj_hdr_ok(h.hdr);
+	if (hdr && !*refuted) hj_settle_probed(ctx, s, ht, h.hdr);
 	return PG_OK;
 }
 
@@ -2836,7 +2863,7 @@ static int hj_readback(pg_ctx* ctx, cudaStream_t s, unsigned long long* acc, con
 static int hj_probe_run(pg_ctx* ctx, pg_stream stream, pg_hashtable* ht,
 		const pg_rel* S_in, const pg_col* proj, int nproj,
 		void* out, uint64_t out_capacity, int flags, int sum_col, pg_join_result* res, const PgPred16* pred,
-		unsigned long long (&checks)[3])
+		HjDenseHdr* checks)
 {
 	if (!ctx || !ht || !res) return pg_fail(ctx, PG_ERR_ARG, "pg_hashjoin_probe: null argument");
 	int rc;
@@ -2864,10 +2891,11 @@ static int hj_probe_run(pg_ctx* ctx, pg_stream stream, pg_hashtable* ht,
 		Sloc.data = part_buf.p;
 	}
 	unsigned long long* acc = nullptr;   // [cursor, count, sum, spare]
-	if ((rc = pg_alloc_async(ctx, s, (void**) &acc, 64))) return rc;
-	PG_CUDA(ctx, cudaMemsetAsync(acc, 0, 64, s));
+	if ((rc = pg_alloc_async(ctx, s, (void**) &acc, sizeof(HjReadback)))) return rc;
+	PG_CUDA(ctx, cudaMemsetAsync(acc, 0, 32, s));
 	const uint64_t ntiles = pg_div_up(S->n, HJ_TILE);
-	unsigned long long host_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+	HjReadback rb = {};
+	unsigned long long (&host_acc)[4] = rb.acc;
 
 	if (view.unique && ht->inline_val) {
 		const char* Sd = (const char*) S->data;
@@ -2886,10 +2914,10 @@ static int hj_probe_run(pg_ctx* ctx, pg_stream stream, pg_hashtable* ht,
 				pg_free_async(ctx, s, counts); pg_free_async(ctx, s, acc);
 				return rc;
 			}
-			if ((rc = hj_readback(ctx, s, acc, hdr, host_acc, &refuted, "pg_hashjoin_probe"))) return rc;
+			if ((rc = hj_readback(ctx, s, acc, ht, hdr, rb, &refuted, "pg_hashjoin_probe"))) return rc;
 			if (refuted) {
 				pg_free_async(ctx, s, counts); pg_free_async(ctx, s, acc);
-				for (int i = 0; i < 3; ++i) checks[i] = host_acc[4 + i];
+				*checks = rb.hdr;
 				return HJ_SPEC_REFUTED;
 			}
 			res->n_out = host_acc[0];
@@ -2912,10 +2940,10 @@ static int hj_probe_run(pg_ctx* ctx, pg_stream stream, pg_hashtable* ht,
 				pg_free_async(ctx, s, acc);
 				return rc;
 			}
-			if ((rc = hj_readback(ctx, s, acc, hdr, host_acc, &refuted, "pg_hashjoin_probe"))) return rc;
+			if ((rc = hj_readback(ctx, s, acc, ht, hdr, rb, &refuted, "pg_hashjoin_probe"))) return rc;
 			if (refuted) {
 				pg_free_async(ctx, s, acc);
-				for (int i = 0; i < 3; ++i) checks[i] = host_acc[4 + i];
+				*checks = rb.hdr;
 				return HJ_SPEC_REFUTED;
 			}
 			res->n_out = host_acc[1];
@@ -2963,11 +2991,11 @@ static int hj_probe(pg_ctx* ctx, pg_stream stream, pg_hashtable* ht,
 		const pg_rel* S, const pg_col* proj, int nproj,
 		void* out, uint64_t out_capacity, int flags, int sum_col, pg_join_result* res, const PgPred16* pred)
 {
-	unsigned long long checks[3];
-	int rc = hj_probe_run(ctx, stream, ht, S, proj, nproj, out, out_capacity, flags, sum_col, res, pred, checks);
+	HjDenseHdr checks;
+	int rc = hj_probe_run(ctx, stream, ht, S, proj, nproj, out, out_capacity, flags, sum_col, res, pred, &checks);
 	if (rc != HJ_NEED_SETTLE && rc != HJ_SPEC_REFUTED) return rc;
-	if ((rc = hj_settle_known(ctx, ht, rc == HJ_SPEC_REFUTED ? checks : nullptr))) return rc;
-	return hj_probe_run(ctx, stream, ht, S, proj, nproj, out, out_capacity, flags, sum_col, res, pred, checks);
+	if ((rc = hj_settle_known(ctx, ht, rc == HJ_SPEC_REFUTED ? &checks : nullptr))) return rc;
+	return hj_probe_run(ctx, stream, ht, S, proj, nproj, out, out_capacity, flags, sum_col, res, pred, &checks);
 }
 
 extern "C" int pg_hashjoin_probe(pg_ctx* ctx, pg_stream stream, pg_hashtable* ht,

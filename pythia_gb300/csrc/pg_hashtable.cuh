@@ -20,7 +20,8 @@ struct HjBuildCols {            // build-projected columns packed into the value
 // side sets the key window and the value base on the device, the fill, store
 // and count kernels read them here, and the store and count kernels record
 // what the table must satisfy. A table whose header says "bad" is rebuilt
-// exactly on its first use (hj_settle).
+// exactly on its first use (hj_settle); a good one is settled by the first probe that
+// reads the header back, or by a use that needs the layout.
 struct HjDenseHdr {
 	long long dmin;              // key of entry 0 (window base)
 	unsigned long long drange;   // window entries (0 when the sample ruled the layout out)
@@ -81,7 +82,8 @@ struct pg_hashtable {
 	HjDenseHdr* hdr;
 	uint32_t* dense32_base;
 	uint32_t* dense32_copy;
-	unsigned long long* small_slots;  // up to 2^20 tuples: slots the build kernel fills when no dense layout fits
+	unsigned long long* small_slots;  // up to 2^20 tuples: slots the build kernel fills when no dense layout fits,
+	                                  // given back by the first use that finds one
 	cudaEvent_t built;          // recorded after the speculative build's kernels (null otherwise)
 	pg_rel rel;                 // the build relation, for an exact rebuild
 };

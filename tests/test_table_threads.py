@@ -88,3 +88,38 @@ def test_first_probes_from_several_threads(ctx, case):
     for s in streams:
         L.pg_stream_destroy(ctx.h, s)
     assert not bad, bad[:5]
+
+
+def _pool_bytes():
+    """Bytes in use in the device's default memory pool."""
+    rt = ctypes.CDLL("libcudart.so.13")
+    pool, used = ctypes.c_void_p(), ctypes.c_uint64()
+    assert rt.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+    assert rt.cudaMemPoolGetAttribute(pool, 7, ctypes.byref(used)) == 0     # cudaMemPoolAttrUsedMemCurrent
+    return used.value
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 3000, 1 << 20])
+def test_probed_dense_table_keeps_only_its_entries(ctx, n):
+    # 2n + n/8 + 4096 entries of 4 bytes and the header; the build's spare hashed
+    # slots (up to 32 bytes a tuple twice over) are gone after the first probe.
+    R = dg.build_relation(n, dg.seed_for(303))
+    S = dg.probe_uniform(1000, R, dg.seed_for(304))
+    dR, dS = ctx.upload(R), ctx.upload(S)
+    rR, rS = ctx.rel(dR, n, 16), ctx.rel(dS, 1000, 16)
+    c, nc = gpu.cols((("P", 8, 8), ("B", 8, 8)))
+    L, ht, res = gpu.lib(), ctypes.c_void_p(), gpu.JoinResult()
+    ctx.sync()
+    before = _pool_bytes()
+    ctx._check(L.pg_hashjoin_build(ctx.h, ctx.stream, ctypes.byref(rR), c, nc, ctypes.byref(ht)))
+    try:
+        for _ in range(2):
+            ctx._check(L.pg_hashjoin_probe(ctx.h, ctx.stream, ht, ctypes.byref(rS), c, nc, None, 0, gpu.JOIN_COUNT, -1,
+                                           ctypes.byref(res)))
+            assert res.n_out == 1000
+            ctx.sync()
+            kept = _pool_bytes() - before
+            assert kept <= 4 * (2 * n + n // 8 + 4096) + 4096, kept
+    finally:
+        L.pg_hashtable_free(ctx.h, ht)
