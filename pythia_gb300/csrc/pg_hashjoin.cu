@@ -399,8 +399,9 @@ __global__ void __launch_bounds__(1024) k_dense_prep16(const uint4* __restrict__
 
 // The same for smaller inputs in one cooperative launch, exactly: ranges over
 // every tuple, window, fill, store and count, with grid barriers where the form
-// for large inputs has launches, and where no dense layout fits (keys too far apart
-// or repeated) the hashed table, which the first use then finds ready. One block
+// for large inputs has launches, 8-byte entries for values that span too much, and
+// where no dense layout fits (keys too far apart or repeated) the hashed table, which
+// the first use then finds ready. One block
 // per 2048 tuples (a single one's barriers are block barriers). Whole joins of
 // 1000 tuples with 10,000: dense keys 73 -> 42 us, far ones 107 -> 78; of 16,000 with
 // 100,000: 84 -> 48 and 112 -> 90 (exact ranges and duplicate counts read back by the
@@ -488,10 +489,30 @@ __global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict
 		if (lane == 0 && c) atomicAdd(&acc->present, (unsigned long long) c);
 		meet();
 		h.present = va->present;
+	} else if (h.flags == 4) {
+		// Dense keys, values that span too much for 4 bytes: 8-byte entries in the
+		// spare slots (16 bytes a slot, at least 64 and twice as many slots as
+		// tuples) and the presence bits in the table's words.
+		const uint32_t range = (uint32_t) span + 1;
+		for (uint32_t i = first; i < (range + 31) / 32; i += stride) table[i] = 0;
+		meet();
+		bool dup = false;
+		#pragma unroll 4
+		for (uint32_t i = first; i < n; i += stride) {
+			const uint4 v = __ldg(R + i);
+			const unsigned long long d = key_of(v) - (unsigned long long) h.dmin;
+			if (d >= range) continue;
+			const uint32_t bit = 1u << (d & 31);
+			if (atomicOr(&table[d >> 5], bit) & bit) dup = true;
+			slots[d] = hj_pack16(v, pk);
+		}
+		if (dup) atomicOr(&acc->dup, 1u);
+		meet();
+		if (!va->dup) h.flags = 64;
 	}
-	// The hashed table, unless the tuples have a dense layout (of wide values: by
-	// the exact build) or a key equal to the empty marker (the exact build's list).
-	if (h.flags != 4 && h.present != n && !va->marker) {
+	// The hashed table, unless the tuples have a dense layout or a key equal to the
+	// empty marker (the exact build's list).
+	if (h.flags != 64 && h.present != n && !va->marker) {
 		const uint32_t mask = (1u << log2cap) - 1;
 		for (uint32_t i = first; i <= mask; i += stride) reinterpret_cast<uint4*>(slots)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
 		meet();
@@ -2430,7 +2451,7 @@ static int hj_settle_known(pg_ctx* ctx, pg_hashtable* ht, const HjDenseHdr* refu
 		PG_CUDA(ctx, cudaMemcpyAsync(&h, ht->hdr, sizeof h, cudaMemcpyDeviceToHost, s));
 		PG_CUDA(ctx, cudaStreamSynchronize(s));
 	}
-	if (!(h.flags & 16)) {       // spare slots that no probe will read
+	if (!(h.flags & (16 | 64))) {       // spare slots that no probe will read
 		pg_free_async(ctx, s, ht->small_slots);
 		ht->small_slots = nullptr;
 	}
@@ -2447,6 +2468,15 @@ static int hj_settle_known(pg_ctx* ctx, pg_hashtable* ht, const HjDenseHdr* refu
 			win = ht->dense32_copy;
 		}
 		hj_settle_good(ht, h, win);
+		return PG_OK;
+	}
+	if (h.flags & 64) {          // the build kernel made the wide dense layout
+		ht->dense_val = ht->small_slots; ht->dense_bits = ht->dense32_base; ht->dense32 = nullptr;
+		ht->small_slots = nullptr; ht->dense32_base = nullptr;
+		ht->dmin = h.dmin; ht->drange = h.kmax - h.kmin + 1;
+		ht->vmin = h.vlo; ht->vlo = h.vlo; ht->vmax = h.vhi;
+		ht->log2cap = 1;
+		ht->spec.store(false, std::memory_order_release);
 		return PG_OK;
 	}
 	// Refuted (a repeated key, a key or value the sample missed): rebuild

@@ -33,7 +33,8 @@ struct HjDenseHdr {
 	int flags;                   // 1 key outside the window, 2 value outside the entry range,
 	                             // 4 sample: window larger than the allocation or values too wide,
 	                             // 8 the keys read span more than any dense table takes,
-	                             // 16 small_slots hold the hashed table (32: of repeated keys)
+	                             // 16 small_slots hold the hashed table (32: of repeated keys),
+	                             // 64 small_slots hold the wide dense values, dense32_base their bits
 	int pad;
 };
 

@@ -123,3 +123,43 @@ def test_probed_dense_table_keeps_only_its_entries(ctx, n):
             assert kept <= 4 * (2 * n + n // 8 + 4096) + 4096, kept
     finally:
         L.pg_hashtable_free(ctx.h, ht)
+
+
+# Values that span 2^32 or more beside dense keys take 8-byte entries, made by the
+# build kernel like the other layouts of up to 2^20 tuples: a join is the build, a
+# probe that finds the header and one that finds the table. Sizes around one block's
+# 2048 tuples and a word of presence bits.
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 2048, 2049, 70_001, 1 << 20])
+@pytest.mark.parametrize("repeated", [False, True])
+def test_small_build_of_wide_values(ctx, n, repeated):
+    R = np.stack([np.random.default_rng(n).permutation(n) - 5, np.arange(n) * 7 - 9], axis=1).astype(np.int64)
+    R[0, 1], R[-1, 1] = np.iinfo(np.int64).min, np.iinfo(np.int64).max
+    if repeated:
+        if n == 1:
+            return
+        R[n // 2, 0] = R[0, 0]
+    S = np.stack([np.arange(-9, n + 3), np.arange(n + 12)], axis=1).astype(np.int64)
+    vals = {}
+    for k, v in R.tolist():
+        vals.setdefault(k, []).append(v)
+    want = sorted((p, v) for k, p in S.tolist() for v in vals.get(k, ()))
+    before = gpu.kernel_launches()
+    t = ctx.build_table(R)
+    try:
+        _, count, total = t.probe(S, flags=gpu.JOIN_COUNT | gpu.JOIN_SUM, sum_col=1)
+        assert repeated or gpu.kernel_launches() - before <= 5      # 7 with an exact rebuild
+        assert count == len(want) and (total - sum(v for _, v in want)) % (1 << 64) == 0
+        got = np.ascontiguousarray(t.probe(S, out_cap=len(want))[0]).view(np.int64).reshape(-1, 2)
+        assert sorted(map(tuple, got.tolist())) == want
+        if not repeated:                                            # the layout of the exact build
+            image = t.serialize()
+            ctx.tune(build_spec=2)
+            try:
+                u = ctx.build_table(R)
+                assert np.array_equal(image, u.serialize())
+                u.free()
+            finally:
+                ctx.tune(build_spec=0)
+    finally:
+        t.free()
