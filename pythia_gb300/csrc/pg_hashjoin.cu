@@ -402,21 +402,28 @@ __global__ void __launch_bounds__(1024) k_dense_prep16(const uint4* __restrict__
 // for large inputs has launches, 8-byte entries for values that span too much, and
 // where no dense layout fits (keys too far apart or repeated) the hashed table, which
 // the first use then finds ready. One block
-// per 2048 tuples (a single one's barriers are block barriers). Whole joins of
-// 1000 tuples with 10,000: dense keys 73 -> 42 us, far ones 107 -> 78; of 16,000 with
-// 100,000: 84 -> 48 and 112 -> 90 (exact ranges and duplicate counts read back by the
+// per 1024 tuples, one a thread (a single one's barriers are block barriers), up to one an
+// SM: with 2048 the walks past repeated keys kept too few SMs busy (20,000 tuples of one
+// key 31 -> 38 ms, now 31; of 20 keys 5.0 -> 5.7, now 3.8). Whole joins of
+// 1000 tuples with 10,000: dense keys 73 -> 42 us, far ones 107 -> 78; of 20,000 with
+// 40,000: 89 -> 53 and 106 -> 90 (exact ranges and duplicate counts read back by the
 // host before). From 65,536 tuples the sampled form, used there before, takes as
-// long for dense keys (140,000 with 800,000: 58 us) and longer for far ones (167,
-// now 87), up to 2^20: the spare hashed slots are 32 MB then.
-#define HJ_SMALL_PER_BLOCK 2048
+// long for dense keys (200,000 with 400,000: 65 us) and longer for far ones (182,
+// now 105), up to 2^20: the spare hashed slots are 32 MB then.
+#define HJ_SMALL_PER_BLOCK 1024
 #define HJ_SMALL_TUPLES (1u << 20)
+// Slots a tuple may walk past. Only keys repeated as often walk so far (the table is
+// at most half full); 2^18 tuples of one key take 0.9 s, a million would take the 15 s
+// of the exact build and hold the other blocks at a barrier for longer than they wait, so
+// the exact build's kernel, which has no barriers, makes those tables.
+#define HJ_SMALL_WALK(n) ((n) > (1u << 18) ? (n) / 16 : 1u << 20)
 
 // What the blocks of k_build_small gather, zero before (G > 1).
 struct HjSmallShared {
 	unsigned long long nkmin, kmax, nvmin, vmax;     // ~smallest and largest key (^ 2^63) and value
 	unsigned long long present;
 	unsigned int marker, dup;
-	unsigned int lost;                               // a block gave up on a barrier
+	unsigned int lost;                               // a walk was too long, or a block gave up on a barrier
 	unsigned int bar;
 };
 
@@ -516,22 +523,29 @@ __global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict
 		const uint32_t mask = (1u << log2cap) - 1;
 		for (uint32_t i = first; i <= mask; i += stride) reinterpret_cast<uint4*>(slots)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
 		meet();
-		bool dup = false;
-		for (uint32_t i = first; i < n; i += stride) {
+		const uint32_t walk = HJ_SMALL_WALK(n);
+		bool dup = false, far = false;
+		for (uint32_t i = first; i < n && !far; i += stride) {
 			const uint4 v = __ldg(R + i);
 			const unsigned long long k = key_of(v);
 			uint32_t s = (uint32_t) hj_slot0((int64_t) k, log2cap);
-			for (uint32_t tries = 0; tries <= mask; ++tries, s = (s + 1) & mask) {       // at most half full
+			far = true;
+			for (uint32_t tries = 0; tries < walk; ++tries, s = (s + 1) & mask) {
 				const unsigned long long old = atomicCAS(&slots[2 * (uint64_t) s], (unsigned long long) PG_EMPTY_KEY, k);
-				if (old == (unsigned long long) PG_EMPTY_KEY) { slots[2 * (uint64_t) s + 1] = hj_pack16(v, pk); break; }
+				if (old == (unsigned long long) PG_EMPTY_KEY) {
+					slots[2 * (uint64_t) s + 1] = hj_pack16(v, pk);
+					far = false;
+					break;
+				}
 				if (old == k) dup = true;
 			}
 		}
 		if (dup) atomicOr(&acc->dup, 1u);
+		if (far) atomicOr(&acc->lost, 1u);
 		meet();
 		h.flags |= 16 | (va->dup ? 32 : 0);
 	}
-	// Past a lost barrier (the status says so) neither layout can be trusted.
+	// Past a lost barrier, or with a tuple left out, no layout can be trusted.
 	if (blockIdx.x == 0 && tid == 0) {
 		if (va->lost) h.flags = 4;
 		*hdr = h;

@@ -163,3 +163,27 @@ def test_small_build_of_wide_values(ctx, n, repeated):
                 ctx.tune(build_spec=0)
     finally:
         t.free()
+
+
+# The tuples of a repeated key walk past each other. Over 2^18 tuples, a key that walks
+# past a sixteenth of them sends the build to the exact build's kernel instead of holding
+# blocks at a barrier, whose wait it could outlast. Without that the first probe makes three
+# launches more than the next: the build, and a probe and its tail that find the header.
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,copies,exact", [(100, 100, False), (9000, 9000, False), (270_000, 8000, False), (270_000, 20_000, True)])
+def test_small_build_of_long_walks(ctx, n, copies, exact):
+    R = np.stack([np.maximum(np.arange(n), copies), np.arange(n)], axis=1).astype(np.int64)
+    R[: copies, 0] = copies
+    S = np.stack([np.arange(copies - 1, n + 2), np.zeros(n + 3 - copies)], axis=1).astype(np.int64)
+    before = gpu.kernel_launches()
+    t = ctx.build_table(R)
+    try:
+        launches = []
+        for _ in range(2):
+            _, count, total = t.probe(S, flags=gpu.JOIN_COUNT | gpu.JOIN_SUM, sum_col=1)
+            assert (count, total) == (n, n * (n - 1) // 2)
+            launches.append(gpu.kernel_launches() - before)
+            before += launches[-1]
+        assert (launches[0] - launches[1] > 3) == exact
+    finally:
+        t.free()
