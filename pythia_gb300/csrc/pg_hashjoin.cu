@@ -429,10 +429,10 @@ struct HjSmallShared {
 
 __global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict__ R, uint32_t n, uint32_t kw,
 		uint32_t pk, uint64_t cap, uint32_t* __restrict__ table, unsigned long long* __restrict__ slots, uint32_t log2cap,
-		HjDenseHdr* __restrict__ hdr, HjSmallShared* g, int* __restrict__ status)
+		HjDenseHdr* __restrict__ hdr, HjSmallShared* g, const int* __restrict__ status)
 {
 	__shared__ unsigned long long red[4][32];
-	__shared__ HjSmallShared mine;
+	__shared__ HjSmallShared mine, seen;
 	const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const uint32_t first = blockIdx.x * 1024 + tid, stride = gridDim.x * 1024;
 	const bool alone = gridDim.x == 1;
@@ -441,9 +441,19 @@ __global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict
 	bool dead = false;
 	HjSmallShared* const acc = alone ? &mine : g;
 	if (alone && tid == 0) mine = HjSmallShared{0, 0, 0, 0, 0, 0, 0, 0, 0};
+	// A barrier that a block gave up on is no error: the build returns before the kernel
+	// has run, and a status would fail whichever call reads it next. The header sends the
+	// table to the exact build. Thread 0 looks at what was gathered for its whole block:
+	// past a lost barrier it still changes, and the block's threads must go the same way.
 	auto meet = [&]() {
-		pg_grid_sync(&g->bar, epoch, dead, spin, status);
-		if (dead) atomicOr(&acc->lost, 1u);          // before this block's next arrival
+		pg_grid_sync(&g->bar, epoch, dead, spin, nullptr);
+		if (tid == 0) {
+			if (dead) atomicOr(&acc->lost, 1u);         // before this block's next arrival
+			const volatile HjSmallShared* const v = acc;
+			seen.nkmin = v->nkmin; seen.kmax = v->kmax; seen.nvmin = v->nvmin; seen.vmax = v->vmax;
+			seen.present = v->present; seen.marker = v->marker; seen.dup = v->dup; seen.lost = v->lost;
+		}
+		__syncthreads();
 	};
 	auto key_of = [&](const uint4& v) { return ((unsigned long long) hj_word4(v, kw + 1) << 32) | hj_word4(v, kw); };
 	unsigned long long lo = ~0ull, hi = 0, vlo = ~0ull, vhi = 0;
@@ -469,9 +479,8 @@ __global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict
 		}
 	}
 	meet();
-	volatile HjSmallShared* const va = acc;
 	HjDenseHdr h;
-	h.n = n; h.present = 0; h.kmin = ~va->nkmin; h.kmax = va->kmax; h.vlo = ~va->nvmin; h.vhi = va->vmax; h.pad = 0;
+	h.n = n; h.present = 0; h.kmin = ~seen.nkmin; h.kmax = seen.kmax; h.vlo = ~seen.nvmin; h.vhi = seen.vmax; h.pad = 0;
 	h.dmin = (long long) (h.kmin ^ (1ull << 63));
 	h.vmin = h.vlo;
 	const unsigned long long span = h.kmax - h.kmin;
@@ -495,7 +504,7 @@ __global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict
 		c = __reduce_add_sync(0xffffffffu, c);
 		if (lane == 0 && c) atomicAdd(&acc->present, (unsigned long long) c);
 		meet();
-		h.present = va->present;
+		h.present = seen.present;
 	} else if (h.flags == 4) {
 		// Dense keys, values that span too much for 4 bytes: 8-byte entries in the
 		// spare slots (16 bytes a slot, at least 64 and twice as many slots as
@@ -515,11 +524,11 @@ __global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict
 		}
 		if (dup) atomicOr(&acc->dup, 1u);
 		meet();
-		if (!va->dup) h.flags = 64;
+		if (!seen.dup) h.flags = 64;
 	}
 	// The hashed table, unless the tuples have a dense layout or a key equal to the
 	// empty marker (the exact build's list).
-	if (h.flags != 64 && h.present != n && !va->marker) {
+	if (h.flags != 64 && h.present != n && !seen.marker) {
 		const uint32_t mask = (1u << log2cap) - 1;
 		for (uint32_t i = first; i <= mask; i += stride) reinterpret_cast<uint4*>(slots)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
 		meet();
@@ -543,11 +552,11 @@ __global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict
 		if (dup) atomicOr(&acc->dup, 1u);
 		if (far) atomicOr(&acc->lost, 1u);
 		meet();
-		h.flags |= 16 | (va->dup ? 32 : 0);
+		h.flags |= 16 | (seen.dup ? 32 : 0);
 	}
 	// Past a lost barrier, or with a tuple left out, no layout can be trusted.
 	if (blockIdx.x == 0 && tid == 0) {
-		if (va->lost) h.flags = 4;
+		if (*(volatile unsigned int*) &acc->lost) h.flags = 4;
 		*hdr = h;
 	}
 }

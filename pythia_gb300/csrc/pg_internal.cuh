@@ -410,7 +410,8 @@ __device__ __forceinline__ void pg_st_relaxed(uint32_t* p, uint32_t v)
 // All blocks of the cooperative launch meet; what they stored before is
 // visible after. Bounded: past the limit the status records PG_ERR_TIMEOUT and
 // this block no longer waits, so callers keep every access in bounds whatever the
-// others have done.
+// others have done. Without a status the caller does something else about `dead` and
+// the context's own limit (`spin`) ends the wait at once.
 __device__ __forceinline__ void pg_grid_sync(uint32_t* bar, uint32_t& epoch, bool& dead, uint32_t spin, int* status)
 {
 	__syncthreads();
@@ -423,8 +424,9 @@ __device__ __forceinline__ void pg_grid_sync(uint32_t* bar, uint32_t& epoch, boo
 			asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
 			if (v >= epoch * gridDim.x) break;
 			++polls;
-			if (polls == (spin ? spin : PG_GRID_SPIN_LIMIT)) pg_set_status(status, PG_ERR_TIMEOUT);
-			if (polls >= PG_GRID_SPIN_LIMIT) { pg_set_status(status, PG_ERR_TIMEOUT); dead = true; }
+			const bool late = polls == (spin ? spin : PG_GRID_SPIN_LIMIT), over = polls >= PG_GRID_SPIN_LIMIT;
+			if (status && (late || over)) pg_set_status(status, PG_ERR_TIMEOUT);
+			dead = over || (late && !status);
 		}
 		__threadfence();
 	}

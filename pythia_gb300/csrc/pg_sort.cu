@@ -305,8 +305,12 @@ k_sort_small(const uint4* __restrict__ in, uint32_t n, uint32_t kw, uint32_t kby
 	if (G > 1) {
 		if (tid == 0) { atomicMax(&mm[0], ~lo); atomicMax(&mm[1], hi); }
 		pg_grid_sync(bar, epoch, dead, spin, status);
-		lo = ~pg_ld_relaxed(mm);
-		hi = pg_ld_relaxed(mm + 1);
+		// One thread's look for the whole block: past a barrier that was given up on the
+		// range still changes, and the block's threads must make the same passes.
+		if (tid == 0) { red[0][0] = ~pg_ld_relaxed(mm); red[1][0] = pg_ld_relaxed(mm + 1); }
+		__syncthreads();
+		lo = red[0][0];
+		hi = red[1][0];
 	}
 	const unsigned long long span = hi - lo;
 	const int passes = span ? (64 - __clzll((long long) span) + 7) / 8 : 0;
