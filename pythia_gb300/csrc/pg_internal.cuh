@@ -48,6 +48,36 @@ int pg_cuda_fail(pg_ctx* ctx, cudaError_t e, const char* what);
 #define PG_BIG_ALLOC (256ull << 20)
 int pg_alloc_async(pg_ctx* ctx, cudaStream_t s, void** p, size_t bytes);
 void pg_free_async(pg_ctx* ctx, cudaStream_t s, void* p);
+
+// A call's scratch on one stream, freed (after the kernels queued on it) when it goes
+// out of scope, whichever way the call returns.
+struct PgScratch {
+	pg_ctx* ctx;
+	cudaStream_t s;
+	void* p[4];
+	int n = 0;
+	PgScratch(pg_ctx* c, cudaStream_t st) : ctx(c), s(st) { }
+	~PgScratch() { for (int i = 0; i < n; ++i) pg_free_async(ctx, s, p[i]); }
+	PgScratch(const PgScratch&) = delete;
+	PgScratch& operator=(const PgScratch&) = delete;
+	int get(void** q, size_t bytes)
+	{
+		if (n == (int) (sizeof p / sizeof p[0])) return PG_ERR_ARG;
+		const int rc = pg_alloc_async(ctx, s, q, bytes);
+		if (!rc) p[n++] = *q;
+		return rc;
+	}
+	// Memory that the caller can do without: true when there is none, and no error is
+	// left behind for the next launch.
+	bool want(void** q, size_t bytes)
+	{
+		if (!get(q, bytes)) return false;
+		cudaGetLastError();
+		*q = nullptr;
+		return true;
+	}
+};
+
 // Reads the sticky status after synchronising `s`; returns its PG_ERR_* code.
 int pg_check_status(pg_ctx* ctx, cudaStream_t s, const char* what);
 // Clears a non-zero status `st` read back by the caller and reports it.

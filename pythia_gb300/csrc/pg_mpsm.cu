@@ -728,7 +728,8 @@ static bool mj_v16(const pg_rel* r)
 // spans: the table's random accesses still cost less than sorting both sides).
 // The window comes from every 1024th tuple widened by 1/64 a side on large
 // inputs, checked by the counting pass, else from every tuple. *handled =
-// false (nothing produced): the caller sorts.
+// false (nothing produced): the caller sorts. So it does where the tables do not fit in
+// memory; the partitioned copies are the first to be done without.
 static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_rel* S, const MjCols& pc, int sum_col,
 		int flags, void* out, uint64_t out_capacity, pg_join_result* res, bool* handled)
 {
@@ -754,8 +755,9 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 	int rc;
 	// [~key min, key max], [rows, sum], [largest count, key outside], two words of
 	// pg_readback, [~value min, value max]
+	PgScratch mem(ctx, s);
 	unsigned long long* mm = nullptr;
-	if ((rc = pg_alloc_async(ctx, s, (void**) &mm, 72))) return rc;
+	if ((rc = mem.get((void**) &mm, 72))) return rc;
 	unsigned long long* agg = mm + 2;
 	unsigned int* meta = reinterpret_cast<unsigned int*>(mm + 4);
 	unsigned long long* vmm = mm + 7;
@@ -779,34 +781,32 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 		if (span >= MJ_MAX_RANGE || span >= std::max<unsigned long long>(MJ_MIN_RANGE + (MJ_MIN_RANGE >> 4), 16 * C->n)) break;
 		const uint32_t range = (uint32_t) span + 1;
 		const long long kmin = (long long) (h[0] ^ (1ull << 63));
+		// [counts, sums of MJ_SCAN counts, values]
+		PgScratch tables(ctx, s), copies(ctx, s);
 		uint32_t* cnt = nullptr;
 		uint64_t* sums = nullptr;
 		unsigned long long* val = nullptr;
-		char* split[2] = {nullptr, nullptr};
-		auto release = [&]() {
-			for (void* p : {(void*) cnt, (void*) sums, (void*) val, (void*) split[0], (void*) split[1]}) pg_free_async(ctx, s, p);
-		};
+		const uint64_t nb = pg_div_up(range, MJ_SCAN);
+		if (tables.want((void**) &cnt, (uint64_t) range * 4)) return PG_OK;
+		if (materialize && (tables.want((void**) &sums, nb * 8) || tables.want((void**) &val, C->n * 8))) return PG_OK;
 		// Rows of more tuples than L2 holds values of: both sides by the top 8 bits of
 		// the window first (without memory for the copies, as they are), then one piece of
 		// the input a block, so that the blocks in flight use the same part of the table.
+		char* split[2] = {nullptr, nullptr};
 		bool parted = false;
-		if (materialize && C->n > MJ_SPLIT_TUPLES && P->n > MJ_SPLIT_TUPLES / 4) {
-			if (pg_alloc_async(ctx, s, (void**) &split[0], C->n * 16) == PG_OK &&
-					pg_alloc_async(ctx, s, (void**) &split[1], P->n * 16) == PG_OK) {
-				pg_hashfn f = {};
-				f.fn = PG_FN_PARAMMODULO;
-				f.nbuckets = 256;
-				f.min = kmin;
-				f.skipbits = range > 256 ? 24 - __builtin_clz(range - 1) : 0;
-				f.k = (int64_t) 255 << f.skipbits;
-				if ((rc = pg_partition_fn(ctx, s, C, f, split[0], nullptr)) ||
-						(rc = pg_partition_fn(ctx, s, P, f, split[1], nullptr))) { release(); pg_free_async(ctx, s, mm); return rc; }
-				parted = true;
-			} else {
-				cudaGetLastError();
-				if (split[0]) { pg_free_async(ctx, s, split[0]); split[0] = nullptr; }
-				split[1] = nullptr;
-			}
+		if (materialize && C->n > MJ_SPLIT_TUPLES && P->n > MJ_SPLIT_TUPLES / 4 &&
+				!copies.want((void**) &split[0], C->n * 16) && !copies.want((void**) &split[1], P->n * 16)) {
+			pg_hashfn f = {};
+			f.fn = PG_FN_PARAMMODULO;
+			f.nbuckets = 256;
+			f.min = kmin;
+			f.skipbits = range > 256 ? 24 - __builtin_clz(range - 1) : 0;
+			f.k = (int64_t) 255 << f.skipbits;
+			rc = pg_partition_fn(ctx, s, C, f, split[0], nullptr);
+			if (!rc) rc = pg_partition_fn(ctx, s, P, f, split[1], nullptr);
+			if (rc && rc != PG_ERR_OOM) return rc;
+			parted = !rc;
+			if (rc) cudaGetLastError();
 		}
 		const char* const cdata = (const char*) (parted ? split[0] : C->data);
 		const char* const pdata = (const char*) (parted ? split[1] : P->data);
@@ -814,7 +814,6 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 			const uint64_t b = pg_div_up(n, per_block);
 			return (int) (parted ? b : std::min<uint64_t>(b, (uint64_t) ctx->sm_count * per_sm));
 		};
-		if ((rc = pg_alloc_async(ctx, s, (void**) &cnt, (uint64_t) range * 4))) return rc;
 		PG_CUDA(ctx, cudaMemsetAsync(cnt, 0, (uint64_t) range * 4, s));
 		const int cblocks = grid(C->n, 256 * MJ_ILP, MJ_BLOCKS_PER_SM), pblocks = grid(P->n, 256 * MJ_ILP, MJ_BLOCKS_PER_SM);
 #define MJ_COUNT(V, VALS) k_mj_count<V, VALS><<<cblocks, 256, 0, s>>>(cdata, C->n, C->width, C->key_off, \
@@ -832,12 +831,13 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 					soff, swords, kmin, range, cnt, agg);
 			PG_LAUNCHED(ctx);
 		} else {
-			const uint64_t nb = pg_div_up(range, MJ_SCAN);
-			if ((rc = pg_alloc_async(ctx, s, (void**) &sums, nb * 8)) ||
-					(rc = pg_alloc_async(ctx, s, (void**) &val, C->n * 8))) { release(); return rc; }
 			k_mj_scan_sums<<<(unsigned) nb, 256, 0, s>>>(cnt, range, sums, meta);
 			PG_LAUNCHED(ctx);
-			if ((rc = pg_scan_u64(ctx, s, sums, nb, nullptr))) { release(); return rc; }
+			if ((rc = pg_scan_u64(ctx, s, sums, nb, nullptr))) {
+				if (rc != PG_ERR_OOM) return rc;
+				cudaGetLastError();
+				return PG_OK;
+			}
 			k_mj_scan_apply<<<(unsigned) nb, 256, 0, s>>>(cnt, range, sums);
 			PG_LAUNCHED(ctx);
 			const int fblocks = grid(C->n, 256, MJ_FILL_BLOCKS_PER_SM);
@@ -852,19 +852,17 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 		}
 		unsigned long long o[4];     // rows, sum, (largest count, key outside)
 		rc = pg_readback(ctx, s, agg, 3, nullptr, o, "pg_mpsm_join");
-		release();
-		if (rc) { pg_free_async(ctx, s, mm); return rc; }
+		if (rc) return rc;
 		if (o[2] >> 32) continue;                                         // the sample missed a key
 		if (materialize && (uint32_t) o[2] > MJ_MAX_RUN) break;
 		res->n_out = o[0];
 		res->sum = (int64_t) o[1];
 		*handled = true;
 		if (materialize && o[0] > out_capacity)
-			rc = pg_fail(ctx, PG_ERR_OUTPUT_FULL, "pg_mpsm_join: output capacity too small");
+			return pg_fail(ctx, PG_ERR_OUTPUT_FULL, "pg_mpsm_join: output capacity too small");
 		break;
 	}
-	pg_free_async(ctx, s, mm);
-	return rc;
+	return PG_OK;
 }
 
 // Whether a side flagged as sorted is, on the device.
