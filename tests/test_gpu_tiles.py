@@ -332,3 +332,28 @@ def test_hashjoin_groupby_shared_tables(ctx, probe, groups, swap):
         got = np.ascontiguousarray(ctx.hashjoin_groupby(R, S, pkey=pkey, val=(val, t), agg=agg))
         want = orc.groupby_exact(joined) if t == "dec" else orc.groupby(joined, val=(8, t), agg=agg)
         assert np.array_equal(orc.canonical(got), orc.canonical(want))
+
+
+# Windows of up to 8192 keys are counted in shared memory when there are eight tuples
+# for each of the blocks' counts and blocks for half the SMs. Either side of both limits,
+# counted on either side, 16- and 24-byte tuples, and one key with most of the tuples.
+@pytest.mark.parametrize("n,keys", [(620_000, 1), (600_000, 1000), (630_000, 1000), (5_100_000, 8192), (5_100_000, 8193)])
+@pytest.mark.parametrize("width", [16, 24])
+def test_mpsm_few_keys_counted_in_shared_memory(ctx, n, keys, width):
+    rng = np.random.default_rng(keys)
+    R = np.stack([rng.integers(0, keys, size=n) - 3] + [rng.integers(-(1 << 62), 1 << 62, size=n)] * (width // 8 - 1), axis=1)
+    R[n // 3:n // 2, 0] = -3
+    R[0, 0], R[-1, 0] = -3, keys - 4
+    S = R[:: n // 700].copy()
+    S[:5, 0] = keys - 3                                     # no match
+    sums, rows = {}, np.bincount(R[:, 0] + 3, minlength=keys + 1)
+    total = np.zeros(keys + 1, dtype=np.uint64)
+    np.add.at(total, R[:, 0] + 3, R[:, 1].astype(np.uint64))
+    k = S[:, 0] + 3
+    want = int(rows[k].sum())
+    sums["B"] = int(total[k].sum(dtype=np.uint64).astype(np.int64))
+    sums["P"] = int((rows[k].astype(np.uint64) * S[:, 1].astype(np.uint64)).sum(dtype=np.uint64).astype(np.int64))
+    for a, b, of in ((R, S, {0: "P", 1: "B"}), (S, R, {0: "B", 1: "P"})):
+        for col in (0, 1):
+            _, got, s = ctx.mpsm(a, b, proj=(("P", 8, 8), ("B", 8, 8)), flags=gpu.JOIN_COUNT | gpu.JOIN_SUM, sum_col=col)
+            assert (got, s) == (want, sums[of[col]])
