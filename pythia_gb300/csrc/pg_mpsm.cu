@@ -604,8 +604,8 @@ k_mj_fill(const char* __restrict__ R, uint64_t n, uint32_t koff, long long kmin,
 	}
 }
 
-// Rows of each probe tuple: one per value of its key's run [end[d - 1],
-// end[d]). A warp looks up 32 T tuples at once, reserves their rows with one
+// Rows of each probe tuple: one per value of its key's run [ends[d - 1],
+// ends[d]). A warp looks up 32 T tuples at once, reserves their rows with one
 // add on the cursor, and writes them 32 at a time, each lane finding its row's
 // tuple by a search over the lanes' offsets, so that a warp stores consecutive
 // rows whatever the runs' lengths. Rows past `cap` are counted only.
@@ -614,13 +614,26 @@ k_mj_fill(const char* __restrict__ R, uint64_t n, uint32_t koff, long long kmin,
 // above with its group-by: no limit on registers 1214 us, with 6 blocks an SM 1160, and
 // two tuples a lane instead of four 1105; of keys with one row 1484, 1513 and 1590, so
 // those take four.
+//
+// A warp's tuples may have thousands of rows each. Those of more than MJ_SLICE_MAX rows
+// in all go on a list instead, MJ_SLICE rows an entry, and a second launch (SLICE) has a
+// warp write an entry's rows. 1000 tuples with 16,000 rows each: 18.97 ms without it,
+// 0.47 with (1.45 sorted, where a thread takes eight rows); 64 such tuples among 4M others 8.4,
+// 0.27 (1.10). The second launch, empty, takes 2 us.
 #define MJ_ROWS_BLOCKS_PER_SM 24
-template <int T>                                      // tuples a lane
+#define MJ_SLICE 2048u
+#define MJ_SLICE_MAX 8192u
+// Entries (tuples' first index / 32 T << 16 | slice) that hold the slices of `cap` rows: more
+// rows than that do not fit the output.
+static uint64_t mj_slices(uint64_t cap) { return cap / (MJ_SLICE / 2) + 16; }
+
+template <int T, bool SLICE>                          // T tuples a lane
 __global__ void __launch_bounds__(256, 6)
 k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin, uint32_t range,
-		const uint32_t* __restrict__ end, const unsigned long long* __restrict__ val, uint32_t wsel,
+		const uint32_t* __restrict__ ends, const unsigned long long* __restrict__ val, uint32_t wsel,
 		uint4* __restrict__ out, uint64_t cap, unsigned long long* __restrict__ cursor, const unsigned int* __restrict__ meta,
-		const unsigned long long* __restrict__ vmm)
+		const unsigned long long* __restrict__ vmm, unsigned long long* __restrict__ list, uint64_t list_cap,
+		unsigned long long* __restrict__ listed)
 {
 	if (meta[0] > MJ_MAX_RUN || meta[1]) return;
 	const unsigned long long vmin = ~vmm[0];
@@ -629,7 +642,10 @@ k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin,
 	const uint64_t pol = pg_policy_evict_first(), keep = pg_policy_keep(4);
 	const uint64_t nwarps = ((uint64_t) gridDim.x * blockDim.x) >> 5;
 	const uint32_t w0 = wsel & 15, w1 = (wsel >> 4) & 15, w2 = (wsel >> 8) & 15, w3 = (wsel >> 12) & 15;
-	for (uint64_t c0 = (((uint64_t) blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (32 * T); c0 < n; c0 += nwarps * (32 * T)) {
+	const uint64_t units = SLICE ? pg_min64(*listed, list_cap) : pg_div_up(n, 32 * T);
+	for (uint64_t u = ((uint64_t) blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < units; u += nwarps) {
+		const unsigned long long entry = SLICE ? list[u] : u << 16;
+		const uint64_t c0 = (entry >> 16) * (32 * T);
 		uint4 t[T];
 		uint32_t lo[T], m[T];
 		#pragma unroll
@@ -640,8 +656,8 @@ k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin,
 			if (i < n) {
 				const uint64_t x = (uint64_t) mj_key<true>(S, i, 16, koff, 8, pol, t[j]) - (uint64_t) kmin;
 				if (x < range) {
-					m[j] = mj_ld32(end + x, keep);
-					if (x) lo[j] = mj_ld32(end + x - 1, keep);
+					m[j] = mj_ld32(ends + x, keep);
+					if (x) lo[j] = mj_ld32(ends + x - 1, keep);
 				}
 			}
 		}
@@ -660,11 +676,26 @@ k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin,
 			total += m[j];
 		}
 		unsigned long long row = 0;
-		if (lane == 0 && total) row = atomicAdd(cursor, (unsigned long long) total);
-		row = __shfl_sync(0xffffffffu, row, 0);
+		if (!SLICE && total > MJ_SLICE_MAX) {
+			const uint32_t pieces = (total + MJ_SLICE - 1) / MJ_SLICE;
+			if (lane == 0) row = atomicAdd(listed, (unsigned long long) pieces);
+			row = __shfl_sync(0xffffffffu, row, 0);
+			for (uint32_t p = lane; p < pieces; p += 32)
+				if (row + p < list_cap) list[row + p] = u << 16 | p;
+				else atomicAdd(cursor, (unsigned long long) pg_min32(MJ_SLICE, total - p * MJ_SLICE));
+			continue;
+		}
+		// Rows [first, last) of the warp's tuples.
+		const uint32_t first = SLICE ? (uint32_t) (entry & 0xFFFF) * MJ_SLICE : 0;
+		const uint32_t last = SLICE ? pg_min32(total, first + MJ_SLICE) : total;
+		if (lane == 0 && last > first) row = atomicAdd(cursor, (unsigned long long) (last - first));
+		row = __shfl_sync(0xffffffffu, row, 0) - first;
+		uint32_t before = 0;                     // rows of the tuples before these 32
 		#pragma unroll
 		for (int j = 0; j < T; ++j) {
-			for (uint32_t r0 = 0; r0 < m[j]; r0 += 32) {
+			const uint32_t begin = SLICE && first > before ? first - before : 0;
+			const uint32_t end = !SLICE ? m[j] : last > before ? pg_min32(m[j], last - before) : 0;
+			for (uint32_t r0 = begin; r0 < end; r0 += 32) {
 				const uint32_t r = r0 + lane;
 				uint32_t x = 0;                  // the last tuple whose offset is <= r (it has rows)
 				#pragma unroll
@@ -672,7 +703,7 @@ k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin,
 					if (__shfl_sync(0xffffffffu, off[j], x + step) <= r) x += step;
 				const uint32_t at = __shfl_sync(0xffffffffu, lo[j], x) + (r - __shfl_sync(0xffffffffu, off[j], x));
 				unsigned long long v = 0;
-				if (r < m[j]) {
+				if (r < end) {
 					if (bytes == 2) v = vmin + mj_ld16(reinterpret_cast<const uint16_t*>(val) + at, keep);
 					else if (bytes == 4) v = vmin + mj_ld32(reinterpret_cast<const uint32_t*>(val) + at, keep);
 					else v = mj_ld64(val + at, keep);
@@ -681,9 +712,10 @@ k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin,
 					return w < 4 ? __shfl_sync(0xffffffffu, mjw_word(t[j], w), x) : w == 4 ? (uint32_t) v : (uint32_t) (v >> 32);
 				};
 				const uint4 o = make_uint4(pick(w0), pick(w1), pick(w2), pick(w3));
-				if (r < m[j] && row + r < cap) pg_st_hint16(out + row + r, o, pol);
+				if (r < end && row + r < cap) pg_st_hint16(out + row + r, o, pol);
 			}
 			row += m[j];
+			if (SLICE) before += m[j];
 		}
 	}
 }
@@ -769,16 +801,16 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 	const pg_rel *C = count_build ? R : S, *P = count_build ? S : R;
 	int rc;
 	// [~key min, key max], [rows, sum], [largest count, key outside], two words of
-	// pg_readback, [~value min, value max]
+	// pg_readback, [~value min, value max], slices listed
 	PgScratch mem(ctx, s);
 	unsigned long long* mm = nullptr;
-	if ((rc = mem.get((void**) &mm, 72))) return rc;
+	if ((rc = mem.get((void**) &mm, 80))) return rc;
 	unsigned long long* agg = mm + 2;
 	unsigned int* meta = reinterpret_cast<unsigned int*>(mm + 4);
 	unsigned long long* vmm = mm + 7;
 	for (int attempt = C->n >= (1ull << 22) ? 0 : 1; attempt < 2; ++attempt) {
 		const uint64_t step = attempt == 0 ? 1024 : 1;
-		PG_CUDA(ctx, cudaMemsetAsync(mm, 0, 72, s));
+		PG_CUDA(ctx, cudaMemsetAsync(mm, 0, 80, s));
 		const int mblocks = (int) std::min<uint64_t>(pg_div_up(pg_div_up(C->n, step), 256), (uint64_t) ctx->sm_count * 8);
 		k_mj_minmax<<<mblocks, 256, 0, s>>>((const char*) C->data, C->n, C->width, C->key_off, C->key_bytes, step, mm, nullptr);
 		PG_LAUNCHED(ctx);
@@ -796,14 +828,18 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 		if (span >= MJ_MAX_RANGE || span >= std::max<unsigned long long>(MJ_MIN_RANGE + (MJ_MIN_RANGE >> 4), 16 * C->n)) break;
 		const uint32_t range = (uint32_t) span + 1;
 		const long long kmin = (long long) (h[0] ^ (1ull << 63));
-		// [counts, sums of MJ_SCAN counts, values]
+		// [counts, sums of MJ_SCAN counts, values, listed slices]
 		PgScratch tables(ctx, s), copies(ctx, s);
 		uint32_t* cnt = nullptr;
 		uint64_t* sums = nullptr;
 		unsigned long long* val = nullptr;
 		const uint64_t nb = pg_div_up(range, MJ_SCAN);
 		if (tables.want((void**) &cnt, (uint64_t) range * 4)) return PG_OK;
-		if (materialize && (tables.want((void**) &sums, nb * 8) || tables.want((void**) &val, C->n * 8))) return PG_OK;
+		unsigned long long* list = nullptr;
+		// (A warp with more rows than an output of at most MJ_SLICE_MAX takes needs no list.)
+		const uint64_t slices = materialize && out_capacity > MJ_SLICE_MAX ? mj_slices(out_capacity) : 0;
+		if (materialize && (tables.want((void**) &sums, nb * 8) || tables.want((void**) &val, C->n * 8) ||
+				(slices && tables.want((void**) &list, slices * 8)))) return PG_OK;
 		// Rows of more tuples than L2 holds values of: both sides by the top 8 bits of
 		// the window first (without memory for the copies, as they are), then one piece of
 		// the input a block, so that the blocks in flight use the same part of the table.
@@ -864,12 +900,16 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 			const int fblocks = grid(C->n, 256, MJ_FILL_BLOCKS_PER_SM);
 			k_mj_fill<<<fblocks, 256, 0, s>>>(cdata, C->n, C->key_off, kmin, range, bp, cnt, val, meta, vmm);
 			PG_LAUNCHED(ctx);
-#define MJ_ROWS(T) k_mj_rows<T><<<grid(P->n, 256 * T, MJ_ROWS_BLOCKS_PER_SM), 256, 0, s>>>(pdata, P->n, P->key_off, kmin, \
-				range, cnt, val, wsel, reinterpret_cast<uint4*>(out), out_capacity, agg, meta, vmm)
-			if (!parted && C->n / 2 >= range) MJ_ROWS(2);
-			else MJ_ROWS(4);
+#define MJ_ROWS(T, SLICE, blocks) do { k_mj_rows<T, SLICE><<<blocks, 256, 0, s>>>(pdata, P->n, P->key_off, kmin, range, cnt, \
+				val, wsel, reinterpret_cast<uint4*>(out), out_capacity, agg, meta, vmm, list, slices, mm + 9); \
+				PG_LAUNCHED(ctx); } while (0)
+			const bool two = !parted && C->n / 2 >= range;
+			if (two) MJ_ROWS(2, false, grid(P->n, 256 * 2, MJ_ROWS_BLOCKS_PER_SM));
+			else MJ_ROWS(4, false, grid(P->n, 256 * 4, MJ_ROWS_BLOCKS_PER_SM));
+			const int sblocks = (int) std::min<uint64_t>(pg_div_up(slices, 8), (uint64_t) ctx->sm_count * 6);
+			if (slices && two) MJ_ROWS(2, true, sblocks);
+			else if (slices) MJ_ROWS(4, true, sblocks);
 #undef MJ_ROWS
-			PG_LAUNCHED(ctx);
 		}
 		unsigned long long o[4];     // rows, sum, (largest count, key outside)
 		rc = pg_readback(ctx, s, agg, 3, nullptr, o, "pg_mpsm_join");

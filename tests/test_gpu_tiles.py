@@ -357,3 +357,34 @@ def test_mpsm_few_keys_counted_in_shared_memory(ctx, n, keys, width):
         for col in (0, 1):
             _, got, s = ctx.mpsm(a, b, proj=(("P", 8, 8), ("B", 8, 8)), flags=gpu.JOIN_COUNT | gpu.JOIN_SUM, sum_col=col)
             assert (got, s) == (want, sums[of[col]])
+
+
+# A warp's probe tuples (64 or 128 of them) with more than 8192 rows in all are written in
+# slices of 2048 rows by a second launch: one row either side of both, tuples of many
+# rows among others, more rows than the output takes (counted, not written), and an
+# output too small for any slice.
+@pytest.mark.parametrize("dup", [1, 5])
+@pytest.mark.parametrize("runs", [[8191], [8192], [8193], [10_240, 10_241], [16_384, 16_384, 3], [4000, 4193, 9000], [130] * 64])
+def test_mpsm_slices_of_long_runs(ctx, runs, dup):
+    rng = np.random.default_rng(sum(runs))
+    others = 3000
+    R = np.concatenate([np.full(x, i) for i, x in enumerate(runs)] + [np.repeat(np.arange(others) + len(runs), dup)])
+    R = np.stack([R, rng.integers(0, 1 << 31, size=R.size)], axis=1).astype(np.int64)
+    R = R[rng.permutation(R.shape[0])]
+    S = np.concatenate([np.arange(len(runs)), rng.integers(len(runs), len(runs) + others + 5, size=500)])
+    S = np.stack([S, np.arange(S.size)], axis=1).astype(np.int64)
+    _mpsm(ctx, R, S)
+    L, res, n = gpu.lib(), gpu.JoinResult(), 0
+    dR, dS = ctx.upload(R), ctx.upload(S)
+    rR, rS = ctx.rel(dR, R.shape[0], 16), ctx.rel(dS, S.shape[0], 16)
+    c, nc = gpu.cols((("P", 8, 8), ("B", 8, 8)))
+    full = int(np.bincount(R[:, 0], minlength=len(runs) + others + 5)[S[:, 0]].sum())
+    for cap in (0, 100, 8192, 8193, full // 2, full - 1):
+        if cap >= full:
+            continue
+        out = ctx.alloc(16 * (cap + 64))
+        ctx._check(L.pg_memset(ctx.h, ctx.stream, out.ptr, 0xA5, 16 * (cap + 64)))
+        rc = L.pg_mpsm_join(ctx.h, ctx.stream, ctypes.byref(rR), ctypes.byref(rS), c, nc, out.ptr, cap,
+                            gpu.JOIN_MATERIALIZE, -1, ctypes.byref(res))
+        assert rc == gpu.PG_ERR_OUTPUT_FULL and res.n_out == full
+        assert (ctx.download(out, 16 * (cap + 64))[16 * cap:] == 0xA5).all()
