@@ -252,31 +252,32 @@ __global__ void k_mj_write(MjSide R, MjSide S, MjCols pc, const uint64_t* __rest
 	}
 }
 
-static int mj_runs(pg_ctx* ctx, cudaStream_t s, const pg_rec* rec, uint64_t n, uint64_t** starts,
-		long long** keys, uint64_t* nruns)
+// Runs of both sides, with one readback of their numbers.
+static int mj_runs(pg_ctx* ctx, cudaStream_t s, const pg_rec* const (&rec)[2], const uint64_t (&n)[2], uint64_t* (&starts)[2],
+		long long* (&keys)[2], uint64_t (&nruns)[2])
 {
 	int rc;
-	const uint64_t nchunks = pg_div_up(std::max<uint64_t>(n, 1), MJ_RUN_CHUNK);
-	uint64_t* cc = nullptr;
-	uint64_t* total = nullptr;
-	if ((rc = pg_alloc_async(ctx, s, (void**) &cc, (nchunks + 1) * 8))) return rc;
-	if ((rc = pg_alloc_async(ctx, s, (void**) &total, 8))) return rc;
-	const int blocks = (int) std::min<uint64_t>(nchunks, (uint64_t) ctx->sm_count * 8);
-	if (n) { k_run_count<<<blocks, MJ_RUN_THREADS, 0, s>>>(rec, n, cc); PG_LAUNCHED(ctx); }
-	else PG_CUDA(ctx, cudaMemsetAsync(cc, 0, 8, s));
-	if ((rc = pg_scan_u64(ctx, s, cc, nchunks, total))) return rc;
-	uint64_t nr = 0;
-	PG_CUDA(ctx, cudaMemcpyAsync(&nr, total, 8, cudaMemcpyDeviceToHost, s));
+	PgScratch mem(ctx, s);
+	uint64_t *cc[2], *total = nullptr;
+	if ((rc = mem.get((void**) &total, 16))) return rc;
+	for (int i = 0; i < 2; ++i) {
+		const uint64_t nchunks = pg_div_up(n[i], MJ_RUN_CHUNK);
+		if ((rc = mem.get((void**) &cc[i], (nchunks + 1) * 8))) return rc;
+		k_run_count<<<(int) std::min<uint64_t>(nchunks, (uint64_t) ctx->sm_count * 8), MJ_RUN_THREADS, 0, s>>>(rec[i], n[i], cc[i]);
+		PG_LAUNCHED(ctx);
+		if ((rc = pg_scan_u64(ctx, s, cc[i], nchunks, total + i))) return rc;
+	}
+	PG_CUDA(ctx, cudaMemcpyAsync(nruns, total, 16, cudaMemcpyDeviceToHost, s));
 	PG_CUDA(ctx, cudaStreamSynchronize(s));
-	uint64_t* st = nullptr;
-	long long* rk = nullptr;
-	if ((rc = pg_alloc_async(ctx, s, (void**) &st, (nr + 1) * 8))) return rc;
-	if ((rc = pg_alloc_async(ctx, s, (void**) &rk, (nr + 1) * 8))) return rc;
-	if (n) { k_run_write<<<blocks, MJ_RUN_THREADS, 0, s>>>(rec, n, cc, st, rk); PG_LAUNCHED(ctx); }
-	PG_CUDA(ctx, cudaMemcpyAsync(st + nr, &n, 8, cudaMemcpyHostToDevice, s));
-	pg_free_async(ctx, s, cc);
-	pg_free_async(ctx, s, total);
-	*starts = st; *keys = rk; *nruns = nr;
+	for (int i = 0; i < 2; ++i) {
+		if ((rc = pg_alloc_async(ctx, s, (void**) &starts[i], (nruns[i] + 1) * 8))) return rc;
+		if ((rc = pg_alloc_async(ctx, s, (void**) &keys[i], (nruns[i] + 1) * 8))) return rc;
+		const uint64_t nchunks = pg_div_up(n[i], MJ_RUN_CHUNK);
+		k_run_write<<<(int) std::min<uint64_t>(nchunks, (uint64_t) ctx->sm_count * 8), MJ_RUN_THREADS, 0, s>>>(rec[i], n[i], cc[i],
+				starts[i], keys[i]);
+		PG_LAUNCHED(ctx);
+		PG_CUDA(ctx, cudaMemcpyAsync(starts[i] + nruns[i], &n[i], 8, cudaMemcpyHostToDevice, s));
+	}
 	return PG_OK;
 }
 
@@ -764,6 +765,47 @@ static bool mj_v16(const pg_rel* r)
 		!(reinterpret_cast<uintptr_t>(r->data) & 15);
 }
 
+// First and last key into mm = [~first, last] (keys ^ 2^63 as unsigned); zeros when
+// they show that the side is not sorted.
+__global__ void k_mj_ends(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, uint32_t kbytes,
+		unsigned long long* __restrict__ mm)
+{
+	const unsigned long long a = (unsigned long long) pg_load_key(in + koff, kbytes) ^ (1ull << 63);
+	const unsigned long long b = (unsigned long long) pg_load_key(in + (n - 1) * W + koff, kbytes) ^ (1ull << 63);
+	mm[0] = a <= b ? ~a : 0;
+	mm[1] = a <= b ? b : 0;
+}
+
+// The sides' flags, and what the device made of them.
+struct MjSorted {
+	bool flagged[2], known, sorted[2];
+};
+
+// Whether the flagged sides are sorted, in one readback, unless that is known.
+static int mj_confirm_sorted(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_rel* S, MjSorted* f)
+{
+	if (f->known || !(f->flagged[0] || f->flagged[1])) return PG_OK;
+	int rc;
+	PgScratch mem(ctx, s);
+	unsigned long long* mm = nullptr;             // [key range, unsorted, spare] of each side
+	if ((rc = mem.get((void**) &mm, 64))) return rc;
+	PG_CUDA(ctx, cudaMemsetAsync(mm, 0, 64, s));
+	for (int i = 0; i < 2; ++i) {
+		if (!f->flagged[i]) continue;
+		const pg_rel* r = i ? S : R;
+		const int blocks = (int) std::min<uint64_t>(pg_div_up(r->n, 256), (uint64_t) ctx->sm_count * 8);
+		k_mj_minmax<<<blocks, 256, 0, s>>>((const char*) r->data, r->n, r->width, r->key_off, r->key_bytes, 1, mm + 4 * i,
+				mm + 4 * i + 2);
+		PG_LAUNCHED(ctx);
+	}
+	unsigned long long h[8];
+	PG_CUDA(ctx, cudaMemcpyAsync(h, mm, 64, cudaMemcpyDeviceToHost, s));
+	PG_CUDA(ctx, cudaStreamSynchronize(s));
+	for (int i = 0; i < 2; ++i) f->sorted[i] = f->flagged[i] && !h[4 * i + 2];
+	f->known = true;
+	return PG_OK;
+}
+
 // Rows of more tuples than this partition both sides first: 64M x 64M with four
 // duplicates a key 6.83 -> 4.40 ms (4-byte values; by sorting both sides in buckets 5.98),
 // 48M with 2-byte values and a group-by 4.76 -> 3.80; 32M 2.33 -> 2.74 with 2-byte values,
@@ -778,7 +820,7 @@ static bool mj_v16(const pg_rel* r)
 // false (nothing produced): the caller sorts. So it does where the tables do not fit in
 // memory; the partitioned copies are the first to be done without.
 static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_rel* S, const MjCols& pc, int sum_col,
-		int flags, void* out, uint64_t out_capacity, pg_join_result* res, bool* handled)
+		int flags, void* out, uint64_t out_capacity, pg_join_result* res, MjSorted* sorted, bool* handled)
 {
 	*handled = false;
 	const bool materialize = (flags & PG_JOIN_MATERIALIZE) != 0;
@@ -789,9 +831,9 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 	if (materialize && sum_col >= 0) {      // the sum as a join of its own, then the rows
 		pg_join_result a;
 		bool done = false;
-		int rs = mj_dense_join(ctx, s, R, S, pc, sum_col, flags & ~PG_JOIN_MATERIALIZE, nullptr, 0, &a, &done);
+		int rs = mj_dense_join(ctx, s, R, S, pc, sum_col, flags & ~PG_JOIN_MATERIALIZE, nullptr, 0, &a, sorted, &done);
 		if (rs || !done) return rs;
-		if ((rs = mj_dense_join(ctx, s, R, S, pc, -1, flags, out, out_capacity, res, handled)) || !*handled) return rs;
+		if ((rs = mj_dense_join(ctx, s, R, S, pc, -1, flags, out, out_capacity, res, sorted, handled)) || !*handled) return rs;
 		res->sum = a.sum;
 		return PG_OK;
 	}
@@ -799,6 +841,7 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 	const bool sum_build = sum_col >= 0 && pc.side[sum_col] == 0;
 	const bool count_build = materialize || (sum_col >= 0 ? !sum_build : R->n <= S->n);
 	const pg_rel *C = count_build ? R : S, *P = count_build ? S : R;
+	const int ci = count_build ? 0 : 1, pi = 1 - ci;
 	int rc;
 	// [~key min, key max], [rows, sum], [largest count, key outside], two words of
 	// pg_readback, [~value min, value max], slices listed
@@ -808,16 +851,23 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 	unsigned long long* agg = mm + 2;
 	unsigned int* meta = reinterpret_cast<unsigned int*>(mm + 4);
 	unsigned long long* vmm = mm + 7;
-	for (int attempt = C->n >= (1ull << 22) ? 0 : 1; attempt < 2; ++attempt) {
+	// -1: from a flagged side's ends; 0: from a sample; 1: from every key.
+	const int first = C->n >= (1ull << 22) ? 0 : 1;
+	for (int attempt = sorted->flagged[ci] ? -1 : first; attempt < 2; attempt = std::max(attempt + 1, first)) {
 		const uint64_t step = attempt == 0 ? 1024 : 1;
 		PG_CUDA(ctx, cudaMemsetAsync(mm, 0, 80, s));
-		const int mblocks = (int) std::min<uint64_t>(pg_div_up(pg_div_up(C->n, step), 256), (uint64_t) ctx->sm_count * 8);
-		k_mj_minmax<<<mblocks, 256, 0, s>>>((const char*) C->data, C->n, C->width, C->key_off, C->key_bytes, step, mm, nullptr);
+		if (attempt < 0) {
+			k_mj_ends<<<1, 1, 0, s>>>((const char*) C->data, C->n, C->width, C->key_off, C->key_bytes, mm);
+		} else {
+			const int mblocks = (int) std::min<uint64_t>(pg_div_up(pg_div_up(C->n, step), 256), (uint64_t) ctx->sm_count * 8);
+			k_mj_minmax<<<mblocks, 256, 0, s>>>((const char*) C->data, C->n, C->width, C->key_off, C->key_bytes, step, mm, nullptr);
+		}
 		PG_LAUNCHED(ctx);
-		unsigned long long h[4];
+		unsigned long long h[2];
 		PG_CUDA(ctx, cudaMemcpyAsync(h, mm, 16, cudaMemcpyDeviceToHost, s));
 		PG_CUDA(ctx, cudaStreamSynchronize(s));
 		h[0] = ~h[0];
+		if (h[0] > h[1]) continue;                                        // not sorted
 		if (step > 1) {
 			const unsigned long long slack = (h[1] - h[0]) / 64 + 64;
 			h[0] = h[0] > slack ? h[0] - slack : 0;
@@ -845,22 +895,26 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 		// the input a block, so that the blocks in flight use the same part of the table.
 		char* split[2] = {nullptr, nullptr};
 		bool parted = false;
-		if (materialize && C->n > MJ_SPLIT_TUPLES && P->n > MJ_SPLIT_TUPLES / 4 &&
-				!copies.want((void**) &split[0], C->n * 16) && !copies.want((void**) &split[1], P->n * 16)) {
+		// A side that is sorted is in pieces as it is.
+		const bool part = materialize && C->n > MJ_SPLIT_TUPLES && P->n > MJ_SPLIT_TUPLES / 4;
+		if (part && (rc = mj_confirm_sorted(ctx, s, R, S, sorted))) return rc;
+		const bool csorted = sorted->sorted[ci], psorted = sorted->sorted[pi];
+		if (part && (csorted || !copies.want((void**) &split[0], C->n * 16)) &&
+				(psorted || !copies.want((void**) &split[1], P->n * 16))) {
 			pg_hashfn f = {};
 			f.fn = PG_FN_PARAMMODULO;
 			f.nbuckets = 256;
 			f.min = kmin;
 			f.skipbits = range > 256 ? 24 - __builtin_clz(range - 1) : 0;
 			f.k = (int64_t) 255 << f.skipbits;
-			rc = pg_partition_fn(ctx, s, C, f, split[0], nullptr);
-			if (!rc) rc = pg_partition_fn(ctx, s, P, f, split[1], nullptr);
+			rc = csorted ? PG_OK : pg_partition_fn(ctx, s, C, f, split[0], nullptr);
+			if (!rc && !psorted) rc = pg_partition_fn(ctx, s, P, f, split[1], nullptr);
 			if (rc && rc != PG_ERR_OOM) return rc;
 			parted = !rc;
 			if (rc) cudaGetLastError();
 		}
-		const char* const cdata = (const char*) (parted ? split[0] : C->data);
-		const char* const pdata = (const char*) (parted ? split[1] : P->data);
+		const char* const cdata = (const char*) (parted && !csorted ? split[0] : C->data);
+		const char* const pdata = (const char*) (parted && !psorted ? split[1] : P->data);
 		auto grid = [&](uint64_t n, uint32_t per_block, uint32_t per_sm) -> int {
 			const uint64_t b = pg_div_up(n, per_block);
 			return (int) (parted ? b : std::min<uint64_t>(b, (uint64_t) ctx->sm_count * per_sm));
@@ -926,24 +980,6 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 	return PG_OK;
 }
 
-// Whether a side flagged as sorted is, on the device.
-static int mj_confirm_sorted(pg_ctx* ctx, cudaStream_t s, const pg_rel* r, bool* sorted)
-{
-	int rc;
-	unsigned long long* mm = nullptr;
-	if ((rc = pg_alloc_async(ctx, s, (void**) &mm, 32))) return rc;
-	PG_CUDA(ctx, cudaMemsetAsync(mm, 0, 32, s));
-	const int blocks = (int) std::min<uint64_t>(pg_div_up(r->n, 256), (uint64_t) ctx->sm_count * 8);
-	k_mj_minmax<<<blocks, 256, 0, s>>>((const char*) r->data, r->n, r->width, r->key_off, r->key_bytes, 1, mm, mm + 2);
-	PG_LAUNCHED(ctx);
-	unsigned long long down = 0;
-	PG_CUDA(ctx, cudaMemcpyAsync(&down, mm + 2, 8, cudaMemcpyDeviceToHost, s));
-	PG_CUDA(ctx, cudaStreamSynchronize(s));
-	pg_free_async(ctx, s, mm);
-	*sorted = !down;
-	return PG_OK;
-}
-
 extern "C" int pg_mpsm_join(pg_ctx* ctx, pg_stream stream, const pg_rel* R, const pg_rel* S,
 		const pg_col* proj, int nproj, void* out, uint64_t out_capacity,
 		int flags, int sum_col, pg_join_result* res)
@@ -972,14 +1008,14 @@ extern "C" int pg_mpsm_join(pg_ctx* ctx, pg_stream stream, const pg_rel* R, cons
 	if (R->n == 0 || S->n == 0) return PG_OK;
 	cudaStream_t s = (cudaStream_t) stream;
 	int rc;
-	bool r_sorted = false, s_sorted = false;   // confirmed on the device
+	MjSorted sorted = {{(flags & PG_JOIN_BUILD_SORTED) != 0, (flags & PG_JOIN_PROBE_SORTED) != 0}, false, {false, false}};
 	if (R->n < (1ull << 32) && S->n < (1ull << 32)) {
 		bool handled = false;
-		if ((rc = mj_dense_join(ctx, s, R, S, pc, sum_col, flags, out, out_capacity, res, &handled))) return rc;
+		if ((rc = mj_dense_join(ctx, s, R, S, pc, sum_col, flags, out, out_capacity, res, &sorted, &handled))) return rc;
 		if (handled) return PG_OK;
-		if ((flags & PG_JOIN_BUILD_SORTED) && (rc = mj_confirm_sorted(ctx, s, R, &r_sorted))) return rc;
-		if ((flags & PG_JOIN_PROBE_SORTED) && (rc = mj_confirm_sorted(ctx, s, S, &s_sorted))) return rc;
+		if ((rc = mj_confirm_sorted(ctx, s, R, S, &sorted))) return rc;
 	}
+	const bool r_sorted = sorted.sorted[0], s_sorted = sorted.sorted[1];
 	// A sorted 16-byte tuple keyed at offset 0 is its own sorted record array.
 	pg_rec *rr = nullptr, *sr = nullptr;
 	const bool r_own = !(r_sorted && pg_sort_mode(R) == 0 && !(reinterpret_cast<uintptr_t>(R->data) & 15));
@@ -990,11 +1026,14 @@ extern "C" int pg_mpsm_join(pg_ctx* ctx, pg_stream stream, const pg_rel* R, cons
 	else sr = (pg_rec*) S->data;
 	MjSide RS{rr, (const char*) R->data, R->width, R->key_off, pg_sort_mode(R), nullptr, 0};
 	MjSide SS{sr, (const char*) S->data, S->width, S->key_off, pg_sort_mode(S), nullptr, 0};
-	uint64_t *rst = nullptr, *sst = nullptr;
-	long long *rk = nullptr, *sk = nullptr;
-	if ((rc = mj_runs(ctx, s, rr, R->n, &rst, &rk, &RS.nruns))) return rc;
-	if ((rc = mj_runs(ctx, s, sr, S->n, &sst, &sk, &SS.nruns))) return rc;
+	uint64_t* starts[2] = {nullptr, nullptr};
+	long long* rkeys[2] = {nullptr, nullptr};
+	uint64_t nruns[2];
+	if ((rc = mj_runs(ctx, s, {rr, sr}, {R->n, S->n}, starts, rkeys, nruns))) return rc;
+	uint64_t *rst = starts[0], *sst = starts[1];
+	long long *rk = rkeys[0], *sk = rkeys[1];
 	RS.run_start = rst; SS.run_start = sst;
+	RS.nruns = nruns[0]; SS.nruns = nruns[1];
 	uint64_t *counts = nullptr, *match = nullptr;
 	unsigned long long* acc = nullptr;  // [total, sum]
 	if ((rc = pg_alloc_async(ctx, s, (void**) &counts, (RS.nruns + 1) * 8))) return rc;

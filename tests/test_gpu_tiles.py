@@ -388,3 +388,35 @@ def test_mpsm_slices_of_long_runs(ctx, runs, dup):
                             gpu.JOIN_MATERIALIZE, -1, ctypes.byref(res))
         assert rc == gpu.PG_ERR_OUTPUT_FULL and res.n_out == full
         assert (ctx.download(out, 16 * (cap + 64))[16 * cap:] == 0xA5).all()
+
+
+# Flagged sides: the window comes from the counted side's ends, and a side confirmed
+# sorted is not partitioned first. Flags that hold, that do not, and a side whose ends
+# do not show that it is not sorted.
+@pytest.mark.parametrize("n,m", [(50_001, 20_003), ((32 << 20) + 3, (8 << 20) + 5)])
+@pytest.mark.parametrize("case", ["sorted", "build_only", "probe_only", "neither", "wide_inside"])
+def test_mpsm_flagged_sides(ctx, n, m, case):
+    rng = np.random.default_rng(n)
+    keys = np.arange(n) * 2 - 9
+    pick = np.sort(rng.integers(0, n, size=m))
+    if case in ("probe_only", "neither"):
+        keys = keys[rng.permutation(n)]
+    if case in ("build_only", "neither"):
+        pick = pick[rng.permutation(m)]
+    if case == "wide_inside":
+        keys[n // 2] = 1 << 45
+    R = np.stack([keys, rng.integers(0, 1 << 20, size=n)], axis=1)
+    S = np.stack([np.sort(keys)[pick] if case != "wide_inside" else keys[pick], np.arange(m)], axis=1)
+    if case in ("build_only", "neither"):
+        S[:, 0] = np.sort(keys)[pick]
+    order = np.argsort(R[:, 0], kind="stable")
+    want = R[order[np.searchsorted(R[order, 0], S[:, 0])], 1]
+    flags = gpu.JOIN_BUILD_SORTED | gpu.JOIN_PROBE_SORTED
+    proj = (("P", 8, 8), ("B", 8, 8))
+    _, count, total = ctx.mpsm(R, S, proj=proj, flags=gpu.JOIN_COUNT | gpu.JOIN_SUM | flags, sum_col=1)
+    assert (count, total) == (m, int(want.sum()))
+    got, rows, _ = ctx.mpsm(R, S, proj=proj, flags=gpu.JOIN_MATERIALIZE | flags)
+    got = np.ascontiguousarray(got).view(np.int64).reshape(-1, 2)
+    seen = np.full(m, -1, dtype=np.int64)
+    seen[got[:, 0]] = got[:, 1]
+    assert rows == m and np.array_equal(seen, want)
