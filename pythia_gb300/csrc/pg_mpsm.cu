@@ -613,8 +613,8 @@ k_mj_fill(const char* __restrict__ R, uint64_t n, uint32_t koff, long long kmin,
 // Bound by DRAM: the values' scattered reads miss L2 under the stream of rows
 // (16M tuples, 64M rows, 4-byte values: 1.36 GB read and 1.07 written). The whole join
 // above with its group-by: no limit on registers 1214 us, with 6 blocks an SM 1160, and
-// two tuples a lane instead of four 1105; of keys with one row 1484, 1513 and 1590, so
-// those take four.
+// two tuples a lane instead of four 1105 (1140 with the slices' checks); of keys with one
+// row 1484, 1513 and 1590, so those take four.
 //
 // A warp's tuples may have thousands of rows each. Those of more than MJ_SLICE_MAX rows
 // in all go on a list instead, MJ_SLICE rows an entry, and a second launch (SLICE) has a
@@ -809,12 +809,15 @@ static int mj_confirm_sorted(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const
 // Rows of more tuples than this partition both sides first: 64M x 64M with four
 // duplicates a key 6.83 -> 4.40 ms (4-byte values; by sorting both sides in buckets 5.98),
 // 48M with 2-byte values and a group-by 4.76 -> 3.80; 32M 2.33 -> 2.74 with 2-byte values,
-// 4.16 -> 3.74 with 4-byte ones.
+// 4.16 -> 3.74 with 4-byte ones (how wide they are is known only after the counting pass,
+// which the copies come before).
 #define MJ_SPLIT_TUPLES (32ull << 20)
 
 // The join by a table of counts when the counted side's keys span a compact
-// range: at most 2^24 values, or 16 times its tuples (64 M x 64 M with 2^30
-// spans: the table's random accesses still cost less than sorting both sides).
+// range: at most 2^24 values (1000 x 1000: sum 62 us against 161 sorted, rows 122
+// against 178), or 16 times its tuples, where the table's random accesses come near the
+// cost of sorting both sides (sum and rows: 16M x 16M 2.50 and 2.69 ms against 3.09 and
+// 3.28, 64M x 64M over 2^30 8.05 and 8.61 against 10.13 and 10.69).
 // The window comes from every 1024th tuple widened by 1/64 a side on large
 // inputs, checked by the counting pass, else from every tuple. *handled =
 // false (nothing produced): the caller sorts. So it does where the tables do not fit in
@@ -891,8 +894,10 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 		if (materialize && (tables.want((void**) &sums, nb * 8) || tables.want((void**) &val, C->n * 8) ||
 				(slices && tables.want((void**) &list, slices * 8)))) return PG_OK;
 		// Rows of more tuples than L2 holds values of: both sides by the top 8 bits of
-		// the window first (without memory for the copies, as they are), then one piece of
-		// the input a block, so that the blocks in flight use the same part of the table.
+		// the window first (without memory for the copies, as they are), then a grid that
+		// goes through them once, in order, so that the blocks in flight use the same part of
+		// the table (the counting pass two: its threads take two tuples half the input apart;
+		// side by side 64M tuples over 2^26 keys took 2% longer).
 		char* split[2] = {nullptr, nullptr};
 		bool parted = false;
 		// A side that is sorted is in pieces as it is.
