@@ -516,8 +516,9 @@ int pg_scan_u64(pg_ctx* ctx, cudaStream_t s, uint64_t* data, uint64_t n, uint64_
 	uint64_t nb = pg_div_up(n, SCAN_TILE);
 	uint64_t* last = nullptr;
 	int rc;
+	PgScratch mem(ctx, s);
 	if (total_dev) {
-		if ((rc = pg_alloc_async(ctx, s, (void**) &last, 8))) return rc;
+		if ((rc = mem.get((void**) &last, 8))) return rc;
 		PG_CUDA(ctx, cudaMemcpyAsync(last, data + n - 1, 8, cudaMemcpyDeviceToDevice, s));
 	}
 	if (nb == 1) {
@@ -525,18 +526,16 @@ int pg_scan_u64(pg_ctx* ctx, cudaStream_t s, uint64_t* data, uint64_t n, uint64_
 		PG_LAUNCHED(ctx);
 	} else {
 		uint64_t* sums = nullptr;
-		if ((rc = pg_alloc_async(ctx, s, (void**) &sums, nb * 8))) return rc;
+		if ((rc = mem.get((void**) &sums, nb * 8))) return rc;
 		k_scan_sums<<<(unsigned) nb, SCAN_THREADS, 0, s>>>(data, n, sums);
 		PG_LAUNCHED(ctx);
 		if ((rc = pg_scan_u64(ctx, s, sums, nb, nullptr))) return rc;
 		k_scan_apply<<<(unsigned) nb, SCAN_THREADS, 0, s>>>(data, n, sums);
 		PG_LAUNCHED(ctx);
-		pg_free_async(ctx, s, sums);
 	}
 	if (total_dev) {
 		k_scan_total<<<1, 1, 0, s>>>(data, last, n, total_dev);
 		PG_LAUNCHED(ctx);
-		pg_free_async(ctx, s, last);
 	}
 	return PG_OK;
 }

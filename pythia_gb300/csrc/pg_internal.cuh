@@ -67,6 +67,13 @@ struct PgScratch {
 		if (!rc) p[n++] = *q;
 		return rc;
 	}
+	// The caller's from now on.
+	void* keep(void* q)
+	{
+		for (int i = 0; i < n; ++i) if (p[i] == q) p[i] = p[--n];
+		return q;
+	}
+	void drop(void* q) { if (q) pg_free_async(ctx, s, keep(q)); }
 	// Memory that the caller can do without: true when there is none, and no error is
 	// left behind for the next launch.
 	bool want(void** q, size_t bytes)

@@ -550,7 +550,8 @@ static int sw_partition_as(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, const 
 	int rc;
 	uint32_t* counts = nullptr;               // [G][256], then the flag of a key outside the window
 	const size_t bytes = (size_t) G * SW_BUCKETS * 4 + 4;
-	if ((rc = pg_alloc_async(ctx, s, (void**) &counts, bytes))) return rc;
+	PgScratch mem(ctx, s);
+	if ((rc = mem.get((void**) &counts, bytes))) return rc;
 	int* outside = reinterpret_cast<int*>(counts + (size_t) G * SW_BUCKETS);
 	PG_CUDA(ctx, cudaMemsetAsync(counts, 0, bytes, s));
 	k_chunk_hist<FN, K0><<<dim3(G, SW_HIST_SPLIT), 512, 0, s>>>((const uint4*) in->data, n, in->key_off / 4, in->key_bytes, f,
@@ -560,13 +561,12 @@ static int sw_partition_as(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, const 
 		int bad = 0;
 		PG_CUDA(ctx, cudaMemcpyAsync(&bad, outside, 4, cudaMemcpyDeviceToHost, s));
 		PG_CUDA(ctx, cudaStreamSynchronize(s));
-		if (bad) { *check->refuted = true; pg_free_async(ctx, s, counts); return PG_OK; }
+		if (bad) { *check->refuted = true; return PG_OK; }
 	}
 	PG_CUDA(ctx, cudaFuncSetAttribute(k_part_sweep<FN, K0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(SwShared)));
 	k_part_sweep<FN, K0><<<G, SW_THREADS, sizeof(SwShared), s>>>((const uint4*) in->data, n, in->key_off / 4, in->key_bytes,
 			f, chunk, counts, offsets, (uint4*) out, ctx->d_status);
 	PG_LAUNCHED(ctx);
-	pg_free_async(ctx, s, counts);
 	return PG_OK;
 }
 
@@ -652,7 +652,8 @@ int pg_partition_fn(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, const pg_hash
 
 	int rc;
 	uint64_t* counts = nullptr;
-	if ((rc = pg_alloc_async(ctx, s, (void**) &counts, (size_t) B * G * 8 + 8))) return rc;
+	PgScratch mem(ctx, s);
+	if ((rc = mem.get((void**) &counts, (size_t) B * G * 8 + 8))) return rc;
 	const bool radix = f.fn == PG_FN_PARAMMODULO, mix = f.fn == PG_FN_MIXRADIX;
 	if (radix)
 		k_part_hist<PG_FN_PARAMMODULO><<<(unsigned) G, 512, B * sizeof(uint32_t), s>>>((const char*) in->data, n, W,
@@ -690,6 +691,5 @@ int pg_partition_fn(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, const pg_hash
 				sizeof(uint64_t), B, cudaMemcpyDeviceToDevice, s));
 		PG_CUDA(ctx, cudaMemcpyAsync(offsets + B, &in->n, sizeof(uint64_t), cudaMemcpyHostToDevice, s));
 	}
-	pg_free_async(ctx, s, counts);
 	return PG_OK;
 }

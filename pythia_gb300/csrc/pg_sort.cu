@@ -175,10 +175,9 @@ __global__ void k_records_to_tuples(const pg_rec* __restrict__ rec, uint64_t n, 
 }
 
 // ---------------------------------------------------------------------------
-// LSD radix path: when the keys span at most 2^32 values, ceil(bits/d) stable
-// 2^d-way partitions on successive d-bit digits of (key - min) (d = 8, or the
-// PG_TUNE_RADIX_BITS knob, 4..12) sort the
-// tuples (pg_partition.cu; each pass reads and writes the relation once). This
+// LSD radix path: ceil(bits / d) stable 2^d-way partitions on successive d-bit
+// digits of (key - min), d = 8 or the PG_TUNE_RADIX_BITS knob (4..12), sort the
+// tuples (pg_partition.cu; each pass reads them twice and writes them once). This
 // is ParameterizedModuloValueHasher::generate's multi-pass radix split
 // (hash.cpp:237-267) driven to completion. Ties keep input order.
 // ---------------------------------------------------------------------------
@@ -444,8 +443,9 @@ static int radix_passes(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, int64_t b
 
 // Sorts `in` into `out` by radix passes when the key span allows; returns
 // PG_OK with *done = false (nothing queued) when it does not. `tmp` holds n
-// tuples of scratch.
-static int radix_sort(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, void* out, void* tmp, bool* done)
+// tuples of scratch; `range`: the key range (sort_key_range), where it is known.
+static int radix_sort(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, void* out, void* tmp, const unsigned long long* range,
+		bool* done)
 {
 	*done = false;
 	const uint64_t n = in->n;
@@ -461,7 +461,7 @@ static int radix_sort(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, void* out, 
 	}
 	int rc;
 	unsigned long long h[2];
-	if (sweep && n >= (1ull << 22)) {
+	if (sweep && n >= (1ull << 22) && !range) {
 		// Large inputs: the window of the digits from every 1024th row, checked
 		// by the first pass, instead of a pass for the exact
 		// range: the aligned power of two around the sample, or the sample
@@ -482,13 +482,13 @@ static int radix_sort(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, void* out, 
 			if (!refuted) { *done = true; return PG_OK; }
 		}
 	}
-	if ((rc = sort_key_range(ctx, s, in, 1, h))) return rc;
+	if (range) { h[0] = range[0]; h[1] = range[1]; }
+	else if ((rc = sort_key_range(ctx, s, in, 1, h))) return rc;
 	const int bits = bits_of(h[1] - h[0]);
-	// LSD radix over the bits of key - min (while they fit 63 bits for other
-	// tuples than 16 bytes, whose digit function masks a signed difference). Bitonic tiles and merge-path
-	// merges instead for wider spans, and for small inputs whose span needs
-	// more than four 8-bit passes: there the few merge passes cost less than
-	// the radix passes (a histogram read and a scatter each).
+	// Tuples that k_part_sweep does not take (other widths, unaligned, other digits) go
+	// by a digit function that masks a signed difference: up to 63 bits. Wider spans go to
+	// the bitonic tiles and merge-path merges, and so do up to 2^18 of them whose span needs
+	// more than four 8-bit passes: the few merges cost less there.
 	if (bits > 63 && !sweep) return PG_OK;
 	if (path == 0 && bits > 32 && n <= (1ull << 18)) return PG_OK;
 	const long long kmin = (long long) (h[0] ^ (1ull << 63));
@@ -529,34 +529,35 @@ int pg_sort_mode(const pg_rel* r)
 
 // Sorts `in` into records; *recs receives a pool allocation of n records
 // (caller frees with pg_free_async on stream s).
-int pg_sort_records(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, pg_rec** recs)
+static int sort_records(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, const unsigned long long* range, pg_rec** recs)
 {
 	const uint64_t n = in->n;
 	int rc;
 	const int mode = pg_sort_mode(in);
+	PgScratch mem(ctx, s);
 	pg_rec *a = nullptr, *b = nullptr;
-	if ((rc = pg_alloc_async(ctx, s, (void**) &a, n * sizeof(pg_rec)))) return rc;
-	if (n == 0) { *recs = a; return PG_OK; }
+	if ((rc = mem.get((void**) &a, n * sizeof(pg_rec)))) return rc;
+	if (n == 0) { *recs = (pg_rec*) mem.keep(a); return PG_OK; }
 	{
 		// Radix path: sort 16-byte records (the tuples themselves when the
 		// layout is a 16-byte tuple keyed at 0).
 		pg_rec* src = nullptr;
 		pg_rel r = *in;
 		if (mode != 0) {
-			if ((rc = pg_alloc_async(ctx, s, (void**) &src, n * sizeof(pg_rec)))) return rc;
+			if ((rc = mem.get((void**) &src, n * sizeof(pg_rec)))) return rc;
 			const int blocks = (int) std::min<uint64_t>(pg_div_up(n, 256), (uint64_t) ctx->sm_count * 16);
 			k_make_records<<<blocks, 256, 0, s>>>((const char*) in->data, n, in->width, in->key_off,
 					in->key_bytes, mode, src);
 			PG_LAUNCHED(ctx);
 			r.data = src; r.width = 16; r.key_off = 0; r.key_bytes = 8;
 		}
-		if ((rc = pg_alloc_async(ctx, s, (void**) &b, n * sizeof(pg_rec)))) return rc;
+		if ((rc = mem.get((void**) &b, n * sizeof(pg_rec)))) return rc;
 		bool done = false;
-		if ((rc = radix_sort(ctx, s, &r, a, b, &done))) return rc;
-		pg_free_async(ctx, s, b);
+		if ((rc = radix_sort(ctx, s, &r, a, b, range, &done))) return rc;
+		mem.drop(b);
 		b = nullptr;
-		if (src) pg_free_async(ctx, s, src);
-		if (done) { *recs = a; return PG_OK; }
+		mem.drop(src);
+		if (done) { *recs = (pg_rec*) mem.keep(a); return PG_OK; }
 	}
 	const uint64_t tiles = pg_div_up(n, TS_TILE);
 	const size_t smem = TS_TILE * (sizeof(pg_rec) + 8 + 2);
@@ -566,16 +567,51 @@ int pg_sort_records(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, pg_rec** recs
 			in->key_bytes, mode, a, bulk_ok, ctx->d_status);
 	PG_LAUNCHED(ctx);
 	if (n > TS_TILE) {
-		if ((rc = pg_alloc_async(ctx, s, (void**) &b, n * sizeof(pg_rec)))) return rc;
+		if ((rc = mem.get((void**) &b, n * sizeof(pg_rec)))) return rc;
 		const unsigned blocks = (unsigned) pg_div_up(n, MG_CHUNK);
 		for (uint64_t L = TS_TILE; L < n; L <<= 1) {
 			k_merge_pass<<<blocks, MG_THREADS, 0, s>>>(a, b, n, L);
 			PG_LAUNCHED(ctx);
 			std::swap(a, b);
 		}
-		pg_free_async(ctx, s, b);
 	}
-	*recs = a;
+	*recs = (pg_rec*) mem.keep(a);
+	return PG_OK;
+}
+
+int pg_sort_records(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, pg_rec** recs)
+{
+	return sort_records(ctx, s, in, nullptr, recs);
+}
+
+// Passes over the tuples themselves, by their width, that cost no more than sorting
+// (key, row) records and gathering the tuples. Both read the exact key range first. A
+// pass over 20M tuples takes 290 us (8 bytes), 350 (12), 500 (24) or 700 (40); over the
+// records 205 to 270, with 480 to 950 to make them and gather. 20M tuples, tuples against
+// records: 8 bytes, 2 and 4 passes 628 against 889 us, 1163 against 1298; 12 bytes, 2: 707
+// and 1005; 24 bytes, 1 to 4: 574, 1029, 1481, 1935 and 955, 1210, 1567, 1776; 40 bytes, 3:
+// 2136 and 1760; 3M of 200 bytes, 2: 924 and 1156, of 100, 3: 819 and 771. Up to 2^20
+// records take one launch, and only the gather of wide tuples costs more: 1M of 100 bytes,
+// 1 and 2 passes 166 and 267 against 217 and 240; of 200, 2: 386 each; of 400, 1 and 2: 422
+// and 771 against 661 and 678. Below 40 MB the round trip for the range costs more than that.
+#define SORT_TUPLE_WIDTH 400        // of which the partition's smallest tiles of 256 fit shared memory
+static int sort_tuple_passes(uint32_t width, uint64_t n)
+{
+	if (n <= SS_MAX_ROWS) return n * width < (40ull << 20) ? -1 : width > 128 && width <= 256 ? 2 : 1;
+	return width <= 8 ? 5 : width <= 12 ? 4 : width <= 24 ? 3 : 2;
+}
+
+// Radix passes over the tuples. *done = false: not taken (the key span, or no memory).
+static int sort_tuples(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, void* out, const unsigned long long* range, bool* done)
+{
+	PgScratch mem(ctx, s);
+	void* tmp = nullptr;
+	*done = false;
+	if (mem.want(&tmp, in->n * in->width)) return PG_OK;
+	const int rc = radix_sort(ctx, s, in, out, tmp, range, done);
+	if (rc != PG_ERR_OOM) return rc;
+	cudaGetLastError();
+	*done = false;
 	return PG_OK;
 }
 
@@ -591,19 +627,32 @@ extern "C" int pg_sort_pages(pg_ctx* ctx, pg_stream stream, const pg_rel* in, vo
 	if (in->n == 0) return PG_OK;
 	pg_rec* recs = nullptr;
 	int rc;
-	// 16-byte tuples sort themselves. Others sort (key, row) records and gather
-	// the rows at the end (10M 24-byte tuples of 50 bits: 1.19 ms, against 1.78
-	// for seven passes over the tuples; knob 1 keeps that form).
-	if (in->width == 16 || ctx->tune[PG_TUNE_SORT_PATH] == 1) {
-		void* tmp = nullptr;
-		if ((rc = pg_alloc_async(ctx, s, &tmp, in->n * in->width))) return rc;
-		bool done = false;
-		rc = radix_sort(ctx, s, in, out, tmp, &done);
-		pg_free_async(ctx, s, tmp);
-		if (rc) return rc;
+	// 16-byte tuples sort themselves; others too where that takes few passes (knob 1:
+	// always), else as (key, row) records with the tuples gathered at the end. Up to 2^20
+	// records sort in one launch. Without memory for one form the other is tried.
+	const int64_t path = ctx->tune[PG_TUNE_SORT_PATH];
+	bool tuples = in->width == 16 || path == 1, done = false;
+	unsigned long long h[2];
+	const unsigned long long* range = nullptr;
+	if (!tuples && path == 0 && in->width <= SORT_TUPLE_WIDTH && in->n < (1ull << 32)) {
+		const int passes = sort_tuple_passes(in->width, in->n);
+		if (passes > 0) {
+			if ((rc = sort_key_range(ctx, s, in, 1, h))) return rc;
+			range = h;
+			tuples = (bits_of(h[1] - h[0]) + 7) / 8 <= passes;
+		}
+	}
+	if (tuples) {
+		if ((rc = sort_tuples(ctx, s, in, out, range, &done))) return rc;
 		if (done) return pg_check_status(ctx, s, "pg_sort_pages");
 	}
-	if ((rc = pg_sort_records(ctx, s, in, &recs))) return rc;
+	rc = sort_records(ctx, s, in, range, &recs);
+	if (rc == PG_ERR_OOM && !tuples && path == 0 && in->width <= SORT_TUPLE_WIDTH) {
+		cudaGetLastError();
+		int rt = sort_tuples(ctx, s, in, out, range, &done);
+		if (rt || done) return rt ? rt : pg_check_status(ctx, s, "pg_sort_pages");
+	}
+	if (rc) return rc;
 	const int mode = pg_sort_mode(in);
 	int blocks = (int) std::min<uint64_t>(pg_div_up(in->n, 256), (uint64_t) ctx->sm_count * 16);
 	k_records_to_tuples<<<blocks, 256, 0, s>>>(recs, in->n, mode, (const char*) in->data, in->width, (char*) out);

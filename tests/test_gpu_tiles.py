@@ -420,3 +420,21 @@ def test_mpsm_flagged_sides(ctx, n, m, case):
     seen = np.full(m, -1, dtype=np.int64)
     seen[got[:, 0]] = got[:, 1]
     assert rows == m and np.array_equal(seen, want)
+
+
+# Tuples other than 16 bytes: radix passes over the tuples where the keys need few,
+# over (key, row) records where they need more, and one launch up to 2^20 (wide tuples
+# again by passes). Either side of each, and of the widths that the passes take.
+@pytest.mark.parametrize("n,width,bits", [((1 << 20) + 1, 8, 30), ((1 << 20) + 1, 12, 32), ((1 << 20) + 1, 12, 33),
+                                          ((1 << 20) + 1, 24, 24), ((1 << 20) + 1, 24, 25), ((1 << 20) + 1, 40, 16),
+                                          ((1 << 20) + 1, 400, 8), ((1 << 20) + 1, 404, 8), (104_857, 400, 8), (104_858, 400, 8),
+                                          (104_858, 400, 9), (209_716, 200, 16), (83_000, 512, 8), ((1 << 20) + 1, 24, 0)])
+def test_sort_of_other_widths(ctx, n, width, bits):
+    rng = np.random.default_rng(width * bits + n)
+    rows = np.zeros((n, width // 4), dtype=np.int32)
+    rows[:, -1] = np.arange(n)
+    kb = 4 if width == 8 else 8
+    keys = rng.integers(0, 1 << bits, size=n) - (1 << bits >> 1)
+    keys[0], keys[1] = -(1 << bits >> 1), (1 << bits) - 1 - (1 << bits >> 1)
+    rows[:, : kb // 4] = keys.astype(np.int64 if kb == 8 else np.int32).view(np.int32).reshape(n, -1)
+    assert np.array_equal(ctx.sort(rows, (0, kb)), rows[np.argsort(keys, kind="stable")])

@@ -101,3 +101,34 @@ def _run(tmp_path, source):
 @pytest.mark.parametrize("n,m", [(100_003, 50_001), ((32 << 20) + 5, (8 << 20) + 3)])
 def test_counted_merge_join(tmp_path, n, m):
     _run(tmp_path, MPSM % (ROOT, n, m, 1 << 31))
+
+
+SORT = COMMON + """
+n, width, bits = %d, %d, %d
+rng = np.random.default_rng(n)
+rows = rng.integers(0, 1 << 30, size=(n, width // 4)).astype(np.int32)
+keys = rng.integers(0, 1 << bits, size=n)
+rows[:, :2] = keys.astype(np.int64).view(np.int32).reshape(n, 2)
+want = rows[np.argsort(keys, kind="stable")]
+dI, dO = ctx.upload(rows), ctx.alloc(rows.nbytes)
+r = ctx.rel(dI, n, width)
+
+def call():
+    return L.pg_sort_pages(ctx.h, ctx.stream, ref(r), dO.ptr)
+
+def right():
+    return np.array_equal(ctx.download(dO, rows.nbytes).view(np.int32).reshape(n, -1), want)
+
+each_failing(call, right, 16 * n)
+"""
+
+
+# One launch of records, passes over the tuples (few digits) and over records (many).
+@pytest.mark.parametrize("n,width,bits", [(50_000, 24, 20), ((1 << 20) + 77, 24, 16), ((1 << 20) + 77, 24, 40),
+                                          ((1 << 20) + 77, 8, 20)])
+def test_sort_of_other_widths(tmp_path, n, width, bits):
+    if width == 8:
+        source = SORT.replace("rows[:, :2]", "rows")
+    else:
+        source = SORT
+    _run(tmp_path, source % (ROOT, n, width, bits))
