@@ -9,7 +9,8 @@
 // output row comes from a warp that adds up the tiles' counts as they are
 // published, and the survivors are written with consecutive lanes on
 // consecutive words: one read of the relation and one write of the survivors.
-// Project stages tiles the same way: one read, one write. Both are bound by
+// Project stages tiles the same way: one read, one write. Tuples wide enough that some of
+// their sectors need not be read are not staged. Both are bound by
 // HBM; 50M 24-byte tuples, half passing, measured 370 us for the filter (0.72
 // of the copy rate; 835 us in two passes with a thread copying each tuple), and
 // 25M of them to 16-byte rows 160 us for the projection (378 us with a
@@ -19,11 +20,26 @@
 #include <cstring>
 
 #define FL_THREADS 256
-#define FL_ITEMS 8
-#define FL_TILE (FL_THREADS * FL_ITEMS)
-#define FL_MAX_WIDTH 1024
+// Wider tuples are not staged: their predicates read the columns' sectors and only
+// the survivors are read whole, a warp a survivor. 600 MB of tuples of 300, 400 and 1000
+// bytes, no survivors: staged 154, 195 and 138 us, unstaged 78, 71 and 51 (131, 115 and 65
+// in two passes); a third pass: 192, 218 and 166 against 151, 118 and 118 (572, 349 and 702);
+// all pass: 274, 264 and 226 against 336, 238 and 274 (2184, 1005 and 1689). At 240 bytes
+// staging is never slower than the two passes were (144 us with no survivors, 153), from
+// 300 it was.
+#define FL_STAGE_WIDTH 240
+#define FL_DIRECT_ROWS 512
 #define FL_TILE_BYTES (24 * 1024)     // eight blocks of 256 threads on an SM
 #define PJ_TILE_BYTES (24 * 1024)
+// A projection of at most a quarter of a wider tuple reads its columns straight from
+// memory: 600 MB of 400-byte tuples, 4, 48, 100 and 200 bytes kept: staged 170, 181, 193 and
+// 206 us, unstaged 58, 72, 131 and 162 (a thread a tuple 57, 158, 748 and 1647); of 1000-byte
+// ones, 8, 248 and 500: 109, 134 and 156 against 33, 95 to 119 and 184; of 136, 32 and 68: 135
+// and 156 against 132 and 218. Up to 128 bytes the sectors are all read anyway (100 bytes, 4
+// kept: 119 both).
+#define PJ_STAGE_WIDTH 128
+#define PJ_STAGE_MAX 1024
+#define PJ_DIRECT_ROWS 512
 #define HJ_PROJ_MAX 16
 
 int pg_pred_prepare(pg_ctx* ctx, const pg_pred* preds, int npred, uint32_t width, PgPredSet* out, bool* has_char)
@@ -71,62 +87,6 @@ bool pg_pred_as16(const pg_pred* preds, int npred, PgPred16* out)
 		out->v[i] = v;
 	}
 	return true;
-}
-
-// Tuples over FL_MAX_WIDTH bytes: survivors per tile of FL_TILE tuples, a scan,
-// and a second evaluation that writes them, a thread a tuple.
-__global__ void __launch_bounds__(FL_THREADS)
-k_filter_count(const char* __restrict__ in, uint64_t n, uint32_t w, const PgPredSet P, uint64_t* __restrict__ counts)
-{
-	__shared__ uint32_t wsum[FL_THREADS / 32];
-	const uint64_t base = (uint64_t) blockIdx.x * FL_TILE;
-	uint32_t c = 0;
-	#pragma unroll
-	for (int j = 0; j < FL_ITEMS; ++j) {
-		const uint64_t i = base + j * FL_THREADS + threadIdx.x;
-		if (i < n && pg_pred_eval(P, in + i * w)) ++c;
-	}
-	#pragma unroll
-	for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-	if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = c;
-	__syncthreads();
-	if (threadIdx.x == 0) {
-		uint32_t t = 0;
-		for (int k = 0; k < FL_THREADS / 32; ++k) t += wsum[k];
-		counts[blockIdx.x] = t;
-	}
-}
-
-__global__ void __launch_bounds__(FL_THREADS)
-k_filter_write(const char* __restrict__ in, uint64_t n, uint32_t w, const PgPredSet P,
-		const uint64_t* __restrict__ offs, char* __restrict__ out)
-{
-	__shared__ uint32_t cnt[FL_ITEMS][FL_THREADS / 32];
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	const uint64_t base = (uint64_t) blockIdx.x * FL_TILE;
-	uint32_t ball[FL_ITEMS];
-	#pragma unroll
-	for (int j = 0; j < FL_ITEMS; ++j) {
-		const uint64_t i = base + j * FL_THREADS + threadIdx.x;
-		ball[j] = __ballot_sync(0xffffffffu, i < n && pg_pred_eval(P, in + i * w));
-		if (lane == 0) cnt[j][warp] = __popc(ball[j]);
-	}
-	__syncthreads();
-	if (threadIdx.x == 0) {
-		uint32_t run = 0;
-		for (int j = 0; j < FL_ITEMS; ++j)
-			for (int k = 0; k < FL_THREADS / 32; ++k) { const uint32_t c = cnt[j][k]; cnt[j][k] = run; run += c; }
-	}
-	__syncthreads();
-	const uint64_t at = offs[blockIdx.x];
-	#pragma unroll
-	for (int j = 0; j < FL_ITEMS; ++j) {
-		if (!((ball[j] >> lane) & 1)) continue;
-		const uint64_t i = base + j * FL_THREADS + threadIdx.x;
-		const uint64_t o = at + cnt[j][warp] + __popc(ball[j] & ((1u << lane) - 1));
-		for (uint32_t b = 0; b < w; b += 4)
-			*reinterpret_cast<uint32_t*>(out + o * w + b) = __ldcs(reinterpret_cast<const uint32_t*>(in + i * w + b));
-	}
 }
 
 // Copies `bytes` (a multiple of 4) of a tile into shared memory: a bulk copy of
@@ -207,19 +167,19 @@ __device__ __forceinline__ void fl_scan_tiles(const uint32_t* __restrict__ count
 	if (lane == 0) *total = run;
 }
 
-// One tile a block (U = unit of the row copies), and one block whose first
+// One tile a block, in shared memory (STAGED) or where it is (U = unit of the row
+// copies), and one block whose first
 // warp scans the tiles' counts: the first to arrive, so it runs whenever a
 // tile waits for it, and every tile that it waits for has been taken by a
 // running block before any later tile.
-template <typename U>
+template <typename U, bool STAGED>
 __global__ void __launch_bounds__(FL_THREADS)
 k_filter(const char* __restrict__ in, uint64_t n, uint32_t w, uint32_t tile_rows, const PgPredSet P,
 		uint32_t* __restrict__ count, unsigned long long* __restrict__ first, unsigned int* __restrict__ ticket,
 		char* __restrict__ out, unsigned long long* __restrict__ total, int* __restrict__ status)
 {
 	extern __shared__ __align__(128) unsigned char fl_sm[];
-	unsigned char* const tile = fl_sm;                                                    // [tile_rows * w]
-	uint32_t* const mask = reinterpret_cast<uint32_t*>(tile + tile_rows * w);             // [tile_rows / 32]
+	uint32_t* const mask = reinterpret_cast<uint32_t*>(fl_sm + (STAGED ? tile_rows * w : 0));   // [tile_rows / 32]
 	uint32_t* const before = mask + tile_rows / 32;                                       // [tile_rows / 32]
 	uint16_t* const sel = reinterpret_cast<uint16_t*>(before + tile_rows / 32);           // [tile_rows]
 	__shared__ __align__(8) uint64_t bar;
@@ -235,10 +195,11 @@ k_filter(const char* __restrict__ in, uint64_t n, uint32_t w, uint32_t tile_rows
 	}
 	const uint64_t t = s_tile - 1;
 	const uint32_t rows = (uint32_t) pg_min64(tile_rows, n - t * tile_rows), chunks = (rows + 31) / 32;
-	fl_load_tile(tile, in + t * tile_rows * w, rows * w, &bar, status);
+	const char* const tile = STAGED ? reinterpret_cast<const char*>(fl_sm) : in + t * tile_rows * w;
+	if (STAGED) fl_load_tile(fl_sm, in + t * tile_rows * w, rows * w, &bar, status);
 	for (uint32_t c = warp; c < chunks; c += FL_THREADS / 32) {
 		const uint32_t i = c * 32 + lane;
-		const uint32_t m = __ballot_sync(0xffffffffu, i < rows && pg_pred_eval(P, reinterpret_cast<const char*>(tile) + i * w));
+		const uint32_t m = __ballot_sync(0xffffffffu, i < rows && pg_pred_eval(P, tile + (STAGED ? i * w : (uint64_t) i * w)));
 		if (lane == 0) mask[c] = m;
 	}
 	__syncthreads();
@@ -282,6 +243,25 @@ k_filter(const char* __restrict__ in, uint64_t n, uint32_t w, uint32_t tile_rows
 	if (s_first + s_count > n) return;                    // the wait gave up
 	U* const dst = reinterpret_cast<U*>(out + s_first * w);
 	const U* const src = reinterpret_cast<const U*>(tile);
+	if (!STAGED) {                                        // a warp Q survivors at once
+		constexpr int Q = sizeof(U) == 8 ? 8 : 4;
+		const uint32_t count = s_count;
+		for (uint32_t k0 = warp; k0 < count; k0 += Q * (FL_THREADS / 32))
+			for (uint32_t u = lane; u < upt; u += 32) {
+				U v[Q];
+				#pragma unroll
+				for (int q = 0; q < Q; ++q) {
+					const uint32_t k = k0 + q * (FL_THREADS / 32);
+					if (k < count) v[q] = __ldcs(src + (uint64_t) sel[k] * upt + u);
+				}
+				#pragma unroll
+				for (int q = 0; q < Q; ++q) {
+					const uint32_t k = k0 + q * (FL_THREADS / 32);
+					if (k < count) __stcs(dst + (uint64_t) k * upt + u, v[q]);
+				}
+			}
+		return;
+	}
 	// The loop starts at a 128-byte boundary of the output, so that a warp's
 	// store covers whole lines.
 	const uint32_t skew = (uint32_t) (reinterpret_cast<uintptr_t>(dst) / sizeof(U)) & (128 / sizeof(U) - 1);
@@ -319,38 +299,35 @@ extern "C" int pg_filter(pg_ctx* ctx, pg_stream stream, const pg_rel* in, const 
 		P.chars = chars;
 	}
 	uint64_t* scratch = nullptr;
-	unsigned long long* count = nullptr;
-	const uint32_t rows = fl_tile_rows(w, FL_TILE_BYTES);
-	const uint64_t ntiles = pg_div_up(in->n, w <= FL_MAX_WIDTH ? rows : FL_TILE);
-	if (w <= FL_MAX_WIDTH && ntiles < (1ull << 31) - 1) {
-		// [total, two words of pg_readback, ticket, first output row of each tile,
-		// survivors of each tile]
-		if ((rc = pg_alloc_async(ctx, s, (void**) &scratch, 32 + ntiles * 12))) return rc;
-		PG_CUDA(ctx, cudaMemsetAsync(scratch, 0, 32 + ntiles * 12, s));
-		unsigned long long* total = reinterpret_cast<unsigned long long*>(scratch);
-		const size_t smem = (size_t) rows * w + rows / 32 * 8 + rows * 2;
-		const uintptr_t o = reinterpret_cast<uintptr_t>(out);
-#define FL_LAUNCH(U) do { \
-		PG_CUDA(ctx, cudaFuncSetAttribute(k_filter<U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)); \
-		k_filter<U><<<(unsigned) ntiles + 1, FL_THREADS, smem, s>>>((const char*) in->data, in->n, w, rows, P, \
-				reinterpret_cast<uint32_t*>(total + 4 + ntiles), total + 4, reinterpret_cast<unsigned int*>(total + 3), (char*) out, total, ctx->d_status); } while (0)
-		if (!(w & 15) && !(o & 15)) FL_LAUNCH(uint4);
-		else if (!(w & 7) && !(o & 7)) FL_LAUNCH(uint2);
-		else FL_LAUNCH(uint32_t);
-#undef FL_LAUNCH
-		PG_LAUNCHED(ctx);
-		count = total;
-	} else {
-		if ((rc = pg_alloc_async(ctx, s, (void**) &scratch, (ntiles + 3) * 8))) return rc;
-		k_filter_count<<<(unsigned) ntiles, FL_THREADS, 0, s>>>((const char*) in->data, in->n, w, P, scratch);
-		PG_LAUNCHED(ctx);
-		if ((rc = pg_scan_u64(ctx, s, scratch, ntiles, scratch + ntiles))) return rc;
-		k_filter_write<<<(unsigned) ntiles, FL_THREADS, 0, s>>>((const char*) in->data, in->n, w, P, scratch, (char*) out);
-		PG_LAUNCHED(ctx);
-		count = reinterpret_cast<unsigned long long*>(scratch + ntiles);
+	const bool staged = w <= FL_STAGE_WIDTH;
+	const uint32_t rows = staged ? fl_tile_rows(w, FL_TILE_BYTES) : FL_DIRECT_ROWS;
+	const uint64_t ntiles = pg_div_up(in->n, rows);
+	if (ntiles >= (1ull << 31) - 1) {
+		pg_free_async(ctx, s, chars);
+		return pg_fail(ctx, PG_ERR_UNSUPPORTED, "pg_filter: too many tuples");
 	}
+	// [total, two words of pg_readback, ticket, first output row of each tile,
+	// survivors of each tile]
+	if ((rc = pg_alloc_async(ctx, s, (void**) &scratch, 32 + ntiles * 12))) { pg_free_async(ctx, s, chars); return rc; }
+	PG_CUDA(ctx, cudaMemsetAsync(scratch, 0, 32 + ntiles * 12, s));
+	unsigned long long* total = reinterpret_cast<unsigned long long*>(scratch);
+	const size_t smem = (staged ? (size_t) rows * w : 0) + rows / 32 * 8 + rows * 2;
+	const uintptr_t base = reinterpret_cast<uintptr_t>(out) | (staged ? 0 : reinterpret_cast<uintptr_t>(in->data));
+#define FL_LAUNCH(U, ST) do { \
+		if (ST) PG_CUDA(ctx, cudaFuncSetAttribute(k_filter<U, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)); \
+		k_filter<U, ST><<<(unsigned) ntiles + 1, FL_THREADS, smem, s>>>((const char*) in->data, in->n, w, rows, P, \
+				reinterpret_cast<uint32_t*>(total + 4 + ntiles), total + 4, reinterpret_cast<unsigned int*>(total + 3), (char*) out, total, ctx->d_status); } while (0)
+#define FL_LAUNCH_AS(ST) do { \
+		if (!((w | base) & 15)) FL_LAUNCH(uint4, ST); \
+		else if (!((w | base) & 7)) FL_LAUNCH(uint2, ST); \
+		else FL_LAUNCH(uint32_t, ST); } while (0)
+	if (staged) FL_LAUNCH_AS(true);
+	else FL_LAUNCH_AS(false);
+#undef FL_LAUNCH_AS
+#undef FL_LAUNCH
+	PG_LAUNCHED(ctx);
 	unsigned long long h[2];
-	rc = pg_readback(ctx, s, count, 1, nullptr, h, "pg_filter");
+	rc = pg_readback(ctx, s, total, 1, nullptr, h, "pg_filter");
 	pg_free_async(ctx, s, scratch);
 	pg_free_async(ctx, s, chars);
 	if (rc) return rc;
@@ -365,10 +342,10 @@ struct ProjCols {
 	uint32_t ow;                  // output words
 };
 
-// A tile of tuples in shared memory, then the output rows in units of U (1, 2
-// or 4 words). A thread keeps to one unit of the row, so its source words are
+// A tile of tuples in shared memory (STAGED) or where it is, then the output rows
+// in units of U (1, 2 or 4 words). A thread keeps to one unit of the row, so its source words are
 // looked up once; consecutive threads store consecutive units.
-template <typename U>
+template <typename U, bool STAGED>
 __global__ void __launch_bounds__(FL_THREADS)
 k_project(const char* __restrict__ in, uint64_t n, uint32_t iw, uint32_t tile_rows, const ProjCols pc,
 		char* __restrict__ out, int* __restrict__ status)
@@ -392,23 +369,23 @@ k_project(const char* __restrict__ in, uint64_t n, uint32_t iw, uint32_t tile_ro
 			k -= pc.words[c];
 		}
 	}
-	fl_load_tile(pj_sm, in + t0 * iw * 4, rows * iw * 4, &bar, status);
+	if (STAGED) fl_load_tile(pj_sm, in + t0 * iw * 4, rows * iw * 4, &bar, status);
 	if (r0 >= lanes) return;
-	const uint32_t* const tile = reinterpret_cast<const uint32_t*>(pj_sm);
+	const uint32_t* const tile = reinterpret_cast<const uint32_t*>(STAGED ? reinterpret_cast<const char*>(pj_sm) : in + t0 * iw * 4);
 	U* const dst = reinterpret_cast<U*>(out + t0 * pc.ow * 4);
 	#pragma unroll 4
 	for (uint32_t r = r0; r < rows; r += lanes) {
-		const uint32_t* const p = tile + r * iw;
+		const uint32_t* const p = tile + (STAGED ? r * iw : (uint64_t) r * iw);
 		U v;
-		if constexpr (UW == 4) v = make_uint4(p[src[0]], p[src[1]], p[src[2]], p[src[3]]);
-		else if constexpr (UW == 2) v = make_uint2(p[src[0]], p[src[1]]);
-		else v = p[src[0]];
+		auto word = [&](uint32_t q) { return STAGED ? p[src[q]] : __ldcs(p + src[q]); };
+		if constexpr (UW == 4) v = make_uint4(word(0), word(1), word(2), word(3));
+		else if constexpr (UW == 2) v = make_uint2(word(0), word(1));
+		else v = word(0);
 		__stcs(dst + r * upt + u, v);
 	}
 }
 
-// Tuples wider than FL_MAX_WIDTH bytes or rows wider than a block's units: one
-// thread per tuple.
+// Rows wider than a block's units: one thread per tuple.
 __global__ void k_project_wide(const uint32_t* __restrict__ in, uint64_t n, uint32_t iw, const ProjCols pc,
 		uint32_t* __restrict__ out)
 {
@@ -447,17 +424,22 @@ extern "C" int pg_project(pg_ctx* ctx, pg_stream stream, const pg_rel* in, const
 	const uint32_t iw = in->width / 4;
 	const uintptr_t o = reinterpret_cast<uintptr_t>(out);
 	const uint32_t uw = (pc.ow & 3) == 0 && !(o & 15) ? 4 : (pc.ow & 1) == 0 && !(o & 7) ? 2 : 1;
-	const uint32_t rows = fl_tile_rows(in->width, PJ_TILE_BYTES);
+	const bool staged = in->width <= PJ_STAGE_WIDTH || (in->width <= PJ_STAGE_MAX && 4 * pc.ow > iw);
+	// (Unstaged: blocks for every SM before rows for every thread.)
+	const uint32_t rows = staged ? fl_tile_rows(in->width, PJ_TILE_BYTES)
+		: (uint32_t) std::min<uint64_t>(PJ_DIRECT_ROWS, std::max<uint64_t>(32, in->n / ((uint64_t) ctx->sm_count * 8) / 32 * 32));
 	const uint64_t ntiles = pg_div_up(in->n, rows);
-	if (in->width <= FL_MAX_WIDTH && pc.ow / uw <= FL_THREADS && ntiles < (1ull << 31) - 1) {
-		const size_t smem = (size_t) rows * in->width;
-#define PJ_LAUNCH(U) do { \
-		PG_CUDA(ctx, cudaFuncSetAttribute(k_project<U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)); \
-		k_project<U><<<(unsigned) ntiles, FL_THREADS, smem, s>>>((const char*) in->data, in->n, iw, rows, pc, (char*) out, \
+	if (pc.ow / uw <= FL_THREADS && ntiles < (1ull << 31) - 1) {
+		const size_t smem = staged ? (size_t) rows * in->width : 0;
+#define PJ_LAUNCH(U, ST) do { \
+		if (ST) PG_CUDA(ctx, cudaFuncSetAttribute(k_project<U, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)); \
+		k_project<U, ST><<<(unsigned) ntiles, FL_THREADS, smem, s>>>((const char*) in->data, in->n, iw, rows, pc, (char*) out, \
 				ctx->d_status); } while (0)
-		if (uw == 4) PJ_LAUNCH(uint4);
-		else if (uw == 2) PJ_LAUNCH(uint2);
-		else PJ_LAUNCH(uint32_t);
+#define PJ_LAUNCH_AS(U) do { if (staged) PJ_LAUNCH(U, true); else PJ_LAUNCH(U, false); } while (0)
+		if (uw == 4) PJ_LAUNCH_AS(uint4);
+		else if (uw == 2) PJ_LAUNCH_AS(uint2);
+		else PJ_LAUNCH_AS(uint32_t);
+#undef PJ_LAUNCH_AS
 #undef PJ_LAUNCH
 	} else {
 		const int grid = (int) std::min<uint64_t>(pg_div_up(in->n, 256), (uint64_t) ctx->sm_count * 16);

@@ -438,3 +438,37 @@ def test_sort_of_other_widths(ctx, n, width, bits):
     keys[0], keys[1] = -(1 << bits >> 1), (1 << bits) - 1 - (1 << bits >> 1)
     rows[:, : kb // 4] = keys.astype(np.int64 if kb == 8 else np.int32).view(np.int32).reshape(n, -1)
     assert np.array_equal(ctx.sort(rows, (0, kb)), rows[np.argsort(keys, kind="stable")])
+
+
+# Tuples over 240 bytes are filtered, and projections of at most a quarter of tuples over
+# 128 bytes made, without staging: tiles of 512 rows. Either side of the widths, of the
+# quarter and of a tile, rows of more units than a block has threads, bases that are and
+# are not aligned to the copies' units.
+@pytest.mark.parametrize("width", [132, 240, 244, 256, 400, 1000, 1024, 1028, 3000])
+@pytest.mark.parametrize("shift", [(0, 0), (4, 0), (0, 8), (8, 8)])
+def test_filter_and_project_of_wide_tuples(ctx, width, shift):
+    L, (si, so) = gpu.lib(), shift
+    quarter = width // 16 * 4
+    for n in (1, 511, 512, 513, 5000):
+        rows = _rows(n, width, width + n)
+        src, dst = ctx.alloc(rows.nbytes + 64), ctx.alloc(rows.nbytes + 64)
+        ctx._check(L.pg_h2d(ctx.h, ctx.stream, src.ptr + si, rows.ctypes.data, rows.nbytes))
+        r = gpu.Rel(src.ptr + si, n, width, 0, 0)
+        for limit in (0, 20, 500, 1000):
+            pr, npr = gpu.preds([("int", "<", 0, limit)])
+            m = ctypes.c_uint64()
+            ctx._check(L.pg_memset(ctx.h, ctx.stream, dst.ptr, 0xA5, rows.nbytes + 64))
+            ctx._check(L.pg_filter(ctx.h, ctx.stream, ctypes.byref(r), pr, npr, dst.ptr + so, ctypes.byref(m)))
+            want = rows[rows[:, 0] < limit]
+            got = ctx.download(dst, rows.nbytes + 64)
+            assert m.value == len(want) and np.array_equal(got[so:so + want.nbytes], want.reshape(-1).view(np.uint8))
+            assert (got[:so] == 0xA5).all() and (got[so + want.nbytes:] == 0xA5).all()
+        for cols in ([(0, 4)], [(width - 8, 8)], [(4, quarter)], [(4, quarter - 4), (width - 8, 8)], [(0, min(width, 1016))] * 2):
+            ow = sum(b for _, b in cols)
+            if ow > width:
+                cols, ow = cols[:1], cols[0][1]
+            c = (gpu.Col * len(cols))(*[gpu.Col(0, o, b) for o, b in cols])
+            ctx._check(L.pg_project(ctx.h, ctx.stream, ctypes.byref(r), c, len(cols), dst.ptr + so))
+            want = np.concatenate([rows[:, o // 4:(o + b) // 4] for o, b in cols], axis=1)
+            got = ctx.download(dst, rows.nbytes + 64)
+            assert np.array_equal(got[so:so + want.nbytes], np.ascontiguousarray(want).reshape(-1).view(np.uint8))
