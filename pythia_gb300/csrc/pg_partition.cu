@@ -8,7 +8,7 @@
 // exactly what the reference produces when its threads read consecutive
 // slices.
 //
-// 16-byte tuples and at most 256 buckets: k_chunk_hist counts tuples per (bucket,
+// 16-byte tuples and at most 256 buckets (sw_wins): k_chunk_hist counts tuples per (bucket,
 // block), an exclusive scan over the bucket-major counts gives every block its first
 // output slot per bucket, and k_part_sweep streams the block's tiles again, ranks
 // their tuples and stores each bucket's rows of a tile as one run.
@@ -343,6 +343,7 @@ __device__ __forceinline__ uint32_t sw_bucket(const pg_hashfn& f, int64_t v, uin
 				f.skipbits & 31) & (uint32_t) f.k;
 	}
 	if (FN == PG_FN_MIXRADIX) return (uint32_t) (pg_mix64((uint64_t) v) >> f.skipbits);
+	if (FN == PG_FN_KNUTH) return (uint32_t) ((((uint64_t) v * 2654435761ull) & (uint64_t) f.k) >> f.skipbits);
 	return pg_hash_value(f, v, kbytes);
 }
 
@@ -530,11 +531,27 @@ k_part_sweep(const uint4* __restrict__ in, uint32_t n, uint32_t kw, uint32_t kby
 	}
 }
 
-// Whether k_part_sweep takes a partition of `in` into `out`.
+// Whether k_part_sweep can take a partition of `in` into `out`.
 static bool sw_takes(const pg_rel* in, const void* out, uint32_t buckets)
 {
 	return in->width == 16 && (in->key_off & 3) == 0 && buckets <= SW_BUCKETS &&
 		!((reinterpret_cast<uintptr_t>(in->data) | reinterpret_cast<uintptr_t>(out)) & 15);
+}
+
+// Whether it is the faster one, for the functions and fan-outs where k_part_scatter's
+// smaller tiles, more blocks and fewer ballots can win. Scatter against sweep: one bucket
+// 64M tuples 438 and 620 us, 3M 63 and 81; two buckets 3M 68 and 77, 500,000 46 and 52, 8M 131
+// and 115, 64M 662 and 545. Functions that both compute twice a tuple and that cost more than
+// the ranking: exactrange into 3 buckets 1094 and 1151 us (64M), 92 and 114 (3M), into 200
+// 1268 and 1214, 111 and 116; bytes into 64 1481 and 1508, 122 and 138, but 500,000 tuples 72
+// and 64.
+static bool sw_wins(const pg_hashfn& f, uint64_t n)
+{
+	switch (f.fn) {
+	case PG_FN_RANGE: case PG_FN_EXACTRANGE: return f.nbuckets > 4;
+	case PG_FN_BYTES: return f.nbuckets > 4 && n < 2500000;
+	default: return f.nbuckets > 2 || (f.nbuckets == 2 && n >= 4000000);
+	}
 }
 
 // `check` (pg_radix_pass): the key window is confirmed before the rows move;
@@ -594,6 +611,7 @@ static int sw_partition(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, pg_hashfn
 		f.k = f.nbuckets - 1;
 		return sw_partition_digit(ctx, s, in, f, lg, out, offsets, nullptr);
 	}
+	if (f.fn == PG_FN_KNUTH) return sw_partition_as<PG_FN_KNUTH, false>(ctx, s, in, f, out, offsets, nullptr);
 	if (f.fn == PG_FN_MIXRADIX) return sw_partition_as<PG_FN_MIXRADIX, false>(ctx, s, in, f, out, offsets, nullptr);
 	return sw_partition_as<PART_FN_ANY, false>(ctx, s, in, f, out, offsets, nullptr);
 }
@@ -637,7 +655,7 @@ int pg_partition_fn(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, const pg_hash
 		if (offsets) PG_CUDA(ctx, cudaMemsetAsync(offsets, 0, (B + 1) * sizeof(uint64_t), s));
 		return PG_OK;
 	}
-	if (sw_takes(in, out, B)) return sw_partition(ctx, s, in, f, out, offsets);
+	if (sw_takes(in, out, B) && sw_wins(f, n)) return sw_partition(ctx, s, in, f, out, offsets);
 	const int NW = B <= 1024 ? 8 : 4;
 	const int64_t tb = ctx->tune[PG_TUNE_PARTITION_TILE];
 	uint32_t tile = (uint32_t) (tb > 0 ? std::min<int64_t>(65536, std::max<int64_t>(8192, tb)) : PART_TILE_BYTES) / W;

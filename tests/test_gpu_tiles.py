@@ -472,3 +472,18 @@ def test_filter_and_project_of_wide_tuples(ctx, width, shift):
             want = np.concatenate([rows[:, o // 4:(o + b) // 4] for o, b in cols], axis=1)
             got = ctx.download(dst, rows.nbytes + 64)
             assert np.array_equal(got[so:so + want.nbytes], np.ascontiguousarray(want).reshape(-1).view(np.uint8))
+
+
+# Either side of the lines between the two partitions of 16-byte tuples: few buckets,
+# functions that cost more than the ranking.
+@pytest.mark.parametrize("fn,kw,n", [("parammodulo", dict(buckets=1), 10_001), ("parammodulo", dict(buckets=2), 3_999_999),
+                                     ("parammodulo", dict(buckets=2), 4_000_000), ("modulo", dict(buckets=4), 10_001),
+                                     ("exactrange", dict(buckets=4, min=0, max=(1 << 40) - 1), 10_001),
+                                     ("exactrange", dict(buckets=5, min=0, max=(1 << 40) - 1), 10_001),
+                                     ("bytes", dict(buckets=4), 10_001), ("bytes", dict(buckets=8), 2_499_999),
+                                     ("bytes", dict(buckets=8), 2_500_000), ("knuth", dict(buckets=256, skipbits=3), 10_001)])
+def test_partition_rules(ctx, fn, kw, n):
+    rows = dg.uniform_keys(n, 1 << 40, dg.seed_for(213))
+    got, offs = ctx.partition(rows, gpu.hashcfg(fn, **kw))
+    want, woffs = orc.partition(rows, orc.hashcfg(fn, **kw))
+    assert np.array_equal(offs, woffs) and np.array_equal(got, want)
