@@ -151,8 +151,7 @@ int pg_check_status(pg_ctx* ctx, cudaStream_t s, const char* what)
 
 __global__ void k_collect(unsigned long long* __restrict__ dst, const int* __restrict__ status, const int* __restrict__ flag)
 {
-	dst[0] = flag ? (unsigned long long) (unsigned) *flag : 0;
-	dst[1] = (unsigned long long) (unsigned) *status;
+	pg_collect(dst, flag, status);
 }
 
 int pg_readback(pg_ctx* ctx, cudaStream_t s, unsigned long long* dev, int n, const int* flag, unsigned long long* host,
@@ -160,6 +159,12 @@ int pg_readback(pg_ctx* ctx, cudaStream_t s, unsigned long long* dev, int n, con
 {
 	k_collect<<<1, 1, 0, s>>>(dev + n, ctx->d_status, flag);
 	PG_LAUNCHED(ctx);
+	return pg_readback_collected(ctx, s, dev, n, host, what);
+}
+
+int pg_readback_collected(pg_ctx* ctx, cudaStream_t s, const unsigned long long* dev, int n, unsigned long long* host,
+		const char* what)
+{
 	unsigned long long h[16];
 	PG_CUDA(ctx, cudaMemcpyAsync(h, dev, (n + 2) * 8, cudaMemcpyDeviceToHost, s));
 	PG_CUDA(ctx, cudaStreamSynchronize(s));

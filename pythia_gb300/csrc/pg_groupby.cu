@@ -196,8 +196,9 @@ __device__ __forceinline__ void gb_write_agg(char* o, uint32_t kbytes, int64_t k
 
 template <int VT, int AGG, bool HASKEY>
 __global__ void k_gb_emit(GbTable t, uint32_t kbytes, char* __restrict__ out, uint64_t cap_rows,
-		unsigned long long* __restrict__ cursor, uint64_t nonkey_rows, PgFx fx)
+		unsigned long long* __restrict__ cursor, uint64_t nonkey_rows, PgFx fx, const int* __restrict__ status)
 {
+	if (blockIdx.x == 0 && threadIdx.x == 0) pg_collect(cursor + 1, GB_DEC ? fx.p + 2 : nullptr, status);
 	const int fx_s = GB_DEC ? fx.p[0] : 0;
 	const uint64_t cap = 1ull << t.log2cap;
 	const uint32_t aw = (AGG == PG_AGG_SUM && VT == PG_VAL_INT) ? 4 : 8;
@@ -518,8 +519,10 @@ k_gb_dense_smem(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t ko
 template <int VT, int AGG>
 __global__ void k_gb_dense_emit(const unsigned long long* __restrict__ acc, PgFx fx,
 		const unsigned char* __restrict__ present, uint64_t range, long long kmin, uint32_t kbytes,
-		char* __restrict__ out, uint64_t cap_rows, unsigned long long* __restrict__ cursor)
+		char* __restrict__ out, uint64_t cap_rows, unsigned long long* __restrict__ cursor, unsigned long long* __restrict__ tail,
+		const int* __restrict__ status)
 {
+	if (blockIdx.x == 0 && threadIdx.x == 0) pg_collect(tail, GB_DEC ? fx.p + 2 : nullptr, status);
 	const int fx_s = GB_DEC ? fx.p[0] : 0;
 	const uint32_t aw = (AGG == PG_AGG_SUM && VT == PG_VAL_INT) ? 4 : 8;
 	const uint32_t ow = kbytes + aw;
@@ -733,10 +736,10 @@ static int gb_dense_window(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint32
 	}
 	const int eblocks = (int) std::min<uint64_t>(pg_div_up(range, 256), (uint64_t) ctx->sm_count * 8);
 	k_gb_dense_emit<VT, AGG><<<eblocks, 256, 0, s>>>(acc, fx, present, range, kmin, in->key_bytes, (char*) out,
-			out_cap, cursor);
+			out_cap, cursor, cursor + 2, ctx->d_status);
 	PG_LAUNCHED(ctx);
 	unsigned long long h[3];
-	rc = pg_readback(ctx, s, cursor, 2, GB_DEC ? fx.p + 2 : nullptr, h, "pg_groupby");
+	rc = pg_readback_collected(ctx, s, cursor, 2, h, "pg_groupby");
 	pg_free_async(ctx, s, mem);
 	*ngroups = h[0];
 	*overflow = h[1] != 0;
@@ -861,11 +864,11 @@ static int gb_run(pg_ctx* ctx, cudaStream_t s, const pg_rel* in, uint32_t voff, 
 		// The groups are written out before the table is known to have held them
 		// all; one that was full is enlarged and filled again.
 		int eblocks = (int) std::min<uint64_t>(pg_div_up(cap + 1, 256), (uint64_t) ctx->sm_count * 8);
-		if (haskey) k_gb_emit<VT, AGG, true><<<eblocks, 256, 0, s>>>(t, in->key_bytes, (char*) out, out_cap, cursor, 0, fx);
-		else k_gb_emit<VT, AGG, false><<<1, 32, 0, s>>>(t, 0, (char*) out, out_cap, cursor, in->n, fx);
+		if (haskey) k_gb_emit<VT, AGG, true><<<eblocks, 256, 0, s>>>(t, in->key_bytes, (char*) out, out_cap, cursor, 0, fx, ctx->d_status);
+		else k_gb_emit<VT, AGG, false><<<1, 32, 0, s>>>(t, 0, (char*) out, out_cap, cursor, in->n, fx, ctx->d_status);
 		PG_LAUNCHED(ctx);
 		unsigned long long h[2];
-		rc = pg_readback(ctx, s, cursor, 1, GB_DEC ? fx.p + 2 : nullptr, h, "pg_groupby");
+		rc = pg_readback_collected(ctx, s, cursor, 1, h, "pg_groupby");
 		pg_free_async(ctx, s, mem);
 		if (rc == PG_ERR_TABLE_FULL) { groups *= 4; continue; }
 		if (rc) return rc;
@@ -938,13 +941,13 @@ int pg_dense_groups_emit(pg_ctx* ctx, cudaStream_t s, const unsigned long long* 
 {
 	const int eblocks = (int) std::min<uint64_t>(pg_div_up(range, 256), (uint64_t) ctx->sm_count * 8);
 	if (agg == PG_AGG_COUNT)
-		k_gb_dense_emit<PG_VAL_LONG, PG_AGG_COUNT><<<eblocks, 256, 0, s>>>(acc, fx, present, range, kmin, kbytes, (char*) out, out_cap, cursor);
+		k_gb_dense_emit<PG_VAL_LONG, PG_AGG_COUNT><<<eblocks, 256, 0, s>>>(acc, fx, present, range, kmin, kbytes, (char*) out, out_cap, cursor, cursor + 1, ctx->d_status);
 	else if (val_type == PG_VAL_INT)
-		k_gb_dense_emit<PG_VAL_INT, PG_AGG_SUM><<<eblocks, 256, 0, s>>>(acc, fx, present, range, kmin, kbytes, (char*) out, out_cap, cursor);
+		k_gb_dense_emit<PG_VAL_INT, PG_AGG_SUM><<<eblocks, 256, 0, s>>>(acc, fx, present, range, kmin, kbytes, (char*) out, out_cap, cursor, cursor + 1, ctx->d_status);
 	else if (val_type == PG_VAL_LONG)
-		k_gb_dense_emit<PG_VAL_LONG, PG_AGG_SUM><<<eblocks, 256, 0, s>>>(acc, fx, present, range, kmin, kbytes, (char*) out, out_cap, cursor);
+		k_gb_dense_emit<PG_VAL_LONG, PG_AGG_SUM><<<eblocks, 256, 0, s>>>(acc, fx, present, range, kmin, kbytes, (char*) out, out_cap, cursor, cursor + 1, ctx->d_status);
 	else
-		k_gb_dense_emit<PG_VAL_DEC, PG_AGG_SUM><<<eblocks, 256, 0, s>>>(acc, fx, present, range, kmin, kbytes, (char*) out, out_cap, cursor);
+		k_gb_dense_emit<PG_VAL_DEC, PG_AGG_SUM><<<eblocks, 256, 0, s>>>(acc, fx, present, range, kmin, kbytes, (char*) out, out_cap, cursor, cursor + 1, ctx->d_status);
 	PG_LAUNCHED(ctx);
 	return PG_OK;
 }

@@ -3520,7 +3520,7 @@ extern "C" int pg_hashjoin_groupby(pg_ctx* ctx, pg_stream stream, pg_hashtable* 
 		if ((rc = pg_dense_groups_emit(ctx, s, acc, fx, present, vrange, (long long) ht->vlo, gbytes, val_type, agg,
 				out, out_capacity, cursor))) return rc;
 		unsigned long long h[2];
-		if ((rc = pg_readback(ctx, s, cursor, 1, dec ? fx.p + 2 : nullptr, h, "pg_hashjoin_groupby"))) {
+		if ((rc = pg_readback_collected(ctx, s, cursor, 1, h, "pg_hashjoin_groupby"))) {
 			pg_free_async(ctx, s, mem);
 			return rc;
 		}

@@ -460,8 +460,9 @@ template <bool V16>
 __global__ void __launch_bounds__(256)
 k_mj_lookup(const char* __restrict__ in, uint64_t n, uint32_t W, uint32_t koff, uint32_t kbytes, uint32_t soff,
 		uint32_t swords, long long kmin, uint32_t range, const uint32_t* __restrict__ cnt,
-		unsigned long long* __restrict__ agg)
+		unsigned long long* __restrict__ agg, const int* __restrict__ status)
 {
+	if (blockIdx.x == 0 && threadIdx.x == 0) pg_collect(agg + 3, nullptr, status);
 	__shared__ unsigned long long red[2][8];
 	const uint64_t stride = (uint64_t) gridDim.x * blockDim.x, pol = pg_policy_evict_first();
 	const uint64_t keep = pg_policy_keep(4);
@@ -634,8 +635,9 @@ k_mj_rows(const char* __restrict__ S, uint64_t n, uint32_t koff, long long kmin,
 		const uint32_t* __restrict__ ends, const unsigned long long* __restrict__ val, uint32_t wsel,
 		uint4* __restrict__ out, uint64_t cap, unsigned long long* __restrict__ cursor, const unsigned int* __restrict__ meta,
 		const unsigned long long* __restrict__ vmm, unsigned long long* __restrict__ list, uint64_t list_cap,
-		unsigned long long* __restrict__ listed)
+		unsigned long long* __restrict__ listed, const int* __restrict__ status)
 {
+	if (!SLICE && blockIdx.x == 0 && threadIdx.x == 0) pg_collect(cursor + 3, nullptr, status);
 	if (meta[0] > MJ_MAX_RUN || meta[1]) return;
 	const unsigned long long vmin = ~vmm[0];
 	const uint32_t bytes = mj_val_bytes(vmm[1] - vmin);
@@ -942,9 +944,9 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 		if (!materialize) {
 			const uint32_t soff = sum_col >= 0 ? pc.off[sum_col] : 0, swords = sum_col >= 0 ? pc.words[sum_col] : 0;
 			if (mj_v16(P)) k_mj_lookup<true><<<pblocks, 256, 0, s>>>((const char*) P->data, P->n, 16, P->key_off, 8, soff,
-					swords, kmin, range, cnt, agg);
+					swords, kmin, range, cnt, agg, ctx->d_status);
 			else k_mj_lookup<false><<<pblocks, 256, 0, s>>>((const char*) P->data, P->n, P->width, P->key_off, P->key_bytes,
-					soff, swords, kmin, range, cnt, agg);
+					soff, swords, kmin, range, cnt, agg, ctx->d_status);
 			PG_LAUNCHED(ctx);
 		} else {
 			k_mj_scan_sums<<<(unsigned) nb, 256, 0, s>>>(cnt, range, sums, meta);
@@ -960,7 +962,7 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 			k_mj_fill<<<fblocks, 256, 0, s>>>(cdata, C->n, C->key_off, kmin, range, bp, cnt, val, meta, vmm);
 			PG_LAUNCHED(ctx);
 #define MJ_ROWS(T, SLICE, blocks) do { k_mj_rows<T, SLICE><<<blocks, 256, 0, s>>>(pdata, P->n, P->key_off, kmin, range, cnt, \
-				val, wsel, reinterpret_cast<uint4*>(out), out_capacity, agg, meta, vmm, list, slices, mm + 9); \
+				val, wsel, reinterpret_cast<uint4*>(out), out_capacity, agg, meta, vmm, list, slices, mm + 9, ctx->d_status); \
 				PG_LAUNCHED(ctx); } while (0)
 			const bool two = !parted && C->n / 2 >= range;
 			if (two) MJ_ROWS(2, false, grid(P->n, 256 * 2, MJ_ROWS_BLOCKS_PER_SM));
@@ -971,7 +973,7 @@ static int mj_dense_join(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, const pg_
 #undef MJ_ROWS
 		}
 		unsigned long long o[4];     // rows, sum, (largest count, key outside)
-		rc = pg_readback(ctx, s, agg, 3, nullptr, o, "pg_mpsm_join");
+		rc = pg_readback_collected(ctx, s, agg, 3, o, "pg_mpsm_join");
 		if (rc) return rc;
 		if (o[2] >> 32) continue;                                         // the sample missed a key
 		if (materialize && (uint32_t) o[2] > MJ_MAX_RUN) break;
