@@ -3452,8 +3452,13 @@ static int hj_groupby_launch(pg_ctx* ctx, cudaStream_t s, const pg_rel* S, const
 {
 	const GbsPlan plan = gbs_plan<VT, AGG>(vrange);
 	auto* const shared = plan.lazy ? k_probe16_groupby_smem<VT, AGG, GB_DEC> : k_probe16_groupby_smem<VT, AGG, false>;
-	int blocks = 0, rc;
-	if ((rc = gbs_blocks(ctx, shared, plan, vrange, S->n, &blocks))) return rc;
+	int blocks = 0, rc, priority = 0;
+	// A stream of raised priority has its call run beside others: blocks of 1024 threads
+	// and up to all of an SM's shared memory wait until that much of an SM is free at once,
+	// where the small blocks below start as the others' end (queries of a few hundred
+	// microseconds beside long ones, serving at 360 queries/s: median 1.15 ms, 0.95 so).
+	PG_CUDA(ctx, cudaStreamGetPriority(s, &priority));
+	if (priority >= 0 && (rc = gbs_blocks(ctx, shared, plan, vrange, S->n, &blocks))) return rc;
 	if (blocks) {
 		shared<<<blocks, GBS_THREADS, plan.bytes, s>>>((const char*) S->data, S->n, S->key_off, tb, voff, goff,
 				(uint32_t) vrange, acc, fx, present);
