@@ -32,7 +32,7 @@
 // values, and values far below the largest add fire-and-forget chunks.
 // Tables in shared memory, where returning adds are cheap, keep less: the dense
 // group-by t2 and its overflows, the hashed one's caches a four-word chained form
-// (pg_fx_chain_add).
+// (pg_fx_chain_add_halves).
 //
 // Host and device: the host test checks quantisation, both table forms' adds
 // and the rounding against exact rational arithmetic.
@@ -224,7 +224,8 @@ PG_FX_HD bool pg_fx_table_add(uint64_t* t, uint64_t stride, const pg_fx4& a, ADD
 // A compact four-word form for tables in shared memory, where returning
 // adds are cheap: t[0], t[1] unsigned, t[2] signed, t[3] its overflows, the
 // sum being t3 2^192 + t2 2^128 + t1 2^64 + t0. Each add returns the old word,
-// whose overflow is the carry into the next word.
+// whose overflow is the carry into the next word. (By whole words; the kernels add by
+// halves, below, and the host test checks both.)
 template <class ADD>
 PG_FX_HD void pg_fx_chain_add(uint64_t* t, uint64_t stride, const pg_fx4& a, ADD add)
 {
@@ -244,6 +245,42 @@ PG_FX_HD void pg_fx_chain_add(uint64_t* t, uint64_t stride, const pg_fx4& a, ADD
 	const int64_t r = (int64_t) l;
 	if (r) q += pg_fx_overflow(add(t + 2 * stride, (uint64_t) r), r);
 	if (q) add(t + 3 * stride, q);
+}
+
+// The form that the kernels use: the same words by their 32-bit halves, q[0] the
+// lower, since a shared 64-bit add is a compare-and-swap loop and a 32-bit one an
+// instruction; ADD(p, v) adds 32 bits and returns the old ones. A carry or overflow goes on
+// with the add that made it, so the words are right once every add is in. Returns the
+// carry out of the 64 bits.
+template <class ADD>
+PG_FX_HD uint32_t pg_fx_add_halves(uint32_t* q, uint64_t v, ADD add)
+{
+	const uint32_t lo = (uint32_t) v, old = add(q, lo);
+	const uint64_t hi = (v >> 32) + ((uint32_t) (old + lo) < lo);          // up to 2^32
+	if ((uint32_t) hi == 0) return (uint32_t) (hi >> 32);
+	const uint32_t oh = add(q + 1, (uint32_t) hi);
+	return (uint32_t) (oh + (uint32_t) hi) < oh;
+}
+
+// Adds a value's count a (its upper word within +-2^60) to the chained table whose word
+// k's halves are q[2 k stride] and q[2 k stride + 1].
+template <class ADD>
+PG_FX_HD void pg_fx_chain_add_halves(uint32_t* q, uint64_t stride, const pg_fx3& a, ADD add)
+{
+	uint64_t c = 0;
+	if (a.w0) c = pg_fx_add_halves(q, a.w0, add);
+	const uint64_t x1 = a.w1 + c;
+	c = x1 < c;
+	if (x1) c += pg_fx_add_halves(q + 2 * stride, x1, add);
+	const uint64_t l = a.w2 + c;                       // within +-2^61
+	if (!l) return;
+	uint32_t* const t2 = q + 4 * stride;
+	const uint32_t lo = (uint32_t) l, old = add(t2, lo);
+	const uint32_t hi = (uint32_t) (l >> 32) + ((uint32_t) (old + lo) < lo);
+	if (!hi) return;
+	const uint32_t oh = add(t2 + 1, hi);
+	const int32_t was = (int32_t) oh, is = (int32_t) (oh + hi);
+	if ((int32_t) hi > 0 ? is < was : is > was) pg_fx_add_halves(q + 6 * stride, (int32_t) hi > 0 ? 1ull : ~0ull, add);
 }
 
 // The count held by a four-word chained table t[k * stride].

@@ -54,40 +54,12 @@ __device__ __forceinline__ void fold_slot(unsigned long long* acc, uint64_t wstr
 	else pg_fx_atomic_add(&acc[slot], wstride, v.f);
 }
 
-// The same with the carry out of the 64 bits.
-__device__ __forceinline__ uint64_t gb_shared_add64_carry(unsigned long long* p, unsigned long long v)
-{
-	unsigned int* const q = reinterpret_cast<unsigned int*>(p);
-	const unsigned int lo = (unsigned int) v, old = atomicAdd(q, lo);
-	const unsigned long long hi = (v >> 32) + (old + lo < lo);          // up to 2^32
-	if ((unsigned int) hi == 0) return hi >> 32;
-	const unsigned int oh = atomicAdd(q + 1, (unsigned int) hi);
-	return oh + (unsigned int) hi < oh;
-}
-
-// Adds count a into four chained words t[k * stride] in shared memory, as
-// pg_fx_chain_add does one add at a time: a carry or overflow goes on with the add
-// that made it. A value near the column's largest is two 32-bit adds on t2, where 64-bit
-// ones were compare-and-swap loops: 20M rows hashed into 10 groups 403 -> 208 us, into
-// 300 408 -> 387, into 100,000 536 -> 514.
+// Adds count a into four chained words t[k * stride] in shared memory. A value near the
+// column's largest is two 32-bit adds on t2, where 64-bit ones were compare-and-swap loops:
+// 20M rows hashed into 10 groups 403 -> 208 us, into 300 408 -> 387, into 100,000 536 -> 514.
 __device__ __forceinline__ void gb_shared_chain_add(unsigned long long* t, uint32_t stride, const pg_fx3& a)
 {
-	uint64_t c = 0;
-	if (a.w0) c = gb_shared_add64_carry(t, a.w0);
-	const uint64_t x1 = a.w1 + c;
-	c = x1 < c;
-	if (x1) c += gb_shared_add64_carry(t + stride, x1);
-	const uint64_t l = a.w2 + c;                       // within +-2^61
-	if (l) {
-		unsigned int* const q = reinterpret_cast<unsigned int*>(t + 2 * stride);
-		const unsigned int lo = (unsigned int) l, old = atomicAdd(q, lo);
-		const unsigned int hi = (unsigned int) (l >> 32) + (old + lo < lo);
-		if (hi) {
-			const unsigned int oh = atomicAdd(q + 1, hi);
-			const int32_t was = (int32_t) oh, is = (int32_t) (oh + hi);
-			if ((int32_t) hi > 0 ? is < was : is > was) gb_shared_add64(t + 3 * stride, (int32_t) hi > 0 ? 1ull : ~0ull);
-		}
-	}
+	pg_fx_chain_add_halves(reinterpret_cast<uint32_t*>(t), stride, a, [](uint32_t* p, uint32_t v) { return atomicAdd(p, v); });
 }
 
 // A dec sum's count from table words acc[slot + k * wstride].

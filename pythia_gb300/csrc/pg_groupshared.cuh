@@ -18,16 +18,11 @@
 #define GBS_MAX_BYTES (224 * 1024)
 #define GBS_LAZY_BYTES (8 * PG_FX_LAZY)
 
-// v added to a 64-bit word in shared memory by its 32-bit halves: a shared
-// 64-bit add is a compare-and-swap loop, a 32-bit one a single instruction, and
-// the upper half needs one only for a carry or a large value. The word is right
-// once every add is in.
+// v added to a 64-bit word in shared memory by its 32-bit halves: the upper half needs
+// an add only for a carry or a large value.
 __device__ __forceinline__ void gb_shared_add64(unsigned long long* p, unsigned long long v)
 {
-	unsigned int* const q = reinterpret_cast<unsigned int*>(p);
-	const unsigned int lo = (unsigned int) v, old = atomicAdd(q, lo);
-	const unsigned int hi = (unsigned int) (v >> 32) + (old + lo < lo);
-	if (hi) atomicAdd(q + 1, hi);
+	pg_fx_add_halves(reinterpret_cast<uint32_t*>(p), v, [](uint32_t* q, uint32_t x) { return atomicAdd(q, x); });
 }
 
 template <int VT, int AGG>
