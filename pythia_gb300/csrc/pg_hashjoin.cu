@@ -427,6 +427,28 @@ struct HjSmallShared {
 	unsigned int bar;
 };
 
+// The blocks of k_build_small meet (`epoch`: how often they have, with this time), and
+// *seen is what they gathered. A barrier that a block gave up on (`dead`) is no error: the
+// build returns before the kernel has run, and a status would fail whichever call reads it
+// next. The header sends the table to the exact build. Thread 0 looks at what was gathered
+// for its whole block: past a lost barrier it still changes, and the block's threads must
+// go the same way. Not inlined: the kernel meets up to seven times, and a small build is
+// over before the code of seven copies has arrived.
+__device__ __noinline__ bool hj_small_meet(HjSmallShared* g, HjSmallShared* acc, HjSmallShared* seen, uint32_t epoch,
+		bool dead, uint32_t spin)
+{
+	uint32_t before = epoch - 1;
+	pg_grid_sync(&g->bar, before, dead, spin, nullptr);
+	if (threadIdx.x == 0) {
+		if (dead) atomicOr(&acc->lost, 1u);         // before this block's next arrival
+		const volatile HjSmallShared* const v = acc;
+		seen->nkmin = v->nkmin; seen->kmax = v->kmax; seen->nvmin = v->nvmin; seen->vmax = v->vmax;
+		seen->present = v->present; seen->marker = v->marker; seen->dup = v->dup;
+	}
+	__syncthreads();
+	return dead;
+}
+
 __global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict__ R, uint32_t n, uint32_t kw,
 		uint32_t pk, uint64_t cap, uint32_t* __restrict__ table, unsigned long long* __restrict__ slots, uint32_t log2cap,
 		HjDenseHdr* __restrict__ hdr, HjSmallShared* g, const int* __restrict__ status)
@@ -441,20 +463,7 @@ __global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict
 	bool dead = false;
 	HjSmallShared* const acc = alone ? &mine : g;
 	if (alone && tid == 0) mine = HjSmallShared{0, 0, 0, 0, 0, 0, 0, 0, 0};
-	// A barrier that a block gave up on is no error: the build returns before the kernel
-	// has run, and a status would fail whichever call reads it next. The header sends the
-	// table to the exact build. Thread 0 looks at what was gathered for its whole block:
-	// past a lost barrier it still changes, and the block's threads must go the same way.
-	auto meet = [&]() {
-		pg_grid_sync(&g->bar, epoch, dead, spin, nullptr);
-		if (tid == 0) {
-			if (dead) atomicOr(&acc->lost, 1u);         // before this block's next arrival
-			const volatile HjSmallShared* const v = acc;
-			seen.nkmin = v->nkmin; seen.kmax = v->kmax; seen.nvmin = v->nvmin; seen.vmax = v->vmax;
-			seen.present = v->present; seen.marker = v->marker; seen.dup = v->dup; seen.lost = v->lost;
-		}
-		__syncthreads();
-	};
+	auto meet = [&]() { dead = hj_small_meet(g, acc, &seen, ++epoch, dead, spin); };
 	auto key_of = [&](const uint4& v) { return ((unsigned long long) hj_word4(v, kw + 1) << 32) | hj_word4(v, kw); };
 	unsigned long long lo = ~0ull, hi = 0, vlo = ~0ull, vhi = 0;
 	int marker = 0;
@@ -2391,11 +2400,13 @@ static int hj_build_spec(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, pg_hashta
 	};
 	// Where the spare slots do not fit in memory the sampled form does without.
 	bool small = R->n <= HJ_SMALL_TUPLES && ctx->tune[PG_TUNE_BUILD_SPEC] != 1;
-	if (small && pg_alloc_async(ctx, s, (void**) &ht->small_slots, 16ull << hj_log2cap(R->n)) != PG_OK) {
+	unsigned long long* spare = nullptr;
+	if (small && pg_alloc_async(ctx, s, (void**) &spare, 16ull << hj_log2cap(R->n)) != PG_OK) {
 		cudaGetLastError();
-		ht->small_slots = nullptr;
+		spare = nullptr;
 		small = false;
 	}
+	ht->small_slots.store(spare);
 	if (small) {
 		ht->log2cap = hj_log2cap(R->n);
 		uint32_t G = (uint32_t) std::min<uint64_t>(pg_div_up(R->n, HJ_SMALL_PER_BLOCK), ctx->sm_count);
@@ -2404,7 +2415,7 @@ static int hj_build_spec(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, pg_hashta
 		const uint4* rd = (const uint4*) R->data;
 		uint32_t n = (uint32_t) R->n, kww = kw, pkk = pk, lg = ht->log2cap;
 		uint64_t capp = cap;
-		void* args[] = {&rd, &n, &kww, &pkk, &capp, &ht->dense32_base, &ht->small_slots, &lg, &ht->hdr, &g, &ctx->d_status};
+		void* args[] = {&rd, &n, &kww, &pkk, &capp, &ht->dense32_base, &spare, &lg, &ht->hdr, &g, &ctx->d_status};
 		PG_CUDA(ctx, cudaLaunchCooperativeKernel((void*) k_build_small, dim3(G), dim3(1024), args, 0, s));
 		PG_LAUNCHED(ctx);
 		return built();
@@ -2446,18 +2457,26 @@ static void hj_settle_good(pg_hashtable* ht, const HjDenseHdr& h, uint32_t* win)
 	ht->spec.store(false, std::memory_order_release);
 }
 
-// After a probe on stream s read back a good header (the build is over then): the
-// table is settled at once where no copy is needed, which always holds for builds of
-// up to 2^20 tuples. Later probes then take it as it is, and the spare slots, 32 of a
-// 1M-tuple table's 41 MB, are given back.
-static void hj_settle_probed(pg_ctx* ctx, cudaStream_t s, pg_hashtable* ht, const HjDenseHdr& h)
+// After a probe read back a good header (the build is over then): the table is settled
+// at once where no copy is needed, which always holds for builds of up to 2^20 tuples.
+// Later probes then take it as it is.
+static void hj_settle_probed(pg_hashtable* ht, const HjDenseHdr& h)
 {
 	if (hj_hdr_rebase(h)) return;
 	std::lock_guard<std::mutex> g(ht->mu);
 	if (!ht->spec.load(std::memory_order_relaxed)) return;
-	pg_free_async(ctx, s, ht->small_slots);
-	ht->small_slots = nullptr;
 	hj_settle_good(ht, h, ht->dense32_base + (h.kmin ^ (1ull << 63)) - (unsigned long long) h.dmin);
+}
+
+// The spare slots of a settled table, which no probe reads (32 of a 1M-tuple table's 41
+// MB), given back by its second probe: a table that is probed once and freed does better
+// to free them then, since freeing it waits for what its stream still holds (2 us of the 41
+// of 1000 tuples joined with 10,000).
+static void hj_free_spare(pg_ctx* ctx, cudaStream_t s, pg_hashtable* ht)
+{
+	if (!ht->small_slots.load(std::memory_order_relaxed)) return;
+	std::lock_guard<std::mutex> g(ht->mu);
+	pg_free_async(ctx, s, ht->small_slots.exchange(nullptr));
 }
 
 // `refuted`: the header as a probe read it back when its checks failed (no second
@@ -2475,8 +2494,7 @@ static int hj_settle_known(pg_ctx* ctx, pg_hashtable* ht, const HjDenseHdr* refu
 		PG_CUDA(ctx, cudaStreamSynchronize(s));
 	}
 	if (!(h.flags & (16 | 64))) {       // spare slots that no probe will read
-		pg_free_async(ctx, s, ht->small_slots);
-		ht->small_slots = nullptr;
+		pg_free_async(ctx, s, ht->small_slots.exchange(nullptr));
 	}
 	if (hj_hdr_ok(h)) {
 		uint32_t* win = ht->dense32_base + (h.kmin ^ (1ull << 63)) - (unsigned long long) h.dmin;
@@ -2494,8 +2512,8 @@ static int hj_settle_known(pg_ctx* ctx, pg_hashtable* ht, const HjDenseHdr* refu
 		return PG_OK;
 	}
 	if (h.flags & 64) {          // the build kernel made the wide dense layout
-		ht->dense_val = ht->small_slots; ht->dense_bits = ht->dense32_base; ht->dense32 = nullptr;
-		ht->small_slots = nullptr; ht->dense32_base = nullptr;
+		ht->dense_val = ht->small_slots.exchange(nullptr); ht->dense_bits = ht->dense32_base; ht->dense32 = nullptr;
+		ht->dense32_base = nullptr;
 		ht->dmin = h.dmin; ht->drange = h.kmax - h.kmin + 1;
 		ht->vmin = h.vlo; ht->vlo = h.vlo; ht->vmax = h.vhi;
 		ht->log2cap = 1;
@@ -2513,8 +2531,7 @@ static int hj_settle_known(pg_ctx* ctx, pg_hashtable* ht, const HjDenseHdr* refu
 		ht->side_cap = HJ_SIDE_CAP0; ht->nside = 0;
 		ht->dense = false; ht->dense_val = nullptr; ht->dense_bits = nullptr; ht->vmin = 0;
 		ht->log2cap = hj_log2cap(ht->rel.n); ht->capacity = 1ull << ht->log2cap;
-		ht->slots = ht->small_slots;
-		ht->small_slots = nullptr;
+		ht->slots = ht->small_slots.exchange(nullptr);
 		ht->unique = (h.flags & 32) == 0;
 		ht->spec.store(false, std::memory_order_release);
 		return PG_OK;
@@ -2553,7 +2570,7 @@ extern "C" int pg_hashjoin_build(pg_ctx* ctx, pg_stream stream, const pg_rel* R,
 	ht->inline_val = bbytes <= 8;
 	ht->rel = *R;
 	ht->spec.store(false); ht->hdr = nullptr; ht->dense32_base = nullptr; ht->dense32_copy = nullptr;
-	ht->built = nullptr; ht->small_slots = nullptr;
+	ht->built = nullptr; ht->small_slots.store(nullptr);
 	const int64_t spec = ctx->tune[PG_TUNE_BUILD_SPEC];
 	if (R->n && ht->inline_val && ctx->tune[PG_TUNE_DENSE] != 2 && spec != 2 && hj_vec16(R, ht->bcols))
 		rc = hj_build_spec(ctx, s, R, ht);
@@ -2581,7 +2598,7 @@ extern "C" int pg_hashtable_free(pg_ctx* ctx, pg_hashtable* ht)
 		pg_free_async(ctx, ht->stream, ht->dense32);
 	}
 	pg_free_async(ctx, ht->stream, ht->hdr);
-	pg_free_async(ctx, ht->stream, ht->small_slots);
+	pg_free_async(ctx, ht->stream, ht->small_slots.load());
 	if (ht->built) cudaEventDestroy(ht->built);
 	delete ht;
 	return PG_OK;
@@ -2907,7 +2924,7 @@ static int hj_readback(pg_ctx* ctx, cudaStream_t s, unsigned long long* acc, pg_
 	PG_CUDA(ctx, cudaStreamSynchronize(s));
 	if (h.status) return pg_status_fail(ctx, s, (int) h.status, what);
 	*refuted = hdr && !hj_hdr_ok(h.hdr);
-	if (hdr && !*refuted) hj_settle_probed(ctx, s, ht, h.hdr);
+	if (hdr && !*refuted) hj_settle_probed(ht, h.hdr);
 	return PG_OK;
 }
 
@@ -2935,6 +2952,7 @@ static int hj_probe_run(pg_ctx* ctx, pg_stream stream, pg_hashtable* ht,
 	const pg_rel* S = &Sloc;
 	HjScratch part_buf(ctx, s);
 	const HjView view = hj_view(*ht);
+	if (!view.spec) hj_free_spare(ctx, s, ht);
 	if (const uint32_t lp = view.spec ? 0 : hj_probe_partition_bits(ctx, ht, S_in->n)) {
 		if ((rc = pg_alloc_async(ctx, s, &part_buf.p, S_in->n * S_in->width))) return rc;
 		pg_hashfn f;

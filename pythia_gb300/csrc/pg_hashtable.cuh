@@ -83,8 +83,8 @@ struct pg_hashtable {
 	HjDenseHdr* hdr;
 	uint32_t* dense32_base;
 	uint32_t* dense32_copy;
-	unsigned long long* small_slots;  // up to 2^20 tuples: slots the build kernel fills when no dense layout fits,
-	                                  // given back by the first use that finds one
+	std::atomic<unsigned long long*> small_slots;  // up to 2^20 tuples: slots the build kernel fills when no dense
+	                                               // layout fits, else given back by the second probe
 	cudaEvent_t built;          // recorded after the speculative build's kernels (null otherwise)
 	pg_rel rel;                 // the build relation, for an exact rebuild
 };

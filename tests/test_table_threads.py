@@ -103,7 +103,7 @@ def _pool_bytes():
 @pytest.mark.parametrize("n", [1, 3000, 1 << 20])
 def test_probed_dense_table_keeps_only_its_entries(ctx, n):
     # 2n + n/8 + 4096 entries of 4 bytes and the header; the build's spare hashed
-    # slots (up to 32 bytes a tuple twice over) are gone after the first probe.
+    # slots (up to 32 bytes a tuple twice over) are gone after the second probe.
     R = dg.build_relation(n, dg.seed_for(303))
     S = dg.probe_uniform(1000, R, dg.seed_for(304))
     dR, dS = ctx.upload(R), ctx.upload(S)
@@ -118,9 +118,9 @@ def test_probed_dense_table_keeps_only_its_entries(ctx, n):
             ctx._check(L.pg_hashjoin_probe(ctx.h, ctx.stream, ht, ctypes.byref(rS), c, nc, None, 0, gpu.JOIN_COUNT, -1,
                                            ctypes.byref(res)))
             assert res.n_out == 1000
-            ctx.sync()
-            kept = _pool_bytes() - before
-            assert kept <= 4 * (2 * n + n // 8 + 4096) + 4096, kept
+        ctx.sync()
+        kept = _pool_bytes() - before
+        assert kept <= 4 * (2 * n + n // 8 + 4096) + 4096, kept
     finally:
         L.pg_hashtable_free(ctx.h, ht)
 
