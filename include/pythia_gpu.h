@@ -81,9 +81,9 @@ typedef struct {
 enum { PG_JOIN_MATERIALIZE = 1, PG_JOIN_COUNT = 2, PG_JOIN_SUM = 4 };
 /* pg_mpsm_join only: that side is already sorted on its key, as a plan's
  * buildpresorted / probepresorted = "yes" states (SortMergeJoinOp::init,
- * operators/join.cpp:750-762). Where the join sorts, the device confirms it and
- * then skips that side's sort; a side that is not sorted is sorted as usual, so the
- * result never depends on the flags. */
+ * operators/join.cpp:750-762). Where the join sorts or partitions that side, the
+ * device confirms it and then skips that; a side that is not sorted is sorted as
+ * usual, so the result never depends on the flags. */
 enum { PG_JOIN_BUILD_SORTED = 8, PG_JOIN_PROBE_SORTED = 16 };
 
 /* ---------------------------------------------------------------------- */
@@ -178,7 +178,8 @@ enum {
 	                                    default, else 32, 64 or 128 (cudaLimitMaxL2FetchGranularity, a limit of
 	                                    the calling process that ends with it) */
 	PG_TUNE_SORT_PATH = 14,          /* page sort and the MPSM's sorts: 0 LSD radix over key - min, in one cooperative
-	                                    launch up to 2^20 tuples, other than 16-byte tuples as (key, row) records;
+	                                    launch up to 2^20 tuples, other than 16-byte tuples as (key, row) records
+	                                    unless the keys need few passes;
 	                                    1 a launch per radix pass over the tuples themselves while the span fits
 	                                    them (63 bits; 64 for 16-byte tuples), else 2 bitonic tiles and merges */
 	PG_TUNE_GROUPBY_ILP = 15,        /* rows in flight per thread of the dense group-by over a global table: 4

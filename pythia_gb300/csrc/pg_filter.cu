@@ -115,6 +115,12 @@ __device__ __forceinline__ void fl_load_tile(unsigned char* dst, const char* src
 // tiles start on 16-byte boundaries.
 static uint32_t fl_tile_rows(uint32_t w, uint32_t bytes) { return std::max<uint32_t>(32, bytes / w / 32 * 32); }
 
+// Rows of a tile that is not staged: blocks for every SM before rows for every thread.
+static uint32_t fl_direct_rows(const pg_ctx* ctx, uint64_t n, uint32_t most)
+{
+	return (uint32_t) std::min<uint64_t>(most, std::max<uint64_t>(32, n / ((uint64_t) ctx->sm_count * 8) / 32 * 32));
+}
+
 #define FL_READY (1ull << 63)       // of a tile's first output row
 #define FL_COUNTED (1u << 31)      // of a tile's count
 #define FL_SPIN_LIMIT (1u << 22)
@@ -300,7 +306,7 @@ extern "C" int pg_filter(pg_ctx* ctx, pg_stream stream, const pg_rel* in, const 
 	}
 	uint64_t* scratch = nullptr;
 	const bool staged = w <= FL_STAGE_WIDTH;
-	const uint32_t rows = staged ? fl_tile_rows(w, FL_TILE_BYTES) : FL_DIRECT_ROWS;
+	const uint32_t rows = staged ? fl_tile_rows(w, FL_TILE_BYTES) : fl_direct_rows(ctx, in->n, FL_DIRECT_ROWS);
 	const uint64_t ntiles = pg_div_up(in->n, rows);
 	if (ntiles >= (1ull << 31) - 1) {
 		pg_free_async(ctx, s, chars);
@@ -425,9 +431,7 @@ extern "C" int pg_project(pg_ctx* ctx, pg_stream stream, const pg_rel* in, const
 	const uintptr_t o = reinterpret_cast<uintptr_t>(out);
 	const uint32_t uw = (pc.ow & 3) == 0 && !(o & 15) ? 4 : (pc.ow & 1) == 0 && !(o & 7) ? 2 : 1;
 	const bool staged = in->width <= PJ_STAGE_WIDTH || (in->width <= PJ_STAGE_MAX && 4 * pc.ow > iw);
-	// (Unstaged: blocks for every SM before rows for every thread.)
-	const uint32_t rows = staged ? fl_tile_rows(in->width, PJ_TILE_BYTES)
-		: (uint32_t) std::min<uint64_t>(PJ_DIRECT_ROWS, std::max<uint64_t>(32, in->n / ((uint64_t) ctx->sm_count * 8) / 32 * 32));
+	const uint32_t rows = staged ? fl_tile_rows(in->width, PJ_TILE_BYTES) : fl_direct_rows(ctx, in->n, PJ_DIRECT_ROWS);
 	const uint64_t ntiles = pg_div_up(in->n, rows);
 	if (pc.ow / uw <= FL_THREADS && ntiles < (1ull << 31) - 1) {
 		const size_t smem = staged ? (size_t) rows * in->width : 0;

@@ -273,7 +273,7 @@ __device__ __forceinline__ void gb_row_kv(const char* __restrict__ in, uint64_t 
 // best: 20M rows in 250,000 groups 320 us, against 530 with six blocks per SM
 // and 1010 with four rows a thread in three resident blocks. Partitioning the
 // rows first (shared-memory tables per partition) took 850 us, and 9.5 ms for
-// 64M rows in 4M groups where this takes 1.3.
+// 64M rows in 4M groups where this takes 1.6.
 // ---------------------------------------------------------------------------
 #define GBH_CACHE_LOG2 8                    // groups kept per block: 256 (4 KB, 10 KB for dec)
 #define GBH_BLOCKS_PER_SM 64

@@ -402,15 +402,17 @@ __global__ void __launch_bounds__(1024) k_dense_prep16(const uint4* __restrict__
 // for large inputs has launches, 8-byte entries for values that span too much, and
 // where no dense layout fits (keys too far apart or repeated) the hashed table, which
 // the first use then finds ready. One block
-// per 1024 tuples, one a thread (a single one's barriers are block barriers), up to one an
-// SM: with 2048 the walks past repeated keys kept too few SMs busy (20,000 tuples of one
-// key 31 -> 38 ms, now 31; of 20 keys 5.0 -> 5.7, now 3.8). Whole joins of
+// per 1024 tuples, one a thread, up to one an SM: with 2048 the walks past repeated keys
+// kept too few SMs busy (20,000 tuples of one key 31 -> 38 ms, now 31; of 20 keys 5.0 -> 5.7,
+// now 3.8). Up to 2048 tuples one block, whose barriers are block barriers (1500 tuples with
+// 3000: 40 us, 49 in two). Whole joins of
 // 1000 tuples with 10,000: dense keys 73 -> 42 us, far ones 107 -> 78; of 20,000 with
 // 40,000: 89 -> 53 and 106 -> 90 (exact ranges and duplicate counts read back by the
 // host before). From 65,536 tuples the sampled form, used there before, takes as
 // long for dense keys (200,000 with 400,000: 65 us) and longer for far ones (182,
 // now 105), up to 2^20: the spare hashed slots are 32 MB then.
 #define HJ_SMALL_PER_BLOCK 1024
+#define HJ_SMALL_ALONE 2048
 #define HJ_SMALL_TUPLES (1u << 20)
 // Slots a tuple may walk past. Only keys repeated as often walk so far (the table is
 // at most half full); 2^18 tuples of one key take 0.9 s, a million would take the 15 s
@@ -428,7 +430,7 @@ struct HjSmallShared {
 };
 
 // The blocks of k_build_small meet (`epoch`: how often they have, with this time), and
-// *seen is what they gathered. A barrier that a block gave up on (`dead`) is no error: the
+// *seen, unless null, is what they gathered. A barrier that a block gave up on (`dead`) is no error: the
 // build returns before the kernel has run, and a status would fail whichever call reads it
 // next. The header sends the table to the exact build. Thread 0 looks at what was gathered
 // for its whole block: past a lost barrier it still changes, and the block's threads must
@@ -439,8 +441,9 @@ __device__ __noinline__ bool hj_small_meet(HjSmallShared* g, HjSmallShared* acc,
 {
 	uint32_t before = epoch - 1;
 	pg_grid_sync(&g->bar, before, dead, spin, nullptr);
+	if (threadIdx.x == 0 && dead) atomicOr(&acc->lost, 1u);         // before this block's next arrival
+	if (!seen) return dead;
 	if (threadIdx.x == 0) {
-		if (dead) atomicOr(&acc->lost, 1u);         // before this block's next arrival
 		const volatile HjSmallShared* const v = acc;
 		seen->nkmin = v->nkmin; seen->kmax = v->kmax; seen->nvmin = v->nvmin; seen->vmax = v->vmax;
 		seen->present = v->present; seen->marker = v->marker; seen->dup = v->dup;
@@ -463,7 +466,7 @@ __global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict
 	bool dead = false;
 	HjSmallShared* const acc = alone ? &mine : g;
 	if (alone && tid == 0) mine = HjSmallShared{0, 0, 0, 0, 0, 0, 0, 0, 0};
-	auto meet = [&]() { dead = hj_small_meet(g, acc, &seen, ++epoch, dead, spin); };
+	auto meet = [&](HjSmallShared* look) { dead = hj_small_meet(g, acc, look, ++epoch, dead, spin); };
 	auto key_of = [&](const uint4& v) { return ((unsigned long long) hj_word4(v, kw + 1) << 32) | hj_word4(v, kw); };
 	unsigned long long lo = ~0ull, hi = 0, vlo = ~0ull, vhi = 0;
 	int marker = 0;
@@ -487,7 +490,7 @@ __global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict
 			if (marker) atomicOr(&acc->marker, 1u);
 		}
 	}
-	meet();
+	meet(&seen);
 	HjDenseHdr h;
 	h.n = n; h.present = 0; h.kmin = ~seen.nkmin; h.kmax = seen.kmax; h.vlo = ~seen.nvmin; h.vhi = seen.vmax; h.pad = 0;
 	h.dmin = (long long) (h.kmin ^ (1ull << 63));
@@ -500,19 +503,19 @@ __global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict
 		const uint32_t range = (uint32_t) h.drange;
 		for (uint32_t i = first; i < (range + 3) / 4; i += stride)
 			reinterpret_cast<uint4*>(table)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
-		meet();
+		meet(nullptr);
 		#pragma unroll 4
 		for (uint32_t i = first; i < n; i += stride) {
 			const uint4 v = __ldg(R + i);
 			const unsigned long long d = key_of(v) - (unsigned long long) h.dmin;
 			if (d < range) table[d] = (uint32_t) (hj_pack16(v, pk) - h.vmin);
 		}
-		meet();
+		meet(nullptr);
 		uint32_t c = 0;
 		for (uint32_t i = first; i < range; i += stride) c += __ldcg(table + i) != 0xFFFFFFFFu;
 		c = __reduce_add_sync(0xffffffffu, c);
 		if (lane == 0 && c) atomicAdd(&acc->present, (unsigned long long) c);
-		meet();
+		meet(&seen);
 		h.present = seen.present;
 	} else if (h.flags == 4) {
 		// Dense keys, values that span too much for 4 bytes: 8-byte entries in the
@@ -520,7 +523,7 @@ __global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict
 		// tuples) and the presence bits in the table's words.
 		const uint32_t range = (uint32_t) span + 1;
 		for (uint32_t i = first; i < (range + 31) / 32; i += stride) table[i] = 0;
-		meet();
+		meet(nullptr);
 		bool dup = false;
 		#pragma unroll 4
 		for (uint32_t i = first; i < n; i += stride) {
@@ -532,7 +535,7 @@ __global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict
 			slots[d] = hj_pack16(v, pk);
 		}
 		if (dup) atomicOr(&acc->dup, 1u);
-		meet();
+		meet(&seen);
 		if (!seen.dup) h.flags = 64;
 	}
 	// The hashed table, unless the tuples have a dense layout or a key equal to the
@@ -540,7 +543,7 @@ __global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict
 	if (h.flags != 64 && h.present != n && !seen.marker) {
 		const uint32_t mask = (1u << log2cap) - 1;
 		for (uint32_t i = first; i <= mask; i += stride) reinterpret_cast<uint4*>(slots)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
-		meet();
+		meet(nullptr);
 		const uint32_t walk = HJ_SMALL_WALK(n);
 		bool dup = false, far = false;
 		for (uint32_t i = first; i < n && !far; i += stride) {
@@ -560,7 +563,7 @@ __global__ void __launch_bounds__(1024, 1) k_build_small(const uint4* __restrict
 		}
 		if (dup) atomicOr(&acc->dup, 1u);
 		if (far) atomicOr(&acc->lost, 1u);
-		meet();
+		meet(&seen);
 		h.flags |= 16 | (seen.dup ? 32 : 0);
 	}
 	// Past a lost barrier, or with a tuple left out, no layout can be trusted.
@@ -1672,8 +1675,9 @@ __device__ __forceinline__ void hj_st_stream(char* p, uint4 v, uint64_t pol)
 // keys: one tuple in flight a thread, straight from global memory, in many short
 // blocks. Random bucket loads bound it (38 of its 54 DRAM bytes a tuple on a
 // 128 MB table, at 0.74 of the copy rate), so what counts is how many warps wait
-// for them at once: 48M probes 520 us, against 580 staged through shared memory
-// with sixteen warps on an SM (k_probe16_warp) and 840 with two tuples a thread
+// for them at once: whole calls of 48M probes of 3M keys 512 us, against 600 staged
+// through shared memory with sixteen warps on an SM (k_probe16_warp), of 20,000 keys 380
+// against 475, of 2M probes or fewer the same; the kernel 840 with two tuples a thread
 // (spills at this occupancy).
 // ---------------------------------------------------------------------------
 #define HA_BLOCKS_PER_SM 64
@@ -2409,7 +2413,7 @@ static int hj_build_spec(pg_ctx* ctx, cudaStream_t s, const pg_rel* R, pg_hashta
 	ht->small_slots.store(spare);
 	if (small) {
 		ht->log2cap = hj_log2cap(R->n);
-		uint32_t G = (uint32_t) std::min<uint64_t>(pg_div_up(R->n, HJ_SMALL_PER_BLOCK), ctx->sm_count);
+		uint32_t G = R->n <= HJ_SMALL_ALONE ? 1 : (uint32_t) std::min<uint64_t>(pg_div_up(R->n, HJ_SMALL_PER_BLOCK), ctx->sm_count);
 		HjSmallShared* g = reinterpret_cast<HjSmallShared*>(ht->hdr + 1);
 		if (G > 1) PG_CUDA(ctx, cudaMemsetAsync(g, 0, sizeof(HjSmallShared), s));
 		const uint4* rd = (const uint4*) R->data;

@@ -544,9 +544,11 @@ static bool sw_takes(const pg_rel* in, const void* out, uint32_t buckets)
 // and 115, 64M 662 and 545. Functions that both compute twice a tuple and that cost more than
 // the ranking: exactrange into 3 buckets 1094 and 1151 us (64M), 92 and 114 (3M), into 200
 // 1268 and 1214, 111 and 116; bytes into 64 1481 and 1508, 122 and 138, but 500,000 tuples 72
-// and 64.
+// and 64. Below 400,000 tuples a block has one tile and the fewer launches win (100,000
+// in 2 buckets 45 and 40, exactrange into 3 46 and 43).
 static bool sw_wins(const pg_hashfn& f, uint64_t n)
 {
+	if (n < 400000) return true;
 	switch (f.fn) {
 	case PG_FN_RANGE: case PG_FN_EXACTRANGE: return f.nbuckets > 4;
 	case PG_FN_BYTES: return f.nbuckets > 4 && n < 2500000;

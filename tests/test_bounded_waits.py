@@ -61,7 +61,7 @@ def test_each_wait_gives_up_and_the_next_call_succeeds(ctx, op):
         ctx.tune(spin_limit=0, **{k: 0 for k in knobs})
 
 
-@pytest.mark.parametrize("n", [1025, 3000, 70_001, 1 << 20])
+@pytest.mark.parametrize("n", [2048, 2049, 3000, 70_001, 1 << 20])
 @pytest.mark.parametrize("case", ["dense", "far", "repeated", "wide"])
 def test_a_build_that_gives_up_on_its_barriers_is_made_again(ctx, n, case):
     R = dg.build_relation(n, dg.seed_for(406))

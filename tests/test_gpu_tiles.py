@@ -477,10 +477,10 @@ def test_filter_and_project_of_wide_tuples(ctx, width, shift):
 # Either side of the lines between the two partitions of 16-byte tuples: few buckets,
 # functions that cost more than the ranking.
 @pytest.mark.parametrize("fn,kw,n", [("parammodulo", dict(buckets=1), 10_001), ("parammodulo", dict(buckets=2), 3_999_999),
-                                     ("parammodulo", dict(buckets=2), 4_000_000), ("modulo", dict(buckets=4), 10_001),
-                                     ("exactrange", dict(buckets=4, min=0, max=(1 << 40) - 1), 10_001),
+                                     ("parammodulo", dict(buckets=2), 4_000_000), ("modulo", dict(buckets=4), 10_001), ("parammodulo", dict(buckets=1), 400_000),
+                                     ("exactrange", dict(buckets=4, min=0, max=(1 << 40) - 1), 400_000),
                                      ("exactrange", dict(buckets=5, min=0, max=(1 << 40) - 1), 10_001),
-                                     ("bytes", dict(buckets=4), 10_001), ("bytes", dict(buckets=8), 2_499_999),
+                                     ("bytes", dict(buckets=4), 399_999), ("bytes", dict(buckets=4), 400_000), ("bytes", dict(buckets=8), 2_499_999),
                                      ("bytes", dict(buckets=8), 2_500_000), ("knuth", dict(buckets=256, skipbits=3), 10_001)])
 def test_partition_rules(ctx, fn, kw, n):
     rows = dg.uniform_keys(n, 1 << 40, dg.seed_for(213))
