@@ -614,14 +614,14 @@ k_mj_fill(const char* __restrict__ R, uint64_t n, uint32_t koff, long long kmin,
 // Bound by DRAM: the values' scattered reads miss L2 under the stream of rows
 // (16M tuples, 64M rows, 4-byte values: 1.36 GB read and 1.07 written). The whole join
 // above with its group-by: no limit on registers 1214 us, with 6 blocks an SM 1160, and
-// two tuples a lane instead of four 1105 (1140 with the slices' checks); of keys with one
+// two tuples a lane instead of four 1105 (1150 with the slices); of keys with one
 // row 1484, 1513 and 1590, so those take four.
 //
 // A warp's tuples may have thousands of rows each. Those of more than MJ_SLICE_MAX rows
 // in all go on a list instead, MJ_SLICE rows an entry, and a second launch (SLICE) has a
 // warp write an entry's rows. 1000 tuples with 16,000 rows each: 18.97 ms without it,
 // 0.47 with (1.45 sorted, where a thread takes eight rows); 64 such tuples among 4M others 8.4,
-// 0.27 (1.10). The second launch, empty, takes 2 us.
+// 0.27 (1.10). The second launch, empty, takes 2 to 4 us.
 #define MJ_ROWS_BLOCKS_PER_SM 24
 #define MJ_SLICE 2048u
 #define MJ_SLICE_MAX 8192u
