@@ -54,7 +54,7 @@ void pg_free_async(pg_ctx* ctx, cudaStream_t s, void* p);
 struct PgScratch {
 	pg_ctx* ctx;
 	cudaStream_t s;
-	void* p[4];
+	void* p[12];
 	int n = 0;
 	PgScratch(pg_ctx* c, cudaStream_t st) : ctx(c), s(st) { }
 	~PgScratch() { for (int i = 0; i < n; ++i) pg_free_async(ctx, s, p[i]); }
@@ -67,6 +67,7 @@ struct PgScratch {
 		if (!rc) p[n++] = *q;
 		return rc;
 	}
+	void own(void* q) { p[n++] = q; }
 	// The caller's from now on.
 	void* keep(void* q)
 	{

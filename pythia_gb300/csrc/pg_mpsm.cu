@@ -252,9 +252,9 @@ __global__ void k_mj_write(MjSide R, MjSide S, MjCols pc, const uint64_t* __rest
 	}
 }
 
-// Runs of both sides, with one readback of their numbers.
-static int mj_runs(pg_ctx* ctx, cudaStream_t s, const pg_rec* const (&rec)[2], const uint64_t (&n)[2], uint64_t* (&starts)[2],
-		long long* (&keys)[2], uint64_t (&nruns)[2])
+// Runs of both sides (starts and keys in `out`), with one readback of their numbers.
+static int mj_runs(pg_ctx* ctx, cudaStream_t s, const pg_rec* const (&rec)[2], const uint64_t (&n)[2], PgScratch& out,
+		uint64_t* (&starts)[2], long long* (&keys)[2], uint64_t (&nruns)[2])
 {
 	int rc;
 	PgScratch mem(ctx, s);
@@ -270,8 +270,8 @@ static int mj_runs(pg_ctx* ctx, cudaStream_t s, const pg_rec* const (&rec)[2], c
 	PG_CUDA(ctx, cudaMemcpyAsync(nruns, total, 16, cudaMemcpyDeviceToHost, s));
 	PG_CUDA(ctx, cudaStreamSynchronize(s));
 	for (int i = 0; i < 2; ++i) {
-		if ((rc = pg_alloc_async(ctx, s, (void**) &starts[i], (nruns[i] + 1) * 8))) return rc;
-		if ((rc = pg_alloc_async(ctx, s, (void**) &keys[i], (nruns[i] + 1) * 8))) return rc;
+		if ((rc = out.get((void**) &starts[i], (nruns[i] + 1) * 8))) return rc;
+		if ((rc = out.get((void**) &keys[i], (nruns[i] + 1) * 8))) return rc;
 		const uint64_t nchunks = pg_div_up(n[i], MJ_RUN_CHUNK);
 		k_run_write<<<(int) std::min<uint64_t>(nchunks, (uint64_t) ctx->sm_count * 8), MJ_RUN_THREADS, 0, s>>>(rec[i], n[i], cc[i],
 				starts[i], keys[i]);
@@ -1027,25 +1027,26 @@ extern "C" int pg_mpsm_join(pg_ctx* ctx, pg_stream stream, const pg_rel* R, cons
 	pg_rec *rr = nullptr, *sr = nullptr;
 	const bool r_own = !(r_sorted && pg_sort_mode(R) == 0 && !(reinterpret_cast<uintptr_t>(R->data) & 15));
 	const bool s_own = !(s_sorted && pg_sort_mode(S) == 0 && !(reinterpret_cast<uintptr_t>(S->data) & 15));
-	if (r_own) { if ((rc = pg_sort_records(ctx, s, R, &rr))) return rc; }
+	PgScratch mem(ctx, s);
+	if (r_own) { if ((rc = pg_sort_records(ctx, s, R, &rr))) return rc; mem.own(rr); }
 	else rr = (pg_rec*) R->data;
-	if (s_own) { if ((rc = pg_sort_records(ctx, s, S, &sr))) return rc; }
+	if (s_own) { if ((rc = pg_sort_records(ctx, s, S, &sr))) return rc; mem.own(sr); }
 	else sr = (pg_rec*) S->data;
 	MjSide RS{rr, (const char*) R->data, R->width, R->key_off, pg_sort_mode(R), nullptr, 0};
 	MjSide SS{sr, (const char*) S->data, S->width, S->key_off, pg_sort_mode(S), nullptr, 0};
 	uint64_t* starts[2] = {nullptr, nullptr};
 	long long* rkeys[2] = {nullptr, nullptr};
 	uint64_t nruns[2];
-	if ((rc = mj_runs(ctx, s, {rr, sr}, {R->n, S->n}, starts, rkeys, nruns))) return rc;
+	if ((rc = mj_runs(ctx, s, {rr, sr}, {R->n, S->n}, mem, starts, rkeys, nruns))) return rc;
 	uint64_t *rst = starts[0], *sst = starts[1];
 	long long *rk = rkeys[0], *sk = rkeys[1];
 	RS.run_start = rst; SS.run_start = sst;
 	RS.nruns = nruns[0]; SS.nruns = nruns[1];
 	uint64_t *counts = nullptr, *match = nullptr;
 	unsigned long long* acc = nullptr;  // [total, sum]
-	if ((rc = pg_alloc_async(ctx, s, (void**) &counts, (RS.nruns + 1) * 8))) return rc;
-	if ((rc = pg_alloc_async(ctx, s, (void**) &match, (RS.nruns + 1) * 8))) return rc;
-	if ((rc = pg_alloc_async(ctx, s, (void**) &acc, 16))) return rc;
+	if ((rc = mem.get((void**) &counts, (RS.nruns + 1) * 8))) return rc;
+	if ((rc = mem.get((void**) &match, (RS.nruns + 1) * 8))) return rc;
+	if ((rc = mem.get((void**) &acc, 16))) return rc;
 	PG_CUDA(ctx, cudaMemsetAsync(acc, 0, 16, s));
 	// One warp per MJ_WARP_RUNS build runs, 8 warps per CTA.
 	int blocks = (int) std::min<uint64_t>(pg_div_up(pg_div_up(RS.nruns, MJ_WARP_RUNS), 8), (uint64_t) ctx->sm_count * 16);
@@ -1068,8 +1069,5 @@ extern "C" int pg_mpsm_join(pg_ctx* ctx, pg_stream stream, const pg_rel* R, cons
 			rc = pg_check_status(ctx, s, "pg_mpsm_join");
 		}
 	}
-	for (void* p : {r_own ? (void*) rr : nullptr, s_own ? (void*) sr : nullptr, (void*) rst, (void*) sst, (void*) rk,
-			(void*) sk, (void*) counts, (void*) match, (void*) acc})
-		pg_free_async(ctx, s, p);
 	return rc;
 }

@@ -132,3 +132,9 @@ def test_sort_of_other_widths(tmp_path, n, width, bits):
     else:
         source = SORT
     _run(tmp_path, source % (ROOT, n, width, bits))
+
+
+# Keys that span too much to be counted: the sort's own scratch.
+def test_sorted_merge_join(tmp_path):
+    source = (MPSM % (ROOT, 30_001, 20_001, 1 << 31)).replace("dR, dS, dO =", "R[:, 0] <<= 30\nS[:, 0] <<= 30\ndR, dS, dO =")
+    _run(tmp_path, source.replace("1 << 14)", "1 << 40)"))
