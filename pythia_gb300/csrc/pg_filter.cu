@@ -391,7 +391,7 @@ k_project(const char* __restrict__ in, uint64_t n, uint32_t iw, uint32_t tile_ro
 	}
 }
 
-// Rows wider than a block's units: one thread per tuple.
+// Rows wider than a block's units, or of few words of wide tuples: one thread per tuple.
 __global__ void k_project_wide(const uint32_t* __restrict__ in, uint64_t n, uint32_t iw, const ProjCols pc,
 		uint32_t* __restrict__ out)
 {
@@ -433,7 +433,13 @@ extern "C" int pg_project(pg_ctx* ctx, pg_stream stream, const pg_rel* in, const
 	const bool staged = in->width <= PJ_STAGE_WIDTH || (in->width <= PJ_STAGE_MAX && 4 * pc.ow > iw);
 	const uint32_t rows = staged ? fl_tile_rows(in->width, PJ_TILE_BYTES) : fl_direct_rows(ctx, in->n, PJ_DIRECT_ROWS);
 	const uint64_t ntiles = pg_div_up(in->n, rows);
-	if (pc.ow / uw <= FL_THREADS && ntiles < (1ull << 31) - 1) {
+	// Unstaged rows of one word, and of up to four of wide or few tuples: a thread a row,
+	// which has all its loads in flight (4 of 136 bytes 99 us against 107 by units, 8: 123 and
+	// 110, of 200 and more 83 to 36 either way; 12 of 1000 47 to 56 and 57, of 400 94 and 87;
+	// 250,000 tuples, 8 of 400 24 and 31; 50,000, 16 of 400 23 and 32).
+	const bool by_row = !staged && (pc.ow == 1 || (pc.ow == 2 && (in->width >= 200 || in->n < 1000000)) ||
+			(pc.ow <= 4 && (in->width >= 900 || in->n < 200000)));
+	if (!by_row && pc.ow / uw <= FL_THREADS && ntiles < (1ull << 31) - 1) {
 		const size_t smem = staged ? (size_t) rows * in->width : 0;
 #define PJ_LAUNCH(U, ST) do { \
 		if (ST) PG_CUDA(ctx, cudaFuncSetAttribute(k_project<U, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)); \

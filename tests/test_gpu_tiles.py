@@ -487,3 +487,14 @@ def test_partition_rules(ctx, fn, kw, n):
     got, offs = ctx.partition(rows, gpu.hashcfg(fn, **kw))
     want, woffs = orc.partition(rows, orc.hashcfg(fn, **kw))
     assert np.array_equal(offs, woffs) and np.array_equal(got, want)
+
+
+# Few words of unstaged tuples are projected a thread a row: few tuples, one word, and up
+# to four words of tuples of 900 bytes and more; units a thread past each line.
+@pytest.mark.parametrize("n,width,keep", [(199_999, 132, 16), (200_000, 132, 16), (200_000, 132, 4), (999_999, 132, 8),
+                                          (1_000_000, 132, 8), (1_000_000, 200, 8), (1_000_000, 196, 8),
+                                          (200_000, 896, 16), (200_000, 900, 16), (200_000, 900, 20), (1, 900, 4)])
+def test_project_few_words(ctx, n, width, keep):
+    rows = _rows(n, width, n + keep)
+    got = ctx.project(rows, [(width - keep, keep)])
+    assert np.array_equal(np.ascontiguousarray(got).view(np.int32).reshape(n, -1), rows[:, (width - keep) // 4:])
